@@ -162,6 +162,10 @@ typedef struct DmoeGemm {
   float act_limit;
   int act_cols;
   int unit_weights;   // combine: the records' weights are left out
+  // != 0: the tokens are the M operand (gemm_wide.cu: CTA pairs on tiles of 256 tokens x 256 weight rows) where the launch
+  // allows it: no multi-GPU hooks, splitk <= 1, no pair, 16-byte aligned output rows; other launches ignore it. bn, streamk,
+  // ws and counters are unused then.
+  int wide;
 } DmoeGemm;
 
 int dmoe_gemm(const DmoeGemm* desc, void* stream);

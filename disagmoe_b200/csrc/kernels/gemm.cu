@@ -25,21 +25,18 @@
 #include <string.h>
 
 #include "dmoe_kernels.h"
+#include "gemm_common.cuh"
 #include "sm100.cuh"
 #include "work_walker.cuh"
 
 namespace dmoe {
 
-constexpr int kBM = 128;       // weight rows per tile (UMMA M)
-constexpr int kBK = 64;        // K elements per stage: 64 bf16 = 128 bytes = one swizzle span
-constexpr int kUmmaK = 16;     // K per tcgen05.mma for 16-bit inputs
 constexpr int kThreads = 192;
 constexpr int kEpiThreads = 128;
 constexpr int kSmemBudget = 220 * 1024;
 constexpr int kTailBytes = 10 * 1024;   // barriers + segment table (2 x kMaxSeg ints)
-constexpr int kMaxSeg = 1024;            // groups x sources
+constexpr int kMaxSeg = kMaxGroups;      // groups x sources
 
-enum { EPI_PLAIN = 0, EPI_SWIGLU = 1, EPI_COMBINE = 2 };
 
 struct GemmArgs {
   const int* offs;   // [G+1] device token offsets, or nullptr for one dense group of T tokens
@@ -144,21 +141,14 @@ __device__ __forceinline__ void trace_stamp(const GemmArgs& a, int i) {
   }
 }
 
-// silu(g) = g sigmoid(g); the tanh form of gelu is g sigmoid(2 sqrt(2 / pi) (g + 0.044715 g^3))
-__device__ __forceinline__ float gate_act(float g, int act) {
-  const float z = act == 0 ? g : 1.5957691216057308f * (g + 0.044715f * g * g * g);
-  return g / (1.f + __expf(-z));
+// gate and up of 32 tokens times the weights of their records (``n`` of them exist)
+__device__ __forceinline__ void weigh(float (&g)[32], float (&u)[32], const int4* recs, int n) {
+  float w[32];
+#pragma unroll
+  for (int j = 0; j < 32; ++j) w[j] = j < n ? __int_as_float(__ldg(&recs[j].z)) : 1.f;
+#pragma unroll
+  for (int j = 0; j < 32; ++j) { g[j] *= w[j]; u[j] *= w[j]; }
 }
-
-// act(g) * u; clamped: min(g, limit) sigmoid(1.702 min(g, limit)) (clamp(u, -limit, limit) + 1)
-__device__ __forceinline__ float gated(float g, float u, int act, float limit) {
-  if (act != 3) return gate_act(g, act) * u;
-  const float m = fminf(g, limit);
-  return __fdividef(m, 1.f + __expf(-1.702f * m)) * (fminf(fmaxf(u, -limit), limit) + 1.f);
-}
-
-// tanh(x) = 1 - 2 / (exp(2x) + 1), good to about 1e-7 absolute
-__device__ __forceinline__ float out_tanh(float x) { return 1.f - __fdividef(2.f, __expf(fminf(2.f * x, 40.f)) + 1.f); }
 
 __device__ __forceinline__ int ld_acquire_sys(const int* p) {
   int v;
@@ -523,12 +513,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUt
               }
             }
           }
-          if (EPI == EPI_SWIGLU) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const float s = a.recs != nullptr && j < jmax ? __int_as_float(__ldg(&a.recs[tok_base + c * 32 + j].z)) : 1.f;
-              acc[j] = gated(acc[j] * s, up[j] * s, a.act, a.act_limit);
-            }
+          if constexpr (EPI == EPI_SWIGLU) {
+            if (a.recs != nullptr) weigh(acc, up, a.recs + tok_base + c * 32, jmax);
+            gated(acc, up, a.act, a.act_limit);
           }
         } else {
           uint32_t v[32];
@@ -538,13 +525,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUt
             tmem_ld32(t0 + BN + c * 32, uu);
             tmem_ld_wait();
             if (et == 0 && c == 0) trace_stamp(a, 8);
+            float up[32];
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const float s = a.recs != nullptr && j < jmax ? __int_as_float(__ldg(&a.recs[tok_base + c * 32 + j].z)) : 1.f;
-              const float g = __uint_as_float(v[j]) * s;
-              const float up = __uint_as_float(uu[j]) * s;
-              acc[j] = gated(g, up, a.act, a.act_limit);
-            }
+            for (int j = 0; j < 32; ++j) { acc[j] = __uint_as_float(v[j]); up[j] = __uint_as_float(uu[j]); }
+            if (a.recs != nullptr) weigh(acc, up, a.recs + tok_base + c * 32, jmax);
+            gated(acc, up, a.act, a.act_limit);
           } else {
             tmem_ld_wait();
             if (et == 0 && c == 0) trace_stamp(a, 8);
@@ -564,7 +549,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUt
         }
         if (EPI == EPI_PLAIN && a.act == 4 && f < a.act_cols) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) acc[j] = gate_act(acc[j], 0);
+          for (int j = 0; j < 32; ++j) acc[j] = gate_act<0>(acc[j]);
         }
         if ((EPI == EPI_PLAIN || EPI == EPI_SWIGLU) && vec) {
           if (jmax <= 0) continue;                   // uniform over the CTA: no barrier is skipped by some threads only
@@ -866,38 +851,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUt
 }
 
 // ------------------------------------------------------------------ host side
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static EncodeTiledFn get_encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  if (fn == nullptr) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qres) == cudaSuccess &&
-        qres == cudaDriverEntryPointSuccess) {
-      fn = reinterpret_cast<EncodeTiledFn>(p);
-    }
-  }
-  return fn;
-}
-
-// Tensor map over a row-major [rows, K] bf16 matrix with a [box_rows, 64] box and the 128-byte swizzle.
-static int make_map_2d(CUtensorMap* map, const void* ptr, long long rows, long long K, long long ld_elems,
-                       int box_rows) {
-  EncodeTiledFn enc = get_encode_fn();
-  if (enc == nullptr) return -1;
-  cuuint64_t gdim[2] = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(rows)};
-  cuuint64_t gstride[1] = {static_cast<cuuint64_t>(ld_elems) * 2};
-  cuuint32_t box[2] = {static_cast<cuuint32_t>(kBK), static_cast<cuuint32_t>(box_rows)};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), gdim, gstride, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? 0 : -2;
-}
-
 static int num_sms() { return device_num_sms(); }
 
 template <int BN, int EPI, bool PAIR = false>
@@ -1029,6 +982,13 @@ extern "C" int dmoe_gemm(const DmoeGemm* d, void* stream_) {
   if ((a.n_wait > 0 || a.n_signal > 0) && a.done_ticket == nullptr) return -17;
   if (a.n_wait > kThreads || (a.n_wait > 0 && (a.wait_flags == nullptr || a.wait_epoch == nullptr))) return -17;
   if (a.n_signal > 0 && (a.signal_ptrs == nullptr || a.signal_epoch == nullptr)) return -17;
+
+  // tokens as the M operand: single-GPU launches with 16-byte output rows; without them the call keeps the kernel of this file
+  const bool alone = d->S == 0 && !d->group_regions && d->n_wait == 0 && d->n_signal == 0 && d->shard_rows == 0 &&
+                     d->rs_bases == nullptr && d->fanout <= 1 && splitk == 1 && !pair && d->trace == nullptr;
+  if (d->wide != 0 && alone && a.epi_vec && d->seg_cnt == nullptr && (!d->w_blocked || (d->K % kBK == 0 && d->F % kBM == 0 &&
+      static_cast<long long>(d->G) * a.w_rows * (d->K / kBK) < (1ll << 31))))
+    return gemm_wide(d, stream);
 
   CUtensorMap tmW, tmX;
   const long long ldx = d->ldx > 0 ? d->ldx : d->K;

@@ -82,8 +82,8 @@ def pick_splitk(T: int, F: int, K: int, bn: int, sms: int = 0) -> int:
     return max(1, min((sms * 128 // 148 + tiles // 2) // tiles, kblocks // 4, 16))
 
 
-def pick_dense(T: int, F: int, K: int, sms: int = 0):
-    """(token tile, split-K factor) of a dense GEMM below one wave of tiles, by a cost model fitted to the tile /
+def dense_cost(T: int, F: int, K: int, sms: int = 0):
+    """(cost in us, token tile, split-K factor) of a dense GEMM below one wave of tiles, by a cost model fitted to the tile /
     split sweep of benchmark/ops/dense_gemm.py on B200. At these sizes a CTA is bound by what its SM can pull from L2
     (~100 GB/s: 16 KB of weights plus bn x 128 B of tokens per K block), so the model counts, per CTA, the bytes of
     its K range times the number of waves, the parked and re-read partial tiles of a split (the last arriver reads
@@ -110,7 +110,12 @@ def pick_dense(T: int, F: int, K: int, sms: int = 0):
                 cost += 128 * bn * 4 / 1e5 + (bn // 32) * sk * 0.35
             if best is None or cost < best[0] - 1e-9:
                 best = (cost, bn, sk)
-    return best[1], best[2]
+    return best
+
+
+def pick_dense(T: int, F: int, K: int, sms: int = 0):
+    """(token tile, split-K factor) of :func:`dense_cost`."""
+    return dense_cost(T, F, K, sms)[1:]
 
 
 def pick_bn(tokens_per_group: int, epi: int) -> int:
@@ -123,7 +128,10 @@ def pick_bn(tokens_per_group: int, epi: int) -> int:
 
 def pick_even_bn(tokens: int, F: int, G: int, sms: int = 0) -> int:
     """Token tile of a grouped GEMM whose G groups have ``tokens`` rows each (the per-head maps of latent attention): the
-    smallest one whose tiles fit one wave of CTAs; below a wave short loops and epilogues count for more than weight re-reads."""
+    smallest one whose tiles fit one wave of CTAs; below a wave short loops and epilogues count for more than weight re-reads.
+    0 (let the grouped GEMM choose) where :func:`want_wide` takes the groups anyway."""
+    if tokens >= 144:
+        return 0
     for bn in (32, 64, 128):
         if (F + 127) // 128 * G * ((tokens + bn - 1) // bn) <= (sms or num_sms()):
             return bn
@@ -140,6 +148,34 @@ def want_streamk(epi: int, F: int, G: int, T: int, bn: int, sms: int) -> bool:
     tiles = ((F + 127) // 128) * max(G, (T + bn - 1) // bn)
     waves = (tiles + sms - 1) // sms
     return tiles / (waves * sms) < 0.85
+
+
+def want_wide(epi: int, T: int, F: int, K: int, G: int, sms: int) -> bool:
+    """Should the tokens be the M operand (csrc/kernels/gemm_wide.cu, 256 x 256 tiles on CTA pairs) instead of the weights?
+
+    Dense: a cost model of both, in us, fitted to a sweep on B200 (K 1024 .. 5632, F 256 .. 32000, T 8 .. 2048; every choice
+    within 5 % of the better kernel). A wide tile takes 0.31 us per K block whatever part of it is used, the other kernel what
+    its SM pulls from L2. Measured (bf16, other kernel -> wide): 4096 x 6144 x 4096 201 -> 149 us (1381 TFLOP/s), 2500 x 4096 x
+    2048 106 -> 40, 1111 x 6144 x 2048 79 -> 31, 256 x 32000 x 4096 89 -> 58; SwiGLU 1024 x 5632 x 2048 59 -> 42.
+
+    Grouped (only the mean group size is known): up to 128 tokens the other kernel's tile fits a group and streams the weights
+    at HBM speed, beyond that it needs a second tile per group. Measured at 64 experts of 1408 x 2048, SwiGLU: 120 tokens each
+    140 -> 154 us, 150: 187 -> 160; 8 experts of 14336 x 4096: 128 tokens 344 -> 393, 160: 456 -> 391. Down-projections with
+    short K loops are bound by the other kernel's transposing epilogue at any size: 64 x (2048 x 1408), 40 tokens each 80 -> 74;
+    with a long loop, 8 x (4096 x 14336), 128 tokens 188 -> 196, 160: 209 -> 193."""
+    kblocks, pairs = (K + 63) // 64, max(1, sms // 2)
+    if G > 1:
+        return T >= 144 * G or (epi != EPI_SWIGLU and K <= 2048 and T >= 16 * G)
+    if T < 64 and epi != EPI_SWIGLU:
+        return False
+    feat = 128 if epi == EPI_SWIGLU else 256
+    tiles = ((F + feat - 1) // feat) * ((T + 255) // 256)
+    wide = 8.0 + (tiles + pairs - 1) // pairs * kblocks * 0.31
+    bn, mt = pick_bn(T, epi), (F + 127) // 128
+    units = mt * ((T + bn - 1) // bn)
+    if epi == EPI_SWIGLU:
+        return wide < 10.0 + (units + sms - 1) // sms * kblocks * (32768 + bn * 128) / 1e5
+    return units >= sms or wide < 3.0 + dense_cost(T, F, K, sms)[0]
 
 
 def _group_hint(T: int, G: int) -> int:
@@ -223,9 +259,10 @@ def rope_table(max_pos: int, hd: int, theta: float, device) -> torch.Tensor:
 
 def _launch(W, X, Y, R, offs, recs, bases, G, T, F, K, epi, bn, splitk, ldy, y_f32, comm: Optional[GemmComm] = None,
             streamk: bool = False, pair: bool = False, w_blocked: bool = False, act: int = 0, act_limit: float = 0.0,
-            act_cols: int = 0, unit_weights: bool = False):
+            act_cols: int = 0, unit_weights: bool = False, wide: bool = False):
     s = scratch(X.device)
     d = _lib.DmoeGemm()
+    d.wide = int(wide)
     d.act_limit, d.act_cols, d.unit_weights = act_limit, act_cols, int(unit_weights)
     d.w_blocked, d.act = int(w_blocked), act
     d.trace = TRACE.data_ptr() if TRACE is not None else None
@@ -303,7 +340,7 @@ def _check_x(x):
 def linear(x: torch.Tensor, w: torch.Tensor, residual: Optional[torch.Tensor] = None,
            out: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None, bn: int = 0,
            splitk: int = 0, comm: Optional["GemmComm"] = None, pair: bool = False, tanh: bool = False,
-           silu_cols: int = 0) -> torch.Tensor:
+           silu_cols: int = 0, wide: Optional[bool] = None) -> torch.Tensor:
     """y[T, F] = x[T, K] @ w[F, K].T (+ residual[T, F]); ``tanh``: of the product; ``silu_cols``: silu of the first so many columns. ``pair``: CTA pairs (tcgen05 cta_group::2) on tiles of 256
     weight rows x ``bn`` (128 / 256) tokens, whole tiles."""
     T, K = x.shape
@@ -338,12 +375,16 @@ def linear(x: torch.Tensor, w: torch.Tensor, residual: Optional[torch.Tensor] = 
     # plain split-K with a factor that fills the SMs. An explicit splitk >= 1 selects split-K with that factor.
     sms = num_sms(x.device)
     auto_sk = 0
+    if wide is None:
+        wide = not (bn or splitk or pair) and want_wide(EPI_PLAIN, T, F, K, 1, sms)
     if not bn:
         bn = pick_bn(T, EPI_PLAIN)
         if ((F + 127) // 128) * ((T + bn - 1) // bn) < sms and not pair:
             bn, auto_sk = pick_dense(T, F, K, sms)
     if pair:
         bn = 256 if bn not in (128, 256) else bn
+        splitk = 1
+    if wide:
         splitk = 1
     streamk = splitk == 0 and STREAM_K and ((F + 127) // 128) * ((T + bn - 1) // bn) >= sms
     if streamk:
@@ -352,7 +393,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, residual: Optional[torch.Tensor] = 
         splitk = splitk or auto_sk or pick_splitk(T, F, K, bn, sms)
     _launch(w, x, out, residual, None, None, None, 1, T, F, K, EPI_PLAIN, bn, splitk,
             F if scatter else out.stride(0), (not scatter) and out.dtype == torch.float32, comm, streamk=streamk,
-            pair=pair, act=ACT_TANH if tanh else ACT_SILU if silu_cols else 0, act_cols=silu_cols)
+            pair=pair, act=ACT_TANH if tanh else ACT_SILU if silu_cols else 0, act_cols=silu_cols, wide=wide)
     return out
 
 
@@ -377,7 +418,7 @@ def _grouped_ref(x, w, offs, swiglu, act="silu", limit=0.0, recs=None):
 def grouped_swiglu(x: torch.Tensor, w13: torch.Tensor, offs: Optional[torch.Tensor], out: Optional[torch.Tensor] = None,
                    bn: int = 0, comm: Optional[GemmComm] = None, streamk: Optional[bool] = None,
                    pair: bool = False, w_blocked: bool = False, act: str = "silu", limit: float = 0.0,
-                   recs: Optional[torch.Tensor] = None) -> torch.Tensor:
+                   recs: Optional[torch.Tensor] = None, wide: Optional[bool] = None) -> torch.Tensor:
     """y[T, I] = act(x @ w13[g, :I].T) * (x @ w13[g, I:].T) for the rows of group g; w13 is [G, 2I, K]. ``recs``: row t of x counts
     with the weight of its record (see :func:`grouped_combine`)."""
     T, K = x.shape
@@ -400,18 +441,20 @@ def grouped_swiglu(x: torch.Tensor, w13: torch.Tensor, offs: Optional[torch.Tens
         out = torch.empty(T, I, dtype=torch.bfloat16, device=x.device)
     if T == 0:
         return out
+    if wide is None:
+        wide = not (bn or pair or streamk or comm is not None) and want_wide(EPI_SWIGLU, T, I, K, G, num_sms(x.device))
     bn = bn or (pick_bn(_group_hint(T, G), EPI_COMBINE) if pair else pick_bn(_group_hint(T, G), EPI_SWIGLU))
     if pair:
         bn = max(bn, 128)
     sk = want_streamk(EPI_SWIGLU, I, G, T, bn, num_sms(x.device)) if streamk is None else streamk
     _launch(w13, x, out, None, offs, recs, None, G, T, I, K, EPI_SWIGLU, bn, 1, out.stride(0), False, comm,
-            streamk=sk, pair=pair, w_blocked=w_blocked, act=ACTS[act], act_limit=limit)
+            streamk=sk, pair=pair, w_blocked=w_blocked, act=ACTS[act], act_limit=limit, wide=wide)
     return out
 
 
 def grouped_linear(x: torch.Tensor, w: torch.Tensor, offs: torch.Tensor, out: Optional[torch.Tensor] = None,
                    bn: int = 0, streamk: Optional[bool] = None, pair: bool = False,
-                   w_blocked: bool = False, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
+                   w_blocked: bool = False, out_dtype: Optional[torch.dtype] = None, wide: Optional[bool] = None) -> torch.Tensor:
     """y[T, F] = x @ w[g].T for the rows of group g; w is [G, F, K]. ``out_dtype``: that of x, or fp32."""
     T, K = x.shape
     G, F, _ = w.shape
@@ -430,12 +473,14 @@ def grouped_linear(x: torch.Tensor, w: torch.Tensor, offs: torch.Tensor, out: Op
         out = torch.empty(T, F, dtype=dt, device=x.device)
     if T == 0:
         return out
+    if wide is None:
+        wide = not (bn or pair or streamk) and want_wide(EPI_PLAIN, T, F, K, G, num_sms(x.device))
     bn = bn or pick_bn(_group_hint(T, G), EPI_PLAIN)
     if pair:
         bn = max(bn, 128)
     sk = want_streamk(EPI_PLAIN, F, G, T, bn, num_sms(x.device)) if streamk is None else streamk
     _launch(w, x, out, None, offs, None, None, G, T, F, K, EPI_PLAIN, bn, 1, out.stride(0), out.dtype == torch.float32,
-            streamk=sk, pair=pair, w_blocked=w_blocked)
+            streamk=sk, pair=pair, w_blocked=w_blocked, wide=wide)
     return out
 
 
@@ -477,7 +522,7 @@ def _bases_aligned(bases: torch.Tensor) -> bool:
 def grouped_combine(x: torch.Tensor, w: torch.Tensor, offs: Optional[torch.Tensor], recs: torch.Tensor,
                     bases: torch.Tensor, ld_out: int, bn: int = 0, outs=None, comm: Optional[GemmComm] = None,
                     streamk: Optional[bool] = None, pair: bool = False, w_blocked: bool = False,
-                    unit_weights: bool = False) -> None:
+                    unit_weights: bool = False, wide: Optional[bool] = None) -> None:
     """GEMM-2 with the combine epilogue: row t of group g becomes ``weight[t] * (x[t] @ w[g].T)`` written to row
     ``recs[t, 1]`` of the buffer ``bases[recs[t, 0]]`` (row stride ``ld_out`` elements).
 
@@ -502,16 +547,18 @@ def grouped_combine(x: torch.Tensor, w: torch.Tensor, offs: Optional[torch.Tenso
     assert recs.dtype == torch.int32 and recs.is_contiguous() and recs.shape[1] == 4 and bases.dtype == torch.int64
     if T == 0:
         return
+    if wide is None:
+        wide = not (bn or pair or streamk or comm is not None) and want_wide(EPI_COMBINE, T, F, K, G, num_sms(x.device))
     bn = bn or pick_bn(_group_hint(T, G), EPI_COMBINE)
     if pair:
         bn = max(bn, 128)
     sk = want_streamk(EPI_COMBINE, F, G, T, bn, num_sms(x.device)) if streamk is None else streamk
     _launch(w, x, None, None, offs, recs, bases, G, T, F, K, EPI_COMBINE, bn, 1, ld_out, False, comm, streamk=sk,
-            pair=pair, w_blocked=w_blocked, unit_weights=unit_weights)
+            pair=pair, w_blocked=w_blocked, unit_weights=unit_weights, wide=wide)
 
 
 def swiglu_linear(x: torch.Tensor, w13: torch.Tensor, out: Optional[torch.Tensor] = None, bn: int = 0,
-                  act: str = "silu") -> torch.Tensor:
+                  act: str = "silu", wide: Optional[bool] = None) -> torch.Tensor:
     """Dense gated up-projection: act(x @ w13[:I].T) * (x @ w13[I:].T); w13 is [2I, K] (a one-group grouped_swiglu)."""
     T, K = x.shape
     I = w13.shape[0] // 2
@@ -530,7 +577,9 @@ def swiglu_linear(x: torch.Tensor, w13: torch.Tensor, out: Optional[torch.Tensor
         out = torch.empty(T, I, dtype=torch.bfloat16, device=x.device)
     if T == 0:
         return out
+    if wide is None:
+        wide = not bn and want_wide(EPI_SWIGLU, T, I, K, 1, num_sms(x.device))
     bn = bn or pick_bn(T, EPI_SWIGLU)
     _launch(w13, x, out, None, None, None, None, 1, T, I, K, EPI_SWIGLU, bn, 1, out.stride(0), False,
-            act=ACTS[act])
+            act=ACTS[act], wide=wide)
     return out
