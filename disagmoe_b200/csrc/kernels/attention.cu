@@ -16,7 +16,7 @@
 // Cache layout: K and V each [num_blocks, block_size, kv_heads, head_dim] bf16.
 // Reference behaviour covered: vLLM paged attention / flash_attn_with_kvcache reached from
 // disagmoe/models/attention.py:150-155,219 with metadata built at disagmoe/frontend/engine.py:429-485.
-#include "dmoe_kernels.h"
+#include "attn_common.cuh"
 #include "mma_sync.cuh"
 
 namespace dmoe {
@@ -49,39 +49,6 @@ __device__ __forceinline__ void cp_async16_stream(uint32_t dst, const void* src,
   asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2, %3;" ::"r"(dst), "l"(src), "r"(sz), "l"(policy)
                : "memory");
 }
-// Options of the EXT instantiations of both kernels (plain ones compile without them):
-//   window > 0: a query at position p sees only keys in (p - window, p];
-//   chunk > 0: it sees only keys of its own chunk of `chunk` positions, counted from position 0;
-//   cap_log2 > 0: score <- cap * tanh(score / cap) before the softmax (cap_log2 = cap * log2 e, cap_in = 2 scale log2 e / cap);
-//   sink != NULL: exp(sink[head]) enters the softmax denominator (no key, no value);
-//   temp_every > 0: scores are multiplied by the query temperature 1 + temp_coef ln(floor((p + 1) / temp_every) + 1);
-//   gate != NULL: head outputs are multiplied by sigmoid(gate[row, head]) (row stride ld_gate);
-//   gq: query heads per kv head where the instantiation leaves it open (GQ = 0).
-// The EXT kernels also keep the softmax weights at fp32 accuracy in the P V product: P = hi + lo, both bf16, two MMAs.
-struct AttnExt {
-  int window, chunk;
-  float cap_in, cap_log2;
-  const float* sink;
-  int gq;
-  const void* gate;
-  long long ld_gate;
-  float temp_coef;
-  int temp_every;
-};
-__device__ __forceinline__ float query_temperature(const AttnExt& x, int p) {
-  return x.temp_every > 0 ? 1.f + x.temp_coef * logf(static_cast<float>((p + 1) / x.temp_every + 1)) : 1.f;
-}
-template <typename T>
-__device__ __forceinline__ float head_gate(const AttnExt& x, long long row, int head) {
-  return x.gate != nullptr ? 1.f / (1.f + expf(-static_cast<float>(static_cast<const T*>(x.gate)[row * x.ld_gate + head]))) : 1.f;
-}
-constexpr float kLog2e = 1.4426950408889634f;
-// first key that a query at position p sees
-__device__ __forceinline__ int first_key(int p, int window, int chunk) {
-  int lo = window > 0 ? max(0, p - window + 1) : 0;
-  if (chunk > 0) lo = max(lo, p / chunk * chunk);
-  return lo;
-}
 // 16-byte chunk c of tile row r in shared memory: rows of 128 bytes and more permute their chunks by groups of eight, rows of
 // 64 bytes (two to a 128-byte line) by groups of four; either way eight rows of one column meet no bank twice.
 template <int NCH>
@@ -89,13 +56,6 @@ __device__ __forceinline__ int swz(int c, int r) {
   static_assert(NCH == 4 || NCH % 8 == 0, "row size");
   return NCH == 4 ? c ^ ((r >> 1) & 3) : c ^ (r & 7);
 }
-// raw q.k -> score in base-2 units. tanh(x) = 1 - 2 / (exp(2x) + 1), good to ~1e-7 absolute.
-template <bool EXT>
-__device__ __forceinline__ float attn_score(float raw, float scale_log2, const AttnExt& x) {
-  if (EXT && x.cap_log2 > 0.f) return x.cap_log2 * (1.f - __fdividef(2.f, exp2f(raw * x.cap_in) + 1.f));
-  return raw * scale_log2;
-}
-
 constexpr int kAttnStages = 3;     // cp.async ring depth, per warp
 constexpr int kAttnStageTok = 16;  // cached tokens per stage and warp (block_size must be a multiple of it)
 constexpr int kAttnWarps = kAttnThreads / 32;
@@ -339,12 +299,7 @@ __global__ void attn_merge_kernel(const float* __restrict__ part_o, const float*
 // row of the sequence, position of the tile's first token}.
 constexpr int kPreKeys = 64;       // keys per pipeline stage
 constexpr int kPreRows = 64;       // query rows per CTA (4 warps x 16)
-
-// 1 / denominator of a row with running maximum m (base 2) and sum l, the sink included; 0 for a row that saw nothing.
-__device__ __forceinline__ float sink_inverse(float m, float l, float sink) {
-  const float sk = sink * kLog2e, M = fmaxf(m, sk), f = exp2f(m - M);
-  return f / (l * f + exp2f(sk - M));
-}
+constexpr int kTileRows = 128;     // query rows of a tile (tokens x query group): one CTA of prefill_attention.cu, two here
 
 template <int HD, int VD, int GQ, bool EXT>
 __global__ void __launch_bounds__(128)
@@ -362,8 +317,10 @@ prefill_attn_kernel(const __nv_bfloat16* __restrict__ q, long long ld_q, const _
   extern __shared__ __align__(128) uint8_t s_pre[];
 
   const int4 tile = tiles[blockIdx.x];
-  const int row0 = tile.x, ntok = tile.y, pos0 = tile.w;
   const int hkv = blockIdx.y, gq = GQ > 0 ? GQ : ext.gq;
+  const int skip = blockIdx.z * (kPreRows / gq);    // tokens of the tile that other CTAs have
+  const int row0 = tile.x + skip, ntok = min(tile.y - skip, kPreRows / gq), pos0 = tile.w + skip;
+  if (ntok <= 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, tq = lane & 3;
   const int* bt = block_tables + static_cast<long long>(tile.z) * max_blocks;
@@ -557,22 +514,6 @@ prefill_attn_kernel(const __nv_bfloat16* __restrict__ q, long long ld_q, const _
   }
 }
 
-// Options of a launch as the kernels take them (softcap <= 0: none; window, chunk <= 0: every key).
-static AttnExt make_ext(float scale, int window, int chunk, float softcap, const float* sink, int gq, const DmoeAttnExtra* extra) {
-  AttnExt x;
-  x.gate = extra != nullptr ? extra->gate : nullptr;
-  x.ld_gate = extra != nullptr ? extra->ld_gate : 0;
-  x.temp_coef = extra != nullptr ? extra->temp_coef : 0.f;
-  x.temp_every = extra != nullptr ? extra->temp_every : 0;
-  x.sink = sink;
-  x.gq = gq;
-  x.window = window > 0 ? window : 0;
-  x.chunk = chunk > 0 ? chunk : 0;
-  x.cap_in = softcap > 0.f ? 2.f * scale * 1.4426950408889634f / softcap : 0.f;
-  x.cap_log2 = softcap > 0.f ? softcap * 1.4426950408889634f : 0.f;
-  return x;
-}
-
 template <int HD, int VD, int GQ, bool EXT>
 static int launch_prefill(const void* q, long long ld_q, const void* kc, const void* vc, const int* bt, int max_blocks,
                           const void* tiles, int n_tiles, int block_size, int n_kv, float scale, void* out,
@@ -584,7 +525,8 @@ static int launch_prefill(const void* q, long long ld_q, const void* kc, const v
                                                  96 * 1024));
   });
   if (crc != 0) return crc;
-  dim3 grid(n_tiles, n_kv);
+  const int gq = GQ > 0 ? GQ : ext.gq, per = kPreRows / gq;
+  dim3 grid(n_tiles, n_kv, (kTileRows / gq + per - 1) / per);
   prefill_attn_kernel<HD, VD, GQ, EXT><<<grid, 128, smem, stream>>>(
       static_cast<const __nv_bfloat16*>(q), ld_q, static_cast<const __nv_bfloat16*>(kc),
       static_cast<const __nv_bfloat16*>(vc), bt, max_blocks, static_cast<const int4*>(tiles), block_size, n_kv,
@@ -696,8 +638,8 @@ extern "C" int dmoe_paged_attention_ext(const void* q, long long ld_q, const voi
 
 // Tokens per tile of dmoe_prefill_attention for a query group of n_q / n_kv heads.
 extern "C" int dmoe_prefill_tile_tokens(int n_q, int n_kv) {
-  if (n_kv < 1 || n_q % n_kv != 0) return 0;
-  return kPreRows / (n_q / n_kv);
+  if (n_kv < 1 || n_q % n_kv != 0 || n_q / n_kv > kPreRows) return 0;
+  return kTileRows / (n_q / n_kv);
 }
 
 template <bool EXT>

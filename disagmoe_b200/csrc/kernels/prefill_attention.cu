@@ -1,0 +1,335 @@
+// Causal attention of prompt rows over the paged cache on tcgen05: S = Q K^T and O += P V with accumulators in TMEM.
+//
+// One CTA owns one tile of up to 128 query rows (consecutive tokens x the query heads of one kv head) and walks the keys its
+// last token sees 128 at a time. K and V pages go straight from the cache to swizzled shared memory by TMA (one box of 64
+// head dimensions per page and half); S lands in TMEM; four warps, one row per thread, apply options and the online softmax
+// and put P back into TMEM over S, from where it is the A operand of P V. The output accumulator stays in TMEM and is only
+// rescaled when a row's maximum grew by more than 2^8 (the sums use the same stale maximum, so nothing is lost). Warp 0
+// loads, warp 1 issues the MMAs. A CTA is a serial chain QK -> softmax -> PV, so two of them share an SM (96 KB of shared
+// memory, 256 TMEM columns each) and one's softmax runs under the other's MMAs.
+//
+// EXT keeps the softmax weights at fp32 accuracy as the mma.sync kernels do: P = hi + lo, both bf16, two products.
+//
+// The mma.sync kernel of attention.cu reached 80-130 TFLOP/s (64 rows per CTA, every warp re-reading all of K and V from
+// shared memory); it stays for other head sizes, page sizes that do not divide 128 keys, and unaligned rows.
+#include <string.h>
+
+#include "attn_common.cuh"
+#include "gemm_common.cuh"
+#include "mma_sync.cuh"
+
+namespace dmoe {
+
+constexpr int kFaRows = 128, kFaKeys = 128, kFaDim = 128;
+constexpr int kFaThreads = 192;
+constexpr int kFaHalf = 128 * 128;                  // bytes of 128 rows x 64 bf16
+constexpr int kFaTile = 2 * kFaHalf;                // one of Q, K, V
+constexpr int kFaSmem = 3 * kFaTile + 1024 /*alignment*/ + 128;
+constexpr float kFaSlack = 8.f;                     // growth of a row's maximum (base 2) that is left in P
+
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+template <bool EXT>
+__global__ void __launch_bounds__(kFaThreads, 2)
+prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
+                  const __nv_bfloat16* __restrict__ q, long long ld_q, const int* __restrict__ block_tables, int max_blocks,
+                  const int4* __restrict__ tiles, int n_tiles, int n_kv, int block_size, float scale_log2, __nv_bfloat16* __restrict__ out,
+                  long long ld_out, AttnExt ext, int* status) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 3 * kFaTile);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
+  int* abort_word = reinterpret_cast<int*>(tmem_slot + 1);
+  const uint32_t sq = smem_u32(smem), sk = sq + kFaTile, sv = sk + kFaTile;
+  // K / V landed, K / V consumed, scores ready, weights ready, output accumulated
+  const uint32_t k_full = smem_u32(bars), v_full = k_full + 8, k_empty = k_full + 16, v_empty = k_full + 24, s_full = k_full + 32,
+                 p_full = k_full + 40, o_full = k_full + 48;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // tiles of a prompt are in order of position: the longest run first
+  const int4 tile = tiles[n_tiles - 1 - blockIdx.x / n_kv];
+  const int hkv = blockIdx.x % n_kv, gq = ext.gq;
+  const int row0 = tile.x, ntok = min(tile.y, kFaRows / gq), pos0 = tile.w;
+  const int* bt = block_tables + static_cast<long long>(tile.z) * max_blocks;
+  const int kmax = pos0 + ntok;
+  const int kb0 = EXT ? first_key(pos0, ext.window, ext.chunk) / kFaKeys : 0;      // first key block anyone sees
+  const int nkb = (kmax + kFaKeys - 1) / kFaKeys - kb0;
+
+  if (threadIdx.x == 0) {
+    *abort_word = 0;
+    for (int i = 0; i < 7; ++i) mbar_init(k_full + 8 * i, i == 5 ? 4 : 1);      // weights: one arrival per softmax warp
+    mbar_fence_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(smem_u32(tmem_slot), 256);
+    tmem_relinquish();
+  }
+  // query row of a softmax thread: its lane of the TMEM quarter that its warp may access
+  const int r = warp >= 2 ? (warp & 3) * 32 + lane : -1;
+  const int tok = r >= 0 ? r / gq : 0, head = hkv * gq + (r >= 0 ? r % gq : 0);
+  const bool live = r >= 0 && tok < ntok;
+  if (warp >= 2) {
+    // the row's head vector into the two halves of the K-major, 128-byte swizzled Q tile
+    const uint4* src = reinterpret_cast<const uint4*>(q + static_cast<long long>(row0 + (live ? tok : 0)) * ld_q + head * kFaDim);
+#pragma unroll
+    for (int c = 0; c < 16; ++c) {
+      const uint4 x = live ? __ldg(src + c) : make_uint4(0, 0, 0, 0);
+      *reinterpret_cast<uint4*>(smem + (c >> 3) * kFaHalf + r * 128 + (((c & 7) ^ (r & 7)) << 4)) = x;
+    }
+    fence_proxy_async_smem();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t t_s = *tmem_slot, t_o = t_s + kFaKeys;      // scores / weights [128 columns], output [128 columns]
+
+  if (warp == 0) {
+    // ------------------------------------------------------------ loads: lane = (page of the block, half of the head)
+    const int pages = kFaKeys / block_size;
+    const int page = lane >> 1, half = lane & 1;
+    for (int j = 0; j < nkb; ++j) {
+      const int key0 = (kb0 + j) * kFaKeys;
+      const int there = min(pages, (kmax - key0 + block_size - 1) / block_size);      // pages that hold visible keys
+      const bool mine = page < there;
+      const int slot = mine ? bt[key0 / block_size + page] * block_size : 0;
+      const uint32_t at = half * kFaHalf + page * block_size * 128;
+      bool ok = true;
+#pragma unroll
+      for (int kv = 0; kv < 2; ++kv) {
+        const uint32_t full = kv ? v_full : k_full;
+        ok = ok && mbar_wait(kv ? v_empty : k_empty, (j & 1) ^ 1, abort_word);
+        if (!__all_sync(0xffffffffu, ok)) break;
+        if (lane == 0) mbar_expect_tx(full, there * block_size * 256);
+        __syncwarp();
+        if (mine) tma_load_3d((kv ? sv : sk) + at, kv ? &tmV : &tmK, half * 64, hkv, slot, full);
+      }
+      if (!__all_sync(0xffffffffu, ok)) break;
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------ MMAs
+    if (lane == 0) {
+      constexpr uint32_t id_qk = umma_idesc_bf16(kFaRows, kFaKeys);
+      constexpr uint32_t id_pv = umma_idesc_bf16(kFaRows, kFaDim) | (1u << 16);      // V is MN-major
+      for (int j = 0; j < nkb; ++j) {
+        const uint32_t ph = j & 1;
+        if (!mbar_wait(k_full, ph, abort_word)) break;
+        tc_fence_after();
+        // the scores overwrite the previous block's weights: the product that read them was issued before
+#pragma unroll
+        for (int k = 0; k < kFaDim / kUmmaK; ++k) {
+          const uint32_t off = (k >> 2) * kFaHalf + (k & 3) * 32;
+          umma_f16(t_s, umma_desc_sw128(sq + off), umma_desc_sw128(sk + off), id_qk, k > 0 ? 1u : 0u);
+        }
+        umma_commit(s_full);
+        umma_commit(k_empty);
+        if (!mbar_wait(p_full, ph, abort_word)) break;
+        if (!mbar_wait(v_full, ph, abort_word)) break;
+        tc_fence_after();
+#pragma unroll
+        for (int part = 0; part < (EXT ? 2 : 1); ++part)
+#pragma unroll
+          for (int k = 0; k < kFaKeys / kUmmaK; ++k)
+            umma_f16_ta(t_o, t_s + part * (kFaKeys / 2) + k * (kUmmaK / 2), umma_desc_sw128_mn(sv + k * kUmmaK * 128, kFaHalf),
+                        id_pv, (j > 0 || part > 0 || k > 0) ? 1u : 0u);
+        umma_commit(o_full);
+        umma_commit(v_empty);
+      }
+    }
+  } else {
+    // ------------------------------------------------------------ softmax: one query row per thread
+    const uint32_t lanes = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    const int qpos = pos0 + tok;
+    const float temp = EXT ? query_temperature(ext, qpos) : 1.f;
+    const int lo = EXT ? first_key(qpos, ext.window, ext.chunk) : 0;
+    // blocks that need no mask: all keys visible to the first and the last token of the tile
+    const int lo_last = EXT ? first_key(kmax - 1, ext.window, ext.chunk) : 0;
+    const float scale = scale_log2 * temp;
+    float m = -INFINITY, l = 0.f;
+    bool ok = true;
+    for (int j = 0; j < nkb; ++j) {
+      const int key0 = (kb0 + j) * kFaKeys;
+      if (!mbar_wait(s_full, j & 1, abort_word)) { ok = false; break; }
+      if (j > 0 && !mbar_wait(o_full, (j - 1) & 1, abort_word)) { ok = false; break; }      // complete by now
+      tc_fence_after();
+      uint32_t s[4][32];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) tmem_ld32(t_s + lanes + i * 32, s[i]);
+      tmem_ld_wait();
+      const bool masked = key0 + kFaKeys - 1 > pos0 || (EXT && key0 < lo_last);
+      float mx = -INFINITY;
+      if (EXT && ext.cap_log2 > 0.f) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int e = 0; e < 32; ++e) s[i][e] = __float_as_uint(attn_score<EXT>(__uint_as_float(s[i][e]) * temp, scale_log2, ext));
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int e = 0; e < 32; ++e) s[i][e] = __float_as_uint(__uint_as_float(s[i][e]) * scale);
+      }
+      if (masked) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int e = 0; e < 32; ++e) {
+            const int key = key0 + i * 32 + e;
+            if (key > qpos || (EXT && key < lo)) s[i][e] = __float_as_uint(-INFINITY);
+          }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float a = __uint_as_float(s[i][0]), b = __uint_as_float(s[i][1]);
+#pragma unroll
+        for (int e = 2; e < 32; e += 2) {
+          a = fmaxf(a, __uint_as_float(s[i][e]));
+          b = fmaxf(b, __uint_as_float(s[i][e + 1]));
+        }
+        mx = fmaxf(mx, fmaxf(a, b));
+      }
+      const bool grow = mx > m + kFaSlack;      // true for the first finite maximum: m is -inf before it
+      if (__any_sync(0xffffffffu, grow)) {
+        const float to = grow ? mx : m;
+        if (j > 0) {
+          const float f = grow ? ex2(m - to) : 1.f;      // -inf - finite: 0, and what it scales is 0
+          l *= f;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            uint32_t o[16];
+            tmem_ld16(t_o + lanes + i * 16, o);
+            tmem_ld_wait();
+#pragma unroll
+            for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * f);
+            tmem_st16(t_o + lanes + i * 16, o);
+          }
+        }
+        m = to;
+      }
+      const float sub = m == -INFINITY ? 0.f : m;      // a row with nothing visible yet: weights 0, not NaN
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        uint32_t hi[16], rest[16];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+          const float p0 = ex2(__uint_as_float(s[i][2 * e]) - sub), p1 = ex2(__uint_as_float(s[i][2 * e + 1]) - sub);
+          sum[e & 3] += p0 + p1;
+          if (EXT) split2(p0, p1, hi[e], rest[e]);
+          else hi[e] = pack_bf16(p0, p1);
+        }
+        tmem_st16(t_s + lanes + i * 16, hi);
+        if (EXT) tmem_st16(t_s + lanes + kFaKeys / 2 + i * 16, rest);
+      }
+      l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+      if (key0 + kFaKeys > kmax) {
+        // keys past the last one: their weights are 0, but 0 times whatever the page holds there need not be
+        if (!mbar_wait(v_full, j & 1, abort_word)) ok = false;
+        const int key = threadIdx.x - 64;
+        if (key0 + key >= kmax) {
+#pragma unroll
+          for (int c = 0; c < 16; ++c)
+            *reinterpret_cast<uint4*>(smem + 2 * kFaTile + (c >> 3) * kFaHalf + key * 128 + ((c & 7) << 4)) = make_uint4(0, 0, 0, 0);
+        }
+        fence_proxy_async_smem();
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_full);
+      if (!ok) break;
+    }
+    if (ok && mbar_wait(o_full, (nkb - 1) & 1, abort_word)) {
+      tc_fence_after();
+      float inv = l > 0.f ? 1.f / l : 0.f;
+      if (EXT && ext.sink != nullptr) inv = sink_inverse(m, l, ext.sink[head]);
+      if (EXT && ext.gate != nullptr && live) inv *= head_gate<__nv_bfloat16>(ext, row0 + tok, head);
+      __nv_bfloat16* y = out + static_cast<long long>(row0 + tok) * ld_out + head * kFaDim;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        uint32_t o[32];
+        tmem_ld32(t_o + lanes + i * 32, o);
+        tmem_ld_wait();
+        if (live) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            uint4 pk;
+            uint32_t* pp = reinterpret_cast<uint32_t*>(&pk);
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              pp[e] = pack_bf16(__uint_as_float(o[c * 8 + 2 * e]) * inv, __uint_as_float(o[c * 8 + 2 * e + 1]) * inv);
+            *reinterpret_cast<uint4*>(y + i * 32 + c * 8) = pk;
+          }
+        }
+      }
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (*abort_word) {
+    if (threadIdx.x == 0 && status != nullptr) atomicCAS(status, kStatusOk, kStatusBarrierTimeout);
+    // give copies that may still be in flight time to land before shared memory is released
+    for (int i = 0; i < 200; ++i) __nanosleep(1000);
+    __syncthreads();
+  }
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(*tmem_slot, 256);
+  }
+}
+
+// The cache [blocks * block_size, n_kv, 128] as boxes of one page x one head x 64 dimensions.
+static int page_map(CUtensorMap* map, const void* cache, long long slots, int n_kv, int block_size) {
+  EncodeTiledFn enc = get_encode_fn();
+  if (enc == nullptr) return -20;
+  cuuint64_t dim[3] = {static_cast<cuuint64_t>(kFaDim), static_cast<cuuint64_t>(n_kv), static_cast<cuuint64_t>(slots)};
+  cuuint64_t stride[2] = {kFaDim * 2, static_cast<cuuint64_t>(n_kv) * kFaDim * 2};
+  cuuint32_t box[3] = {64, 1, static_cast<cuuint32_t>(block_size)};
+  cuuint32_t step[3] = {1, 1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(cache), dim, stride, box, step,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : -21;
+}
+
+template <bool EXT>
+static int launch_tc(const CUtensorMap& tmK, const CUtensorMap& tmV, const void* q, long long ld_q, const int* bt, int max_blocks,
+                     const void* tiles, int n_tiles, int block_size, int n_kv, float scale, void* out, long long ld_out, AttnExt ext,
+                     int* status, cudaStream_t stream) {
+  static PerDeviceOnce configured;
+  const int crc = configured.run([] {
+    return static_cast<int>(cudaFuncSetAttribute(prefill_tc_kernel<EXT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFaSmem));
+  });
+  if (crc != 0) return crc;
+  prefill_tc_kernel<EXT><<<n_kv * n_tiles, kFaThreads, kFaSmem, stream>>>(
+      tmK, tmV, static_cast<const __nv_bfloat16*>(q), ld_q, bt, max_blocks, static_cast<const int4*>(tiles), n_tiles, n_kv,
+      block_size, scale * kLog2e, static_cast<__nv_bfloat16*>(out), ld_out, ext, status);
+  return static_cast<int>(cudaGetLastError());
+}
+
+}  // namespace dmoe
+
+using namespace dmoe;
+
+extern "C" int dmoe_prefill_attention_tc(const void* q, long long ld_q, const void* kcache, const void* vcache, int n_blocks,
+                                         const int* block_tables, int max_blocks, const void* tiles, int n_tiles, int block_size,
+                                         int n_q, int n_kv, int plain, float scale, int window, int chunk, float softcap,
+                                         const float* sink, void* out, long long ld_out, const DmoeAttnExtra* extra, int* status,
+                                         void* stream_) {
+  if (n_tiles == 0) return 0;
+  if (n_kv < 1 || n_q % n_kv != 0 || n_q / n_kv > kFaRows || n_tiles < 0 || static_cast<long long>(n_tiles) * n_kv > 0x7fffffff || tiles == nullptr || n_blocks < 1 ||
+      block_size < 8 || kFaKeys % block_size != 0)
+    return -10;
+  CUtensorMap tmK, tmV;
+  const long long slots = static_cast<long long>(n_blocks) * block_size;
+  int rc = page_map(&tmK, kcache, slots, n_kv, block_size);
+  if (rc == 0) rc = page_map(&tmV, vcache, slots, n_kv, block_size);
+  if (rc != 0) return rc;
+  const AttnExt ext = make_ext(scale, window, chunk, softcap, sink, n_q / n_kv, extra);
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  if (plain) return launch_tc<false>(tmK, tmV, q, ld_q, block_tables, max_blocks, tiles, n_tiles, block_size, n_kv, scale, out, ld_out, ext, status, stream);
+  return launch_tc<true>(tmK, tmV, q, ld_q, block_tables, max_blocks, tiles, n_tiles, block_size, n_kv, scale, out, ld_out, ext, status, stream);
+}

@@ -43,6 +43,7 @@ class StepBuffers(TokenBuffers):
         self.prefill_tiles = z(cap, 4, dt=torch.int32)
         self.ctx_len_decode = z(cap, dt=torch.int32)
         self.n_prefill_tiles = 0
+        self.n_loose: Optional[int] = None
 
 
 class FusedModelExecutor(StepExecutor):
@@ -93,7 +94,7 @@ class FusedModelExecutor(StepExecutor):
         cfg = self.cfg
         meta = AttnMeta(buf.positions[:T], buf.slots[:T], self.block_tables, buf.bt_row[:T], buf.ctx_len[:T],
                         max_ctx=max_ctx, prefill_tiles=buf.prefill_tiles, n_prefill_tiles=buf.n_prefill_tiles,
-                        ctx_len_decode=buf.ctx_len_decode[:T])
+                        ctx_len_decode=buf.ctx_len_decode[:T], n_loose=buf.n_loose)
         resid = buf.resid[:T]
         F.embed(buf.ids[:T], self.embed_w, out=resid)
         parts = None
@@ -127,11 +128,11 @@ class FusedModelExecutor(StepExecutor):
             a0 = self.attn[self.layer_ids[0]]
             tiles, covered = F.build_prefill_tiles(bt_row, positions, F.prefill_tile_tokens(a0.num_heads, a0.num_kv_heads))
             if len(tiles):
-                buf.n_prefill_tiles = len(tiles)
+                buf.n_prefill_tiles, buf.n_loose = len(tiles), F.loose_rows(covered)
                 buf.prefill_tiles[:len(tiles)].copy_(tiles, non_blocking=True)
                 cd = torch.as_tensor(ctx_len).clone()
                 cd[covered] = 0
                 buf.ctx_len_decode[:T].copy_(cd, non_blocking=True)
 
     def _end_prefill(self, buf: StepBuffers) -> None:
-        buf.n_prefill_tiles = 0
+        buf.n_prefill_tiles, buf.n_loose = 0, None

@@ -159,7 +159,7 @@ class LayerListExecutor(StepExecutor):
                 buf.prefill_tiles[n] = (tiles.to(self.device), len(tiles))
                 cd = torch.as_tensor(ctx_len).clone()
                 cd[covered] = 0              # which rows are tiled does not depend on the tile size
-                buf.ctx_len_decode, buf.n_untiled = cd.to(self.device), int((~covered).sum())
+                buf.ctx_len_decode, buf.n_untiled = cd.to(self.device), F.loose_rows(covered)
 
     def _end_prefill(self, buf: LayerListBuffers) -> None:
         buf.segments, buf.prefill_tiles, buf.ctx_len_decode, buf.latent, buf.block_offs = None, {}, None, {}, {}

@@ -40,6 +40,8 @@ class AttnMeta:
     prefill_tiles: Optional[torch.Tensor] = None
     n_prefill_tiles: int = 0
     ctx_len_decode: Optional[torch.Tensor] = None
+    # with tiles: rows from here on are all covered by them (None: not known)
+    n_loose: Optional[int] = None
 
 
 @dataclass
@@ -167,15 +169,18 @@ class MoEAttention(torch.nn.Module):
             F.rope_kv_append(qkv, meta.positions, meta.slots, kc, vc, self.num_heads, self.num_kv_heads,
                              self.head_dim, cfg.rope_theta)
         T = qkv.shape[0]
+        tiled = qkv.is_cuda and meta.n_prefill_tiles > 0
+        n = T if not tiled or meta.n_loose is None else meta.n_loose
         splits = 1
         if qkv.is_cuda:
-            splits = F.pick_attn_splits(T, self.num_kv_heads, meta.max_ctx or cfg.max_seq_len, kc.shape[1])
-        tiled = qkv.is_cuda and meta.n_prefill_tiles > 0
-        attn = F.paged_attention(qkv[:, :self.q_size], kc, vc, meta.block_tables, meta.bt_row,
-                                 meta.ctx_len_decode if tiled else meta.ctx_len,
-                                 self.num_heads, self.num_kv_heads, self.head_dim, splits=splits)
+            splits = F.pick_attn_splits(n, self.num_kv_heads, meta.max_ctx or cfg.max_seq_len, kc.shape[1])
+        attn = torch.empty(T, self.q_size, dtype=qkv.dtype, device=qkv.device)
+        if n:
+            F.paged_attention(qkv[:n, :self.q_size], kc, vc, meta.block_tables, meta.bt_row[:n] if meta.bt_row is not None else None,
+                              (meta.ctx_len_decode if tiled else meta.ctx_len)[:n], self.num_heads, self.num_kv_heads, self.head_dim,
+                              out=attn[:n], splits=splits)
         if tiled:
-            # prompt segments: one pass over the sequence's K / V per tile of 64 query rows instead of one per row
+            # prompt segments: one pass over the sequence's K / V per tile of query rows instead of one per row
             F.prefill_attention(qkv[:, :self.q_size], kc, vc, meta.block_tables, meta.prefill_tiles,
                                 meta.n_prefill_tiles, self.num_heads, self.num_kv_heads, self.head_dim, attn)
         if self.tp_size == 1:

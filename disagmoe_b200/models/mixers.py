@@ -376,18 +376,18 @@ class SoftmaxAttention(Mixer):
         cuda = self.tiled()
         tiles, n_tiles = meta.prefill_tiles.get(F.prefill_tile_tokens(m.heads, m.kv_heads), (None, 0)) \
             if cuda and meta.prefill_tiles else (None, 0)
-        splits = 1
-        if cuda:
-            reach = min(meta.max_ctx, m.window or meta.max_ctx, m.chunk or meta.max_ctx)
-            splits = F.pick_attn_splits(q.shape[0], m.kv_heads, reach, kc.shape[1])
-        attn = None
-        if n_tiles == 0 or meta.num_decode_tokens > 0:
-            attn = F.paged_attention(q, kc, vc, meta.block_tables, meta.bt_row,
-                                     meta.ctx_len_decode if n_tiles else meta.ctx_len, m.heads, m.kv_heads, self.dk,
-                                     splits=splits, **opt)
+        T = q.shape[0]
+        n = meta.num_decode_tokens if n_tiles else T         # rows from n on are all tiled
+        attn = torch.empty(T, m.heads * self.dv, dtype=q.dtype, device=q.device)
+        if n:
+            splits = 1
+            if cuda:
+                reach = min(meta.max_ctx, m.window or meta.max_ctx, m.chunk or meta.max_ctx)
+                splits = F.pick_attn_splits(n, m.kv_heads, reach, kc.shape[1])
+            F.paged_attention(q[:n], kc, vc, meta.block_tables, meta.bt_row[:n], (meta.ctx_len_decode if n_tiles else meta.ctx_len)[:n],
+                              m.heads, m.kv_heads, self.dk, out=attn[:n], splits=splits,
+                              **{**opt, "gate": gate[:n] if gate is not None else None})
         if n_tiles:
-            if attn is None:
-                attn = torch.empty(q.shape[0], m.heads * self.dv, dtype=q.dtype, device=q.device)
             F.prefill_attention(q, kc, vc, meta.block_tables, tiles, n_tiles, m.heads, m.kv_heads, self.dk, attn, **opt)
         return attn
 

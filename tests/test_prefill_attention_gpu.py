@@ -1,0 +1,73 @@
+"""Prompt attention on tcgen05 (heads of 128) vs fp32 PyTorch: edges of query and key tiles, page sizes, garbage beyond the keys."""
+import pytest
+import torch
+
+from disagmoe_b200.config import QueryTemperature
+from disagmoe_b200.ops import functional as F
+from disagmoe_b200.ops import gemm, reference
+
+pytestmark = pytest.mark.gpu
+
+HD = 128
+# (block-table row, first position, tokens)
+SEGS = [(0, 0, 300), (1, 0, 128), (2, 137, 70), (3, 0, 8), (4, 31, 129), (5, 255, 9), (6, 127, 257)]
+
+
+def _run(n_q, n_kv, bs, poison=False, seed=0, **opt):
+    torch.manual_seed(seed)
+    maxb, rows, pos = 512 // bs, [], []
+    for r, p0, n in SEGS:
+        rows += [r] * n
+        pos += list(range(p0, p0 + n))
+    T, nb = len(rows), 7 * maxb
+    bf = lambda *s: torch.randn(*s, device="cuda").to(torch.bfloat16)
+    q, kc, vc = bf(T, n_q * HD), bf(nb, bs, n_kv, HD), bf(nb, bs, n_kv, HD)
+    bt = torch.randperm(nb, device="cuda").view(7, maxb).int()
+    bt_row = torch.tensor(rows, dtype=torch.int32, device="cuda")
+    ctx = torch.tensor(pos, dtype=torch.int32, device="cuda") + 1
+    if "gate" in opt:
+        opt["gate"] = bf(T, n_q)
+    if "sink" in opt:
+        opt["sink"] = torch.randn(n_q, device="cuda")
+    ref = reference.paged_attention(q, kc, vc, bt, bt_row, ctx, n_q, n_kv, HD, opt.get("scale"), opt.get("window"), opt.get("softcap"),
+                                    opt.get("sink"), opt.get("chunk"), opt.get("q_temp"), opt.get("gate"))
+    if poison:
+        # what a page holds behind the last cached token must not matter
+        for r, p0, n in SEGS:
+            for p in range(p0 + n, maxb * bs):
+                for c in (kc, vc):
+                    c[bt[r, p // bs].long(), p % bs] = float("nan")
+    tiles, covered = F.build_prefill_tiles(rows, pos, F.prefill_tile_tokens(n_q, n_kv))
+    assert bool(covered.all()) and F.loose_rows(covered) == 0
+    out = torch.full((T, n_q * HD), 9.0, dtype=torch.bfloat16, device="cuda")
+    assert F._prefill_on_tcgen05(q, kc, vc, out, HD, HD)
+    F.prefill_attention(q, kc, vc, bt, tiles.cuda(), len(tiles), n_q, n_kv, HD, out, **opt)
+    assert gemm.check_status() == 0
+    return out.float(), ref.float()
+
+
+def _close(y, ref, tol):
+    bound = ref.abs() * tol + ref.pow(2).mean().sqrt() * tol
+    bad = int(((y - ref).abs() > bound).sum())
+    assert bad == 0, f"{bad} of {ref.numel()} off, max {(y - ref).abs().max().item():.4g}"
+
+
+@pytest.mark.parametrize("n_q,n_kv", [(2, 2), (8, 2), (8, 1), (6, 2), (64, 1)])
+@pytest.mark.parametrize("bs", [8, 16, 64, 128])
+def test_plain(n_q, n_kv, bs):
+    # softmax weights and outputs are rounded to bf16 once each: two roundings of 2^-9, some on sums of several terms
+    _close(*_run(n_q, n_kv, bs, poison=True, fp32_weights=n_q // n_kv in (3, 64)), tol=2 ** -6)
+
+
+@pytest.mark.parametrize("opt", [
+    dict(window=64), dict(window=1, sink=None), dict(window=200, softcap=20.0), dict(chunk=96), dict(chunk=128, window=40),
+    dict(sink=None, gate=None), dict(q_temp=QueryTemperature(0.3, 50), scale=0.2), dict(fp32_weights=True, scale=3.0),
+])
+def test_options(opt):
+    # fp32 softmax weights: one rounding of the output, 2^-9 relative, and twice that for the bf16 reference it is compared in
+    _close(*_run(8, 2, 16, poison=True, **opt), tol=2 ** -7)
+
+
+def test_loose_rows():
+    assert F.loose_rows(torch.tensor([True, False, True])) == 2 and F.loose_rows(torch.zeros(4, dtype=torch.bool)) == 4
+    assert F.loose_rows(torch.ones(3, dtype=torch.bool)) == 0
