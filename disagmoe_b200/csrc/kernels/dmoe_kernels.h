@@ -18,6 +18,9 @@ typedef struct DmoeRouter {
   int E, K, renorm, sigmoid, groups, keep;
   float wscale;
 } DmoeRouter;
+// Logits h @ weight.T (+ logit_bias [E]) of normalised bf16 rows on the tensor cores, and the choice of experts (router.cu); H a
+// multiple of 256, 16-byte aligned rows. logits [T, E]: optional copy of the logits.
+int dmoe_router(const void* h, long long ld_h, int T, int H, const DmoeRouter* r, const float* logit_bias, float* logits, void* stream);
 // Token shift: n_mix outputs h + (before - h) mu per row, `before` = the row before in the sequence, kept per slot in `last`.
 // singles: int4 {row, 1, slot, position}; NULL: one-token segment i is row i, as in DmoeRecur.
 typedef struct DmoeShift {
@@ -184,6 +187,9 @@ int dmoe_rope_kv_append(void* qkv, long long ld, const int* positions, const lon
 int dmoe_rope_table(void* table, int max_pos, int hd, float theta, void* stream);
 int dmoe_embed(const int* ids, const void* table, void* out, int T, int H, int vocab, long long ld_out, void* stream);
 int dmoe_argmax(const void* logits, int is_f32, long long ld, int T, int V, int* ids, void* stream);
+// resid[t] += sh[t] * sigmoid(y[t] . w): bf16 rows of H elements, 16-byte aligned.
+int dmoe_gated_add(void* resid, long long ld_r, const void* sh, long long ld_s, const void* y, long long ld_y, const void* w, int T, int H,
+                   void* stream);
 int dmoe_permute_rows(const void* src, long long ld_src, void* dst, long long ld_dst, const int* map, int n, int H,
                       int repeat, int gather, void* stream);
 int dmoe_gather_ptrs(const void* ptrs, void* dst, long long ld_dst, int n, int H, void* stream);

@@ -3,6 +3,7 @@
 // whole segments, per-head query / key norm + partial rotary embedding + value mixing + paged KV append, rotary table from arbitrary frequencies, act(gate) * up,
 // and a CUDA-core GEMM, dense or over row groups, for fp32 operands (and for bf16 shapes the tcgen05 kernel's TMA cannot
 // address).
+#include "router_choose.cuh"
 #include "dmoe_kernels.h"
 #include "row_pack.cuh"
 
@@ -166,7 +167,6 @@ __device__ __forceinline__ int4 single_segment(const A& s, long long i) {
   return make_int4(static_cast<int>(i), s.kv_slots[i] >= 0 ? 1 : 0, s.rows[i], s.positions[i]);
 }
 constexpr int kSumThreads = 256, kSumWarps = kSumThreads / 32;
-constexpr int kMaxExperts = 256, kMaxTop = 32;
 
 // add += sum over the two sides of row / root mean square (with the scale: inv) * weights, columns v * VEC ..
 template <typename T, int VEC>
@@ -383,72 +383,8 @@ __global__ void __launch_bounds__(kSumThreads) sum_norm_kernel(const SumNormArgs
   __syncthreads();
   const long long tok = static_cast<long long>(blockIdx.x) * TPC + warp;
   if (warp >= TPC || tok >= a.n) return;
-  float* lg = slog[warp];
-  float* score = sscore[warp];
-  float mx = -INFINITY, den = 0.f;
-  if (a.sigmoid) {
-    for (int e = lane; e < a.E; e += 32) {
-      score[e] = 1.f / (1.f + expf(-lg[e]));
-      lg[e] = score[e] + (a.correction != nullptr ? a.correction[e] : 0.f);
-    }
-    __syncwarp();
-    if (a.keep < a.groups) {
-      const int per = a.E / a.groups;
-      float* sum = sgroup[warp];
-      for (int g = lane; g < a.groups; g += 32) {
-        float first = -INFINITY, second = -INFINITY;
-        for (int e = g * per; e < (g + 1) * per; ++e) {
-          const float c = lg[e];
-          if (c > first) { second = first; first = c; }
-          else if (c > second) second = c;
-        }
-        sum[g] = per > 1 ? first + second : first;
-      }
-      __syncwarp();
-      for (int g = lane; g < a.groups; g += 32) {
-        int ahead = 0;
-        for (int q = 0; q < a.groups; ++q) ahead += sum[q] > sum[g] || (sum[q] == sum[g] && q < g);
-        if (ahead >= a.keep)
-          for (int e = g * per; e < (g + 1) * per; ++e) lg[e] = -INFINITY;
-      }
-      __syncwarp();
-    }
-  } else {
-    for (int e = lane; e < a.E; e += 32) mx = fmaxf(mx, lg[e]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    for (int e = lane; e < a.E; e += 32) den += expf(lg[e] - mx);
-    den = warp_sum(den);
-  }
-  int my_id = -1;           // lane k keeps the k-th choice
-  float my_w = 0.f, total = 0.f;
-  for (int k = 0; k < a.K; ++k) {
-    float best = -INFINITY;
-    int bi = 0x7fffffff;
-    for (int e = lane; e < a.E; e += 32)
-      if (lg[e] > best) { best = lg[e]; bi = e; }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-    }
-    float s = a.sigmoid ? (bi < a.E ? score[bi] : 0.f) : expf(best - mx) / den;
-    if (bi >= a.E) {        // no finite logit left: the lowest expert not chosen yet, so that the ids stay valid
-      for (bi = 0; __any_sync(0xffffffffu, my_id == bi);) ++bi;
-      s = 0.f;
-    }
-    if (lane == k) { my_id = bi; my_w = s; }
-    total += s;
-    __syncwarp();
-    if (lane == 0) lg[bi] = -INFINITY;
-    __syncwarp();
-  }
-  if (lane < a.K) {
-    a.ids[tok * a.K + lane] = my_id;
-    a.wts[tok * a.K + lane] = (a.renorm && total > 0.f ? my_w / total : my_w) * a.wscale;
-    if (a.counts != nullptr) atomicAdd(&a.counts[my_id], 1);
-  }
+  choose_experts(slog[warp], sscore[warp], sgroup[warp], a.E, a.K, a.renorm, a.sigmoid, a.groups, a.keep, a.correction, a.wscale, lane,
+                 a.ids + tok * a.K, a.wts + tok * a.K, a.counts);
 }
 
 // Token shift of a batch that holds longer segments: rows h (fp32) -> S mixed rows h + (before - h) mu_s, `before` = the row before

@@ -218,9 +218,7 @@ class MoEAttention(torch.nn.Module):
         if self.shared_gate is None:
             return self._ffn(y, self.shared_w13, self.shared_w2, resid)
         sh = self._ffn(y, self.shared_w13, self.shared_w2, None)
-        g = torch.sigmoid(y.float() @ self.shared_gate.float().T)
-        resid.copy_((resid.float() + sh.float() * g).to(resid.dtype))
-        return resid
+        return F.gated_add(resid, sh, y, self.shared_gate)
 
     def dense_ffn(self, resid: torch.Tensor, h: Optional[torch.Tensor] = None) -> torch.Tensor:
         """resid += mlp(rmsnorm(resid)) for a layer with a dense FFN, in place (h: the normalised rows if the

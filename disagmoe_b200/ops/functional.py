@@ -264,6 +264,19 @@ def gather_ptrs(ptrs: torch.Tensor, n: int, H: int, out: torch.Tensor) -> torch.
     return out
 
 
+def separate_router(T: int, H: int, E: int, h: torch.Tensor, weight: torch.Tensor) -> bool:
+    """Should the router run as a kernel of its own on the tensor cores (csrc/kernels/router.cu) behind the norm, instead of inside
+    it on the CUDA cores? Measured on B200 (norm + router in one kernel -> in two): 4096 rows of 4096, 8 experts 98 -> 41 us; 1111 rows of
+    2048, 64 experts 82 -> 22; 3000 rows of 2048, 64 experts, after a sum 108 -> 45; 37 rows of 2048, 60 experts 22 -> 16. One row and 8
+    experts take 7.5 us in one kernel, which a second launch does not beat."""
+    return H % 256 == 0 and E <= 256 and (E > 16 or T >= 128) and h.stride(0) % 8 == 0 and h.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0
+
+
+def _router(h: torch.Tensor, rd, bias: Optional[torch.Tensor] = None, logits: Optional[torch.Tensor] = None) -> None:
+    _lib.check(_lib.lib().dmoe_router(_vp(h), c_ll(h.stride(0)), c_int(h.shape[0]), c_int(h.shape[1]), ctypes.byref(rd), _vp(bias),
+                                      _vp(logits), _st()), "dmoe_router")
+
+
 def route(x: torch.Tensor, norm_w: Optional[torch.Tensor], eps: float, gate_w: torch.Tensor, top_k: int,
           renormalize: bool = True, y: Optional[torch.Tensor] = None, counts: Optional[torch.Tensor] = None,
           want_logits: bool = False, logit_bias: Optional[torch.Tensor] = None):
@@ -287,6 +300,14 @@ def route(x: torch.Tensor, norm_w: Optional[torch.Tensor], eps: float, gate_w: t
     logits = torch.empty(T, E, dtype=torch.float32, device=x.device) if want_logits else None
     assert gate_w.is_contiguous() and gate_w.dtype == torch.bfloat16 and x.stride(1) == 1
     assert logit_bias is None or (logit_bias.dtype == torch.float32 and logit_bias.is_cuda and logit_bias.numel() == E)
+    if x.dtype == torch.bfloat16 and top_k <= min(8, E) and separate_router(T, H, E, y, gate_w):
+        # the same kernel without its router, then the router on the normalised rows
+        _lib.check(_lib.lib().dmoe_route_ex(
+            _vp(x), c_ll(x.stride(0)), _vp(norm_w), c_float(eps), None, c_int(T), c_int(H), c_int(0), c_int(0), c_int(0), _vp(y),
+            c_ll(y.stride(0)), None, None, None, None, c_int(0), c_ll(0), None, c_ll(0), c_int(0), c_int(0), None, _st()), "dmoe_route_ex")
+        rd = _lib.DmoeRouter(gate_w.data_ptr(), None, ids.data_ptr(), w.data_ptr(), _lib.ptr(counts), E, top_k, int(renormalize), 0, 1, 1, 1.0)
+        _router(y, rd, logit_bias, logits)
+        return y, ids, w, logits
     _lib.check(_lib.lib().dmoe_route(
         _vp(x), c_ll(x.stride(0)), _vp(norm_w), c_float(eps), _vp(gate_w), c_int(T), c_int(H), c_int(E), c_int(top_k),
         c_int(int(renormalize)), _vp(y), c_ll(y.stride(0)), _vp(ids), _vp(w), _vp(logits), _vp(counts),
@@ -310,6 +331,20 @@ class DispatchBuffers:
     @property
     def counts(self):
         return self.ws[: self.E]
+
+
+def gated_add(resid: torch.Tensor, sh: torch.Tensor, y: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+    """resid += sh * sigmoid(y @ w.T), in place (w [1, H]): the gated shared expert. bf16 rows on the GPU are one launch."""
+    rows = (resid, sh, y)
+    if resid.is_cuda and all(t.dtype == torch.bfloat16 and t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in rows) \
+            and w.dtype == torch.bfloat16 and w.is_contiguous() and w.data_ptr() % 16 == 0 and resid.shape[1] % 8 == 0:
+        T, H = resid.shape
+        _lib.check(_lib.lib().dmoe_gated_add(_vp(resid), c_ll(resid.stride(0)), _vp(sh), c_ll(sh.stride(0)), _vp(y), c_ll(y.stride(0)),
+                                             _vp(w), c_int(T), c_int(H), _st()), "dmoe_gated_add")
+        return resid
+    g = torch.sigmoid(y.float() @ w.float().T)
+    resid.copy_((resid.float() + sh.float() * g).to(resid.dtype))
+    return resid
 
 
 def dispatch_local(y: torch.Tensor, topk_ids: torch.Tensor, topk_w: torch.Tensor, buf: DispatchBuffers) -> None:
@@ -715,6 +750,8 @@ def sum_norm(resid: torch.Tensor, y, parts: Optional[torch.Tensor], w: torch.Ten
                              int(router.renormalize), int(router.sigmoid), router.groups, router.keep, router.scale)
     if shift is not None and not two_steps:
         sd = shift.descriptor(n)
+    after = rd is not None and dtype == torch.bfloat16 and rd.K <= min(32, rd.E) and rd.groups >= 1 and rd.keep >= 1 and \
+        rd.E % rd.groups == 0 and separate_router(n, W, rd.E, h, router.weight)
     x = cd = None
     if bias is not None or gate is not None or sides is not None or conv is not None:
         x = _lib.DmoeSumExtra()
@@ -738,8 +775,11 @@ def sum_norm(resid: torch.Tensor, y, parts: Optional[torch.Tensor], w: torch.Ten
         _f32(dtype), _vp(resid), _vp(y), c_ll(y.stride(0) if y is not None else 0), _vp(parts),
         c_int(parts.shape[1] if parts is not None else 0), c_ll(parts.stride(0) if parts is not None else 0),
         c_ll(parts.stride(1) if parts is not None else 0), c_float(mult), _vp(w), c_int(int(centred)), c_float(eps), _vp(rows),
-        _vp(h), c_int(int(two_steps)), c_ll(W), c_int(n), c_int(W), ctypes.byref(rd) if rd else None,
-        ctypes.byref(sd) if sd else None, ctypes.byref(x) if x else None, _st()), "dmoe_sum_norm")
+        _vp(h), c_int(int(two_steps)), c_ll(W), c_int(n), c_int(W),
+        ctypes.byref(rd) if rd and not after else None, ctypes.byref(sd) if sd else None, ctypes.byref(x) if x else None, _st()),
+        "dmoe_sum_norm")
+    if after:
+        _router(h, rd)
     if conv is not None and cd is None:
         seq_conv(h[0], conv.w, conv.ring, conv.segs, residual=True, out=h[1])
     return (token_shift(h, shift, dtype) if two_steps else h), ids, wts
