@@ -133,6 +133,8 @@ __device__ __forceinline__ RowFactors row_factors(const DmoeRecur& a, const floa
 template <typename T, int MODE, bool CONV, int VEC>
 __global__ void __launch_bounds__(kStepThreads, 2)
 step_kernel(const DmoeRecur a, int vt) {
+  pdl_trigger();
+  pdl_wait();
   constexpr bool DELTA = MODE == kDelta;
   extern __shared__ __align__(16) float s_mem[];
   const int tid = threadIdx.x, lane = tid & 31;
@@ -261,6 +263,8 @@ step_kernel(const DmoeRecur a, int vt) {
 template <typename T, int MODE, bool CONV, int NT>
 __global__ void __launch_bounds__(NT, 3 * kStepThreads / NT)
 stream_step_kernel(const DmoeRecur a) {
+  pdl_trigger();
+  pdl_wait();
   constexpr bool DELTA = MODE == kDelta;
   extern __shared__ __align__(128) float s_stream[];
   __shared__ __align__(8) unsigned long long s_bar;
