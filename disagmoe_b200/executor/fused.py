@@ -129,10 +129,10 @@ class FusedModelExecutor(StepExecutor):
             tiles, covered = F.build_prefill_tiles(bt_row, positions, F.prefill_tile_tokens(a0.num_heads, a0.num_kv_heads))
             if len(tiles):
                 buf.n_prefill_tiles, buf.n_loose = len(tiles), F.loose_rows(covered)
-                buf.prefill_tiles[:len(tiles)].copy_(tiles, non_blocking=True)
+                buf.prefill_tiles[:len(tiles)].copy_(tiles.pin_memory(), non_blocking=True)
                 cd = torch.as_tensor(ctx_len).clone()
                 cd[covered] = 0
-                buf.ctx_len_decode[:T].copy_(cd, non_blocking=True)
+                buf.ctx_len_decode[:T].copy_(cd.pin_memory(), non_blocking=True)
 
     def _end_prefill(self, buf: StepBuffers) -> None:
         buf.n_prefill_tiles, buf.n_loose = 0, None

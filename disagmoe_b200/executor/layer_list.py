@@ -27,6 +27,7 @@ from ..models.mixers import (GatedFeedForward, LatentTables, RoutedBuffers, Rout
                              make_mixer)
 from ..ops import functional as F
 from ..ops import gemm
+from ..ops._lib import upload
 from ..ops.recurrent import MAX_TAPS, RecurrentState, SegmentTables, build_segments, decode_segments
 from .step import StepExecutor, TokenBuffers
 
@@ -156,16 +157,16 @@ class LayerListExecutor(StepExecutor):
                 continue
             tiles, covered = F.build_prefill_tiles(bt_row, positions, n)
             if len(tiles):
-                buf.prefill_tiles[n] = (tiles.to(self.device), len(tiles))
+                buf.prefill_tiles[n] = (upload(tiles, self.device), len(tiles))
                 cd = torch.as_tensor(ctx_len).clone()
                 cd[covered] = 0              # which rows are tiled does not depend on the tile size
-                buf.ctx_len_decode, buf.n_untiled = cd.to(self.device), F.loose_rows(covered)
+                buf.ctx_len_decode, buf.n_untiled = upload(cd, self.device), F.loose_rows(covered)
 
     def _end_prefill(self, buf: LayerListBuffers) -> None:
         buf.segments, buf.prefill_tiles, buf.ctx_len_decode, buf.latent, buf.block_offs = None, {}, None, {}, {}
 
     def _block_offs(self, T: int) -> Dict[int, torch.Tensor]:
-        return {n: (torch.arange(n + 1, dtype=torch.int32) * T).to(self.device) for n in self.blocks_of_rows}
+        return {n: upload(torch.arange(n + 1, dtype=torch.int32) * T, self.device) for n in self.blocks_of_rows}
 
     def _decode_tables(self, T: int) -> Tuple[Dict[Tuple, LatentTables], Dict[int, torch.Tensor]]:
         """Latent tables and block offsets, made once per batch size: graphs replay on them."""

@@ -107,7 +107,7 @@ class StepExecutor:
         self._fill(buf, T, ids, positions, slots, ctx_len, bt_row)
         self._begin_prefill(buf, T, positions, ctx_len, bt_row)
         if out_rows is not None:
-            buf.out_rows = torch.tensor(out_rows, dtype=torch.int32).to(self.device)
+            buf.out_rows = _lib.upload(torch.tensor(out_rows, dtype=torch.int32), self.device)
         try:
             return self._forward(buf, T, int(ctx_len.max()), want_logits)
         finally:

@@ -17,6 +17,7 @@ from ..config import (AttentionSpec, ChannelDeltaSpec, GatedLinearSpec, GatedUni
                       LayerListConfig, MatrixMemorySpec, SideBySideSpec, WkvSpec)
 from ..ops import functional as F
 from ..ops import gemm
+from ..ops._lib import upload
 from ..ops.recurrent import (GatedUnit, Recurrence, RecurrentState, SegmentTables, recurrent_attention, unit_recurrence)
 from .attention import AttnMeta
 from .experts import ExpertStack
@@ -69,7 +70,7 @@ class LatentTables:
         recs = torch.zeros(heads * n, 4, dtype=torch.int32)
         recs[:, 1] = (rows[None].long() * heads + torch.arange(heads)[:, None]).reshape(-1).int()
         recs[:, 2] = torch.ones(1).view(torch.int32)
-        return (torch.arange(heads + 1, dtype=torch.int32) * n).to(device), recs.to(device)
+        return upload(torch.arange(heads + 1, dtype=torch.int32) * n, device), upload(recs, device)
 
     @classmethod
     def decode(cls, m: LatentAttentionSpec, T: int, device) -> "LatentTables":
@@ -99,8 +100,8 @@ class LatentTables:
             keys[a:b, 0], keys[a:b, 1] = row[begins[i]], np.arange(lo[i], hi[i])
         base = torch.from_numpy(np.repeat(at[:-1] - lo, ends - begins + 1).astype(np.int32))
         keys = torch.from_numpy(keys)
-        t = cls(len(rows), loose.to(device), rows.to(device), None, None, tiles.to(device),
-                base.to(device), len(tiles), keys.to(device), len(keys))
+        up = lambda x: upload(x, device)
+        t = cls(len(rows), up(loose), up(rows), None, None, up(tiles), up(base), len(tiles), up(keys), len(keys))
         if len(rows):
             t.offs, t.recs = cls._per_head(rows, m.heads, device)
         return t

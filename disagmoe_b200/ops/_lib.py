@@ -135,7 +135,14 @@ def lib():
 
 
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream of the current device, without the Python stream object (every launch asks for it)."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+
+
+def upload(t: torch.Tensor, device) -> torch.Tensor:
+    """A host table on the device. To a GPU it goes through pinned memory, in stream order: a copy from pageable memory makes the
+    host wait for everything that is queued, and a step has several tables."""
+    return t.pin_memory().to(device, non_blocking=True) if torch.device(device).type == "cuda" else t.to(device)
 
 
 LAUNCHES = 0   # entry-point calls that launched kernels of this library (a graph replay adds its captured count)

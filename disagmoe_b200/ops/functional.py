@@ -494,9 +494,9 @@ def build_prefill_tiles(bt_row, positions, tile_tokens: int, min_len: int = 8):
         if b - a < min_len:
             continue
         covered[a:b] = True
-        for t0 in range(a, b, tile_tokens):
-            tiles.append((t0, min(tile_tokens, b - t0), int(rows[a]), int(pos[t0])))
-    t = torch.tensor(tiles, dtype=torch.int32).reshape(-1, 4)
+        t0 = np.arange(a, b, tile_tokens)
+        tiles.append(np.stack([t0, np.minimum(tile_tokens, b - t0), np.full_like(t0, rows[a]), pos[t0]], 1))
+    t = torch.from_numpy(np.concatenate(tiles).astype(np.int32)) if tiles else torch.zeros(0, 4, dtype=torch.int32)
     return t, torch.from_numpy(covered)
 
 

@@ -14,6 +14,7 @@ operands (and bf16 operands whose rows are not 16-byte aligned) the CUDA-core ke
 from __future__ import annotations
 
 import ctypes
+from functools import lru_cache
 from typing import Optional
 
 import torch
@@ -82,14 +83,14 @@ def pick_splitk(T: int, F: int, K: int, bn: int, sms: int = 0) -> int:
     return max(1, min((sms * 128 // 148 + tiles // 2) // tiles, kblocks // 4, 16))
 
 
-def dense_cost(T: int, F: int, K: int, sms: int = 0):
+@lru_cache(maxsize=4096)
+def dense_cost(T: int, F: int, K: int, sms: int):
     """(cost in us, token tile, split-K factor) of a dense GEMM below one wave of tiles, by a cost model fitted to the tile /
     split sweep of benchmark/ops/dense_gemm.py on B200. At these sizes a CTA is bound by what its SM can pull from L2
     (~100 GB/s: 16 KB of weights plus bn x 128 B of tokens per K block), so the model counts, per CTA, the bytes of
     its K range times the number of waves, the parked and re-read partial tiles of a split (the last arriver reads
     them chunk by chunk, latency-bound) and a fixed launch + pipeline-fill cost. It reproduces the order of the
     measured configurations (QKV and o_proj of Mixtral at 64-512 tokens)."""
-    sms = sms or num_sms()
     kblocks = (K + 63) // 64
     mt = (F + 127) // 128
     best = None
@@ -115,7 +116,7 @@ def dense_cost(T: int, F: int, K: int, sms: int = 0):
 
 def pick_dense(T: int, F: int, K: int, sms: int = 0):
     """(token tile, split-K factor) of :func:`dense_cost`."""
-    return dense_cost(T, F, K, sms)[1:]
+    return dense_cost(T, F, K, sms or num_sms())[1:]
 
 
 def pick_bn(tokens_per_group: int, epi: int) -> int:
@@ -152,6 +153,7 @@ def want_streamk(epi: int, F: int, G: int, T: int, bn: int, sms: int) -> bool:
     return tiles / (waves * sms) < 0.85
 
 
+@lru_cache(maxsize=4096)
 def want_wide(epi: int, T: int, F: int, K: int, G: int, sms: int) -> bool:
     """Should the tokens be the M operand (csrc/kernels/gemm_wide.cu, 256 x 256 tiles on CTA pairs) instead of the weights?
 
@@ -263,28 +265,45 @@ def _launch(W, X, Y, R, offs, recs, bases, G, T, F, K, epi, bn, splitk, ldy, y_f
             streamk: bool = False, pair: bool = False, w_blocked: bool = False, act: int = 0, act_limit: float = 0.0,
             act_cols: int = 0, unit_weights: bool = False, wide: bool = False):
     s = scratch(X.device)
-    d = _lib.DmoeGemm()
-    d.wide = int(wide)
-    d.act_limit, d.act_cols, d.unit_weights = act_limit, act_cols, int(unit_weights)
-    d.w_blocked, d.act = int(w_blocked), act
-    d.trace = TRACE.data_ptr() if TRACE is not None else None
-    d.streamk, d.n_counters = int(streamk and splitk <= 1 and not pair), s.counters.numel()
-    d.pair = int(pair)
-    d.combine_vec = int(epi == EPI_COMBINE and F % 8 == 0 and ldy % 8 == 0 and _bases_aligned(bases))
+    d = _lib.DmoeGemm()           # zeros: only what a launch has is filled in
+    if wide:
+        d.wide = 1
+    if act:
+        d.act, d.act_limit, d.act_cols = act, act_limit, act_cols
+    if unit_weights:
+        d.unit_weights = 1
+    if w_blocked:
+        d.w_blocked = 1
+    if TRACE is not None:
+        d.trace = TRACE.data_ptr()
+    if streamk and splitk <= 1 and not pair:
+        d.streamk = 1
+    d.n_counters = s.counters.numel()
+    if pair:
+        d.pair = 1
     if comm is not None:
         comm.fill(d)
-    d.W, d.X, d.Y, d.R = W.data_ptr(), X.data_ptr(), _lib.ptr(Y), _lib.ptr(R)
-    d.offs, d.recs, d.bases = _lib.ptr(offs), _lib.ptr(recs), _lib.ptr(bases)
+    d.W, d.X = W.data_ptr(), X.data_ptr()
+    if Y is not None:
+        d.Y = Y.data_ptr()
+    if R is not None:
+        d.R, d.ldr = R.data_ptr(), R.stride(0)
+    if offs is not None:
+        d.offs = offs.data_ptr()
+    if recs is not None:
+        d.recs = recs.data_ptr()
+    if bases is not None:
+        d.bases = bases.data_ptr()
+        d.combine_vec = int(epi == EPI_COMBINE and F % 8 == 0 and ldy % 8 == 0 and _bases_aligned(bases))
     if splitk > 1:
         need = _lib.lib().dmoe_gemm_workspace_bytes(T, F, bn, splitk)
         s.ensure(need)
-    d.ws, d.counters, d.status = s.ws.data_ptr(), s.counters.data_ptr(), s.status.data_ptr()
-    d.ws_bytes = s.ws.numel()
-    d.ldx = X.stride(0)
-    d.ldy = ldy
-    d.ldr = R.stride(0) if R is not None else 0
+    d.ws, d.counters, d.status, d.ws_bytes = s.ws.data_ptr(), s.counters.data_ptr(), s.status.data_ptr(), s.ws.numel()
+    d.ldx, d.ldy = X.stride(0), ldy
     d.G, d.T, d.F, d.K = G, T, F, K
-    d.epi, d.bn, d.splitk, d.y_f32 = epi, bn, splitk, int(y_f32)
+    d.epi, d.bn, d.splitk = epi, bn, splitk
+    if y_f32:
+        d.y_f32 = 1
     _lib.check(_lib.lib().dmoe_gemm(ctypes.byref(d), _lib.stream_ptr()), "dmoe_gemm")
 
 

@@ -60,9 +60,9 @@ def build_segments(bt_row, positions, device) -> SegmentTables:
             continue
         chunks += [(c, min(CHUNK, b - c), len(multi), i) for i, c in enumerate(range(a, b, CHUNK))]
         multi.append(seg)
-    table = torch.tensor(singles + multi + chunks, dtype=torch.int32).reshape(-1, 4)
+    table = torch.from_numpy(np.array(singles + multi + chunks, dtype=np.int32).reshape(-1, 4))
     if torch.device(device).type == "cuda":
-        table = table.to(device)
+        table = _lib.upload(table, device)
     s, m = len(singles), len(multi)
     return SegmentTables(s, m, len(chunks), max((x[1] for x in multi), default=0), table[:s], table[s:s + m], table[s + m:])
 
