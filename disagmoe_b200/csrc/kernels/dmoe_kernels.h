@@ -252,6 +252,12 @@ int dmoe_latent_prefill(const void* q, long long ld_q, const void* kv, long long
 // (<= dmoe_prefill_tile_tokens), block-table row, position of the first token}; the tokens of a tile are consecutive
 // rows at consecutive positions of one sequence, whose K / V (own tokens included) are already in the paged cache.
 int dmoe_prefill_tile_tokens(int n_q, int n_kv);
+// dmoe_latent_prefill on tcgen05 (prefill_attention.cu) for heads of 128 + 64 rotated numbers and values of 128; n_keys rows of kv
+// and lat; 16-byte aligned rows.
+int dmoe_latent_prefill_tc(const void* q, long long ld_q, const void* kv, long long ld_kv, const void* lat, long long ld_lat,
+                           long long n_keys, const void* tiles, const int* base, int n_tiles, int heads, int rankp, float scale,
+                           int window, const float* sink, const void* gate, long long ld_gate, void* out, long long ld_out, int* status,
+                           void* stream);
 // The same on tcgen05 (prefill_attention.cu) for heads of 128: pages of block_size tokens that divide 128 keys (at least 8),
 // 16-byte aligned rows of q, out and the caches ([n_blocks, block_size, n_kv, 128]). plain != 0: no options, softmax weights in
 // bf16 (dmoe_prefill_attention); else those of dmoe_prefill_attention_ext. status: device word, see DmoeGemm.

@@ -413,8 +413,8 @@ latent_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ 
 }
 
 // ---------------------------------------------------------------------------------------------------------------------------
-// Prompt runs over expanded keys and values: a CTA of four warps has 64 consecutive tokens of one head (16 per warp as MMA
-// rows), keys 64 at a time, double buffered. KD / VD: key (unrotated + rotated) and value sizes rounded up to the tile's.
+// Prompt runs over expanded keys and values in head sizes that prefill_attention.cu does not take: a tile is up to 128 consecutive
+// tokens of one head, a CTA of four warps has 64 of them (16 per warp as MMA rows), keys 64 at a time, double buffered. KD / VD: key (unrotated + rotated) and value sizes rounded up to the tile's.
 constexpr int kLpKeys = 64;
 
 template <int KD, int VD>
@@ -428,7 +428,9 @@ latent_prefill_kernel(const bf16* __restrict__ q, long long ld_q, const bf16* __
   constexpr int KS = KD / 16, NT = VD / 8;
   extern __shared__ __align__(128) uint8_t smem[];
   const int4 tile = tiles[blockIdx.x];
-  const int row0 = tile.x, ntok = tile.y, pos0 = tile.w, head = blockIdx.y;
+  const int skip = blockIdx.z * 64;                       // tokens of the tile that the other CTA has
+  const int row0 = tile.x + skip, ntok = min(tile.y - skip, 64), pos0 = tile.w + skip, head = blockIdx.y;
+  if (ntok <= 0) return;
   const long long kbase = base[blockIdx.x];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, tq = lane & 3;
@@ -623,7 +625,7 @@ static int launch_latent_prefill(const void* q, long long ld_q, const void* kv, 
     return static_cast<int>(cudaFuncSetAttribute(latent_prefill_kernel<KD, VD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   });
   if (rc != 0) return rc;
-  latent_prefill_kernel<KD, VD><<<dim3(n_tiles, heads), 128, smem, stream>>>(
+  latent_prefill_kernel<KD, VD><<<dim3(n_tiles, heads, 2), 128, smem, stream>>>(
       static_cast<const bf16*>(q), ld_q, static_cast<const bf16*>(kv), ld_kv, static_cast<const bf16*>(lat), ld_lat,
       static_cast<const int4*>(tiles), base, dimp, rotp, rankp, vdimp, scale * kLog2e, window, sink,
       static_cast<const bf16*>(gate), ld_gate, static_cast<bf16*>(out), ld_out);

@@ -10,6 +10,11 @@
 //
 // EXT keeps the softmax weights at fp32 accuracy as the mma.sync kernels do: P = hi + lo, both bf16, two products.
 //
+// LATENT: the same for prompt runs of latent attention over expanded keys and values (latent_attention.cu has the layout): a
+// tile is 128 tokens of one head, a key is 128 numbers of its expanded row and the 64 rotated ones of its cache row, and the
+// keys of a sequence are consecutive rows, so that a box holds 128 of them. With 128 KB of shared memory one CTA fits an SM.
+// Measured on B200: 3000 tokens of 16 heads, window 1024, 166 us with mma.sync, 71 us here.
+//
 // The mma.sync kernel of attention.cu reached 80-130 TFLOP/s (64 rows per CTA, every warp re-reading all of K and V from
 // shared memory); it stays for other head sizes, page sizes that do not divide 128 keys, and unaligned rows.
 #include <string.h>
@@ -24,7 +29,9 @@ constexpr int kFaRows = 128, kFaKeys = 128, kFaDim = 128;
 constexpr int kFaThreads = 192;
 constexpr int kFaHalf = 128 * 128;                  // bytes of 128 rows x 64 bf16
 constexpr int kFaTile = 2 * kFaHalf;                // one of Q, K, V
-constexpr int kFaSmem = 3 * kFaTile + 1024 /*alignment*/ + 128;
+constexpr int kFaRot = 64;                          // rotated part of a latent key
+constexpr int fa_smem(bool lat) { return 3 * kFaTile + (lat ? 2 * kFaHalf : 0) + 1024 /*alignment*/ + 128; }
+enum { FA_PLAIN = 0, FA_EXT = 1, FA_LATENT = 2 };
 constexpr float kFaSlack = 8.f;                     // growth of a row's maximum (base 2) that is left in P
 
 __device__ __forceinline__ float ex2(float x) {
@@ -33,18 +40,29 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
-template <bool EXT>
-__global__ void __launch_bounds__(kFaThreads, 2)
+__device__ __forceinline__ void fa_load(uint32_t dst, const CUtensorMap* m, int x, int y, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y), "r"(bar)
+      : "memory");
+}
+
+// LATENT: tmK is the map of the expanded keys and values, tmV that of the cache rows, base the row of position 0 per tile
+template <int KIND>
+__global__ void __launch_bounds__(kFaThreads, KIND == FA_LATENT ? 1 : 2)
 prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                   const __nv_bfloat16* __restrict__ q, long long ld_q, const int* __restrict__ block_tables, int max_blocks,
                   const int4* __restrict__ tiles, int n_tiles, int n_kv, int block_size, float scale_log2, __nv_bfloat16* __restrict__ out,
-                  long long ld_out, AttnExt ext, int* status) {
+                  long long ld_out, AttnExt ext, const int* __restrict__ base, int rankp, int* status) {
+  constexpr bool EXT = KIND != FA_PLAIN, LAT = KIND == FA_LATENT;
+  constexpr int kQd = kFaDim + (LAT ? kFaRot : 0);                 // numbers of a query / key
+  constexpr int kQk = kFaTile + (LAT ? kFaHalf : 0);               // bytes of Q, K
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 3 * kFaTile);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 2 * kQk + kFaTile);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
   int* abort_word = reinterpret_cast<int*>(tmem_slot + 1);
-  const uint32_t sq = smem_u32(smem), sk = sq + kFaTile, sv = sk + kFaTile;
+  const uint32_t sq = smem_u32(smem), sk = sq + kQk, sv = sk + kQk;
   // K / V landed, K / V consumed, scores ready, weights ready, output accumulated
   const uint32_t k_full = smem_u32(bars), v_full = k_full + 8, k_empty = k_full + 16, v_empty = k_full + 24, s_full = k_full + 32,
                  p_full = k_full + 40, o_full = k_full + 48;
@@ -54,10 +72,11 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
   const int4 tile = tiles[n_tiles - 1 - blockIdx.x / n_kv];
   const int hkv = blockIdx.x % n_kv, gq = ext.gq;
   const int row0 = tile.x, ntok = min(tile.y, kFaRows / gq), pos0 = tile.w;
-  const int* bt = block_tables + static_cast<long long>(tile.z) * max_blocks;
+  const int* bt = LAT ? nullptr : block_tables + static_cast<long long>(tile.z) * max_blocks;
   const int kmax = pos0 + ntok;
-  const int kb0 = EXT ? first_key(pos0, ext.window, ext.chunk) / kFaKeys : 0;      // first key block anyone sees
-  const int nkb = (kmax + kFaKeys - 1) / kFaKeys - kb0;
+  // first key block: from the first key that anyone sees, at the start of a page
+  const int first = EXT ? first_key(pos0, ext.window, ext.chunk) : 0, kbase = LAT ? first : first / kFaKeys * kFaKeys;
+  const int nkb = (kmax - kbase + kFaKeys - 1) / kFaKeys;
 
   if (threadIdx.x == 0) {
     *abort_word = 0;
@@ -74,9 +93,9 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
   const bool live = r >= 0 && tok < ntok;
   if (warp >= 2) {
     // the row's head vector into the two halves of the K-major, 128-byte swizzled Q tile
-    const uint4* src = reinterpret_cast<const uint4*>(q + static_cast<long long>(row0 + (live ? tok : 0)) * ld_q + head * kFaDim);
+    const uint4* src = reinterpret_cast<const uint4*>(q + static_cast<long long>(row0 + (live ? tok : 0)) * ld_q + head * kQd);
 #pragma unroll
-    for (int c = 0; c < 16; ++c) {
+    for (int c = 0; c < kQd / 8; ++c) {
       const uint4 x = live ? __ldg(src + c) : make_uint4(0, 0, 0, 0);
       *reinterpret_cast<uint4*>(smem + (c >> 3) * kFaHalf + r * 128 + (((c & 7) ^ (r & 7)) << 4)) = x;
     }
@@ -88,26 +107,46 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
   const uint32_t t_s = *tmem_slot, t_o = t_s + kFaKeys;      // scores / weights [128 columns], output [128 columns]
 
   if (warp == 0) {
-    // ------------------------------------------------------------ loads: lane = (page of the block, half of the head)
-    const int pages = kFaKeys / block_size;
-    const int page = lane >> 1, half = lane & 1;
-    for (int j = 0; j < nkb; ++j) {
-      const int key0 = (kb0 + j) * kFaKeys;
-      const int there = min(pages, (kmax - key0 + block_size - 1) / block_size);      // pages that hold visible keys
-      const bool mine = page < there;
-      const int slot = mine ? bt[key0 / block_size + page] * block_size : 0;
-      const uint32_t at = half * kFaHalf + page * block_size * 128;
-      bool ok = true;
-#pragma unroll
-      for (int kv = 0; kv < 2; ++kv) {
-        const uint32_t full = kv ? v_full : k_full;
-        ok = ok && mbar_wait(kv ? v_empty : k_empty, (j & 1) ^ 1, abort_word);
-        if (!__all_sync(0xffffffffu, ok)) break;
-        if (lane == 0) mbar_expect_tx(full, there * block_size * 256);
-        __syncwarp();
-        if (mine) tma_load_3d((kv ? sv : sk) + at, kv ? &tmV : &tmK, half * 64, hkv, slot, full);
+    // ------------------------------------------------------------ loads
+    if (LAT) {
+      // one box of 128 keys per 64 numbers
+      if (lane == 0) {
+        const int at = base[n_tiles - 1 - blockIdx.x / n_kv], col = hkv * (2 * kFaDim);
+        for (int j = 0; j < nkb; ++j) {
+          const int row = at + kbase + j * kFaKeys;
+          if (!mbar_wait(k_empty, (j & 1) ^ 1, abort_word)) break;
+          mbar_expect_tx(k_full, kQk);
+          fa_load(sk, &tmK, col, row, k_full);
+          fa_load(sk + kFaHalf, &tmK, col + 64, row, k_full);
+          fa_load(sk + 2 * kFaHalf, &tmV, rankp, row, k_full);
+          if (!mbar_wait(v_empty, (j & 1) ^ 1, abort_word)) break;
+          mbar_expect_tx(v_full, kFaTile);
+          fa_load(sv, &tmK, col + kFaDim, row, v_full);
+          fa_load(sv + kFaHalf, &tmK, col + kFaDim + 64, row, v_full);
+        }
       }
-      if (!__all_sync(0xffffffffu, ok)) break;
+    } else {
+      // lane = (page of the block, half of the head)
+      const int pages = kFaKeys / block_size;
+      const int page = lane >> 1, half = lane & 1;
+      for (int j = 0; j < nkb; ++j) {
+        const int key0 = kbase + j * kFaKeys;
+        const int there = min(pages, (kmax - key0 + block_size - 1) / block_size);      // pages that hold visible keys
+        const bool mine = page < there;
+        const int slot = mine ? bt[key0 / block_size + page] * block_size : 0;
+        const uint32_t at = half * kFaHalf + page * block_size * 128;
+        bool ok = true;
+#pragma unroll
+        for (int kv = 0; kv < 2; ++kv) {
+          const uint32_t full = kv ? v_full : k_full;
+          ok = ok && mbar_wait(kv ? v_empty : k_empty, (j & 1) ^ 1, abort_word);
+          if (!__all_sync(0xffffffffu, ok)) break;
+          if (lane == 0) mbar_expect_tx(full, there * block_size * 256);
+          __syncwarp();
+          if (mine) tma_load_3d((kv ? sv : sk) + at, kv ? &tmV : &tmK, half * 64, hkv, slot, full);
+        }
+        if (!__all_sync(0xffffffffu, ok)) break;
+      }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMAs
@@ -120,7 +159,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         tc_fence_after();
         // the scores overwrite the previous block's weights: the product that read them was issued before
 #pragma unroll
-        for (int k = 0; k < kFaDim / kUmmaK; ++k) {
+        for (int k = 0; k < kQd / kUmmaK; ++k) {
           const uint32_t off = (k >> 2) * kFaHalf + (k & 3) * 32;
           umma_f16(t_s, umma_desc_sw128(sq + off), umma_desc_sw128(sk + off), id_qk, k > 0 ? 1u : 0u);
         }
@@ -151,7 +190,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     float m = -INFINITY, l = 0.f;
     bool ok = true;
     for (int j = 0; j < nkb; ++j) {
-      const int key0 = (kb0 + j) * kFaKeys;
+      const int key0 = kbase + j * kFaKeys;
       if (!mbar_wait(s_full, j & 1, abort_word)) { ok = false; break; }
       if (j > 0 && !mbar_wait(o_full, (j - 1) & 1, abort_word)) { ok = false; break; }      // complete by now
       tc_fence_after();
@@ -232,7 +271,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         if (key0 + key >= kmax) {
 #pragma unroll
           for (int c = 0; c < 16; ++c)
-            *reinterpret_cast<uint4*>(smem + 2 * kFaTile + (c >> 3) * kFaHalf + key * 128 + ((c & 7) << 4)) = make_uint4(0, 0, 0, 0);
+            *reinterpret_cast<uint4*>(smem + 2 * kQk + (c >> 3) * kFaHalf + key * 128 + ((c & 7) << 4)) = make_uint4(0, 0, 0, 0);
         }
         fence_proxy_async_smem();
       }
@@ -295,18 +334,19 @@ static int page_map(CUtensorMap* map, const void* cache, long long slots, int n_
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : -21;
 }
 
-template <bool EXT>
+template <int KIND>
 static int launch_tc(const CUtensorMap& tmK, const CUtensorMap& tmV, const void* q, long long ld_q, const int* bt, int max_blocks,
                      const void* tiles, int n_tiles, int block_size, int n_kv, float scale, void* out, long long ld_out, AttnExt ext,
-                     int* status, cudaStream_t stream) {
+                     const int* base, int rankp, int* status, cudaStream_t stream) {
+  constexpr int smem = fa_smem(KIND == FA_LATENT);
   static PerDeviceOnce configured;
   const int crc = configured.run([] {
-    return static_cast<int>(cudaFuncSetAttribute(prefill_tc_kernel<EXT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFaSmem));
+    return static_cast<int>(cudaFuncSetAttribute(prefill_tc_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   });
   if (crc != 0) return crc;
-  prefill_tc_kernel<EXT><<<n_kv * n_tiles, kFaThreads, kFaSmem, stream>>>(
+  prefill_tc_kernel<KIND><<<n_kv * n_tiles, kFaThreads, smem, stream>>>(
       tmK, tmV, static_cast<const __nv_bfloat16*>(q), ld_q, bt, max_blocks, static_cast<const int4*>(tiles), n_tiles, n_kv,
-      block_size, scale * kLog2e, static_cast<__nv_bfloat16*>(out), ld_out, ext, status);
+      block_size, scale * kLog2e, static_cast<__nv_bfloat16*>(out), ld_out, ext, base, rankp, status);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -330,6 +370,22 @@ extern "C" int dmoe_prefill_attention_tc(const void* q, long long ld_q, const vo
   if (rc != 0) return rc;
   const AttnExt ext = make_ext(scale, window, chunk, softcap, sink, n_q / n_kv, extra);
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  if (plain) return launch_tc<false>(tmK, tmV, q, ld_q, block_tables, max_blocks, tiles, n_tiles, block_size, n_kv, scale, out, ld_out, ext, status, stream);
-  return launch_tc<true>(tmK, tmV, q, ld_q, block_tables, max_blocks, tiles, n_tiles, block_size, n_kv, scale, out, ld_out, ext, status, stream);
+  if (plain) return launch_tc<FA_PLAIN>(tmK, tmV, q, ld_q, block_tables, max_blocks, tiles, n_tiles, block_size, n_kv, scale, out, ld_out, ext, nullptr, 0, status, stream);
+  return launch_tc<FA_EXT>(tmK, tmV, q, ld_q, block_tables, max_blocks, tiles, n_tiles, block_size, n_kv, scale, out, ld_out, ext, nullptr, 0, status, stream);
+}
+
+extern "C" int dmoe_latent_prefill_tc(const void* q, long long ld_q, const void* kv, long long ld_kv, const void* lat, long long ld_lat,
+                                      long long n_keys, const void* tiles, const int* base, int n_tiles, int heads, int rankp,
+                                      float scale, int window, const float* sink, const void* gate, long long ld_gate, void* out,
+                                      long long ld_out, int* status, void* stream) {
+  if (n_tiles == 0) return 0;
+  if (heads < 1 || n_tiles < 0 || n_keys < 1 || static_cast<long long>(n_tiles) * heads > 0x7fffffff || rankp % 8 != 0) return -10;
+  CUtensorMap tmKV, tmL;
+  if (make_map_2d(&tmKV, kv, n_keys, static_cast<long long>(heads) * 2 * kFaDim, ld_kv, kFaKeys) != 0 ||
+      make_map_2d(&tmL, lat, n_keys, rankp + kFaRot, ld_lat, kFaKeys) != 0)
+    return -20;
+  const DmoeAttnExtra extra = {gate, ld_gate, 0.f, 0};
+  const AttnExt ext = make_ext(scale, window, 0, 0.f, sink, 1, &extra);
+  return launch_tc<FA_LATENT>(tmKV, tmL, q, ld_q, nullptr, 0, tiles, n_tiles, kFaKeys, heads, scale, out, ld_out, ext, base, rankp, status,
+                              static_cast<cudaStream_t>(stream));
 }

@@ -81,7 +81,7 @@ class LatentTables:
         lay, T = latent_layout(m), len(positions)
         if not (device.type == "cuda" and lay.tiled(dtype)):
             return cls.decode(m, T, device)
-        tiles, covered = F.build_prefill_tiles(bt_row, positions, 64, lay.min_run())
+        tiles, covered = F.build_prefill_tiles(bt_row, positions, 128, lay.min_run())
         if len(tiles) == 0:
             return cls.decode(m, T, device)
         rows = (~covered).nonzero()[:, 0].int()

@@ -994,6 +994,13 @@ def latent_prefill(q: torch.Tensor, kv: torch.Tensor, lat: torch.Tensor, tiles: 
     _check_sink(sink, lay.heads)
     assert gate is None or (gate.dtype == torch.bfloat16 and gate.stride(1) == 1)
     assert tiles.dtype == base.dtype == torch.int32 and kv.stride(1) == lat.stride(1) == 1
+    if (lay.dimp, lay.rotp, lay.vdimp) == (128, 64, 128) and all(t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (q, kv, lat, out)):
+        _lib.check(_lib.lib().dmoe_latent_prefill_tc(
+            _vp(q), c_ll(q.stride(0)), _vp(kv), c_ll(kv.stride(0)), _vp(lat), c_ll(lat.stride(0)), c_ll(min(kv.shape[0], lat.shape[0])),
+            _vp(tiles), _vp(base), c_int(n_tiles), c_int(lay.heads), c_int(lay.rankp), c_float(scale), c_int(window or 0), _vp(sink),
+            _vp(gate), c_ll(gate.stride(0) if gate is not None else 0), _vp(out), c_ll(out.stride(0)), _vp(scratch(q.device).status),
+            _st()), "dmoe_latent_prefill_tc")
+        return out
     _lib.check(_lib.lib().dmoe_latent_prefill(
         _vp(q), c_ll(q.stride(0)), _vp(kv), c_ll(kv.stride(0)), _vp(lat), c_ll(lat.stride(0)), _vp(tiles), _vp(base),
         c_int(n_tiles), c_int(lay.heads), c_int(lay.dimp), c_int(lay.rotp), c_int(lay.rankp), c_int(lay.vdimp), c_float(scale),

@@ -71,3 +71,55 @@ def test_options(opt):
 def test_loose_rows():
     assert F.loose_rows(torch.tensor([True, False, True])) == 2 and F.loose_rows(torch.zeros(4, dtype=torch.bool)) == 4
     assert F.loose_rows(torch.ones(3, dtype=torch.bool)) == 0
+
+
+@pytest.mark.parametrize("window", [None, 1, 64, 200])
+@pytest.mark.parametrize("extras", [False, True])
+def test_latent(window, extras):
+    """Expanded keys and values of several runs, rows of garbage before, between and behind them."""
+    torch.manual_seed(3)
+    H, rankp, scale = 3, 72, 0.07
+    lay = F.LatentLayout(H, 128, 64, 128, rankp)
+    bf = lambda *s: torch.randn(*s, device="cuda").to(torch.bfloat16)
+    runs = [(0, 0, 300), (1, 50, 129), (2, 400, 16), (3, 0, 128)]      # (row, first position, tokens)
+    rows, pos = [], []
+    for r, p0, n in runs:
+        rows += [r] * n
+        pos += list(range(p0, p0 + n))
+    T = len(rows)
+    tiles, covered = F.build_prefill_tiles(rows, pos, 128, 8)
+    assert bool(covered.all())
+    lo = {r: max(0, p0 - window + 1) if window else 0 for r, p0, n in runs}
+    start, at = {}, 5
+    for r, p0, n in runs:
+        start[r] = at - lo[r]
+        at += p0 + n - lo[r] + 5
+    base = torch.tensor([start[int(t[2])] for t in tiles], dtype=torch.int32, device="cuda")
+    kv, lat = bf(at, H * 256), bf(at, rankp + 64 + 8)[:, :rankp + 64]
+    live = torch.zeros(at, dtype=torch.bool, device="cuda")
+    for r, p0, n in runs:
+        live[start[r] + lo[r]:start[r] + p0 + n] = True
+    kv[~live], lat[~live] = float("nan"), float("nan")
+    q = bf(T, H * 192 + 16)
+    sink = torch.randn(H, device="cuda") if extras else None
+    gate = bf(T, H) if extras else None
+    out = torch.full((T, H * 128), 9.0, dtype=torch.bfloat16, device="cuda")
+    F.latent_prefill(q, kv, lat, tiles.cuda(), base, len(tiles), lay, scale, window, sink, out, gate)
+    assert gemm.check_status() == 0
+    t0 = 0
+    for r, p0, n in runs:
+        keys = torch.arange(lo[r], p0 + n, device="cuda")
+        kr, p = (start[r] + keys).long(), torch.arange(p0, p0 + n, device="cuda")
+        hide = keys[None] > p[:, None]
+        if window:
+            hide |= keys[None] <= p[:, None] - window
+        for h in range(H):
+            k = torch.cat([kv[kr, h * 256:h * 256 + 128], lat[kr, rankp:]], 1).double()
+            s = (q[t0:t0 + n, h * 192:(h + 1) * 192].double() @ k.T * scale).masked_fill(hide, -float("inf"))
+            if extras:
+                s = torch.cat([s, sink[h].double().expand(n, 1)], 1)
+            o = torch.softmax(s, -1)[:, :len(keys)] @ kv[kr, h * 256 + 128:(h + 1) * 256].double()
+            if extras:
+                o = o * torch.sigmoid(gate[t0:t0 + n, h, None].double())
+            _close(out[t0:t0 + n, h * 128:(h + 1) * 128].double(), o, tol=2 ** -8)
+        t0 += n
