@@ -103,6 +103,7 @@ struct GemmArgs {
   // 7 tear-down reached; 8-12 inside the first epilogue chunk: TMEM read done, staged to shared memory, barrier passed,
   // rows stored, second barrier passed; 13-15 in the producer: work walker initialised, L2 policies made, first stage free
   unsigned long long* trace;
+  DenseWalk dense;
 };
 
 // PAIR: the kernel runs as clusters of two CTAs on one tile of 256 weight rows (two m-tiles) x BN tokens with
@@ -271,7 +272,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUt
     // ------------------------------------------------------------ TMA producer
     if (lane == 0) {
       WorkWalker tw;
-      tw.init(s_start, s_cnt, a.G, S, MT, BN, kblocks, a.splitk, a.streamk, work_cta, work_grid);
+      if (a.dense.units > 0) tw.init_dense(a.dense, a.T, BN, kblocks, a.splitk, work_cta);
+      else tw.init(s_start, s_cnt, a.G, S, MT, BN, kblocks, a.splitk, a.streamk, work_cta, work_grid);
       trace_stamp(a, 13);
       if (a.n_wait > 0) asm volatile("fence.proxy.async;" ::: "memory");  // peers' generic stores -> TMA reads
       const uint64_t pol_w = l2_policy_evict_first();
@@ -348,7 +350,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUt
     // ------------------------------------------------------------ MMA issuer (pair mode: the even CTA's only)
     if (lane == 0 && leader) {
       WorkWalker tw;
-      tw.init(s_start, s_cnt, a.G, S, MT, BN, kblocks, a.splitk, a.streamk, work_cta, work_grid);
+      if (a.dense.units > 0) tw.init_dense(a.dense, a.T, BN, kblocks, a.splitk, work_cta);
+      else tw.init(s_start, s_cnt, a.G, S, MT, BN, kblocks, a.splitk, a.streamk, work_cta, work_grid);
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;
@@ -413,7 +416,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUt
     const int row = q * 32 + lane;          // accumulator lane = feature within the tile
     const int et = threadIdx.x - 64;        // 0..127
     WorkWalker tw;
-    tw.init(s_start, s_cnt, a.G, S, MT, BN, kblocks, a.splitk, a.streamk, work_cta, work_grid);
+    if (a.dense.units > 0) tw.init_dense(a.dense, a.T, BN, kblocks, a.splitk, work_cta);
+    else tw.init(s_start, s_cnt, a.G, S, MT, BN, kblocks, a.splitk, a.streamk, work_cta, work_grid);
     constexpr size_t kSlotF4 = static_cast<size_t>(C::kNumA) * (BN / 4) * kBM;   // float4 per workspace slot
     int it = 0;
     bool ok = true;
@@ -1018,6 +1022,10 @@ extern "C" int dmoe_gemm(const DmoeGemm* d, void* stream_) {
     if (grid * 2 * slot_bytes > d->ws_bytes || max_tiles / splitk > n_counters) streamk = 0;
   }
   a.streamk = streamk;
+
+  memset(&a.dense, 0, sizeof(a.dense));
+  if (d->G == 1 && d->offs == nullptr && d->S == 0 && d->seg_cnt == nullptr && !streamk && !pair && mtiles > 0)
+    a.dense = DenseWalk::make(d->T, static_cast<int>(mt), bn, kblocks, splitk, mtiles < num_sms() ? mtiles : num_sms());
 
 #define DMOE_LAUNCH(BN_, EPI_) return launch<BN_, EPI_>(tmW, tmX, a, mtiles, stream)
 #define DMOE_LAUNCH_PAIR(BN_, EPI_) return launch<BN_, EPI_, true>(tmW, tmX, a, mtiles, stream)

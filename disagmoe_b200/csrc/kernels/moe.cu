@@ -209,27 +209,33 @@ dispatch_kernel(const U* __restrict__ y, long long ld_y, const int* __restrict__
                 const float* __restrict__ topk_w, int T, int K, int units, int E, int experts_per_rank, int my_rank,
                 int* __restrict__ ws, int* __restrict__ offs, void* const* __restrict__ x_bases, long long ld_dst,
                 void* const* __restrict__ rec_bases, int dst_capacity, int* __restrict__ status) {
-  __shared__ int s_base[kMaxExperts + 1];
+  __shared__ int s_base[kMaxExperts + 1], s_before[kMaxExperts + 1];
   int* counts = ws;
   int* cursor = ws + E;
   int* ticket = ws + 2 * E;
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {
     int run = 0;
-    for (int e = 0; e < E; ++e) {
-      if (e % experts_per_rank == 0) run = 0;  // every destination rank's buffer starts at row 0
-      s_base[e] = run;
-      run += counts[e];
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      const int e = e0 + threadIdx.x, c = e < E ? counts[e] : 0;
+      int sum = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, sum, o);
+        if (static_cast<int>(threadIdx.x) >= o) sum += x;
+      }
+      if (e < E) s_before[e] = run + sum - c;
+      run += __shfl_sync(0xffffffffu, sum, 31);
     }
+    if (threadIdx.x == 0) s_before[E] = run;
   }
   __syncthreads();
-  if (blockIdx.x == 0 && offs != nullptr) {
+  for (int e = threadIdx.x; e <= E; e += blockDim.x) {
+    // every destination rank's buffer starts at row 0
+    if (e < E) s_base[e] = s_before[e] - s_before[e / experts_per_rank * experts_per_rank];
     // offsets of the local (rank-0-relative) view: global exclusive scan, used by a colocated engine
-    if (threadIdx.x == 0) {
-      int run = 0;
-      for (int e = 0; e < E; ++e) { offs[e] = run; run += counts[e]; }
-      offs[E] = run;
-    }
+    if (blockIdx.x == 0 && offs != nullptr) offs[e] = s_before[e];
   }
+  __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   const int npairs = T * K;
   for (int p = blockIdx.x * nw + warp; p < npairs; p += gridDim.x * nw) {

@@ -17,7 +17,7 @@ constexpr int kRtRows = 16, kRtSlices = 8, kRtThreads = 512;
 
 // NT: groups of 8 experts per pass and warp
 template <int NT>
-__global__ void __launch_bounds__(kRtThreads)
+__global__ void __launch_bounds__(kRtThreads, 2)
 router_kernel(const __nv_bfloat16* __restrict__ h, long long ld_h, int T, int H, const DmoeRouter r, const float* __restrict__ bias,
               float* __restrict__ logits_out) {
   extern __shared__ float s_part[];                        // [slices][rows][E8]

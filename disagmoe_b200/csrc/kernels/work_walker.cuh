@@ -37,6 +37,35 @@ struct WorkUnit {
   int slot;        // workspace slot where this unit parks its partial accumulator (when ncontrib > 1)
 };
 
+// n / d for 0 <= n < 2^22 by a product with the rounded reciprocal r = 1 / d: the quotient is off by one at most
+DMOE_HD int div_by(int n, int d, float r) {
+  int q = static_cast<int>(static_cast<float>(n) * r);
+  const int rest = n - q * d;
+  q += rest >= d ? 1 : rest < 0 ? -1 : 0;
+  return q;
+}
+
+// A launch of one group of T rows without stream-K: what the walker would work out on the device, made by the host. A decode-size
+// launch lasts ten microseconds and every role starts with this arithmetic: four integer divisions took a microsecond each time.
+struct DenseWalk {
+  int units, step, ntn, kb_per;      // units 0: not such a launch
+  float inv_splitk, inv_ntn;
+
+  // the units that WorkWalker::init deals out, see there
+  static DenseWalk make(int T, int MT, int BN, int kblocks, int splitk, int grid) {
+    DenseWalk d;
+    d.ntn = (T + BN - 1) / BN;
+    d.units = MT * d.ntn * splitk;
+    d.kb_per = (kblocks + splitk - 1) / splitk;
+    const int w = (d.units + grid - 1) / grid;
+    d.step = w > 0 ? (d.units + w - 1) / w : 1;
+    d.inv_splitk = 1.f / static_cast<float>(splitk);
+    d.inv_ntn = 1.f / static_cast<float>(d.ntn > 0 ? d.ntn : 1);
+    if (d.units >= (1 << 22)) d.units = 0;
+    return d;
+  }
+};
+
 struct WorkWalker {
   const int* seg_start;  // [S * G] absolute first row of segment (s, g)
   const int* seg_cnt;    // [S * G]
@@ -49,6 +78,14 @@ struct WorkWalker {
   // of the remaining tiles (ids from tile0 on); `total` counts the remainder's iterations
   int it, it_end, total, it_begin;
   int active, cta, grid, waves, wave, tile0;
+
+  DenseWalk dense;
+  int rows;                             // of the one group of a dense launch
+
+  DMOE_HD void init_dense(const DenseWalk& d, int T, int BN_, int kblocks_, int splitk_, int cta_) {
+    dense = d; rows = T; BN = BN_; kblocks = kblocks_; splitk = splitk_; streamk = 0;
+    lin = cta_ < d.step ? cta_ : d.units;      // an idle CTA's first unit is already past the end
+  }
 
   DMOE_HD static int min_i(int a, int b) { return a < b ? a : b; }
 
@@ -69,7 +106,7 @@ struct WorkWalker {
   DMOE_HD void init(const int* s_start, const int* s_cnt, int G_, int S_, int MT_, int BN_, int kblocks_, int splitk_,
                     int streamk_, int cta_, int grid_) {
     seg_start = s_start; seg_cnt = s_cnt; G = G_; S = S_; MT = MT_; BN = BN_; kblocks = kblocks_;
-    splitk = splitk_ < 1 ? 1 : splitk_; streamk = streamk_; cta = cta_;
+    splitk = splitk_ < 1 ? 1 : splitk_; streamk = streamk_; cta = cta_; dense.units = 0;
     kb_per = (kblocks + splitk - 1) / splitk;
     lin = cta_; lin_step = grid_;
     it = it_end = it_begin = total = 0; active = 1; grid = grid_; waves = wave = tile0 = 0;
@@ -140,6 +177,23 @@ struct WorkWalker {
 
   // The next unit of this CTA; false when it has none left.
   DMOE_HD bool next(WorkUnit& u) {
+    if (dense.units > 0) {
+      if (lin >= dense.units) return false;
+      const int tile = div_by(lin, splitk, dense.inv_splitk), ks = lin - tile * splitk;
+      u.tile = tile;
+      u.g = 0;
+      u.m = div_by(tile, dense.ntn, dense.inv_ntn);
+      u.n = tile - u.m * dense.ntn;
+      u.row0 = u.n * BN;
+      u.ntok = min_i(BN, rows - u.row0);
+      u.kb0 = ks * dense.kb_per;
+      u.kb1 = min_i(kblocks, u.kb0 + dense.kb_per);
+      u.ncontrib = splitk;
+      u.c_first = 0;
+      u.slot = lin;
+      lin += dense.step;
+      return true;
+    }
     if (!streamk) {
       const int tile = lin / splitk;
       if (lin < 0 || !locate(tile, u)) return false;

@@ -165,11 +165,12 @@ def want_wide(epi: int, T: int, F: int, K: int, G: int, sms: int) -> bool:
     Grouped (only the mean group size is known): up to 128 tokens the other kernel's tile fits a group and streams the weights
     at HBM speed, beyond that it needs a second tile per group. Measured at 64 experts of 1408 x 2048, SwiGLU: 120 tokens each
     140 -> 154 us, 150: 187 -> 160; 8 experts of 14336 x 4096: 128 tokens 344 -> 393, 160: 456 -> 391. Down-projections with
-    short K loops are bound by the other kernel's transposing epilogue at any size: 64 x (2048 x 1408), 40 tokens each 80 -> 74;
-    with a long loop, 8 x (4096 x 14336), 128 tokens 188 -> 196, 160: 209 -> 193."""
+    short K loops are bound by the other kernel's transposing epilogue at any size: 60 x (2048 x 1408), 8 rows in all 30 -> 20,
+    148 rows 75 -> 64, 600 rows 76 -> 69; with a long loop, 8 x (4096 x 14336), 2 rows 47 -> 77, 128 rows 149 -> 181, 160 rows
+    each 209 -> 193."""
     kblocks, pairs = (K + 63) // 64, max(1, sms // 2)
     if G > 1:
-        return T >= 144 * G or (epi != EPI_SWIGLU and K <= 2048 and T >= 16 * G)
+        return T >= 144 * G or (epi != EPI_SWIGLU and K <= 2048)
     if T < 64 and epi != EPI_SWIGLU:
         return False
     feat = 128 if epi == EPI_SWIGLU else 256
@@ -179,7 +180,7 @@ def want_wide(epi: int, T: int, F: int, K: int, G: int, sms: int) -> bool:
     units = mt * ((T + bn - 1) // bn)
     if epi == EPI_SWIGLU:
         return wide < 10.0 + (units + sms - 1) // sms * kblocks * (32768 + bn * 128) / 1e5
-    return units >= sms or wide < 3.0 + dense_cost(T, F, K, sms)[0]
+    return units >= sms or wide < 1.4 + dense_cost(T, F, K, sms)[0]
 
 
 def _group_hint(T: int, G: int) -> int:
