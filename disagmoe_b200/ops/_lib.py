@@ -142,7 +142,8 @@ def stream_ptr() -> int:
 def upload(t: torch.Tensor, device) -> torch.Tensor:
     """A host table on the device. To a GPU it goes through pinned memory, in stream order: a copy from pageable memory makes the
     host wait for everything that is queued, and a step has several tables."""
-    return t.pin_memory().to(device, non_blocking=True) if torch.device(device).type == "cuda" else t.to(device)
+    kind = getattr(device, "type", None) or torch.device(device).type
+    return t.pin_memory().to(device, non_blocking=True) if kind == "cuda" and torch.cuda.is_available() else t.to(device)
 
 
 LAUNCHES = 0   # entry-point calls that launched kernels of this library (a graph replay adds its captured count)
