@@ -183,6 +183,14 @@ def want_wide(epi: int, T: int, F: int, K: int, G: int, sms: int) -> bool:
     return units >= sms or wide < 1.4 + dense_cost(T, F, K, sms)[0]
 
 
+def _wide_rows(F: int, out: Optional[torch.Tensor], residual: Optional[torch.Tensor], comm: "Optional[GemmComm]") -> bool:
+    """Launches of gemm_wide.cu: on one GPU, rows that move 16 bytes at a time (others keep their split of K)."""
+    rows16 = lambda t: t is None or (t.stride(0) * t.element_size() % 16 == 0 and t.data_ptr() % 16 == 0)
+    alone = comm is None or (comm.seg_cnt is None and not (comm.S or comm.n_wait or comm.n_signal or comm.shard_rows or comm.group_regions)
+                             and comm.rs_bases is None and comm.fanout <= 1)
+    return alone and F % 8 == 0 and rows16(out) and rows16(residual)
+
+
 def _group_hint(T: int, G: int) -> int:
     """Token-tile hint for a grouped GEMM whose group sizes are only known on the device: the mean group size plus
     head-room for routing imbalance, so that most groups fit one token tile (a second tile re-reads the weights)."""
@@ -398,7 +406,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, residual: Optional[torch.Tensor] = 
     sms = num_sms(x.device)
     auto_sk = 0
     if wide is None:
-        wide = not (bn or splitk or pair) and want_wide(EPI_PLAIN, T, F, K, 1, sms)
+        wide = not (bn or splitk or pair) and want_wide(EPI_PLAIN, T, F, K, 1, sms) and _wide_rows(F, out, residual, comm)
     if not bn:
         bn = pick_bn(T, EPI_PLAIN)
         if ((F + 127) // 128) * ((T + bn - 1) // bn) < sms and not pair:

@@ -1,0 +1,40 @@
+"""Which GEMM kernel a call takes: the rule on sizes, rows and multi-GPU hooks (no GPU)."""
+import pytest
+import torch
+
+from disagmoe_b200.ops import gemm
+
+SMS = 148
+
+
+@pytest.mark.parametrize("epi,T,F,K,G,wide", [
+    (gemm.EPI_PLAIN, 4096, 6144, 4096, 1, True), (gemm.EPI_PLAIN, 1, 32000, 4096, 1, False), (gemm.EPI_PLAIN, 63, 32000, 4096, 1, False),
+    (gemm.EPI_PLAIN, 256, 32000, 4096, 1, True), (gemm.EPI_PLAIN, 300, 256, 5632, 1, False), (gemm.EPI_PLAIN, 2048, 2048, 2048, 1, True),
+    (gemm.EPI_SWIGLU, 256, 5632, 2048, 1, True), (gemm.EPI_SWIGLU, 64, 14336, 4096, 1, False), (gemm.EPI_SWIGLU, 100, 1408, 2048, 64, False),
+    (gemm.EPI_SWIGLU, 144 * 8, 14336, 4096, 8, True), (gemm.EPI_COMBINE, 2, 4096, 14336, 8, False), (gemm.EPI_COMBINE, 148, 2048, 1408, 60, True),
+])
+def test_measured_choices(epi, T, F, K, G, wide):
+    assert gemm.want_wide(epi, T, F, K, G, SMS) is wide
+
+
+def test_rows_and_hooks():
+    y = torch.empty(4, 64, dtype=torch.bfloat16)
+    assert gemm._wide_rows(64, y, y, None) and gemm._wide_rows(64, None, None, gemm.GemmComm())
+    assert not gemm._wide_rows(60, None, None, None)                       # rows end inside 16 bytes
+    assert not gemm._wide_rows(56, y[:, 1:57], None, None)                 # unaligned rows
+    assert not gemm._wide_rows(64, y, torch.empty(4, 65, dtype=torch.bfloat16)[:, :64], None)
+    for hooks in (dict(n_wait=1), dict(n_signal=1), dict(shard_rows=4), dict(group_regions=True), dict(fanout=2), dict(rs_bases=y),
+                  dict(seg_cnt=y, S=1)):
+        assert not gemm._wide_rows(64, y, None, gemm.GemmComm(**hooks))
+
+
+def test_dense_walk_division():
+    """div_by of work_walker.cuh in fp32: exact over its range for every divisor a launch can have."""
+    import numpy as np
+    n = np.concatenate([np.arange(0, 1 << 16), np.random.default_rng(0).integers(0, 1 << 22, 1 << 16)]).astype(np.int64)
+    for d in list(range(1, 130)) + [148, 255, 1000, 4097]:
+        r = np.float32(1.0) / np.float32(d)
+        q = (n.astype(np.float32) * r).astype(np.int64)
+        rest = n - q * d
+        q += np.where(rest >= d, 1, np.where(rest < 0, -1, 0))
+        assert np.array_equal(q, n // d)
