@@ -258,12 +258,11 @@ int dmoe_latent_prefill_tc(const void* q, long long ld_q, const void* kv, long l
                            long long n_keys, const void* tiles, const int* base, int n_tiles, int heads, int rankp, float scale,
                            int window, const float* sink, const void* gate, long long ld_gate, void* out, long long ld_out, int* status,
                            void* stream);
-// The same on tcgen05 (prefill_attention.cu) for heads of 128: pages of block_size tokens that divide 128 keys (at least 8),
-// 16-byte aligned rows of q, out and the caches ([n_blocks, block_size, n_kv, 128]). plain != 0: no options, softmax weights in
-// bf16 (dmoe_prefill_attention); else those of dmoe_prefill_attention_ext. status: device word, see DmoeGemm.
+// dmoe_prefill_attention_ext on tcgen05 (prefill_attention.cu) for heads of 128: pages of block_size tokens that divide 128 keys (at
+// least 8), 16-byte aligned rows of q, out and the caches ([n_blocks, block_size, n_kv, 128]). status: device word, see DmoeGemm.
 int dmoe_prefill_attention_tc(const void* q, long long ld_q, const void* kcache, const void* vcache, int n_blocks,
                               const int* block_tables, int max_blocks, const void* tiles, int n_tiles, int block_size, int n_q,
-                              int n_kv, int plain, float scale, int window, int chunk, float softcap, const float* sink, void* out,
+                              int n_kv, float scale, int window, int chunk, float softcap, const float* sink, void* out,
                               long long ld_out, const DmoeAttnExtra* extra, int* status, void* stream);
 int dmoe_prefill_attention(const void* q, long long ld_q, const void* kcache, const void* vcache,
                            const int* block_tables, int max_blocks, const void* tiles, int n_tiles, int block_size,

@@ -8,15 +8,18 @@
 // loads, warp 1 issues the MMAs. A CTA is a serial chain QK -> softmax -> PV, so two of them share an SM (96 KB of shared
 // memory, 256 TMEM columns each) and one's softmax runs under the other's MMAs.
 //
-// EXT keeps the softmax weights at fp32 accuracy as the mma.sync kernels do: P = hi + lo, both bf16, two products.
+// The softmax weights keep fp32 accuracy: P = hi + lo, both bf16, two products.
 //
 // LATENT: the same for prompt runs of latent attention over expanded keys and values (latent_attention.cu has the layout): a
 // tile is 128 tokens of one head, a key is 128 numbers of its expanded row and the 64 rotated ones of its cache row, and the
 // keys of a sequence are consecutive rows, so that a box holds 128 of them. With 128 KB of shared memory one CTA fits an SM.
 // Measured on B200: 3000 tokens of 16 heads, window 1024, 166 us with mma.sync, 71 us here.
 //
-// The mma.sync kernel of attention.cu reached 80-130 TFLOP/s (64 rows per CTA, every warp re-reading all of K and V from
-// shared memory); it stays for other head sizes, page sizes that do not divide 128 keys, and unaligned rows.
+// Measured on B200 against the mma.sync kernel of attention.cu (64 rows per CTA, every warp re-reading all of K and V from shared
+// memory): 4096 tokens of 16 heads, window 1024, soft cap 362 -> 130 us; 3000 tokens, sinks 293 -> 76 us. That kernel stays for
+// other head sizes, page sizes that do not divide 128 keys, unaligned rows, and for attention without options, whose weights are
+// rounded to bf16 relative to a running maximum per 64 keys: another order of blocks rounds them differently, and decoders with
+// few large experts then choose other experts for nearly tied rows.
 #include <string.h>
 
 #include "attn_common.cuh"
@@ -31,7 +34,7 @@ constexpr int kFaHalf = 128 * 128;                  // bytes of 128 rows x 64 bf
 constexpr int kFaTile = 2 * kFaHalf;                // one of Q, K, V
 constexpr int kFaRot = 64;                          // rotated part of a latent key
 constexpr int fa_smem(bool lat) { return 3 * kFaTile + (lat ? 2 * kFaHalf : 0) + 1024 /*alignment*/ + 128; }
-enum { FA_PLAIN = 0, FA_EXT = 1, FA_LATENT = 2 };
+enum { FA_PAGED = 0, FA_LATENT = 1 };
 constexpr float kFaSlack = 8.f;                     // growth of a row's maximum (base 2) that is left in P
 
 __device__ __forceinline__ float ex2(float x) {
@@ -54,7 +57,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                   const __nv_bfloat16* __restrict__ q, long long ld_q, const int* __restrict__ block_tables, int max_blocks,
                   const int4* __restrict__ tiles, int n_tiles, int n_kv, int block_size, float scale_log2, __nv_bfloat16* __restrict__ out,
                   long long ld_out, AttnExt ext, const int* __restrict__ base, int rankp, int* status) {
-  constexpr bool EXT = KIND != FA_PLAIN, LAT = KIND == FA_LATENT;
+  constexpr bool LAT = KIND == FA_LATENT;
   constexpr int kQd = kFaDim + (LAT ? kFaRot : 0);                 // numbers of a query / key
   constexpr int kQk = kFaTile + (LAT ? kFaHalf : 0);               // bytes of Q, K
   extern __shared__ uint8_t smem_raw[];
@@ -75,7 +78,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
   const int* bt = LAT ? nullptr : block_tables + static_cast<long long>(tile.z) * max_blocks;
   const int kmax = pos0 + ntok;
   // first key block: from the first key that anyone sees, at the start of a page
-  const int first = EXT ? first_key(pos0, ext.window, ext.chunk) : 0, kbase = LAT ? first : first / kFaKeys * kFaKeys;
+  const int first = first_key(pos0, ext.window, ext.chunk), kbase = LAT ? first : first / kFaKeys * kFaKeys;
   const int nkb = (kmax - kbase + kFaKeys - 1) / kFaKeys;
 
   if (threadIdx.x == 0) {
@@ -169,7 +172,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         if (!mbar_wait(v_full, ph, abort_word)) break;
         tc_fence_after();
 #pragma unroll
-        for (int part = 0; part < (EXT ? 2 : 1); ++part)
+        for (int part = 0; part < 2; ++part)
 #pragma unroll
           for (int k = 0; k < kFaKeys / kUmmaK; ++k)
             umma_f16_ta(t_o, t_s + part * (kFaKeys / 2) + k * (kUmmaK / 2), umma_desc_sw128_mn(sv + k * kUmmaK * 128, kFaHalf),
@@ -182,10 +185,10 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     // ------------------------------------------------------------ softmax: one query row per thread
     const uint32_t lanes = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const int qpos = pos0 + tok;
-    const float temp = EXT ? query_temperature(ext, qpos) : 1.f;
-    const int lo = EXT ? first_key(qpos, ext.window, ext.chunk) : 0;
+    const float temp = query_temperature(ext, qpos);
+    const int lo = first_key(qpos, ext.window, ext.chunk);
     // blocks that need no mask: all keys visible to the first and the last token of the tile
-    const int lo_last = EXT ? first_key(kmax - 1, ext.window, ext.chunk) : 0;
+    const int lo_last = first_key(kmax - 1, ext.window, ext.chunk);
     const float scale = scale_log2 * temp;
     float m = -INFINITY, l = 0.f;
     bool ok = true;
@@ -198,13 +201,13 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
 #pragma unroll
       for (int i = 0; i < 4; ++i) tmem_ld32(t_s + lanes + i * 32, s[i]);
       tmem_ld_wait();
-      const bool masked = key0 + kFaKeys - 1 > pos0 || (EXT && key0 < lo_last);
+      const bool masked = key0 + kFaKeys - 1 > pos0 || key0 < lo_last;
       float mx = -INFINITY;
-      if (EXT && ext.cap_log2 > 0.f) {
+      if (ext.cap_log2 > 0.f) {
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-          for (int e = 0; e < 32; ++e) s[i][e] = __float_as_uint(attn_score<EXT>(__uint_as_float(s[i][e]) * temp, scale_log2, ext));
+          for (int e = 0; e < 32; ++e) s[i][e] = __float_as_uint(attn_score<true>(__uint_as_float(s[i][e]) * temp, scale_log2, ext));
       } else {
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -217,7 +220,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
 #pragma unroll
           for (int e = 0; e < 32; ++e) {
             const int key = key0 + i * 32 + e;
-            if (key > qpos || (EXT && key < lo)) s[i][e] = __float_as_uint(-INFINITY);
+            if (key > qpos || key < lo) s[i][e] = __float_as_uint(-INFINITY);
           }
       }
 #pragma unroll
@@ -257,11 +260,10 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         for (int e = 0; e < 16; ++e) {
           const float p0 = ex2(__uint_as_float(s[i][2 * e]) - sub), p1 = ex2(__uint_as_float(s[i][2 * e + 1]) - sub);
           sum[e & 3] += p0 + p1;
-          if (EXT) split2(p0, p1, hi[e], rest[e]);
-          else hi[e] = pack_bf16(p0, p1);
+          split2(p0, p1, hi[e], rest[e]);
         }
         tmem_st16(t_s + lanes + i * 16, hi);
-        if (EXT) tmem_st16(t_s + lanes + kFaKeys / 2 + i * 16, rest);
+        tmem_st16(t_s + lanes + kFaKeys / 2 + i * 16, rest);
       }
       l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
       if (key0 + kFaKeys > kmax) {
@@ -284,8 +286,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     if (ok && mbar_wait(o_full, (nkb - 1) & 1, abort_word)) {
       tc_fence_after();
       float inv = l > 0.f ? 1.f / l : 0.f;
-      if (EXT && ext.sink != nullptr) inv = sink_inverse(m, l, ext.sink[head]);
-      if (EXT && ext.gate != nullptr && live) inv *= head_gate<__nv_bfloat16>(ext, row0 + tok, head);
+      if (ext.sink != nullptr) inv = sink_inverse(m, l, ext.sink[head]);
+      if (ext.gate != nullptr && live) inv *= head_gate<__nv_bfloat16>(ext, row0 + tok, head);
       __nv_bfloat16* y = out + static_cast<long long>(row0 + tok) * ld_out + head * kFaDim;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -356,7 +358,7 @@ using namespace dmoe;
 
 extern "C" int dmoe_prefill_attention_tc(const void* q, long long ld_q, const void* kcache, const void* vcache, int n_blocks,
                                          const int* block_tables, int max_blocks, const void* tiles, int n_tiles, int block_size,
-                                         int n_q, int n_kv, int plain, float scale, int window, int chunk, float softcap,
+                                         int n_q, int n_kv, float scale, int window, int chunk, float softcap,
                                          const float* sink, void* out, long long ld_out, const DmoeAttnExtra* extra, int* status,
                                          void* stream_) {
   if (n_tiles == 0) return 0;
@@ -370,8 +372,7 @@ extern "C" int dmoe_prefill_attention_tc(const void* q, long long ld_q, const vo
   if (rc != 0) return rc;
   const AttnExt ext = make_ext(scale, window, chunk, softcap, sink, n_q / n_kv, extra);
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  if (plain) return launch_tc<FA_PLAIN>(tmK, tmV, q, ld_q, block_tables, max_blocks, tiles, n_tiles, block_size, n_kv, scale, out, ld_out, ext, nullptr, 0, status, stream);
-  return launch_tc<FA_EXT>(tmK, tmV, q, ld_q, block_tables, max_blocks, tiles, n_tiles, block_size, n_kv, scale, out, ld_out, ext, nullptr, 0, status, stream);
+  return launch_tc<FA_PAGED>(tmK, tmV, q, ld_q, block_tables, max_blocks, tiles, n_tiles, block_size, n_kv, scale, out, ld_out, ext, nullptr, 0, status, stream);
 }
 
 extern "C" int dmoe_latent_prefill_tc(const void* q, long long ld_q, const void* kv, long long ld_kv, const void* lat, long long ld_lat,

@@ -459,7 +459,8 @@ def loose_rows(covered: torch.Tensor) -> int:
 
 
 def _prefill_on_tcgen05(q, kcache, vcache, out, hd: int, vd: int) -> bool:
-    """Shapes of csrc/kernels/prefill_attention.cu: heads of 128, pages that divide a block of 128 keys, 16-byte rows."""
+    """Shapes of csrc/kernels/prefill_attention.cu (attention with options): heads of 128, pages that divide a block of 128 keys,
+    16-byte rows."""
     bs = kcache.shape[1]
     return hd == vd == 128 and bs >= 8 and 128 % bs == 0 and q.stride(0) % 8 == 0 and out.stride(0) % 8 == 0 and \
         kcache.is_contiguous() and vcache.is_contiguous() and all(t.data_ptr() % 16 == 0 for t in (q, out, kcache, vcache))
@@ -517,12 +518,12 @@ def prefill_attention(q: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tenso
     options = window or chunk or softcap or fp32_weights or sink is not None or q_temp is not None or gate is not None or \
         hd != vd or n_q // n_kv not in (1, 2, 4, 8)
     x = _attn_extra(q_temp, gate, q.dtype)
-    if _prefill_on_tcgen05(q, kcache, vcache, out, hd, vd):
+    if options and _prefill_on_tcgen05(q, kcache, vcache, out, hd, vd):
         from .gemm import scratch
         _lib.check(_lib.lib().dmoe_prefill_attention_tc(
             _vp(q), c_ll(q.stride(0)), _vp(kcache), _vp(vcache), c_int(kcache.shape[0]), _vp(block_tables),
             c_int(block_tables.stride(0)), _vp(tiles), c_int(n_tiles), c_int(kcache.shape[1]), c_int(n_q), c_int(n_kv),
-            c_int(int(not options)), c_float(scale), c_int(window or 0), c_int(chunk or 0), c_float(softcap or 0.0), _vp(sink),
+            c_float(scale), c_int(window or 0), c_int(chunk or 0), c_float(softcap or 0.0), _vp(sink),
             _vp(out), c_ll(out.stride(0)), ctypes.byref(x) if x else None, _vp(scratch(q.device).status), _st()),
             "dmoe_prefill_attention_tc")
         return out

@@ -54,9 +54,9 @@ def _close(y, ref, tol):
 
 @pytest.mark.parametrize("n_q,n_kv", [(2, 2), (8, 2), (8, 1), (6, 2), (64, 1)])
 @pytest.mark.parametrize("bs", [8, 16, 64, 128])
-def test_plain(n_q, n_kv, bs):
-    # softmax weights and outputs are rounded to bf16 once each: two roundings of 2^-9, some on sums of several terms
-    _close(*_run(n_q, n_kv, bs, poison=True, fp32_weights=n_q // n_kv in (3, 64)), tol=2 ** -6)
+def test_groups_and_pages(n_q, n_kv, bs):
+    # fp32 softmax weights: one rounding of the output, 2^-9 relative, and twice that for the bf16 reference it is compared in
+    _close(*_run(n_q, n_kv, bs, poison=True, fp32_weights=True), tol=2 ** -7)
 
 
 @pytest.mark.parametrize("opt", [
