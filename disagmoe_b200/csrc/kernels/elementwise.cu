@@ -194,6 +194,7 @@ __global__ void __launch_bounds__(kArgThreads)
 argmax_kernel(const T* __restrict__ logits, long long ld, int V, int* __restrict__ ids, int parts) {
   __shared__ float sv[32], part_v[kArgParts];
   __shared__ int si[32], part_i[kArgParts];
+  if (parts > 1) cluster_arrive();
   const long long t = blockIdx.x / parts;
   const int part = blockIdx.x % parts;
   const T* row = logits + t * ld;
@@ -222,6 +223,7 @@ argmax_kernel(const T* __restrict__ logits, long long ld, int V, int* __restrict
     if (threadIdx.x == 0) ids[t] = bi;
     return;
   }
+  cluster_wait();      // the first CTA's shared memory may be written once that CTA is known to run; the scan hides the wait
   if (threadIdx.x == 0) {
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(mapa_rank(smem_u32(&part_v[part]), 0)), "f"(best) : "memory");
     asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(mapa_rank(smem_u32(&part_i[part]), 0)), "r"(bi) : "memory");

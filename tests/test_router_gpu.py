@@ -77,6 +77,17 @@ def test_argmax(T, V, dtype, off):
     assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("T", [1, 40, 295])
+@pytest.mark.parametrize("V,dtype", [(8192, torch.float32), (8203, torch.bfloat16), (32000, torch.float32)])
+def test_argmax_over_the_runs_of_a_row(T, V, dtype):
+    """Rows that several CTAs of a cluster share, from one to just below two per SM: the maximum stands in every run in turn."""
+    x = torch.zeros(T, V, dtype=dtype, device="cuda")
+    at = (torch.arange(T, device="cuda") * 1031 + 17) % V
+    x[torch.arange(T, device="cuda"), at] = 1.0
+    for _ in range(20):
+        assert torch.equal(F.argmax(x).long(), at)
+
+
 @pytest.mark.parametrize("T,H", [(1, 8), (37, 2048), (300, 264)])
 def test_gated_add(T, H):
     torch.manual_seed(H)
