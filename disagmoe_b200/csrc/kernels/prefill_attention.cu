@@ -159,8 +159,10 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
       for (int j = 0; j < nkb; ++j) {
         const uint32_t ph = j & 1;
         if (!mbar_wait(k_full, ph, abort_word)) break;
+        // the scores overwrite the previous block's weights, which the product before reads from tensor memory. The order of two
+        // products is only given for the same accumulator, so that one has to be complete
+        if (j > 0 && !mbar_wait(o_full, ph ^ 1, abort_word)) break;
         tc_fence_after();
-        // the scores overwrite the previous block's weights: the product that read them was issued before
 #pragma unroll
         for (int k = 0; k < kQd / kUmmaK; ++k) {
           const uint32_t off = (k >> 2) * kFaHalf + (k & 3) * 32;

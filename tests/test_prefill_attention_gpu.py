@@ -13,10 +13,10 @@ HD = 128
 SEGS = [(0, 0, 300), (1, 0, 128), (2, 137, 70), (3, 0, 8), (4, 31, 129), (5, 255, 9), (6, 127, 257)]
 
 
-def _run(n_q, n_kv, bs, poison=False, seed=0, **opt):
+def _run(n_q, n_kv, bs, poison=False, seed=0, segs=SEGS, span=512, **opt):
     torch.manual_seed(seed)
-    maxb, rows, pos = 512 // bs, [], []
-    for r, p0, n in SEGS:
+    maxb, rows, pos = span // bs, [], []
+    for r, p0, n in segs:
         rows += [r] * n
         pos += list(range(p0, p0 + n))
     T, nb = len(rows), 7 * maxb
@@ -33,7 +33,7 @@ def _run(n_q, n_kv, bs, poison=False, seed=0, **opt):
                                     opt.get("sink"), opt.get("chunk"), opt.get("q_temp"), opt.get("gate"))
     if poison:
         # what a page holds behind the last cached token must not matter
-        for r, p0, n in SEGS:
+        for r, p0, n in segs:
             for p in range(p0 + n, maxb * bs):
                 for c in (kc, vc):
                     c[bt[r, p // bs].long(), p % bs] = float("nan")
@@ -66,6 +66,13 @@ def test_groups_and_pages(n_q, n_kv, bs):
 def test_options(opt):
     # fp32 softmax weights: one rounding of the output, 2^-9 relative, and twice that for the bf16 reference it is compared in
     _close(*_run(8, 2, 16, poison=True, **opt), tol=2 ** -7)
+
+
+def test_many_key_blocks():
+    """Two CTAs per SM, each with up to 32 key blocks: scores of a block take the place of the weights before."""
+    # fp32 softmax weights: one rounding of the output, 2^-9 relative, and twice that for the bf16 reference it is compared in
+    segs = [(0, 3000, 1096), (1, 2047, 300), (2, 0, 2049), (3, 4088, 8)]
+    _close(*_run(8, 2, 16, segs=segs, span=4096, scale=0.5, fp32_weights=True), tol=2 ** -7)
 
 
 def test_loose_rows():
