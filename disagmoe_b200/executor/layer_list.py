@@ -173,6 +173,8 @@ class LayerListExecutor(StepExecutor):
         if T not in self.decode_tables:
             self.decode_tables[T] = ({k: LatentTables.decode(m, T, self.device) for k, m in self.latent_specs.items()},
                                      self._block_offs(T))
+            if self.device.type == "cuda":
+                torch.cuda.current_stream(self.device).synchronize()      # the uploads: other streams read the tables as well
         return self.decode_tables[T]
 
     def _forward(self, buf: LayerListBuffers, T: int, max_ctx: int, want_logits: bool):
