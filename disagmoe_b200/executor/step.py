@@ -100,11 +100,15 @@ class StepExecutor:
 
     def prefill(self, ids, positions, slots, ctx_len, bt_row, want_logits=False, out_rows: Optional[List[int]] = None):
         """Eager pass over prompt tokens (any number of sequences packed together, decode rows among them). Host tensors
-        in, device out. ``out_rows``: the rows to sample (and whose logits to return), in this order; None = all."""
+        in, device out; the inputs may be refilled when the call is back. ``out_rows``: the rows to sample (and whose logits to
+        return), in this order; None = all."""
         T = ids.shape[0]
         assert T <= self.prefill_buf.cap, f"{T} prefill tokens exceed the buffer ({self.prefill_buf.cap})"
         buf = self.prefill_buf
         self._fill(buf, T, ids, positions, slots, ctx_len, bt_row)
+        copied = torch.cuda.Event() if self.device.type == "cuda" else None
+        if copied is not None:
+            copied.record(torch.cuda.current_stream(self.device))
         self._begin_prefill(buf, T, positions, ctx_len, bt_row)
         if out_rows is not None:
             buf.out_rows = _lib.upload(torch.tensor(out_rows, dtype=torch.int32), self.device)
@@ -113,6 +117,8 @@ class StepExecutor:
         finally:
             buf.out_rows = None
             self._end_prefill(buf)
+            if copied is not None:
+                copied.synchronize()      # pinned inputs are read by the copies; the launches are queued by now
 
     def capture(self, sizes: Optional[List[int]] = None) -> None:
         """Warm-up (compiles nothing, but sizes scratch buffers and sets kernel attributes) and graph capture."""
