@@ -147,7 +147,7 @@ def want_streamk(epi: int, F: int, G: int, T: int, bn: int, sms: int) -> bool:
     eight experts: 64 tiles for 148 SMs, 77 us with whole tiles, 47 us with a stream-K tail.)"""
     if not STREAM_K or epi == EPI_SWIGLU:
         return False
-    active = G * (1.0 - (1.0 - 1.0 / G) ** T)       # groups that T evenly routed rows are expected to reach
+    active = G * (1.0 - (1.0 - 1.0 / G) ** max(T, 1))       # groups that T evenly routed rows are expected to reach
     tiles = ((F + 127) // 128) * max(round(active), (T + bn - 1) // bn)
     waves = (tiles + sms - 1) // sms
     return tiles / (waves * sms) < 0.85

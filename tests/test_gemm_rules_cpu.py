@@ -17,6 +17,12 @@ def test_measured_choices(epi, T, F, K, G, wide):
     assert gemm.want_wide(epi, T, F, K, G, SMS) is wide
 
 
+@pytest.mark.parametrize("G", [1, 2, 8, 64])
+def test_stream_k_of_no_expected_rows(G):
+    """An expert rank whose share of the arriving rows rounds to none still asks for a rule: 32 tiles leave most SMs idle."""
+    assert gemm.want_streamk(gemm.EPI_COMBINE, 4096, G, 0, 32, SMS)
+
+
 def test_rows_and_hooks():
     y = torch.empty(4, 64, dtype=torch.bfloat16)
     assert gemm._wide_rows(64, y, y, None) and gemm._wide_rows(64, None, None, gemm.GemmComm())
