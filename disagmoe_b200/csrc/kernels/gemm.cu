@@ -989,7 +989,7 @@ extern "C" int dmoe_gemm(const DmoeGemm* d, void* stream_) {
 
   // tokens as the M operand: single-GPU launches with 16-byte output rows; without them the call keeps the kernel of this file
   const bool alone = d->S == 0 && !d->group_regions && d->n_wait == 0 && d->n_signal == 0 && d->shard_rows == 0 &&
-                     d->rs_bases == nullptr && d->fanout <= 1 && splitk == 1 && !pair && d->trace == nullptr;
+                     d->rs_bases == nullptr && d->fanout <= 1 && d->clear_n == 0 && splitk == 1 && !pair && d->trace == nullptr;
   if (d->wide != 0 && alone && a.epi_vec && d->seg_cnt == nullptr && (!d->w_blocked || (d->K % kBK == 0 && d->F % kBM == 0 &&
       static_cast<long long>(d->G) * a.w_rows * (d->K / kBK) < (1ll << 31))))
     return gemm_wide(d, stream);

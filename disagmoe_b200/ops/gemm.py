@@ -187,7 +187,7 @@ def _wide_rows(F: int, out: Optional[torch.Tensor], residual: Optional[torch.Ten
     """Launches of gemm_wide.cu: on one GPU, rows that move 16 bytes at a time (others keep their split of K)."""
     rows16 = lambda t: t is None or (t.stride(0) * t.element_size() % 16 == 0 and t.data_ptr() % 16 == 0)
     alone = comm is None or (comm.seg_cnt is None and not (comm.S or comm.n_wait or comm.n_signal or comm.shard_rows or comm.group_regions)
-                             and comm.rs_bases is None and comm.fanout <= 1)
+                             and comm.rs_bases is None and comm.fanout <= 1 and comm.clear is None)
     return alone and F % 8 == 0 and rows16(out) and rows16(residual)
 
 

@@ -30,7 +30,7 @@ def test_rows_and_hooks():
     assert not gemm._wide_rows(56, y[:, 1:57], None, None)                 # unaligned rows
     assert not gemm._wide_rows(64, y, torch.empty(4, 65, dtype=torch.bfloat16)[:, :64], None)
     for hooks in (dict(n_wait=1), dict(n_signal=1), dict(shard_rows=4), dict(group_regions=True), dict(fanout=2), dict(rs_bases=y),
-                  dict(seg_cnt=y, S=1)):
+                  dict(seg_cnt=y, S=1), dict(clear=torch.ones(4, dtype=torch.int32), done_ticket=torch.zeros(1, dtype=torch.int32))):
         assert not gemm._wide_rows(64, y, None, gemm.GemmComm(**hooks))
 
 

@@ -37,6 +37,15 @@ def test_linear_variants(T, O, K):
     _close(out, ref + r.float())
 
 
+@pytest.mark.parametrize("wide", [None, True])
+def test_counters_to_clear(wide):
+    """Only the other kernel zeroes the counters that a launch is given: it keeps such a launch, whatever is asked for."""
+    x, w = _rand(1024, 512), _rand(2048, 512, scale=512 ** -0.5)
+    cnt, ticket = torch.full((37,), 5, dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    _close(gemm.linear(x, w, wide=wide, comm=gemm.GemmComm(done_ticket=ticket, clear=cnt)), x.float() @ w.float().T)
+    assert int(cnt.abs().sum()) == 0 and int(ticket) == 0
+
+
 @pytest.mark.parametrize("counts,I,K,blocked", [
     ([1, 0, 255, 256], 128, 64, True), ([257, 128, 0, 129], 264, 200, False), ([0, 0, 0], 128, 64, True),
     ([600, 3, 40, 512, 0, 90] * 11, 256, 192, True),
