@@ -3,10 +3,18 @@
 // One CTA has 16 rows; eighths of the width x halves of the experts go to its 16 warps, so that a router weight is read once
 // per 16 rows (straight from L2 as 16-byte pieces in the order the mma fragments want: the order of k inside a step does not
 // matter as long as both operands share it) and no row passes through shared memory. At decode batches a handful of CTAs runs
-// and the time is the latency of the weight reads: four steps of the width are in flight per warp. Partial logits are added in
-// a fixed order, then every warp chooses for one row. The kernels that norm the rows (moe.cu: route_kernel, layer_ops.cu: sum_norm_kernel) have a router of their own on
-// the CUDA cores, bound by its fp32 multiply-adds and shared-memory reads; ops/functional.py: separate_router says where each
-// is used. Products of bf16 values are exact and sums are fp32 in both.
+// and the time is the latency of the weight reads: the loop is unrolled by four steps of the width, and one CTA per SM leaves
+// 128 registers per thread for their loads (37 rows x 60 experts of 2048: 16.4 us with two CTAs per SM, 14.3 with one).
+//
+// The logits choose experts, so they are as exact as fp32 multiply-adds. The tensor core truncates what it adds to an
+// accumulator; chained over the width that made the errors three to eight times as large (4096 wide: 4.8e-7 of the logits'
+// root mean square, against 9.4e-8 for the CUDA cores). Every mma therefore starts from zero, and its 16 products are added in
+// rounded fp32: first over four steps of the width, then over those; the eight slices are added in fp64. Errors against fp64,
+// root mean square, CUDA cores -> here: 4096 wide 9.4e-8 -> 7.1e-8, 2048 wide 7.9e-8 -> 6.5e-8, 256 wide 5.6e-8 -> 4.4e-8.
+//
+// Afterwards every warp chooses for one row. The kernels that norm the rows (moe.cu: route_kernel, layer_ops.cu: sum_norm_kernel)
+// have a router of their own on the CUDA cores, bound by its fp32 multiply-adds and shared-memory reads; ops/functional.py:
+// separate_router says where each is used.
 #include "dmoe_kernels.h"
 #include "mma_sync.cuh"
 #include "router_choose.cuh"
@@ -17,7 +25,7 @@ constexpr int kRtRows = 16, kRtSlices = 8, kRtThreads = 512;
 
 // NT: groups of 8 experts per pass and warp
 template <int NT>
-__global__ void __launch_bounds__(kRtThreads, 2)
+__global__ void __launch_bounds__(kRtThreads, 1)
 router_kernel(const __nv_bfloat16* __restrict__ h, long long ld_h, int T, int H, const DmoeRouter r, const float* __restrict__ bias,
               float* __restrict__ logits_out) {
   extern __shared__ float s_part[];                        // [slices][rows][E8]
@@ -31,7 +39,7 @@ router_kernel(const __nv_bfloat16* __restrict__ h, long long ld_h, int T, int H,
   const __nv_bfloat16* x0 = h + (v0 ? row0 + g : 0) * ld_h + k0;
   const __nv_bfloat16* x1 = h + (v1 ? row0 + g + 8 : 0) * ld_h + k0;
   for (int e0 = warp / kRtSlices * 8 * NT; e0 < E; e0 += 16 * NT) {
-    float acc[NT][4] = {};
+    float acc[NT][4] = {}, run[NT][4] = {};
     const __nv_bfloat16* w[NT];
 #pragma unroll
     for (int n = 0; n < NT; ++n) w[n] = W + static_cast<long long>(min(e0 + n * 8 + g, E - 1)) * H + k0;
@@ -45,14 +53,23 @@ router_kernel(const __nv_bfloat16* __restrict__ h, long long ld_h, int T, int H,
       const uint32_t lo[4] = {a0.x, a1.x, a0.y, a1.y}, hi[4] = {a0.z, a1.z, a0.w, a1.w};
 #pragma unroll
       for (int n = 0; n < NT; ++n) {
-        mma_bf16_16816(acc[n], lo, b[n].x, b[n].y);
-        mma_bf16_16816(acc[n], hi, b[n].z, b[n].w);
+        float t[4] = {}, u[4] = {};
+        mma_bf16_16816(t, lo, b[n].x, b[n].y);
+        mma_bf16_16816(u, hi, b[n].z, b[n].w);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) run[n][i] += t[i] + u[i];
+        if (k % 128 == 96) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) { acc[n][i] += run[n][i]; run[n][i] = 0.f; }
+        }
       }
     }
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
       const int e = e0 + n * 8 + 2 * tq;
       if (e >= E8) continue;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[n][i] += run[n][i];
       float* p = s_part + (slice * kRtRows + g) * E8 + e;
       *reinterpret_cast<float2*>(p) = make_float2(acc[n][0], acc[n][1]);
       *reinterpret_cast<float2*>(p + 8 * E8) = make_float2(acc[n][2], acc[n][3]);
@@ -63,9 +80,10 @@ router_kernel(const __nv_bfloat16* __restrict__ h, long long ld_h, int T, int H,
   const long long t = row0 + j;
   if (t >= T) return;
   for (int e = lane; e < E; e += 32) {
-    float z = 0.f;
+    double sum = 0.;
 #pragma unroll
-    for (int p = 0; p < kRtSlices; ++p) z += s_part[(p * kRtRows + j) * E8 + e];
+    for (int p = 0; p < kRtSlices; ++p) sum += s_part[(p * kRtRows + j) * E8 + e];
+    float z = static_cast<float>(sum);
     if (bias != nullptr) z += bias[e];
     if (logits_out != nullptr) logits_out[t * E + e] = z;
     s_lg[j][e] = z;

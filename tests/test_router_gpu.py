@@ -30,6 +30,25 @@ def test_softmax_router(T, H, E, K):
     assert torch.equal(counts.long(), torch.bincount(ids.reshape(-1).long(), minlength=E))
 
 
+@pytest.mark.parametrize("kind", ["normal", "outliers", "offset"])
+@pytest.mark.parametrize("T,H,E", [(1111, 2048, 64), (37, 2048, 60), (2048, 4096, 8), (300, 256, 33), (300, 8192, 17), (300, 1024, 256)])
+def test_logits_no_less_exact_than_on_the_cuda_cores(T, H, E, kind, monkeypatch):
+    """Errors against fp64 of the same rows on the tensor cores and in the fused kernel's fp32 multiply-adds."""
+    torch.manual_seed(H + E)
+    x, gw = torch.randn(T, H, device="cuda"), torch.randn(E, H, device="cuda") * H ** -0.5
+    if kind == "outliers":
+        x[:, ::97] *= 30
+    if kind == "offset":
+        x, gw = x + 3, gw + 0.05
+    x, gw, nw, err = x.bfloat16(), gw.bfloat16(), _bf(H).abs() + 0.5, []
+    for separate in (True, False):
+        monkeypatch.setattr(F, "separate_router", lambda *a: separate)
+        y, _, _, logits = F.route(x, nw, 1e-5, gw, 2, want_logits=True)
+        err.append((logits.double() - y.double() @ gw.double().T).pow(2).mean().sqrt())
+    # the errors are sums of many rounding errors: their mean square over some thousand logits moves by a few percent
+    assert float(err[0]) <= 1.05 * float(err[1])
+
+
 @pytest.mark.parametrize("T", [3, 161, 700])
 @pytest.mark.parametrize("E,top,groups,keep,sigmoid", [(64, 6, 8, 3, True), (24, 2, 1, 1, True), (64, 6, 1, 1, False)])
 def test_router_behind_sum_norm(T, E, top, groups, keep, sigmoid, monkeypatch):
