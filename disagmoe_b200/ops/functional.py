@@ -266,10 +266,13 @@ def gather_ptrs(ptrs: torch.Tensor, n: int, H: int, out: torch.Tensor) -> torch.
 
 def separate_router(T: int, H: int, E: int, h: torch.Tensor, weight: torch.Tensor) -> bool:
     """Should the router run as a kernel of its own on the tensor cores (csrc/kernels/router.cu) behind the norm, instead of inside
-    it on the CUDA cores? Measured on B200 (norm + router in one kernel -> in two): 4096 rows of 4096, 8 experts 98 -> 41 us; 1111 rows of
-    2048, 64 experts 82 -> 22; 3000 rows of 2048, 64 experts, after a sum 108 -> 45; 37 rows of 2048, 60 experts 22 -> 16. One row and 8
-    experts take 7.5 us in one kernel, which a second launch does not beat."""
-    return H % 256 == 0 and E <= 256 and (E > 16 or T >= 128) and h.stride(0) % 8 == 0 and h.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0
+    it on the CUDA cores? The fused kernel pays for the router per row, the second launch costs about 3 us. Measured on B200 with cold
+    caches (norm + router, one kernel -> two): a router of 65,536 numbers and more wins at any number of rows (1 .. 148 rows, 64 experts of
+    2048 27 -> 20 us, 32 of 2048 17.0 -> 15.3, 64 of 1024 18.2 -> 15.3; but 24 of 1024 12.2 -> 13.3, 8 of 4096 14.3 -> 17.0); below it
+    the rows decide, at about 10 million products (8 of 4096: 256 rows 15.1 -> 17.4, 320 rows 17.1 -> 17.4, 448 rows 20.0 -> 17.1, 1024
+    rows 32.7 -> 21.2; 8 of 2048: 448 rows 14.0 -> 14.3, 640 rows 20.5 -> 15.4). After a sum the lines lie at the same sizes."""
+    return H % 256 == 0 and E <= 256 and (E * H >= 65536 or T * E * H >= 10_000_000) and h.stride(0) % 8 == 0 and \
+        h.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0
 
 
 def _router(h: torch.Tensor, rd, bias: Optional[torch.Tensor] = None, logits: Optional[torch.Tensor] = None) -> None:

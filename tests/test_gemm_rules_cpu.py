@@ -1,7 +1,8 @@
-"""Which GEMM kernel a call takes: the rule on sizes, rows and multi-GPU hooks (no GPU)."""
+"""Which GEMM and which router kernel a call takes: the rules on sizes, rows and multi-GPU hooks (no GPU)."""
 import pytest
 import torch
 
+from disagmoe_b200.ops import functional as F
 from disagmoe_b200.ops import gemm
 
 SMS = 148
@@ -21,6 +22,16 @@ def test_measured_choices(epi, T, F, K, G, wide):
 def test_stream_k_of_no_expected_rows(G):
     """An expert rank whose share of the arriving rows rounds to none still asks for a rule: 32 tiles leave most SMs idle."""
     assert gemm.want_streamk(gemm.EPI_COMBINE, 4096, G, 0, 32, SMS)
+
+
+@pytest.mark.parametrize("T,H,E,separate", [
+    (1, 2048, 64, True), (1, 2048, 60, True), (37, 2048, 32, True), (96, 1024, 64, True), (1, 4096, 8, False), (256, 4096, 8, False),
+    (448, 4096, 8, True), (448, 2048, 8, False), (640, 2048, 8, True), (148, 1024, 24, False), (512, 256, 24, False), (64, 2000, 64, False),
+])
+def test_measured_router_choices(T, H, E, separate):
+    rows, weight = torch.empty(2, H, dtype=torch.bfloat16), torch.empty(E, H, dtype=torch.bfloat16)
+    assert F.separate_router(T, H, E, rows, weight) is separate
+    assert not F.separate_router(T, H, E, torch.empty(2, H + 8, dtype=torch.bfloat16)[:, 1:H + 1], weight)      # unaligned rows
 
 
 def test_rows_and_hooks():

@@ -13,12 +13,12 @@ def _bf(*s, scale=1.0):
 
 @pytest.mark.parametrize("T", [1, 15, 16, 17, 300])
 @pytest.mark.parametrize("H,E,K", [(256, 17, 3), (2048, 60, 4), (4096, 64, 8), (512, 256, 8), (2048, 33, 1)])
-def test_softmax_router(T, H, E, K):
+def test_softmax_router(T, H, E, K, monkeypatch):
+    monkeypatch.setattr(F, "separate_router", lambda *a: True)
     torch.manual_seed(T)
     x, nw, gw = _bf(T, H), _bf(H), _bf(E, H, scale=H ** -0.5)
     bias = torch.randn(E, device="cuda")
     counts = torch.zeros(E, dtype=torch.int32, device="cuda")
-    assert F.separate_router(T, H, E, x, gw)
     y, ids, w, logits = F.route(x, nw, 1e-5, gw, K, True, counts=counts, want_logits=True, logit_bias=bias)
     exact = y.double() @ gw.double().T + bias.double()
     # fp32 sums of exact products: a few units of 2^-24 of the sum of their sizes (the tensor core truncates when it aligns them)
@@ -59,8 +59,7 @@ def test_router_behind_sum_norm(T, E, top, groups, keep, sigmoid, monkeypatch):
     corr = torch.randn(E, device="cuda") * 0.1 if sigmoid else None
     weight, out = _bf(E, W, scale=W ** -0.5), []
     for fused in (False, True):
-        if fused:
-            monkeypatch.setattr(F, "separate_router", lambda *a: False)
+        monkeypatch.setattr(F, "separate_router", lambda *a: not fused)
         r = F.Router(weight, top, sigmoid, torch.zeros(E, dtype=torch.int32, device="cuda"), sigmoid, corr, groups, keep, 2.5)
         h, ids, wts = F.sum_norm(resid.clone(), y, None, w, 1e-6, torch.bfloat16, False, router=r)
         assert torch.equal(r.counts.long(), torch.bincount(ids.reshape(-1).long(), minlength=E))
