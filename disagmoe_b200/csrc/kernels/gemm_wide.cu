@@ -351,10 +351,13 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
 #pragma unroll
               for (int j = 0; j < 32; ++j) o[j] = out_tanh(o[j]);
             }
-            if (a.act == 4) {
+            const int silu = a.act == 4 ? a.act_cols - f0 - c * 32 : 0;      // columns of this chunk that take it
+            if (silu >= 32) {
 #pragma unroll
-              for (int j = 0; j < 32; ++j)
-                if (f0 + c * 32 + j < a.act_cols) o[j] = gate_act<0>(o[j]);
+              for (int j = 0; j < 32; ++j) o[j] = gate_act<0>(o[j]);
+            } else if (silu > 0) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) o[j] = j < silu ? gate_act<0>(o[j]) : o[j];
             }
             if (res != nullptr) {
 #pragma unroll

@@ -37,6 +37,23 @@ def test_linear_variants(T, O, K):
     _close(out, ref + r.float())
 
 
+@pytest.mark.parametrize("wide", [False, True])
+def test_silu_divides_exactly(wide):
+    """Of a product with the identity the activation is all that rounds: the quotient to nearest (0.5 units of 2^-24), its denominator
+    and the exponential. Their errors' root mean square measured 0.77 units, and 0.93 with an approximate quotient."""
+    torch.manual_seed(0)
+    x = _rand(4096, 256, scale=0.1)
+    y = gemm.linear(x, torch.eye(256, device="cuda").bfloat16(), out_dtype=torch.float32, silu_cols=256, wide=wide).double()
+    want = torch.nn.functional.silu(x.double())
+    err = ((y - want) / want)[want != 0] * 2.0 ** 24
+    assert float(err.pow(2).mean().sqrt()) < 0.85 and float(err.abs().max()) < 5
+    # signed zeros, infinities and NaN as the division has them
+    edge = torch.tensor([0.0, -0.0, float("inf"), float("nan"), -200.0, 300.0, -88.0, 1.0], device="cuda").bfloat16()
+    y = gemm.linear(edge.repeat(8).diag(), torch.eye(64, device="cuda").bfloat16(), out_dtype=torch.float32, silu_cols=64, wide=wide)
+    assert bool(y[3].isnan().all()) and bool(y[2, 2].isposinf()) and float(y[5, 5]) == 300.0
+    assert -1e-35 < float(y[6, 6]) < 0 and float(y[4, 4]) == 0 and float(y[0].abs().max()) == 0
+
+
 @pytest.mark.parametrize("wide", [None, True])
 def test_counters_to_clear(wide):
     """Only the other kernel zeroes the counters that a launch is given: it keeps such a launch, whatever is asked for."""
