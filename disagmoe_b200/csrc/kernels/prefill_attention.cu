@@ -37,12 +37,6 @@ constexpr int fa_smem(bool lat) { return 3 * kFaTile + (lat ? 2 * kFaHalf : 0) +
 enum { FA_PAGED = 0, FA_LATENT = 1 };
 constexpr float kFaSlack = 8.f;                     // growth of a row's maximum (base 2) that is left in P
 
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 __device__ __forceinline__ void fa_load(uint32_t dst, const CUtensorMap* m, int x, int y, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
@@ -204,12 +198,14 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
       for (int i = 0; i < 4; ++i) tmem_ld32(t_s + lanes + i * 32, s[i]);
       tmem_ld_wait();
       const bool masked = key0 + kFaKeys - 1 > pos0 || key0 < lo_last;
-      float mx = -INFINITY;
+      float mx = -INFINITY, mul = 1.f;      // scores are s times mul: the factor goes into the exponent's subtraction where it can
       if (ext.cap_log2 > 0.f) {
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
           for (int e = 0; e < 32; ++e) s[i][e] = __float_as_uint(attn_score<true>(__uint_as_float(s[i][e]) * temp, scale_log2, ext));
+      } else if (scale > 0.f) {
+        mul = scale;
       } else {
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -235,11 +231,12 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         }
         mx = fmaxf(mx, fmaxf(a, b));
       }
+      mx *= mul;
       const bool grow = mx > m + kFaSlack;      // true for the first finite maximum: m is -inf before it
       if (__any_sync(0xffffffffu, grow)) {
         const float to = grow ? mx : m;
         if (j > 0) {
-          const float f = grow ? ex2(m - to) : 1.f;      // -inf - finite: 0, and what it scales is 0
+          const float f = grow ? exp2f(m - to) : 1.f;      // -inf - finite: 0, and what it scales is 0
           l *= f;
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
@@ -260,7 +257,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         uint32_t hi[16], rest[16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
-          const float p0 = ex2(__uint_as_float(s[i][2 * e]) - sub), p1 = ex2(__uint_as_float(s[i][2 * e + 1]) - sub);
+          // exp2f and not the instruction alone, which makes 0 of weights below 2^-126
+          const float p0 = exp2f(fmaf(__uint_as_float(s[i][2 * e]), mul, -sub)), p1 = exp2f(fmaf(__uint_as_float(s[i][2 * e + 1]), mul, -sub));
           sum[e & 3] += p0 + p1;
           split2(p0, p1, hi[e], rest[e]);
         }

@@ -1,4 +1,6 @@
 """Prompt attention on tcgen05 (heads of 128) vs fp32 PyTorch: edges of query and key tiles, page sizes, garbage beyond the keys."""
+import math
+
 import pytest
 import torch
 
@@ -73,6 +75,23 @@ def test_many_key_blocks():
     # fp32 softmax weights: one rounding of the output, 2^-9 relative, and twice that for the bf16 reference it is compared in
     segs = [(0, 3000, 1096), (1, 2047, 300), (2, 0, 2049), (3, 4088, 8)]
     _close(*_run(8, 2, 16, segs=segs, span=4096, scale=0.5, fp32_weights=True), tol=2 ** -7)
+
+
+@pytest.mark.parametrize("shift", [-120, -127, -130, -133])
+def test_weights_below_the_normal_range(shift):
+    """A key that is 2^shift of the largest weight still counts: its value is as large as bf16 has them, those of all others are 0."""
+    n_q, bs, n = 2, 16, 130
+    q, kc, vc = (torch.zeros(s, dtype=torch.bfloat16, device="cuda") for s in ((n, n_q * HD), (9, bs, n_q, HD), (9, bs, n_q, HD)))
+    q[:, ::HD] = 1.0
+    kc[0, 3, :, 0], vc[0, 3] = float(shift), 2.0 ** 127
+    bt, out = torch.arange(9, device="cuda").int()[None], torch.empty(n, n_q * HD, dtype=torch.bfloat16, device="cuda")
+    tiles, _ = F.build_prefill_tiles([0] * n, range(n), F.prefill_tile_tokens(n_q, n_q))
+    F.prefill_attention(q, kc, vc, bt, tiles.cuda(), len(tiles), n_q, n_q, HD, out, scale=math.log(2.0), fp32_weights=True)
+    t = torch.arange(n, device="cuda", dtype=torch.float64)
+    want = torch.where(t >= 3, 2.0 ** (127 + shift) / t.clamp(min=1), t * 0)
+    # powers of two down to bf16's smallest, 2^-133: one rounding of the output and the fp32 division by the sum
+    assert gemm.check_status() == 0
+    torch.testing.assert_close(out.double(), want[:, None].expand_as(out), rtol=2.0 ** -7, atol=0.0)
 
 
 def test_loose_rows():
