@@ -43,15 +43,3 @@ def test_rows_and_hooks():
     for hooks in (dict(n_wait=1), dict(n_signal=1), dict(shard_rows=4), dict(group_regions=True), dict(fanout=2), dict(rs_bases=y),
                   dict(seg_cnt=y, S=1), dict(clear=torch.ones(4, dtype=torch.int32), done_ticket=torch.zeros(1, dtype=torch.int32))):
         assert not gemm._wide_rows(64, y, None, gemm.GemmComm(**hooks))
-
-
-def test_dense_walk_division():
-    """div_by of work_walker.cuh in fp32: exact over its range for every divisor a launch can have."""
-    import numpy as np
-    n = np.concatenate([np.arange(0, 1 << 16), np.random.default_rng(0).integers(0, 1 << 22, 1 << 16)]).astype(np.int64)
-    for d in list(range(1, 130)) + [148, 255, 1000, 4097]:
-        r = np.float32(1.0) / np.float32(d)
-        q = (n.astype(np.float32) * r).astype(np.int64)
-        rest = n - q * d
-        q += np.where(rest >= d, 1, np.where(rest < 0, -1, 0))
-        assert np.array_equal(q, n // d)

@@ -114,5 +114,10 @@ def test_gated_add(T, H):
     got = F.gated_add(resid.clone(), sh, y, w).double()
     # one bf16 rounding of the sum (half a unit in the last of 8 bits) and the fp32 gate
     assert bool(((got - want).abs() <= want.abs() * 2.0 ** -7.99 + 1e-5).all())
-    wide = torch.cat([resid, resid], 1)[:, :H + 1][:, 1:]      # unaligned rows take the general path
-    assert F.gated_add(wide.clone(), sh, y, w).shape == (T, H)
+    # unaligned rows take the general path
+    base = torch.cat([resid, resid], 1)
+    v = base[:, 1:H + 1]
+    assert v.data_ptr() % 16 != 0
+    want = v.double() + sh.double() * torch.sigmoid(y.double() @ w.double().T)
+    got = F.gated_add(v, sh, y, w).double()
+    assert bool(((got - want).abs() <= want.abs() * 2.0 ** -7.99 + 1e-5).all())
