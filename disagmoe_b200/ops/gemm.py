@@ -158,9 +158,12 @@ def want_wide(epi: int, T: int, F: int, K: int, G: int, sms: int) -> bool:
     """Should the tokens be the M operand (csrc/kernels/gemm_wide.cu, 256 x 256 tiles on CTA pairs) instead of the weights?
 
     Dense: a cost model of both, in us, fitted to a sweep on B200 (K 1024 .. 5632, F 256 .. 32000, T 8 .. 2048; the choice is within
-    5 % of the better of these two kernels). A wide tile takes 0.31 us per K block whatever part of it is used, the other kernel what
+    8 % of the better of these two kernels, K below 1024 within 15 %). A wide tile takes 0.31 us per K block whatever part of it is used, the other kernel what
     its SM pulls from L2. Measured (bf16, other kernel -> wide): 4096 x 6144 x 4096 201 -> 149 us (1381 TFLOP/s), 2500 x 4096 x
-    2048 106 -> 40, 1111 x 6144 x 2048 79 -> 31, 256 x 32000 x 4096 89 -> 58; SwiGLU 1024 x 5632 x 2048 59 -> 42.
+    2048 106 -> 40, 1111 x 6144 x 2048 79 -> 31, 256 x 32000 x 4096 89 -> 58; SwiGLU 1024 x 5632 x 2048 59 -> 42. A few rows of SwiGLU
+    gain by the wider tile's faster K blocks (1 row, 2048 x 4096 38 -> 32, 16 rows, 8192 x 7168 82 -> 65), but pay 2 us more per launch
+    (1 row, 2048 x 256 11.2 -> 12.6, 4096 x 1024 17.4 -> 17.4), and more where the tiles of a wave want more than HBM gives (1 row,
+    8192 x 1024 17.4 -> 19.3, 8192 x 7168 69 -> 78; 8 rows, 8192 x 4096 47 -> 49).
 
     Grouped (only the mean group size is known): up to 128 tokens the other kernel's tile fits a group and streams the weights
     at HBM speed, beyond that it needs a second tile per group. Measured at 64 experts of 1408 x 2048, SwiGLU: 120 tokens each
@@ -174,6 +177,8 @@ def want_wide(epi: int, T: int, F: int, K: int, G: int, sms: int) -> bool:
     if G > 1:
         return T >= 144 * G or (epi != EPI_SWIGLU and K <= 2048 and (F * K <= 4_400_000 or G >= 60))
     if T < 64 and epi != EPI_SWIGLU:
+        return False
+    if T <= 32 and (K < 1024 or F > 4096 and K < (8192 if T <= 8 else 4096)):      # SwiGLU: see above
         return False
     feat = 128 if epi == EPI_SWIGLU else 256
     tiles = ((F + feat - 1) // feat) * ((T + 255) // 256)

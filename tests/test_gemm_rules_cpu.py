@@ -13,6 +13,8 @@ SMS = 148
     (gemm.EPI_PLAIN, 256, 32000, 4096, 1, True), (gemm.EPI_PLAIN, 300, 256, 5632, 1, False), (gemm.EPI_PLAIN, 2048, 2048, 2048, 1, True),
     (gemm.EPI_SWIGLU, 256, 5632, 2048, 1, True), (gemm.EPI_SWIGLU, 64, 14336, 4096, 1, False), (gemm.EPI_SWIGLU, 100, 1408, 2048, 64, False),
     (gemm.EPI_SWIGLU, 144 * 8, 14336, 4096, 8, True), (gemm.EPI_COMBINE, 2, 4096, 14336, 8, False), (gemm.EPI_COMBINE, 148, 2048, 1408, 60, True),
+    (gemm.EPI_SWIGLU, 1, 2048, 256, 1, False), (gemm.EPI_SWIGLU, 16, 8192, 1024, 1, False), (gemm.EPI_SWIGLU, 1, 8192, 7168, 1, False),
+    (gemm.EPI_SWIGLU, 16, 8192, 7168, 1, True), (gemm.EPI_SWIGLU, 1, 2048, 4096, 1, True), (gemm.EPI_SWIGLU, 37, 5632, 2048, 1, True),
     (gemm.EPI_COMBINE, 24, 6144, 2048, 16, False), (gemm.EPI_COMBINE, 24, 4096, 1408, 16, False), (gemm.EPI_COMBINE, 24, 4096, 1408, 60, True),
     (gemm.EPI_COMBINE, 74, 4096, 1024, 8, True), (gemm.EPI_PLAIN, 96, 2048, 2816, 64, False),
 ])
