@@ -172,9 +172,12 @@ __global__ void embed_kernel(const int* __restrict__ ids, const __nv_bfloat16* _
   for (int i = threadIdx.x; i < H / 8; i += blockDim.x) dst[i] = src[i];
 }
 
-// ids[t] = argmax_v logits[t, v] (first maximum wins). logits fp32 or bf16. A row is cut into `parts` runs, one per CTA of a
-// cluster, whose maxima meet in the first CTA's shared memory: one CTA per row left most SMs idle at decode batches and walked
-// the row one dependent 4-byte load at a time (37 rows of 151,936: 44 us on B200, now 6 us). VEC values per load (1: unaligned rows).
+// ids[t] = argmax_v logits[t, v] (first maximum wins). logits fp32 or bf16, VEC values per load (1: unaligned rows). Where a batch
+// leaves most SMs idle, a row is cut into `parts` runs, one per CTA of a cluster, whose maxima meet in the first CTA's shared memory.
+// Cutting pays while the clusters find place side by side, about two CTAs per SM; beyond that, and for short rows, their launches cost
+// more than the scans they shorten. Measured on B200 with cold caches, 1 / 2 / 4 / 8 parts: 1 row of 151,936 27 / 18 / 14 / 11 us,
+// 37 rows 28 / 21 / 16 / 14, 100 rows 33 / 25 / 22 / 29, 256 rows 44 / 49 / 49 / 55; 32,000: 1 row 11 / 10 / 10 / 8, 100 rows 13 / 12 / 12
+// / 16, 256 rows 15 / 19 / 23 / 28; 16,384: 1 row 9.1 / 8.5 / 8.3 / 8.2, 37 rows (warm) 3.1 / 3.3 / 3.5 / 3.9.
 constexpr int kArgThreads = 512, kArgParts = 8;
 
 __device__ __forceinline__ void arg_take(float x, int v, float& best, int& bi) {
@@ -237,8 +240,8 @@ argmax_kernel(const T* __restrict__ logits, long long ld, int V, int* __restrict
 
 template <typename T, int VEC>
 static int launch_argmax(const void* logits, long long ld, int T_, int V, int* ids, cudaStream_t stream) {
-  // enough rows for every SM: one CTA each
-  const int parts = T_ >= 2 * device_num_sms() || V < 8192 ? 1 : kArgParts;
+  int parts = 1;
+  while (V >= 24000 && parts < kArgParts && 2 * parts * T_ <= 2 * device_num_sms()) parts *= 2;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3(static_cast<unsigned>(T_) * parts);

@@ -95,10 +95,10 @@ def test_argmax(T, V, dtype, off):
     assert torch.equal(got, want)
 
 
-@pytest.mark.parametrize("T", [1, 40, 295])
-@pytest.mark.parametrize("V,dtype", [(8192, torch.float32), (8203, torch.bfloat16), (32000, torch.float32)])
+@pytest.mark.parametrize("T", [1, 37, 38, 74, 75, 148, 149, 300])
+@pytest.mark.parametrize("V,dtype", [(8192, torch.float32), (24011, torch.bfloat16), (32000, torch.float32)])
 def test_argmax_over_the_runs_of_a_row(T, V, dtype):
-    """Rows that several CTAs of a cluster share, from one to just below two per SM: the maximum stands in every run in turn."""
+    """Rows that 8, 4, 2 CTAs of a cluster share, and those that one CTA scans: the maximum stands in every run in turn."""
     x = torch.zeros(T, V, dtype=dtype, device="cuda")
     at = (torch.arange(T, device="cuda") * 1031 + 17) % V
     x[torch.arange(T, device="cuda"), at] = 1.0
