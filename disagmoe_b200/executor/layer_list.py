@@ -45,7 +45,8 @@ class LayerListBuffers(TokenBuffers):
         self.block_offs: Dict[int, torch.Tensor] = {}        # likewise
         self.resid = torch.zeros(cap, cfg.hidden_size, dtype=torch.float32, device=device)
         self.segments: Optional[SegmentTables] = None        # None: decode step, every row its own segment
-        self.prefill_tiles: Dict[int, Tuple[torch.Tensor, int]] = {}    # tokens per tile -> (table, tiles)
+        # tokens per tile -> (table, tiles, their reach by (window, chunk))
+        self.prefill_tiles: Dict[int, Tuple[torch.Tensor, int, Dict[Tuple, int]]] = {}
         self.ctx_len_decode: Optional[torch.Tensor] = None
         self.n_untiled = 0
 
@@ -148,19 +149,25 @@ class LayerListExecutor(StepExecutor):
         buf.latent = {k: LatentTables.prefill(m, bt_row, positions, self.device, self.dtype)
                       for k, m in self.latent_specs.items()}
         buf.block_offs = self._block_offs(T)
+        built = {}
         for mixer in self.attentions:
             m = mixer.spec
             if not mixer.tiled():
                 continue
             n = F.prefill_tile_tokens(m.heads, m.kv_heads)
-            if n in buf.prefill_tiles:
+            if n not in built:
+                built[n] = F.build_prefill_tiles(bt_row, positions, n)
+            tiles, covered = built[n]
+            if not len(tiles):
                 continue
-            tiles, covered = F.build_prefill_tiles(bt_row, positions, n)
-            if len(tiles):
-                buf.prefill_tiles[n] = (upload(tiles, self.device), len(tiles))
+            if n not in buf.prefill_tiles:
+                buf.prefill_tiles[n] = (upload(tiles, self.device), len(tiles), {})
                 cd = torch.as_tensor(ctx_len).clone()
                 cd[covered] = 0              # which rows are tiled does not depend on the tile size
                 buf.ctx_len_decode, buf.n_untiled = upload(cd, self.device), F.loose_rows(covered)
+            reach = buf.prefill_tiles[n][2]
+            if (m.window, m.chunk) not in reach:
+                reach[m.window, m.chunk] = F.tile_reach(tiles, m.window, m.chunk)
 
     def _end_prefill(self, buf: LayerListBuffers) -> None:
         buf.segments, buf.prefill_tiles, buf.ctx_len_decode, buf.latent, buf.block_offs = None, {}, None, {}, {}

@@ -56,6 +56,7 @@ class LatentTables:
     tiles: Optional[torch.Tensor] = None      # int32 [n_tiles, 4], see ops.functional.build_prefill_tiles
     base: Optional[torch.Tensor] = None       # int32 [n_tiles]: workspace row of position 0 of the tile's sequence
     n_tiles: int = 0
+    reach: int = 0                            # most keys of a tile, see ops.functional.tile_reach
     keys: Optional[torch.Tensor] = None       # int32 [n_keys, 2] = (block-table row, position) of every workspace row
     n_keys: int = 0
 
@@ -101,7 +102,7 @@ class LatentTables:
         base = torch.from_numpy(np.repeat(at[:-1] - lo, ends - begins + 1).astype(np.int32))
         keys = torch.from_numpy(keys)
         up = lambda x: upload(x, device)
-        t = cls(len(rows), up(loose), up(rows), None, None, up(tiles), up(base), len(tiles), up(keys), len(keys))
+        t = cls(len(rows), up(loose), up(rows), None, None, up(tiles), up(base), len(tiles), F.tile_reach(tiles, m.window), up(keys), len(keys))
         if len(rows):
             t.offs, t.recs = cls._per_head(rows, m.heads, device)
         return t
@@ -375,8 +376,8 @@ class SoftmaxAttention(Mixer):
         opt = dict(scale=m.scale, window=m.window, chunk=m.chunk, softcap=m.softcap, fp32_weights=True, sink=self.sink,
                    q_temp=m.q_temp, gate=gate)
         cuda = self.tiled()
-        tiles, n_tiles = meta.prefill_tiles.get(F.prefill_tile_tokens(m.heads, m.kv_heads), (None, 0)) \
-            if cuda and meta.prefill_tiles else (None, 0)
+        tiles, n_tiles, reaches = meta.prefill_tiles.get(F.prefill_tile_tokens(m.heads, m.kv_heads), (None, 0, None)) \
+            if cuda and meta.prefill_tiles else (None, 0, None)
         T = q.shape[0]
         n = meta.num_decode_tokens if n_tiles else T         # rows from n on are all tiled
         attn = torch.empty(T, m.heads * self.dv, dtype=q.dtype, device=q.device)
@@ -389,7 +390,8 @@ class SoftmaxAttention(Mixer):
                               m.heads, m.kv_heads, self.dk, out=attn[:n], splits=splits,
                               **{**opt, "gate": gate[:n] if gate is not None else None})
         if n_tiles:
-            F.prefill_attention(q, kc, vc, meta.block_tables, tiles, n_tiles, m.heads, m.kv_heads, self.dk, attn, **opt)
+            F.prefill_attention(q, kc, vc, meta.block_tables, tiles, n_tiles, m.heads, m.kv_heads, self.dk, attn, **opt,
+                                reach=reaches[m.window, m.chunk])
         return attn
 
 
@@ -477,7 +479,7 @@ class LatentAttention(Mixer):
         if t.n_tiles:
             lat = F.latent_gather(cache, meta.block_tables, t.keys, t.n_keys)
             kvx = gemm.linear(lat[:, :lay.rankp], self.expand)
-            F.latent_prefill(y, kvx, lat, t.tiles, t.base, t.n_tiles, lay, m.scale, m.window, self.sink, attn, gate)
+            F.latent_prefill(y, kvx, lat, t.tiles, t.base, t.n_tiles, lay, m.scale, m.window, self.sink, attn, gate, t.reach)
         return gemm.linear(attn, self.o)
 
 

@@ -504,14 +504,26 @@ def build_prefill_tiles(bt_row, positions, tile_tokens: int, min_len: int = 8):
     return t, torch.from_numpy(covered)
 
 
+def tile_reach(tiles: torch.Tensor, window: Optional[int] = None, chunk: Optional[int] = None) -> int:
+    """Most keys that a tile of a host table (:func:`build_prefill_tiles`) looks at, from the first that its first token sees on."""
+    import numpy as np
+    t = tiles.numpy()
+    first = np.maximum(0, t[:, 3] - window + 1) if window else np.zeros_like(t[:, 3])
+    if chunk:
+        first = np.maximum(first, t[:, 3] // chunk * chunk)
+    return int((t[:, 3] + t[:, 1] - first).max()) if len(t) else 0
+
+
 def prefill_attention(q: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tensor, block_tables: torch.Tensor,
                       tiles: torch.Tensor, n_tiles: int, n_q: int, n_kv: int, hd: int, out: torch.Tensor,
                       scale: Optional[float] = None, window: Optional[int] = None, softcap: Optional[float] = None,
                       fp32_weights: bool = False, sink: Optional[torch.Tensor] = None,
-                      chunk: Optional[int] = None, q_temp=None, gate: Optional[torch.Tensor] = None) -> torch.Tensor:
+                      chunk: Optional[int] = None, q_temp=None, gate: Optional[torch.Tensor] = None,
+                      reach: Optional[int] = None) -> torch.Tensor:
     """Causal attention of the prompt tokens named by ``tiles`` (device int32 [>= n_tiles, 4], see
     :func:`build_prefill_tiles`) over the paged cache, which already holds their own K / V; writes their rows of
-    ``out``. Every tile streams its sequence's K / V once (the per-token kernel streams it once per row)."""
+    ``out``. Every tile streams its sequence's K / V once (the per-token kernel streams it once per row). ``reach``
+    (:func:`tile_reach`), where the caller knows it, chooses between two kernels of attention with options."""
     if n_tiles == 0:
         return out
     assert q.is_cuda and tiles.is_cuda and tiles.dtype == torch.int32 and tiles.is_contiguous()
@@ -521,7 +533,12 @@ def prefill_attention(q: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tenso
     options = window or chunk or softcap or fp32_weights or sink is not None or q_temp is not None or gate is not None or \
         hd != vd or n_q // n_kv not in (1, 2, 4, 8)
     x = _attn_extra(q_temp, gate, q.dtype)
-    if options and _prefill_on_tcgen05(q, kcache, vcache, out, hd, vd):
+    # A CTA of the tcgen05 kernel needs 10 us before its first result and 3 us per 128 keys then, one of the mma.sync kernel 6 us and
+    # 9 us; a chip full of them meets at fewer keys. Measured on B200 (warm, mma.sync -> tcgen05), 16 / 4 heads: one prompt of 64 tokens 7.2
+    # -> 12.9 us, 192: 15.2 -> 17.1, 256: 19.3 -> 16.3; 16 prompts of 64 9.5 -> 13.5, of 100 20.5 -> 17.0; 48 of 64 23 -> 27, of 96 40 -> 31;
+    # window 64: one prompt of 1000 13.5 -> 18.5, 4 of 500 24.4 -> 22.4, one of 3000 35.0 -> 34.3; window 200: of 1000 25.7 -> 22.6.
+    if options and (reach is None or reach > 192 or reach >= 95 and n_tiles * n_kv >= 192) and \
+            _prefill_on_tcgen05(q, kcache, vcache, out, hd, vd):
         from .gemm import scratch
         _lib.check(_lib.lib().dmoe_prefill_attention_tc(
             _vp(q), c_ll(q.stride(0)), _vp(kcache), _vp(vcache), c_int(kcache.shape[0]), _vp(block_tables),
@@ -990,15 +1007,17 @@ def latent_gather(cache: torch.Tensor, block_tables: torch.Tensor, keys: torch.T
 
 def latent_prefill(q: torch.Tensor, kv: torch.Tensor, lat: torch.Tensor, tiles: torch.Tensor, base: torch.Tensor, n_tiles: int,
                    lay: LatentLayout, scale: float, window: Optional[int], sink: Optional[torch.Tensor],
-                   out: torch.Tensor, gate: Optional[torch.Tensor] = None) -> torch.Tensor:
+                   out: torch.Tensor, gate: Optional[torch.Tensor] = None, reach: Optional[int] = None) -> torch.Tensor:
     """Causal attention of the prompt tokens named by ``tiles`` over expanded keys and values: kv [keys, heads x (key
     unrotated | value)], rotated key parts in the gathered cache rows ``lat`` [keys, row]; the key at position p of tile i's
     sequence is row base[i] + p. q: projection rows with rotated queries. Writes the tokens' rows of out [T, heads x vdimp], scaled by sigmoid(gate)
-    per head where ``gate`` [T, heads] is given."""
+    per head where ``gate`` [T, heads] is given. ``reach`` (:func:`tile_reach`), where the caller knows it, chooses between two kernels."""
     _check_sink(sink, lay.heads)
     assert gate is None or (gate.dtype == torch.bfloat16 and gate.stride(1) == 1)
     assert tiles.dtype == base.dtype == torch.int32 and kv.stride(1) == lat.stride(1) == 1
-    if (lay.dimp, lay.rotp, lay.vdimp) == (128, 64, 128) and all(t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (q, kv, lat, out)):
+    # Measured on B200 (warm, mma.sync -> tcgen05), 16 heads: one prompt of 64 tokens 6.6 -> 9.9 us, 128: 9.0 -> 10.6, 192: 11.9 -> 13.4,
+    # 256: 14.6 -> 13.9, 512: 25.8 -> 20.9; 16 prompts of 64 9.2 -> 20, of 128 20.4 -> 21.7, of 192 38 -> 46, of 256 56 -> 48.
+    if (reach is None or reach > 192) and (lay.dimp, lay.rotp, lay.vdimp) == (128, 64, 128) and all(t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (q, kv, lat, out)):
         _lib.check(_lib.lib().dmoe_latent_prefill_tc(
             _vp(q), c_ll(q.stride(0)), _vp(kv), c_ll(kv.stride(0)), _vp(lat), c_ll(lat.stride(0)), c_ll(min(kv.shape[0], lat.shape[0])),
             _vp(tiles), _vp(base), c_int(n_tiles), c_int(lay.heads), c_int(lay.rankp), c_float(scale), c_int(window or 0), _vp(sink),

@@ -47,3 +47,15 @@ def test_rows_and_hooks():
     for hooks in (dict(n_wait=1), dict(n_signal=1), dict(shard_rows=4), dict(group_regions=True), dict(fanout=2), dict(rs_bases=y),
                   dict(seg_cnt=y, S=1), dict(clear=torch.ones(4, dtype=torch.int32), done_ticket=torch.zeros(1, dtype=torch.int32))):
         assert not gemm._wide_rows(64, y, None, gemm.GemmComm(**hooks))
+
+
+def test_reach_of_prompt_tiles():
+    """Tiles of 32 tokens: the last of 100 tokens sees all of them; a window or a chunk cuts what its first token sees."""
+    tiles, _ = F.build_prefill_tiles([0] * 100 + [1] * 20, list(range(100)) + list(range(40, 60)), 32)
+    assert F.tile_reach(tiles) == 100 and F.tile_reach(tiles, window=10) == 9 + 32 and F.tile_reach(tiles, window=1) == 32
+    assert F.tile_reach(tiles, chunk=64) == 64 and F.tile_reach(tiles, chunk=1000) == 100 and F.tile_reach(tiles, 10, 64) == 9 + 32
+    assert F.tile_reach(tiles[:0]) == 0
+    for t in tiles.tolist():                         # against the keys of every token of every tile
+        for window, chunk in ((None, None), (10, None), (None, 24), (5, 24)):
+            first = min(max(0, p - window + 1 if window else 0, p // chunk * chunk if chunk else 0) for p in range(t[3], t[3] + t[1]))
+            assert F.tile_reach(tiles[tiles[:, 0] == t[0]], window, chunk) == t[3] + t[1] - first

@@ -70,6 +70,14 @@ def test_options(opt):
     _close(*_run(8, 2, 16, poison=True, **opt), tol=2 ** -7)
 
 
+@pytest.mark.parametrize("opt", [dict(window=64), dict(sink=None, gate=None), dict(chunk=96, softcap=20.0)])
+def test_short_reach(opt):
+    """Prompts of few keys take the mma.sync kernel, two of whose CTAs share a tile of 128 rows."""
+    segs = [(0, 0, 90), (1, 0, 8), (2, 30, 33)]
+    # fp32 softmax weights: one rounding of the output, 2^-9 relative, and twice that for the bf16 reference it is compared in
+    _close(*_run(8, 2, 16, segs=segs, reach=90, **opt), tol=2 ** -7)
+
+
 def test_many_key_blocks():
     """Two CTAs per SM, each with up to 32 key blocks: scores of a block take the place of the weights before."""
     # fp32 softmax weights: one rounding of the output, 2^-9 relative, and twice that for the bf16 reference it is compared in
