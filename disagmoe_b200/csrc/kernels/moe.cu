@@ -209,7 +209,7 @@ dispatch_kernel(const U* __restrict__ y, long long ld_y, const int* __restrict__
                 const float* __restrict__ topk_w, int T, int K, int units, int E, int experts_per_rank, int my_rank,
                 int* __restrict__ ws, int* __restrict__ offs, void* const* __restrict__ x_bases, long long ld_dst,
                 void* const* __restrict__ rec_bases, int dst_capacity, int* __restrict__ status) {
-  __shared__ int s_base[kMaxExperts + 1], s_before[kMaxExperts + 1];
+  __shared__ int s_before[kMaxExperts + 1];      // rows of the experts before
   int* counts = ws;
   int* cursor = ws + E;
   int* ticket = ws + 2 * E;
@@ -229,13 +229,9 @@ dispatch_kernel(const U* __restrict__ y, long long ld_y, const int* __restrict__
     if (threadIdx.x == 0) s_before[E] = run;
   }
   __syncthreads();
-  for (int e = threadIdx.x; e <= E; e += blockDim.x) {
-    // every destination rank's buffer starts at row 0
-    if (e < E) s_base[e] = s_before[e] - s_before[e / experts_per_rank * experts_per_rank];
-    // offsets of the local (rank-0-relative) view: global exclusive scan, used by a colocated engine
-    if (blockIdx.x == 0 && offs != nullptr) offs[e] = s_before[e];
-  }
-  __syncthreads();
+  // offsets of the local (rank-0-relative) view: global exclusive scan, used by a colocated engine
+  if (blockIdx.x == 0 && offs != nullptr)
+    for (int e = threadIdx.x; e <= E; e += blockDim.x) offs[e] = s_before[e];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   const int npairs = T * K;
   for (int p = blockIdx.x * nw + warp; p < npairs; p += gridDim.x * nw) {
@@ -248,7 +244,7 @@ dispatch_kernel(const U* __restrict__ y, long long ld_y, const int* __restrict__
     if (lane == 0) slot = atomicAdd(&cursor[e], 1);
     slot = __shfl_sync(0xffffffffu, slot, 0);
     const int rank = e / experts_per_rank;
-    const int row = s_base[e] + slot;
+    const int row = s_before[e] - s_before[rank * experts_per_rank] + slot;      // every destination rank's buffer starts at row 0
     if (row >= dst_capacity) {
       if (lane == 0 && status != nullptr) atomicCAS(status, kStatusOk, kStatusCapacity);
       continue;
