@@ -149,7 +149,7 @@ class LayerListExecutor(StepExecutor):
         buf.latent = {k: LatentTables.prefill(m, bt_row, positions, self.device, self.dtype)
                       for k, m in self.latent_specs.items()}
         buf.block_offs = self._block_offs(T)
-        built = {}
+        built, longest = {}, 0
         for mixer in self.attentions:
             m = mixer.spec
             if not mixer.tiled():
@@ -163,11 +163,12 @@ class LayerListExecutor(StepExecutor):
             if n not in buf.prefill_tiles:
                 buf.prefill_tiles[n] = (upload(tiles, self.device), len(tiles), {})
                 cd = torch.as_tensor(ctx_len).clone()
+                longest = int(cd[covered].max())
                 cd[covered] = 0              # which rows are tiled does not depend on the tile size
                 buf.ctx_len_decode, buf.n_untiled = upload(cd, self.device), F.loose_rows(covered)
             reach = buf.prefill_tiles[n][2]
             if (m.window, m.chunk) not in reach:
-                reach[m.window, m.chunk] = F.tile_reach(tiles, m.window, m.chunk)
+                reach[m.window, m.chunk] = F.tile_reach(longest, n, m.window, m.chunk)
 
     def _end_prefill(self, buf: LayerListBuffers) -> None:
         buf.segments, buf.prefill_tiles, buf.ctx_len_decode, buf.latent, buf.block_offs = None, {}, None, {}, {}

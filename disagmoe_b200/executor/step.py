@@ -23,6 +23,7 @@ class TokenBuffers:
         self.slots = z(cap, dt=torch.int64)
         self.logits = z(logit_rows, cfg.vocab_size, dt=torch.float32)
         self.out_rows: Optional[torch.Tensor] = None      # rows whose logits are wanted (None: all), set per step
+        self.copied = torch.cuda.Event() if device.type == "cuda" else None      # behind the copies of a prompt step's inputs
 
 
 class StepExecutor:
@@ -106,9 +107,8 @@ class StepExecutor:
         assert T <= self.prefill_buf.cap, f"{T} prefill tokens exceed the buffer ({self.prefill_buf.cap})"
         buf = self.prefill_buf
         self._fill(buf, T, ids, positions, slots, ctx_len, bt_row)
-        copied = torch.cuda.Event() if self.device.type == "cuda" else None
-        if copied is not None:
-            copied.record(torch.cuda.current_stream(self.device))
+        if buf.copied is not None:
+            buf.copied.record(torch.cuda.current_stream(self.device))
         self._begin_prefill(buf, T, positions, ctx_len, bt_row)
         if out_rows is not None:
             buf.out_rows = _lib.upload(torch.tensor(out_rows, dtype=torch.int32), self.device)
@@ -117,8 +117,8 @@ class StepExecutor:
         finally:
             buf.out_rows = None
             self._end_prefill(buf)
-            if copied is not None:
-                copied.synchronize()      # pinned inputs are read by the copies; the launches are queued by now
+            if buf.copied is not None:
+                buf.copied.synchronize()      # pinned inputs are read by the copies; the launches are queued by now
 
     def capture(self, sizes: Optional[List[int]] = None) -> None:
         """Warm-up (compiles nothing, but sizes scratch buffers and sets kernel attributes) and graph capture."""

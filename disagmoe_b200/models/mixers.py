@@ -56,7 +56,7 @@ class LatentTables:
     tiles: Optional[torch.Tensor] = None      # int32 [n_tiles, 4], see ops.functional.build_prefill_tiles
     base: Optional[torch.Tensor] = None       # int32 [n_tiles]: workspace row of position 0 of the tile's sequence
     n_tiles: int = 0
-    reach: int = 0                            # most keys of a tile, see ops.functional.tile_reach
+    reach: int = 0                            # keys of a tile at most, see ops.functional.tile_reach
     keys: Optional[torch.Tensor] = None       # int32 [n_keys, 2] = (block-table row, position) of every workspace row
     n_keys: int = 0
 
@@ -102,7 +102,7 @@ class LatentTables:
         base = torch.from_numpy(np.repeat(at[:-1] - lo, ends - begins + 1).astype(np.int32))
         keys = torch.from_numpy(keys)
         up = lambda x: upload(x, device)
-        t = cls(len(rows), up(loose), up(rows), None, None, up(tiles), up(base), len(tiles), F.tile_reach(tiles, m.window), up(keys), len(keys))
+        t = cls(len(rows), up(loose), up(rows), None, None, up(tiles), up(base), len(tiles), F.tile_reach(int(hi.max()), 128, m.window), up(keys), len(keys))
         if len(rows):
             t.offs, t.recs = cls._per_head(rows, m.heads, device)
         return t

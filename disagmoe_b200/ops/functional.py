@@ -504,14 +504,12 @@ def build_prefill_tiles(bt_row, positions, tile_tokens: int, min_len: int = 8):
     return t, torch.from_numpy(covered)
 
 
-def tile_reach(tiles: torch.Tensor, window: Optional[int] = None, chunk: Optional[int] = None) -> int:
-    """Most keys that a tile of a host table (:func:`build_prefill_tiles`) looks at, from the first that its first token sees on."""
-    import numpy as np
-    t = tiles.numpy()
-    first = np.maximum(0, t[:, 3] - window + 1) if window else np.zeros_like(t[:, 3])
-    if chunk:
-        first = np.maximum(first, t[:, 3] // chunk * chunk)
-    return int((t[:, 3] + t[:, 1] - first).max()) if len(t) else 0
+def tile_reach(longest: int, tile_tokens: int, window: Optional[int] = None, chunk: Optional[int] = None) -> int:
+    """At most so many keys a tile looks at, from the first that its first token sees on; ``longest``: context of the last row of all."""
+    reach = longest
+    if window:
+        reach = min(reach, window - 1 + tile_tokens)
+    return min(reach, chunk - 1 + tile_tokens) if chunk else reach
 
 
 def prefill_attention(q: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tensor, block_tables: torch.Tensor,

@@ -50,12 +50,11 @@ def test_rows_and_hooks():
 
 
 def test_reach_of_prompt_tiles():
-    """Tiles of 32 tokens: the last of 100 tokens sees all of them; a window or a chunk cuts what its first token sees."""
+    """Against the keys of every token of every tile: never less, and no more than the worst place of a window or chunk makes it."""
     tiles, _ = F.build_prefill_tiles([0] * 100 + [1] * 20, list(range(100)) + list(range(40, 60)), 32)
-    assert F.tile_reach(tiles) == 100 and F.tile_reach(tiles, window=10) == 9 + 32 and F.tile_reach(tiles, window=1) == 32
-    assert F.tile_reach(tiles, chunk=64) == 64 and F.tile_reach(tiles, chunk=1000) == 100 and F.tile_reach(tiles, 10, 64) == 9 + 32
-    assert F.tile_reach(tiles[:0]) == 0
-    for t in tiles.tolist():                         # against the keys of every token of every tile
-        for window, chunk in ((None, None), (10, None), (None, 24), (5, 24)):
-            first = min(max(0, p - window + 1 if window else 0, p // chunk * chunk if chunk else 0) for p in range(t[3], t[3] + t[1]))
-            assert F.tile_reach(tiles[tiles[:, 0] == t[0]], window, chunk) == t[3] + t[1] - first
+    for window, chunk in ((None, None), (1, None), (10, None), (200, None), (None, 24), (None, 64), (5, 24), (50, 64)):
+        first = lambda p: max(p - window + 1 if window else 0, p // chunk * chunk if chunk else 0, 0)
+        most = max(pos + n - first(pos) for _, n, _, pos in tiles.tolist())
+        reach = F.tile_reach(100, 32, window, chunk)
+        assert most <= reach <= min(100, 32 + min(window or 100, chunk or 100) - 1)
+    assert F.tile_reach(90, 32) == 90 and F.tile_reach(90, 32, window=10) == 41
