@@ -14,10 +14,10 @@ constexpr int kMaxGroups = 1024;
 enum { EPI_PLAIN = 0, EPI_SWIGLU = 1, EPI_COMBINE = 2 };
 
 // n / (1 + e) for e >= 0, rounded to nearest where the quotient is of normal size (3 of 2^30 random ones were a unit off the
-// operator's); signed zeros, infinities and NaN as the division has them. The quotient by an approximate reciprocal is corrected by its remainder, which a fused multiply-add gives exactly (P.
-// Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", 1990); both sides are scaled so that the
-// reciprocal stays normal. Straight code: the operator's slow path, which zero rows of a ragged tile take, and its branch keep the
-// chains of an epilogue thread from overlapping. Measured on B200, SwiGLU of 2500 x 5632 x 2048: 119 us with the operator, 88 us here;
+// operator's); signed zeros, infinities and NaN as the division has them. The quotient by an approximate reciprocal is corrected
+// by its remainder, which a fused multiply-add gives exactly (P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990); both sides are scaled so that the reciprocal stays normal. Straight code: the operator's slow
+// path, which zero rows of a ragged tile take, and its branch keep the chains of an epilogue thread from overlapping. Measured on B200, SwiGLU of 2500 x 5632 x 2048: 119 us with the operator, 88 us here;
 // one row of 5632 x 2048: 50 us with the operator, 27 us here.
 __device__ __forceinline__ float over_1p(float n, float e) {
   constexpr float kScale = 0.0625f;

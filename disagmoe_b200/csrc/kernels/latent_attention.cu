@@ -413,8 +413,9 @@ latent_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ 
 }
 
 // ---------------------------------------------------------------------------------------------------------------------------
-// Prompt runs over expanded keys and values in head sizes that prefill_attention.cu does not take: a tile is up to 128 consecutive
-// tokens of one head, a CTA of four warps has 64 of them (16 per warp as MMA rows), keys 64 at a time, double buffered. KD / VD: key (unrotated + rotated) and value sizes rounded up to the tile's.
+// Prompt runs over expanded keys and values, in head sizes that prefill_attention.cu does not take and of prompts too short for
+// it: a tile is up to 128 consecutive tokens of one head, a CTA of four warps has 64 of them (16 per warp as MMA rows), keys 64 at
+// a time, double buffered. KD / VD: key (unrotated + rotated) and value sizes rounded up to the tile's.
 constexpr int kLpKeys = 64;
 
 template <int KD, int VD>

@@ -6,7 +6,8 @@
 // and put P back into TMEM over S, from where it is the A operand of P V. The output accumulator stays in TMEM and is only
 // rescaled when a row's maximum grew by more than 2^8 (the sums use the same stale maximum, so nothing is lost). Warp 0
 // loads, warp 1 issues the MMAs. A CTA is a serial chain QK -> softmax -> PV, so two of them share an SM (96 KB of shared
-// memory, 256 TMEM columns each) and one's softmax runs under the other's MMAs.
+// memory, 256 TMEM columns each) and one's softmax runs under the other's MMAs. Weights as the A operand in TMEM and the rescale
+// that waits for a growth of 2^8 are published ideas of attention on this chip (T. Dao et al., FlashAttention-4, 2025).
 //
 // The softmax weights keep fp32 accuracy: P = hi + lo, both bf16, two products.
 //

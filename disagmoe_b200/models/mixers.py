@@ -102,7 +102,8 @@ class LatentTables:
         base = torch.from_numpy(np.repeat(at[:-1] - lo, ends - begins + 1).astype(np.int32))
         keys = torch.from_numpy(keys)
         up = lambda x: upload(x, device)
-        t = cls(len(rows), up(loose), up(rows), None, None, up(tiles), up(base), len(tiles), F.tile_reach(int(hi.max()), 128, m.window), up(keys), len(keys))
+        t = cls(len(rows), up(loose), up(rows), None, None, up(tiles), up(base), len(tiles),
+                F.tile_reach(int(hi.max()), 128, m.window), up(keys), len(keys))
         if len(rows):
             t.offs, t.recs = cls._per_head(rows, m.heads, device)
         return t

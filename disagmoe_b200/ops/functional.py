@@ -1009,13 +1009,15 @@ def latent_prefill(q: torch.Tensor, kv: torch.Tensor, lat: torch.Tensor, tiles: 
     """Causal attention of the prompt tokens named by ``tiles`` over expanded keys and values: kv [keys, heads x (key
     unrotated | value)], rotated key parts in the gathered cache rows ``lat`` [keys, row]; the key at position p of tile i's
     sequence is row base[i] + p. q: projection rows with rotated queries. Writes the tokens' rows of out [T, heads x vdimp], scaled by sigmoid(gate)
-    per head where ``gate`` [T, heads] is given. ``reach`` (:func:`tile_reach`), where the caller knows it, chooses between two kernels."""
+    per head where ``gate`` [T, heads] is given. ``reach`` (:func:`tile_reach`), where the caller knows it, chooses between two
+    kernels."""
     _check_sink(sink, lay.heads)
     assert gate is None or (gate.dtype == torch.bfloat16 and gate.stride(1) == 1)
     assert tiles.dtype == base.dtype == torch.int32 and kv.stride(1) == lat.stride(1) == 1
     # Measured on B200 (warm, mma.sync -> tcgen05), 16 heads: one prompt of 64 tokens 6.6 -> 9.9 us, 128: 9.0 -> 10.6, 192: 11.9 -> 13.4,
     # 256: 14.6 -> 13.9, 512: 25.8 -> 20.9; 16 prompts of 64 9.2 -> 20, of 128 20.4 -> 21.7, of 192 38 -> 46, of 256 56 -> 48.
-    if (reach is None or reach > 192) and (lay.dimp, lay.rotp, lay.vdimp) == (128, 64, 128) and all(t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (q, kv, lat, out)):
+    if (reach is None or reach > 192) and (lay.dimp, lay.rotp, lay.vdimp) == (128, 64, 128) and \
+            all(t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (q, kv, lat, out)):
         _lib.check(_lib.lib().dmoe_latent_prefill_tc(
             _vp(q), c_ll(q.stride(0)), _vp(kv), c_ll(kv.stride(0)), _vp(lat), c_ll(lat.stride(0)), c_ll(min(kv.shape[0], lat.shape[0])),
             _vp(tiles), _vp(base), c_int(n_tiles), c_int(lay.heads), c_int(lay.rankp), c_float(scale), c_int(window or 0), _vp(sink),

@@ -158,12 +158,12 @@ def want_wide(epi: int, T: int, F: int, K: int, G: int, sms: int) -> bool:
     """Should the tokens be the M operand (csrc/kernels/gemm_wide.cu, 256 x 256 tiles on CTA pairs) instead of the weights?
 
     Dense: a cost model of both, in us, fitted to a sweep on B200 (K 1024 .. 5632, F 256 .. 32000, T 8 .. 2048; the choice is within
-    8 % of the better of these two kernels, K below 1024 within 15 %). A wide tile takes 0.31 us per K block whatever part of it is used, the other kernel what
-    its SM pulls from L2. Measured (bf16, other kernel -> wide): 4096 x 6144 x 4096 201 -> 149 us (1381 TFLOP/s), 2500 x 4096 x
-    2048 106 -> 40, 1111 x 6144 x 2048 79 -> 31, 256 x 32000 x 4096 89 -> 58; SwiGLU 1024 x 5632 x 2048 59 -> 42. A few rows of SwiGLU
-    gain by the wider tile's faster K blocks (1 row, 2048 x 4096 38 -> 32, 16 rows, 8192 x 7168 82 -> 65), but pay 2 us more per launch
-    (1 row, 2048 x 256 11.2 -> 12.6, 4096 x 1024 17.4 -> 17.4), and more where the tiles of a wave want more than HBM gives (1 row,
-    8192 x 1024 17.4 -> 19.3, 8192 x 7168 69 -> 78; 8 rows, 8192 x 4096 47 -> 49).
+    8 % of the better of these two kernels, K below 1024 within 15 %). A wide tile takes 0.31 us per K block whatever part of it is
+    used, the other kernel what its SM pulls from L2. Measured (bf16, other kernel -> wide): 4096 x 6144 x 4096 201 -> 149 us (1381
+    TFLOP/s), 2500 x 4096 x 2048 106 -> 40, 1111 x 6144 x 2048 79 -> 31, 256 x 32000 x 4096 89 -> 58; SwiGLU 1024 x 5632 x 2048 59 ->
+    42. A few rows of SwiGLU gain by the wider tile's faster K blocks (1 row, 2048 x 4096 38 -> 32, 16 rows, 8192 x 7168 82 -> 65),
+    but pay 2 us more per launch (1 row, 2048 x 256 11.2 -> 12.6, 4096 x 1024 17.4 -> 17.4), and more where the tiles of a wave want
+    more than HBM gives (1 row, 8192 x 1024 17.4 -> 19.3, 8192 x 7168 69 -> 78; 8 rows, 8192 x 4096 47 -> 49).
 
     Grouped (only the mean group size is known): up to 128 tokens the other kernel's tile fits a group and streams the weights
     at HBM speed, beyond that it needs a second tile per group. Measured at 64 experts of 1408 x 2048, SwiGLU: 120 tokens each
@@ -171,8 +171,8 @@ def want_wide(epi: int, T: int, F: int, K: int, G: int, sms: int) -> bool:
     short K loops are bound by the other kernel's transposing epilogue at any size. Sweep over 8 .. 64 experts, F 2048 .. 6144, K 512
     .. 7168, 2 rows in all .. 140 per expert: with F K to 4.4 million 0.92 .. 1.9 times as fast, 1.17 on average (60 x (2048 x 1408):
     16 rows 46 -> 34, 148 rows 81 -> 70; 8 x (4096 x 1024): 74 rows 28 -> 25); above that a badly filled wave of long tiles can make it
-    0.8 times as fast with few experts (16 x (6144 x 2048): 24 rows 74 -> 88), while 60 and 64 experts still gain to K 2048 (0.96 .. 1.5; 60 x
-    (4096 x 2048): 64 rows 136 -> 131); from K 2816 on nothing is gained (8 x (4096 x 14336): 2 rows 47 -> 77, 128 rows 149 -> 181)."""
+    0.8 times as fast with few experts (16 x (6144 x 2048): 24 rows 74 -> 88), while 60 and 64 experts still gain to K 2048 (0.96 ..
+    1.5; 60 x (4096 x 2048): 64 rows 136 -> 131); from K 2816 on nothing is gained (8 x (4096 x 14336): 2 rows 47 -> 77, 128 rows 149 -> 181)."""
     kblocks, pairs = (K + 63) // 64, max(1, sms // 2)
     if G > 1:
         return T >= 144 * G or (epi != EPI_SWIGLU and K <= 2048 and (F * K <= 4_400_000 or G >= 60))
@@ -378,8 +378,8 @@ def linear(x: torch.Tensor, w: torch.Tensor, residual: Optional[torch.Tensor] = 
            out: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None, bn: int = 0,
            splitk: int = 0, comm: Optional["GemmComm"] = None, pair: bool = False, tanh: bool = False,
            silu_cols: int = 0, wide: Optional[bool] = None) -> torch.Tensor:
-    """y[T, F] = x[T, K] @ w[F, K].T (+ residual[T, F]); ``tanh``: of the product; ``silu_cols``: silu of the first so many columns. ``pair``: CTA pairs (tcgen05 cta_group::2) on tiles of 256
-    weight rows x ``bn`` (128 / 256) tokens, whole tiles."""
+    """y[T, F] = x[T, K] @ w[F, K].T (+ residual[T, F]); ``tanh``: of the product; ``silu_cols``: silu of the first so
+    many columns. ``pair``: CTA pairs (tcgen05 cta_group::2) on tiles of 256 weight rows x ``bn`` (128 / 256) tokens, whole tiles."""
     T, K = x.shape
     F = w.shape[0]
     if not x.is_cuda:
