@@ -14,13 +14,13 @@
 // LATENT: the same for prompt runs of latent attention over expanded keys and values (latent_attention.cu has the layout): a
 // tile is 128 tokens of one head, a key is 128 numbers of its expanded row and the 64 rotated ones of its cache row, and the
 // keys of a sequence are consecutive rows, so that a box holds 128 of them. With 128 KB of shared memory one CTA fits an SM.
-// Measured on B200: 3000 tokens of 16 heads, window 1024, 166 us with mma.sync, 71 us here.
+// Measured on B200 (1965 MHz), mma.sync -> here: 3000 tokens of 16 heads, window 1024, 199 -> 94 us; 4096 without, 604 -> 215 us.
 //
-// Measured on B200 against the mma.sync kernel of attention.cu (64 rows per CTA, every warp re-reading all of K and V from shared
-// memory): 4096 tokens of 16 heads, window 1024, soft cap 362 -> 130 us; 3000 tokens, sinks 293 -> 76 us. That kernel stays for
-// other head sizes, page sizes that do not divide 128 keys, unaligned rows, and for attention without options, whose weights are
-// rounded to bf16 relative to a running maximum per 64 keys: another order of blocks rounds them differently, and decoders with
-// few large experts then choose other experts for nearly tied rows.
+// Measured on B200 (1965 MHz) against the mma.sync kernel of attention.cu (64 rows per CTA, every warp re-reading all of K and V
+// from shared memory): 4096 tokens of 16 heads, window 1024, soft cap 371 -> 137 us; 3000 tokens, sinks 432 -> 111 us. That kernel
+// stays for other head sizes, page sizes that do not divide 128 keys, unaligned rows, prompts of few keys, and for attention without
+// options, whose weights are rounded to bf16 relative to a running maximum per 64 keys: another order of blocks rounds them
+// differently, and decoders with few large experts then choose other experts for nearly tied rows.
 #include <string.h>
 
 #include "attn_common.cuh"
