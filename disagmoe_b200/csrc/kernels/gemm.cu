@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const GemmArgs a) {
   using C = Cfg<BN, EPI, PAIR>;
   // pair mode: rank of this CTA in its pair (the even CTA issues the MMAs), work is dealt out per pair
-  const uint32_t prank = PAIR ? cluster_ctarank() : 0u;
+  const uint32_t prank = PAIR ? __shfl_sync(0xffffffffu, cluster_ctarank(), 0) : 0u;
   const bool leader = prank == 0;
   const int work_cta = PAIR ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
   const int work_grid = PAIR ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
@@ -181,7 +181,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUt
   float* epi_stage = reinterpret_cast<float*>(tail + kTailBytes);    // [32][kBM] (plain epilogue only)
   const int S = (a.S > 0 && !a.group_regions) ? a.S : 1;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform_warp();
   const int lane = threadIdx.x & 31;
   const int MT1 = (a.F + kBM - 1) / kBM;              // 128-row weight tiles
   const int MT = PAIR ? (MT1 + 1) / 2 : MT1;          // work tiles along M (pairs of them in pair mode)
@@ -265,62 +265,67 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUt
   __syncthreads();
   if (PAIR) cluster_sync_all();      // both CTAs' barriers are initialised before either is signalled from outside
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   if (threadIdx.x == 0) trace_stamp(a, 1);
 
+  // Warps 0 and 1 run converged, with values that are uniform for the compiler; only the copies, MMAs and commits are left to an
+  // elected lane (sm100.cuh: elect_one says why).
+  const auto uni = [](int x) { return __shfl_sync(0xffffffffu, x, 0); };
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      WorkWalker tw;
-      if (a.dense.units > 0) tw.init_dense(a.dense, a.T, BN, kblocks, a.splitk, work_cta);
-      else tw.init(s_start, s_cnt, a.G, S, MT, BN, kblocks, a.splitk, a.streamk, work_cta, work_grid);
-      trace_stamp(a, 13);
-      if (a.n_wait > 0) asm volatile("fence.proxy.async;" ::: "memory");  // peers' generic stores -> TMA reads
-      const uint64_t pol_w = l2_policy_evict_first();
-      const uint64_t pol_x = l2_policy_evict_last();
-      trace_stamp(a, 14);
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      bool traced = false;
-      unsigned long long shard_ready = 0;     // bit s: shard s of X has landed (all-gather prologue)
-      const int shard_want = (a.shard_rows > 0) ? *a.wait_epoch + 1 : 0;
-      WorkUnit u;
-      while (ok && tw.next(u)) {
-        const int ntok_ = u.ntok;
-        // pair mode: this CTA stages the token rows of its half of the MMA's N extent (the even CTA the first half)
-        int n_eff = (u.ntok + 31) & ~31;
-        n_eff = n_eff > BN ? BN : n_eff;
-        const int xrow = u.row0 + (PAIR ? static_cast<int>(prank) * (n_eff / 2) : 0);
-        const int wrow = u.g * a.w_rows + (PAIR ? 2 * u.m + static_cast<int>(prank) : u.m) * kBM;
-        const int kb0 = u.kb0, kb1 = u.kb1;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(smem_u32(&empty_bar[stage]), phase ^ 1, abort_word, bar_budget)) { ok = false; break; }
-          if (a.trace != nullptr && !traced) trace_stamp(a, 15);
-          // pair mode: the bytes of both CTAs are counted on the even CTA's barrier, which its producer arms
-          const uint32_t fb = PAIR ? mapa_rank(smem_u32(&full_bar[stage]), 0) : smem_u32(&full_bar[stage]);
-          uint8_t* st = smem + stage * C::kStageBytes;
+    WorkWalker tw;
+    if (a.dense.units > 0) tw.init_dense(a.dense, a.T, BN, kblocks, a.splitk, work_cta);
+    else tw.init(s_start, s_cnt, a.G, S, MT, BN, kblocks, a.splitk, a.streamk, work_cta, work_grid);
+    if (lane == 0) trace_stamp(a, 13);
+    if (a.n_wait > 0) asm volatile("fence.proxy.async;" ::: "memory");  // peers' generic stores -> TMA reads
+    const uint64_t pol_w = l2_policy_evict_first();
+    const uint64_t pol_x = l2_policy_evict_last();
+    if (lane == 0) trace_stamp(a, 14);
+    // pair mode: the bytes of both CTAs are counted on the even CTA's barriers, which its producer arms
+    const uint32_t full0 = PAIR ? uni(mapa_rank(smem_u32(full_bar), 0)) : smem_u32(full_bar);
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    bool traced = false;
+    unsigned long long shard_ready = 0;     // bit s: shard s of X has landed (all-gather prologue)
+    const int shard_want = (a.shard_rows > 0) ? *a.wait_epoch + 1 : 0;
+    WorkUnit u;
+    while (ok && tw.next(u)) {
+      // pair mode: this CTA stages the token rows of its half of the MMA's N extent (the even CTA the first half)
+      int n_eff = (u.ntok + 31) & ~31;
+      n_eff = n_eff > BN ? BN : n_eff;
+      const int xrow = uni(u.row0 + (PAIR ? static_cast<int>(prank) * (n_eff / 2) : 0));
+      const int wrow = uni(u.g * a.w_rows + (PAIR ? 2 * u.m + static_cast<int>(prank) : u.m) * kBM);
+      const int kb0 = uni(u.kb0), kb1 = uni(u.kb1);
+      for (int kb = kb0; kb < kb1; ++kb) {
+        ok = mbar_wait_warp(smem_u32(&empty_bar[stage]), phase ^ 1, abort_word, bar_budget);
+        if (!ok) break;
+        if (a.trace != nullptr && !traced && lane == 0) trace_stamp(a, 15);
+        const uint32_t fb = full0 + 8 * stage, st = smem_u32(smem) + stage * C::kStageBytes;
+        const auto load = [&](uint32_t dst, const CUtensorMap* m, int x, int y, uint64_t pol) {
+          if (PAIR) tma_load_2d_pair(dst, m, x, y, fb, pol);
+          else tma_load_2d(dst, m, x, y, fb, pol);
+        };
+        // blocked weights: the map is a [tiles * K blocks * 128, 64] matrix, tile (t, kb) starts at row (t * kblocks + kb) * 128
+        const int x = a.w_blocked ? 0 : kb * kBK;
+        const int y = a.w_blocked ? (wrow / kBM * kblocks + kb) * kBM : wrow;
+        const bool gated = a.shard_rows > 0 && kb == kb0;
+        if (elect_one()) {
           if (!PAIR) mbar_expect_tx(fb, C::kStageBytes);
           else if (leader) mbar_expect_tx(smem_u32(&full_bar[stage]), 2 * C::kStageBytes);
-          auto load = [&](uint32_t dst, const CUtensorMap* m, int x, int y, uint64_t pol) {
-            if (PAIR) tma_load_2d_pair(dst, m, x, y, fb, pol);
-            else tma_load_2d(dst, m, x, y, fb, pol);
-          };
-          if (a.w_blocked) {
-            // blocked weights: the map is a [tiles * K blocks * 128, 64] matrix, tile (t, kb) starts at row (t * kblocks + kb) * 128
-            const int wt = wrow / kBM;
-            load(smem_u32(st), &tmW, 0, (wt * kblocks + kb) * kBM, pol_w);
-            if (EPI == EPI_SWIGLU) load(smem_u32(st + C::kABytes), &tmW, 0, ((wt + a.F / kBM) * kblocks + kb) * kBM, pol_w);
-          } else {
-            load(smem_u32(st), &tmW, kb * kBK, wrow, pol_w);
-            if (EPI == EPI_SWIGLU) load(smem_u32(st + C::kABytes), &tmW, kb * kBK, wrow + a.F, pol_w);
-          }
-          if (a.shard_rows > 0 && kb == kb0) {
-            // the weight tile is already on its way; the token tile may only be fetched once every peer whose rows
-            // it covers has published them (the peers' stores are generic-proxy writes: fence before the TMA read)
+          load(st, &tmW, x, y, pol_w);
+          if (EPI == EPI_SWIGLU) load(st + C::kABytes, &tmW, x, a.w_blocked ? y + a.F / kBM * kblocks * kBM : y + a.F, pol_w);
+          if (!gated) load(st + C::kNumA * C::kABytes, &tmX, kb * kBK, xrow, pol_x);
+        }
+        __syncwarp();
+        if (gated) {
+          // the weight tile is already on its way; the token tile may only be fetched once every peer whose rows
+          // it covers has published them (the peers' stores are generic-proxy writes: fence before the TMA read)
+          int landed = 1;
+          if (lane == 0) {
             const int s0 = u.row0 / a.shard_rows;
-            const int s1 = min((u.row0 + ntok_ - 1) / a.shard_rows, a.n_wait - 1);
-            for (int sh = s0; sh <= s1 && ok; ++sh) {
+            const int s1 = min((u.row0 + u.ntok - 1) / a.shard_rows, a.n_wait - 1);
+            for (int sh = s0; sh <= s1 && landed; ++sh) {
               if ((shard_ready >> sh) & 1ull) continue;
               const long long t0 = clock64();
               while (ld_acquire_sys(a.wait_flags + sh) < shard_want) {
@@ -328,27 +333,31 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUt
                     (a.status != nullptr && *reinterpret_cast<volatile int*>(a.status) != kStatusOk)) {
                   if (a.status != nullptr) atomicCAS(a.status, kStatusOk, kStatusFlagTimeout);
                   *abort_word = 1;
-                  ok = false;
+                  landed = 0;
                   break;
                 }
                 __nanosleep(64);
               }
-              if (ok) {
-                shard_ready |= 1ull << sh;
-                asm volatile("fence.proxy.async;" ::: "memory");
-              }
+              if (landed) shard_ready |= 1ull << sh;
             }
-            if (!ok) break;
           }
-          load(smem_u32(st + C::kNumA * C::kABytes), &tmX, kb * kBK, xrow, pol_x);
-          if (a.trace != nullptr && !traced) { trace_stamp(a, 2); traced = true; }
-          if (++stage == C::kStages) { stage = 0; phase ^= 1; }
+          ok = uni(landed) != 0;
+          if (!ok) break;
+          __syncwarp();
+          asm volatile("fence.proxy.async;" ::: "memory");
+          if (elect_one()) load(st + C::kNumA * C::kABytes, &tmX, kb * kBK, xrow, pol_x);
+          __syncwarp();
         }
+        if (a.trace != nullptr && !traced) {
+          if (lane == 0) trace_stamp(a, 2);
+          traced = true;
+        }
+        if (++stage == C::kStages) { stage = 0; phase ^= 1; }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (pair mode: the even CTA's only)
-    if (lane == 0 && leader) {
+    if (leader) {
       WorkWalker tw;
       if (a.dense.units > 0) tw.init_dense(a.dense, a.T, BN, kblocks, a.splitk, work_cta);
       else tw.init(s_start, s_cnt, a.G, S, MT, BN, kblocks, a.splitk, a.streamk, work_cta, work_grid);
@@ -360,53 +369,52 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUt
       for (; ok && tw.next(u); ++it) {
         const int buf = it % C::kAccBufs;
         const uint32_t bphase = (it / C::kAccBufs) & 1;
-        if (PAIR) {
-          if (!mbar_wait_cluster(smem_u32(&tempty_bar[buf]), bphase ^ 1, abort_word, bar_budget)) { ok = false; break; }
-        } else if (!mbar_wait(smem_u32(&tempty_bar[buf]), bphase ^ 1, abort_word, bar_budget)) { ok = false; break; }
+        ok = __all_sync(0xffffffffu, PAIR ? mbar_wait_cluster(smem_u32(&tempty_bar[buf]), bphase ^ 1, abort_word, bar_budget)
+                                          : mbar_wait(smem_u32(&tempty_bar[buf]), bphase ^ 1, abort_word, bar_budget));
+        if (!ok) break;
         tc_fence_after();
         const uint32_t d0 = tmem_base + buf * C::kAccCols;
         // a ragged token tile only pays for the MMA columns it has (N is a run-time field of the instruction)
         const int nq = PAIR ? 32 : 16;
-        int n_eff = (u.ntok + nq - 1) & ~(nq - 1);
+        int n_eff = (uni(u.ntok) + nq - 1) & ~(nq - 1);
         n_eff = n_eff < nq ? nq : (n_eff > BN ? BN : n_eff);
         const uint32_t idesc = umma_idesc_bf16(PAIR ? 2 * kBM : kBM, n_eff);
-        const int kb0 = u.kb0, kb1 = u.kb1;
+        const int kb0 = uni(u.kb0), kb1 = uni(u.kb1);
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(smem_u32(&full_bar[stage]), phase, abort_word, bar_budget)) { ok = false; break; }
-          if (a.trace != nullptr && it == 0 && kb == kb0) trace_stamp(a, 3);
+          ok = mbar_wait_warp(smem_u32(&full_bar[stage]), phase, abort_word, bar_budget);
+          if (!ok) break;
+          if (a.trace != nullptr && it == 0 && kb == kb0 && lane == 0) trace_stamp(a, 3);
           tc_fence_after();
-          const uint32_t sa = smem_u32(smem + stage * C::kStageBytes);
-          const uint64_t da = umma_desc_sw128(sa);
-          const uint64_t db = umma_desc_sw128(sa + C::kNumA * C::kABytes);
+          const uint32_t sa = smem_u32(smem) + stage * C::kStageBytes;
+          if (elect_one()) {
+            const uint64_t da = umma_desc_sw128(sa);
+            const uint64_t db = umma_desc_sw128(sa + C::kNumA * C::kABytes);
 #pragma unroll
-          for (int k = 0; k < kBK / kUmmaK; ++k) {
-            const uint32_t acc = (kb > kb0 || k > 0) ? 1u : 0u;
-            // advancing K by 16 bf16 = 32 bytes inside the 128-byte swizzle span: +2 in the (>>4) address field
-            if (PAIR) umma_f16_pair(d0, da + 2 * k, db + 2 * k, idesc, acc);
-            else umma_f16(d0, da + 2 * k, db + 2 * k, idesc, acc);
-            if (EPI == EPI_SWIGLU) {
-              const uint64_t da2 = umma_desc_sw128(sa + C::kABytes);
-              if (PAIR) umma_f16_pair(d0 + BN, da2 + 2 * k, db + 2 * k, idesc, acc);
-              else umma_f16(d0 + BN, da2 + 2 * k, db + 2 * k, idesc, acc);
+            for (int k = 0; k < kBK / kUmmaK; ++k) {
+              const uint32_t acc = (kb > kb0 || k > 0) ? 1u : 0u;
+              // advancing K by 16 bf16 = 32 bytes inside the 128-byte swizzle span: +2 in the (>>4) address field
+              if (PAIR) umma_f16_pair(d0, da + 2 * k, db + 2 * k, idesc, acc);
+              else umma_f16(d0, da + 2 * k, db + 2 * k, idesc, acc);
+              if (EPI == EPI_SWIGLU) {
+                const uint64_t da2 = umma_desc_sw128(sa + C::kABytes);
+                if (PAIR) umma_f16_pair(d0 + BN, da2 + 2 * k, db + 2 * k, idesc, acc);
+                else umma_f16(d0 + BN, da2 + 2 * k, db + 2 * k, idesc, acc);
+              }
             }
+            // frees the smem stage when these MMAs retire (pair mode: in both CTAs, one arrival each)
+            if (PAIR) umma_commit_both(smem_u32(&empty_bar[stage]));
+            else umma_commit(smem_u32(&empty_bar[stage]));
           }
-          // frees the smem stage when these MMAs retire (pair mode: in both CTAs, one arrival each)
-          if (PAIR) {
-            umma_commit_pair(mapa_rank(smem_u32(&empty_bar[stage]), 0));
-            umma_commit_pair(mapa_rank(smem_u32(&empty_bar[stage]), 1));
-          } else {
-            umma_commit(smem_u32(&empty_bar[stage]));
-          }
+          __syncwarp();
           if (++stage == C::kStages) { stage = 0; phase ^= 1; }
         }
         if (ok) {
-          if (PAIR) {
-            umma_commit_pair(mapa_rank(smem_u32(&tfull_bar[buf]), 0));
-            umma_commit_pair(mapa_rank(smem_u32(&tfull_bar[buf]), 1));
-          } else {
-            umma_commit(smem_u32(&tfull_bar[buf]));
-            trace_stamp(a, 4);
+          if (elect_one()) {
+            if (PAIR) umma_commit_both(smem_u32(&tfull_bar[buf]));
+            else umma_commit(smem_u32(&tfull_bar[buf]));
           }
+          __syncwarp();
+          if (!PAIR && lane == 0) trace_stamp(a, 4);
         }
       }
     }

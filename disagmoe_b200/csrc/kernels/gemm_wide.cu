@@ -4,7 +4,8 @@
 // that layout is bound by what an SM can pull from L2 (~58 of 64 bytes per clock): a 128 x 256 tile of one CTA stages 48 KB
 // per 512 tensor cycles, and every output chunk has to be transposed through shared memory. Here a cluster of two CTAs
 // computes a tile of 256 tokens x 256 weight rows with tcgen05.mma.cta_group::2: each CTA stages its own 128 token rows and
-// HALF of the weight rows (32 KB per 512 tensor cycles, six stages), and a TMEM lane is a token, so an epilogue thread owns
+// HALF of the weight rows (32 KB per 512 tensor cycles, three stages of two K blocks: a round of the issuing warp
+// takes about 400 cycles, and was what bounded a K block when every block had a round of its own), and a TMEM lane is a token, so an epilogue thread owns
 // consecutive features of one output row: no transposition, no barrier between the epilogue warps. For SwiGLU the even CTA
 // stages 128 gate rows and the odd one the matching 128 up rows; gate and up of a feature then sit 128 TMEM columns apart
 // in the same lane.
@@ -24,9 +25,11 @@ namespace dmoe {
 constexpr int kWThreads = 192;
 constexpr int kWTokens = 2 * kBM;                        // tokens per tile
 constexpr int kWCols = 256;                              // accumulator columns = weight rows per tile
-constexpr int kWStages = 6;
+constexpr int kWSub = 2;                                 // K blocks per stage
+constexpr int kWStages = 3;
 constexpr int kWOperandBytes = kBM * kBK * 2;            // 128 rows x 64 bf16: one CTA's tokens or its half of the weights
-constexpr int kWStageBytes = 2 * kWOperandBytes;
+constexpr int kWSubBytes = 2 * kWOperandBytes;           // tokens, then weights of one K block
+constexpr int kWStageBytes = kWSub * kWSubBytes;
 constexpr int kWBarBytes = 256;
 constexpr int kWSmemBytes = kWStages * kWStageBytes + 1024 /*alignment slack*/ + kWBarBytes + (2 * kMaxGroups + 1) * 4;
 
@@ -98,9 +101,9 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   int* s_start = reinterpret_cast<int*>(smem + kWStages * kWStageBytes + kWBarBytes);      // [G] first row
   int* s_tile0 = s_start + kMaxGroups;                                                     // [G + 1] first tile
 
-  const uint32_t prank = cluster_ctarank();
+  const int prank = __shfl_sync(0xffffffffu, static_cast<int>(cluster_ctarank()), 0);
   const bool leader = prank == 0;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   constexpr int kFeat = EPI == EPI_SWIGLU ? kWCols / 2 : kWCols;      // output features per tile
   const int NT = (a.F + kFeat - 1) / kFeat;
@@ -159,67 +162,86 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   __syncthreads();
   cluster_sync_all();      // both CTAs' barriers are initialised before either is signalled from outside
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   WideTile u;
   u.g = 0;
   // the rows of a group end where the next one starts; the last one ends at T, or where offs says
   const int t_end = a.offs != nullptr ? a.offs[a.G] : a.T;
 
+  const int steps = (kblocks + kWSub - 1) / kWSub;
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      const uint64_t pol_first = l2_policy_evict_first(), pol_last = l2_policy_evict_last();
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int tile = pair; ok && u.locate(tile, s_start, s_tile0, a.G, NT, t_end); tile += pairs) {
-        const bool both = u.ntok > kBM;             // the odd CTA has token rows of its own
-        const bool mine = leader || both;
-        // a weight tile that one token tile reads streams through L2, one that several read stays
-        const uint64_t pol_w = s_tile0[u.g + 1] - s_tile0[u.g] == NT ? pol_first : pol_last;
-        const int xrow = u.row0 + static_cast<int>(prank) * kBM;
-        const int wrow = u.g * a.w_rows + (EPI == EPI_SWIGLU ? u.n * kFeat + static_cast<int>(prank) * a.F
-                                                             : u.n * kFeat + static_cast<int>(prank) * kBM);
-        for (int kb = 0; kb < kblocks; ++kb) {
-          if (!mbar_wait(smem_u32(&empty_bar[stage]), phase ^ 1, abort_word)) { ok = false; break; }
-          // the bytes of both CTAs are counted on the even CTA's barrier, which its producer arms
-          const uint32_t fb = mapa_rank(smem_u32(&full_bar[stage]), 0);
-          if (leader) mbar_expect_tx(smem_u32(&full_bar[stage]), (both ? 4 : 3) * kWOperandBytes);
-          const uint32_t st = smem_u32(smem + stage * kWStageBytes);
-          if (a.w_blocked) tma_load_2d_pair(st + kWOperandBytes, &tmW, 0, (wrow / kBM * kblocks + kb) * kBM, fb, pol_w);
-          else tma_load_2d_pair(st + kWOperandBytes, &tmW, kb * kBK, wrow, fb, pol_w);
-          if (mine) tma_load_2d_pair(st, &tmX, kb * kBK, xrow, fb, pol_last);
-          if (++stage == kWStages) { stage = 0; phase ^= 1; }
+    const uint64_t pol_first = l2_policy_evict_first(), pol_last = l2_policy_evict_last();
+    // the bytes of both CTAs are counted on the even CTA's barriers, which its producer arms
+    const uint32_t full0 = __shfl_sync(0xffffffffu, mapa_rank(smem_u32(full_bar), 0), 0);
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int tile = pair; ok && u.locate(tile, s_start, s_tile0, a.G, NT, t_end); tile += pairs) {
+      const bool both = __shfl_sync(0xffffffffu, u.ntok, 0) > kBM;             // the odd CTA has token rows of its own
+      const bool mine = leader || both;
+      // a weight tile that one token tile reads streams through L2, one that several read stays
+      const bool once = __shfl_sync(0xffffffffu, s_tile0[u.g + 1] - s_tile0[u.g], 0) == NT;
+      const int xrow = __shfl_sync(0xffffffffu, u.row0, 0) + prank * kBM;
+      const int wrow = __shfl_sync(0xffffffffu, u.g * a.w_rows + u.n * kFeat, 0) + prank * (EPI == EPI_SWIGLU ? a.F : kBM);
+      for (int i = 0; i < steps; ++i) {
+        ok = mbar_wait_warp(smem_u32(&empty_bar[stage]), phase ^ 1, abort_word);
+        if (!ok) break;
+        const uint32_t fb = full0 + 8 * stage, st = smem_u32(smem) + stage * kWStageBytes;
+        const int kb = i * kWSub, n = min(kWSub, kblocks - kb);
+        if (elect_one()) {
+          if (leader) mbar_expect_tx(smem_u32(&full_bar[stage]), n * (both ? 4 : 3) * kWOperandBytes);
+#pragma unroll
+          for (int j = 0; j < kWSub; ++j) {
+            if (j < n) {
+              const uint32_t sx = st + j * kWSubBytes;
+              const int x = a.w_blocked ? 0 : (kb + j) * kBK, y = a.w_blocked ? (wrow / kBM * kblocks + kb + j) * kBM : wrow;
+              tma_load_2d_pair(sx + kWOperandBytes, &tmW, x, y, fb, once ? pol_first : pol_last);
+              if (mine) tma_load_2d_pair(sx, &tmX, (kb + j) * kBK, xrow, fb, pol_last);
+            }
+          }
         }
+        __syncwarp();
+        if (++stage == kWStages) { stage = 0; phase ^= 1; }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (the even CTA's)
-    if (lane == 0 && leader) {
+    if (leader) {
       constexpr uint32_t idesc = umma_idesc_bf16(2 * kBM, kWCols);
+      const int tiles = __shfl_sync(0xffffffffu, s_tile0[a.G], 0);
       int stage = 0, it = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int tile = pair; ok && tile < s_tile0[a.G]; tile += pairs, ++it) {
+      for (int tile = pair; ok && tile < tiles; tile += pairs, ++it) {
         const int buf = it & 1;
-        if (!mbar_wait_cluster(smem_u32(&tempty_bar[buf]), ((it >> 1) & 1) ^ 1, abort_word, DMOE_WAIT_CYCLES)) break;
+        ok = __all_sync(0xffffffffu, mbar_wait_cluster(smem_u32(&tempty_bar[buf]), ((it >> 1) & 1) ^ 1, abort_word, DMOE_WAIT_CYCLES));
+        if (!ok) break;
         tc_fence_after();
         const uint32_t d0 = tmem_base + buf * kWCols;
-        for (int kb = 0; kb < kblocks; ++kb) {
-          if (!mbar_wait(smem_u32(&full_bar[stage]), phase, abort_word)) { ok = false; break; }
+        for (int i = 0; i < steps; ++i) {
+          ok = mbar_wait_warp(smem_u32(&full_bar[stage]), phase, abort_word);
+          if (!ok) break;
           tc_fence_after();
-          const uint32_t st = smem_u32(smem + stage * kWStageBytes);
-          const uint64_t da = umma_desc_sw128(st), db = umma_desc_sw128(st + kWOperandBytes);
+          const uint32_t st = smem_u32(smem) + stage * kWStageBytes;
+          const int n = min(kWSub, kblocks - i * kWSub);
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < kBK / kUmmaK; ++k) umma_f16_pair(d0, da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-          umma_commit_pair(mapa_rank(smem_u32(&empty_bar[stage]), 0));
-          umma_commit_pair(mapa_rank(smem_u32(&empty_bar[stage]), 1));
+            for (int j = 0; j < kWSub; ++j) {
+              if (j < n) {
+                const uint64_t da = umma_desc_sw128(st + j * kWSubBytes), db = umma_desc_sw128(st + j * kWSubBytes + kWOperandBytes);
+#pragma unroll
+                for (int k = 0; k < kBK / kUmmaK; ++k)
+                  umma_f16_pair(d0, da + 2 * k, db + 2 * k, idesc, (i > 0 || j > 0 || k > 0) ? 1u : 0u);
+              }
+            }
+            umma_commit_both(smem_u32(&empty_bar[stage]));
+          }
+          __syncwarp();
           if (++stage == kWStages) { stage = 0; phase ^= 1; }
         }
-        if (ok) {
-          umma_commit_pair(mapa_rank(smem_u32(&tfull_bar[buf]), 0));
-          umma_commit_pair(mapa_rank(smem_u32(&tfull_bar[buf]), 1));
-        }
+        if (ok && elect_one()) umma_commit_both(smem_u32(&tfull_bar[buf]));
+        __syncwarp();
       }
     }
   } else {
@@ -231,7 +253,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       if (!mbar_wait(smem_u32(&tfull_bar[buf]), (it >> 1) & 1, abort_word)) break;
       tc_fence_after();
       const uint32_t t0 = tmem_base + buf * kWCols + (static_cast<uint32_t>(q * 32) << 16);
-      const int first = static_cast<int>(prank) * kBM + q * 32;      // first token of this warp inside the tile
+      const int first = prank * kBM + q * 32;      // first token of this warp inside the tile
       const bool ok_row = first + lane < u.ntok;
       const long long t = u.row0 + first + lane;
       const int f0 = u.n * kFeat;

@@ -78,6 +78,21 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   }
 }
 
+// One lane of a converged warp. The instructions that TMA, tcgen05.mma and tcgen05.commit compile to take their addresses and
+// descriptors from uniform registers. Code that the whole warp runs with values the compiler knows to be equal in all lanes, and
+// in which only those instructions are left to an elected lane, has them there; inside `if (lane == 0)` each is made uniform
+// first: 640 cycles per round of wait, four MMAs and commit instead of 405.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0); }
+// mbar_wait of a whole warp: the same answer in every lane
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_word, long long budget = DMOE_WAIT_CYCLES) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_word, budget));
+}
+
 // Flag store of a release pattern: the caller has executed a system-scope fence (__threadfence_system) after the data
 // writes; the flags themselves then go out as relaxed system-scope stores, so that signalling n destinations costs one
 // fence and n independent stores instead of n fence + store pairs in a row (st.release implies a fence each time).
@@ -213,6 +228,8 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
   return r;
 }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+// without the release (0.3 us), for what is ordered by other means
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -282,10 +299,12 @@ __device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t desc_a, 
       "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// One arrival on `bar_cluster` (a shared::cluster address: this CTA's barrier or the other CTA's) when every
-// tcgen05.mma issued so far by this thread has finished in both CTAs.
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar_cluster) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_cluster) : "memory");
+// One arrival on the barrier at this shared-memory offset in each CTA of the pair when every tcgen05.mma issued so far by this
+// thread has finished in both.
+__device__ __forceinline__ void umma_commit_both(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+               "h"(static_cast<uint16_t>(3))
+               : "memory");
 }
 
 // Shared-memory matrix descriptor for a K-major bf16 tile stored as rows of 128 bytes with the 128-byte
