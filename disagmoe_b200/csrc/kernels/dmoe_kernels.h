@@ -169,6 +169,10 @@ typedef struct DmoeGemm {
   // allows it: no multi-GPU hooks, splitk <= 1, no pair, 16-byte aligned output rows; other launches ignore it. bn, streamk,
   // ws and counters are unused then.
   int wide;
+  // > 0: one tile of 128 weight rows x bn tokens (any multiple of 16 up to 256) per cluster of `cluster` CTAs (1 .. 8) that share
+  // K (gemm_split.cu) where the launch qualifies as above, is dense, plain or SwiGLU, and its weights are row-major; otherwise the
+  // launch picks a token tile of its own
+  int cluster;
 } DmoeGemm;
 
 int dmoe_gemm(const DmoeGemm* desc, void* stream);

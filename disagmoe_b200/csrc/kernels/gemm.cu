@@ -925,7 +925,7 @@ extern "C" int dmoe_gemm(const DmoeGemm* d, void* stream_) {
   if (d->G < 1 || d->G > kMaxSeg || d->K % 8 != 0 || d->F < 1 || d->T < 0) return -10;
   if (d->T == 0) return 0;
   const int epi = d->epi;
-  int bn = d->bn;
+  int bn = d->cluster > 0 ? 0 : d->bn;
   if (bn == 0) bn = dmoe_gemm_pick_bn((d->T + d->G - 1) / d->G, epi);
   if (bn != 32 && bn != 64 && bn != 128 && bn != 256) return -11;
   const bool pair = d->pair != 0;
@@ -1001,6 +1001,9 @@ extern "C" int dmoe_gemm(const DmoeGemm* d, void* stream_) {
   if (d->wide != 0 && alone && a.epi_vec && d->seg_cnt == nullptr && (!d->w_blocked || (d->K % kBK == 0 && d->F % kBM == 0 &&
       static_cast<long long>(d->G) * a.w_rows * (d->K / kBK) < (1ll << 31))))
     return gemm_wide(d, stream);
+  if (d->cluster > 0 && alone && a.epi_vec && d->seg_cnt == nullptr && !d->w_blocked && d->G == 1 && d->offs == nullptr &&
+      d->recs == nullptr && epi != EPI_COMBINE)
+    return gemm_split(d, stream);
 
   CUtensorMap tmW, tmX;
   const long long ldx = d->ldx > 0 ? d->ldx : d->K;

@@ -92,5 +92,7 @@ inline int make_map_2d(CUtensorMap* map, const void* ptr, long long rows, long l
 
 // gemm_wide.cu: the same product with the tokens as the M operand (see there). Checks have been made by dmoe_gemm.
 int gemm_wide(const DmoeGemm* d, cudaStream_t stream);
+// gemm_split.cu: dense launches of one wave, K cut over a cluster. Checks as above, but for the token tile.
+int gemm_split(const DmoeGemm* d, cudaStream_t stream);
 
 }  // namespace dmoe

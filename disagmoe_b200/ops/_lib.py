@@ -41,6 +41,7 @@ class DmoeGemm(ctypes.Structure):
         ("combine_vec", ctypes.c_int), ("w_blocked", ctypes.c_int), ("act", ctypes.c_int),
         ("trace", ctypes.c_void_p),
         ("act_limit", ctypes.c_float), ("act_cols", ctypes.c_int), ("unit_weights", ctypes.c_int), ("wide", ctypes.c_int),
+        ("cluster", ctypes.c_int),
     ]
 
 

@@ -190,6 +190,82 @@ def want_wide(epi: int, T: int, F: int, K: int, G: int, sms: int) -> bool:
     return units >= sms or wide < 1.4 + dense_cost(T, F, K, sms)[0]
 
 
+def dense_wide_cost(T: int, F: int, K: int, epi: int, sms: int) -> float:
+    """us of a dense product in csrc/kernels/gemm_wide.cu, fitted to the sweep of :func:`split_plan` (within 6 % on average)."""
+    feat = 128 if epi == EPI_SWIGLU else 256
+    waves = -(-(-(-F // feat) * -(-T // 256)) // max(1, sms // 2))
+    return 2.7 + waves * (4.3 + 0.31 * -(-K // 64))
+
+
+# CTAs of csrc/kernels/gemm_split.cu that a B200 holds at once in clusters of 1 .. 8, with the small amount of shared memory (two per
+# SM) and the large one; fewer than two per SM and one, because a cluster stays inside a group of SMs
+_SPLIT_SMALL = (296, 296, 279, 284, 280, 270, 259, 264)
+_SPLIT_LARGE = (148, 148, 135, 132, 130, 132, 105, 120)
+
+
+def split_plan(T: int, F: int, K: int, epi: int, sms: int):
+    """(cost in us, token tile, CTAs per cluster) of a dense product in csrc/kernels/gemm_split.cu, or None where other kernels are
+    faster: all its CTAs have to find place at once, or it has one tile of up to 64 tokens and the weights stream through it (an LM
+    head).
+
+    The cost model is fitted to a sweep on B200 (T 1 .. 4096, F 16 .. 151936, K 16 .. 14336; launches back to back, weights from HBM); its
+    choice is 2.8 % slower than the best tile and cluster on average. Measured, this module's other kernels -> the choice, us: 1 x 4096 x
+    4096 13.9 -> 9.7, 37 x 2048 x 2048 10.3 -> 6.6, 37 x 6144 x 2048 14.6 -> 9.6, 37 x 2048 x 5632 14.1 -> 9.1, SwiGLU 37 x 5632 x 2048 17.7
+    -> 11.8, 96 x 2048 x 10944 22.6 -> 14.5, 256 x 4096 x 4096 22.0 -> 16.0, 576 x 2048 x 5632 29.4 -> 22.0, 1111 x 2048 x 2048 17.8 -> 14.7, 3
+    x 32000 x 4096 54.1 -> 42.4, 37 x 151936 x 2048 111 -> 104. A second wave costs as much as the first: 96 x 10944 x 2048 SwiGLU (171
+    CTAs of one per SM) 22.6 -> 26.3, 1111 x 2816 x 2048 SwiGLU 28.6 -> 36.4, 192 x 32000 x 2048 32.5 -> 42.5.
+
+    Sizes are rounded up to a grid of tokens, so that few plans serve prompts of all lengths."""
+    grid = 16 if T <= 256 else 32 if T <= 1024 else 64
+    return _split_plan(-(-T // grid) * grid, F, K, epi, sms)
+
+
+@lru_cache(maxsize=4096)
+def _split_plan(T: int, F: int, K: int, epi: int, sms: int):
+    gate = epi == EPI_SWIGLU
+    mt, kblocks = -(-F // (64 if gate else 128)), -(-K // 64)
+    small, large = ([n * sms // 148 for n in t] for t in (_SPLIT_SMALL, _SPLIT_LARGE))
+    stream = F * K * (4 if gate else 2) / 6.6e6
+    best = None
+    if mt > small[0]:
+        shapes = [(1, T)] if T <= 64 else []
+    elif mt * -(-T // 256) > small[0]:
+        shapes = []
+    else:
+        shapes = []
+        for S in range(1, min(8, kblocks) + 1):
+            lo, hi = -(-T // (256 if S == 1 else 208)), min(small[S - 1] // (mt * S), -(-T // 16))
+            # a dozen counts of token tiles at most; partial rows sent and received have to fit shared memory: 208 tokens
+            shapes += [(S, -(-(-(-T // nt)) // 16) * 16) for nt in range(lo, hi + 1, max(1, (hi - lo) // 12))]
+    for S, bn in shapes:
+        per = -(-kblocks // S)
+        if -(-kblocks // per) != S:
+            continue                      # a smaller cluster has the same shares
+        units, steps, stage = mt * S * -(-T // bn), -(-per // 2), 32768 + 256 * bn
+        one = bn > 80 or (per > 4 and units <= large[S - 1])      # one CTA per SM
+        cap = (large if one else small)[S - 1]
+        if units > cap and (S > 1 or bn < T or T > 64):
+            continue
+        waves, shared = -(-units // cap), 2 if not one and units > sms else 1
+        flight = min(steps, (230400 if one else 114176) // stage, 6)
+        body = max(waves * steps * max(0.226, shared * stage / 1.27e5, 0.81 / flight), stream)
+        adds = -(-(-(-bn // S) * (8 if gate else 16)) // 192)
+        cost = 3.4 + body + 0.0098 * bn + (0.0167 * bn if S > 1 else 0.0) + waves * adds * 0.285 + (0.51 if shared > 1 else 0.0) + \
+            (0.1 if bn < T else 0.0)
+        if best is None or cost < best[0]:
+            best = (cost, bn, S)
+    return best
+
+
+@lru_cache(maxsize=4096)
+def _dense_plan(T: int, F: int, K: int, epi: int, sms: int):
+    """(wide, split plan) of a dense launch on one GPU that leaves the choice of kernel to this module."""
+    wide, plan = want_wide(epi, T, F, K, 1, sms), split_plan(T, F, K, epi, sms)
+    if plan is not None and (not wide or plan[0] < dense_wide_cost(T, F, K, epi, sms)):
+        return False, plan
+    return wide, None
+
+
 def _wide_rows(F: int, out: Optional[torch.Tensor], residual: Optional[torch.Tensor], comm: "Optional[GemmComm]") -> bool:
     """Launches of gemm_wide.cu: on one GPU, rows that move 16 bytes at a time (others keep their split of K)."""
     rows16 = lambda t: t is None or (t.stride(0) * t.element_size() % 16 == 0 and t.data_ptr() % 16 == 0)
@@ -279,9 +355,11 @@ def rope_table(max_pos: int, hd: int, theta: float, device) -> torch.Tensor:
 
 def _launch(W, X, Y, R, offs, recs, bases, G, T, F, K, epi, bn, splitk, ldy, y_f32, comm: Optional[GemmComm] = None,
             streamk: bool = False, pair: bool = False, w_blocked: bool = False, act: int = 0, act_limit: float = 0.0,
-            act_cols: int = 0, unit_weights: bool = False, wide: bool = False):
+            act_cols: int = 0, unit_weights: bool = False, wide: bool = False, cluster: int = 0):
     s = scratch(X.device)
     d = _lib.DmoeGemm()           # zeros: only what a launch has is filled in
+    if cluster:
+        d.cluster = cluster
     if wide:
         d.wide = 1
     if act:
@@ -377,9 +455,10 @@ def _check_x(x):
 def linear(x: torch.Tensor, w: torch.Tensor, residual: Optional[torch.Tensor] = None,
            out: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None, bn: int = 0,
            splitk: int = 0, comm: Optional["GemmComm"] = None, pair: bool = False, tanh: bool = False,
-           silu_cols: int = 0, wide: Optional[bool] = None) -> torch.Tensor:
+           silu_cols: int = 0, wide: Optional[bool] = None, cluster: Optional[int] = None) -> torch.Tensor:
     """y[T, F] = x[T, K] @ w[F, K].T (+ residual[T, F]); ``tanh``: of the product; ``silu_cols``: silu of the first so
-    many columns. ``pair``: CTA pairs (tcgen05 cta_group::2) on tiles of 256 weight rows x ``bn`` (128 / 256) tokens, whole tiles."""
+    many columns. ``pair``: CTA pairs (tcgen05 cta_group::2) on tiles of 256 weight rows x ``bn`` (128 / 256) tokens, whole tiles.
+    ``cluster``: tiles of 128 weight rows x ``bn`` tokens (any multiple of 16), K cut over so many CTAs (csrc/kernels/gemm_split.cu)."""
     T, K = x.shape
     F = w.shape[0]
     if not x.is_cuda:
@@ -412,8 +491,16 @@ def linear(x: torch.Tensor, w: torch.Tensor, residual: Optional[torch.Tensor] = 
     # plain split-K with a factor that fills the SMs. An explicit splitk >= 1 selects split-K with that factor.
     sms = num_sms(x.device)
     auto_sk = 0
-    if wide is None:
-        wide = not (bn or splitk or pair) and want_wide(EPI_PLAIN, T, F, K, 1, sms) and _wide_rows(F, out, residual, comm)
+    if wide is None and not cluster:
+        wide = False
+        if not (bn or splitk or pair) and _wide_rows(F, out, residual, comm):
+            wide, plan = _dense_plan(T, F, K, EPI_PLAIN, sms)
+            if plan is not None:
+                _, bn, cluster = plan
+    if cluster:
+        _launch(w, x, out, residual, None, None, None, 1, T, F, K, EPI_PLAIN, bn, 1, out.stride(0), out.dtype == torch.float32, comm,
+                act=ACT_TANH if tanh else ACT_SILU if silu_cols else 0, act_cols=silu_cols, cluster=cluster)
+        return out
     if not bn:
         bn = pick_bn(T, EPI_PLAIN)
         if ((F + 127) // 128) * ((T + bn - 1) // bn) < sms and not pair:
@@ -595,7 +682,7 @@ def grouped_combine(x: torch.Tensor, w: torch.Tensor, offs: Optional[torch.Tenso
 
 
 def swiglu_linear(x: torch.Tensor, w13: torch.Tensor, out: Optional[torch.Tensor] = None, bn: int = 0,
-                  act: str = "silu", wide: Optional[bool] = None) -> torch.Tensor:
+                  act: str = "silu", wide: Optional[bool] = None, cluster: Optional[int] = None) -> torch.Tensor:
     """Dense gated up-projection: act(x @ w13[:I].T) * (x @ w13[I:].T); w13 is [2I, K] (a one-group grouped_swiglu)."""
     T, K = x.shape
     I = w13.shape[0] // 2
@@ -614,8 +701,15 @@ def swiglu_linear(x: torch.Tensor, w13: torch.Tensor, out: Optional[torch.Tensor
         out = torch.empty(T, I, dtype=torch.bfloat16, device=x.device)
     if T == 0:
         return out
-    if wide is None:
-        wide = not bn and want_wide(EPI_SWIGLU, T, I, K, 1, num_sms(x.device))
+    if wide is None and not cluster:
+        wide = False
+        if not bn:
+            wide, plan = _dense_plan(T, I, K, EPI_SWIGLU, num_sms(x.device))
+            if plan is not None and _wide_rows(I, out, None, None):
+                _, bn, cluster = plan
+    if cluster:
+        _launch(w13, x, out, None, None, None, None, 1, T, I, K, EPI_SWIGLU, bn, 1, out.stride(0), False, act=ACTS[act], cluster=cluster)
+        return out
     bn = bn or pick_bn(T, EPI_SWIGLU)
     _launch(w13, x, out, None, None, None, None, 1, T, I, K, EPI_SWIGLU, bn, 1, out.stride(0), False,
             act=ACTS[act], wide=wide)

@@ -1,0 +1,88 @@
+"""Dense GEMM with K cut over a cluster (csrc/kernels/gemm_split.cu) vs fp64 PyTorch: edges of tiles, shares and shared memory."""
+import pytest
+import torch
+
+from disagmoe_b200.ops import functional as F
+from disagmoe_b200.ops import gemm, reference
+
+pytestmark = pytest.mark.gpu
+
+
+def _bf(*s):
+    return torch.randn(*s, device="cuda").to(torch.bfloat16)
+
+
+def _close(y, ref, K, bits=8):
+    """One rounding of the output (half a unit: 2^-8 relative in bf16, 2^-24 in fp32) and fp32 sums of K products of size 1 / K in any order."""
+    bound = ref.abs() * 2.0 ** -bits + 2.0 ** -22 * K ** 0.5 + 1e-6
+    bad = ((y.double() - ref).abs() > bound).sum().item()
+    assert bad == 0 and gemm.check_status() == 0, f"{bad} of {ref.numel()} off, max {(y.double() - ref).abs().max().item():.3g}"
+
+
+@pytest.mark.parametrize("bn,cluster", [(16, 1), (16, 8), (32, 4), (48, 5), (80, 2), (96, 3), (128, 2), (208, 8), (256, 1)])
+@pytest.mark.parametrize("T,N,K", [(1, 8, 8), (15, 136, 72), (17, 128, 64), (97, 264, 520), (300, 144, 1096), (33, 1024, 2048)])
+def test_tiles_and_clusters(T, N, K, bn, cluster):
+    torch.manual_seed(T + N + K)
+    x, w, r = _bf(T, K), _bf(N, K) * K ** -0.5, _bf(T, N)
+    ref = x.double() @ w.double().T
+    wide_x = torch.cat([x, _bf(T, 16)], 1)[:, :K]                        # rows further apart than they are long
+    out = torch.full((T + 1, N + 8), 7.0, dtype=torch.bfloat16, device="cuda")
+    gemm.linear(wide_x, w, out=out[:T, :N], bn=bn, cluster=cluster)
+    _close(out[:T, :N], ref, K)
+    assert bool((out[T] == 7.0).all()) and bool((out[:, N:] == 7.0).all())
+    y = r.clone()
+    gemm.linear(x, w, residual=y, out=y, bn=bn, cluster=cluster)         # in place
+    _close(y, ref + r.double(), K)
+    _close(gemm.linear(x, w, bn=bn, cluster=cluster, out_dtype=torch.float32), ref, K, bits=22)
+    s = ref.clone()
+    s[:, :N // 2] *= torch.sigmoid(s[:, :N // 2])
+    # the activation adds the error of its exponential, 2^-21 relative
+    _close(gemm.linear(x, w, bn=bn, cluster=cluster, silu_cols=N // 2, out_dtype=torch.float32), s, K, bits=19)
+
+
+@pytest.mark.parametrize("bn,cluster", [(16, 2), (48, 8), (144, 3), (256, 1)])
+@pytest.mark.parametrize("T,I,K", [(1, 8, 64), (37, 72, 520), (150, 200, 1024)])
+def test_gated(T, I, K, bn, cluster):
+    torch.manual_seed(T)
+    x, w = _bf(T, K), _bf(2 * I, K) * K ** -0.5
+    h = x.double() @ w.double().T
+    ref = h[:, :I] * torch.sigmoid(h[:, :I]) * h[:, I:]
+    _close(gemm.swiglu_linear(x, w, bn=bn, cluster=cluster), ref, K)
+
+
+@pytest.mark.parametrize("hd,n_q,n_kv", [(128, 4, 1), (64, 6, 2)])
+@pytest.mark.parametrize("T,bn,cluster", [(1, 16, 4), (50, 32, 3), (200, 112, 2)])
+def test_rope_append(T, bn, cluster, hd, n_q, n_kv):
+    torch.manual_seed(T)
+    K, bs, N = 512, 16, (n_q + 2 * n_kv) * hd
+    x, w = _bf(T, K), _bf(N, K) * K ** -0.5
+    pos = torch.randint(0, 500, (T,), device="cuda", dtype=torch.int32)
+    slots = torch.randperm(400, device="cuda")[:T]
+    slots[::7] = -1
+    caches = [torch.full((25, bs, n_kv, hd), 5.0, dtype=torch.bfloat16, device="cuda") for _ in range(4)]
+    table = gemm.rope_table(512, hd, 1e4, "cuda")
+    y = torch.zeros(T, N, dtype=torch.bfloat16, device="cuda")
+    gemm.linear(x, w, out=y, bn=bn, cluster=cluster, comm=gemm.GemmComm(rope=gemm.RopeAppend(table, pos, slots, *caches[:2], n_q, n_kv, hd)))
+    z = gemm.linear(x, w, bn=bn, cluster=cluster)
+    reference.rope_kv_append(z, pos, slots, *caches[2:], n_q, n_kv, hd, 1e4)
+    # the reference rotates in fp32 with its own sines: a unit of the last place of bf16
+    for a, b in ((y[:, :n_q * hd], z[:, :n_q * hd]), (caches[0], caches[2]), (caches[1], caches[3])):
+        torch.testing.assert_close(a.float(), b.float(), rtol=2 ** -7, atol=2 ** -7)
+    assert gemm.check_status() == 0
+
+
+@pytest.mark.parametrize("T,N,K,gate", [(1, 4096, 4096, False), (37, 6144, 2048, False), (64, 32000, 512, False), (65, 2816, 1024, True),
+                                        (300, 2048, 1096, False), (1111, 1024, 256, False)])
+def test_chosen_plan_agrees_with_the_other_kernels(T, N, K, gate):
+    torch.manual_seed(N)
+    assert gemm.split_plan(T, N, K, gemm.EPI_SWIGLU if gate else gemm.EPI_PLAIN, gemm.num_sms("cuda")) is not None
+    x, w = _bf(T, K), _bf(2 * N if gate else N, K) * K ** -0.5
+    y, z = (gemm.swiglu_linear(x, w), gemm.swiglu_linear(x, w, wide=False)) if gate else (gemm.linear(x, w), gemm.linear(x, w, wide=False))
+    torch.testing.assert_close(y.float(), z.float(), rtol=2 ** -7, atol=2 ** -9)      # two roundings of nearly equal sums
+    assert gemm.check_status() == 0
+
+
+def test_launch_that_does_not_qualify():
+    """Rows that do not move 16 bytes at a time keep the kernel that stores them one by one."""
+    x, w = _bf(9, 128), _bf(20, 128)
+    _close(gemm.linear(x, w, bn=16, cluster=2, out_dtype=torch.float32), x.double() @ w.double().T, 128 * 128, bits=20)
