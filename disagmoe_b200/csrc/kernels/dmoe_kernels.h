@@ -263,11 +263,12 @@ int dmoe_latent_prefill_tc(const void* q, long long ld_q, const void* kv, long l
                            int window, const float* sink, const void* gate, long long ld_gate, void* out, long long ld_out, int* status,
                            void* stream);
 // dmoe_prefill_attention_ext on tcgen05 (prefill_attention.cu) for heads of 128: pages of block_size tokens that divide 128 keys (at
-// least 8), 16-byte aligned rows of q, out and the caches ([n_blocks, block_size, n_kv, 128]). status: device word, see DmoeGemm.
+// least 8), 16-byte aligned rows of q, out and the caches ([n_blocks, block_size, n_kv, 128]). exact != 0 (no options): weights rounded
+// to bf16 as dmoe_prefill_attention does. status: device word, see DmoeGemm.
 int dmoe_prefill_attention_tc(const void* q, long long ld_q, const void* kcache, const void* vcache, int n_blocks,
                               const int* block_tables, int max_blocks, const void* tiles, int n_tiles, int block_size, int n_q,
                               int n_kv, float scale, int window, int chunk, float softcap, const float* sink, void* out,
-                              long long ld_out, const DmoeAttnExtra* extra, int* status, void* stream);
+                              long long ld_out, const DmoeAttnExtra* extra, int exact, int* status, void* stream);
 int dmoe_prefill_attention(const void* q, long long ld_q, const void* kcache, const void* vcache,
                            const int* block_tables, int max_blocks, const void* tiles, int n_tiles, int block_size,
                            int n_q, int n_kv, int hd, float scale, void* out, long long ld_out, void* stream);

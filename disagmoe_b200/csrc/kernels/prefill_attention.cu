@@ -1,26 +1,28 @@
 // Causal attention of prompt rows over the paged cache on tcgen05: S = Q K^T and O += P V with accumulators in TMEM.
 //
-// One CTA owns one tile of up to 128 query rows (consecutive tokens x the query heads of one kv head) and walks the keys its
-// last token sees 128 at a time. K and V pages go straight from the cache to swizzled shared memory by TMA (one box of 64
-// head dimensions per page and half); S lands in TMEM; four warps, one row per thread, apply options and the online softmax
-// and put P back into TMEM over S, from where it is the A operand of P V. The output accumulator stays in TMEM and is only
-// rescaled when a row's maximum grew by more than 2^8 (the sums use the same stale maximum, so nothing is lost). Warp 0
-// loads, warp 1 issues the MMAs. A CTA is a serial chain QK -> softmax -> PV, so two of them share an SM (96 KB of shared
-// memory, 256 TMEM columns each) and one's softmax runs under the other's MMAs. Weights as the A operand in TMEM and the rescale
-// that waits for a growth of 2^8 are published ideas of attention on this chip (T. Dao et al., FlashAttention-4, 2025).
+// One CTA owns one tile of up to 128 query rows (consecutive tokens x the query heads of one kv head). K and V pages go straight
+// from the cache to swizzled shared memory by TMA, 128 keys at a time (one box of 64 head dimensions per page and half), and are
+// worked through 64 keys at a time: S lands in TMEM; four warps, one row per thread, apply options and the online softmax and put P
+// back into TMEM over S, from where it is the A operand of P V. Two score buffers of 64 columns: the scores of the next 64 keys are
+// there when a thread is done with these, and Q K^T and P V run under the softmax. The output accumulator stays in TMEM. Warp 0
+// loads, warp 1 issues the MMAs. Two CTAs share an SM (96 KB of shared memory, 256 TMEM columns each). Weights as the A operand in
+// TMEM, and rescaling the output only when a row's maximum grew by more than 2^8 (the sums use the same stale maximum, so nothing is
+// lost), are published ideas of attention on this chip (T. Dao et al., FlashAttention-4, 2025).
 //
-// The softmax weights keep fp32 accuracy: P = hi + lo, both bf16, two products.
+// With options the softmax weights keep fp32 accuracy: P = hi + lo, both bf16, two products. EXACT, without options: weights are
+// rounded to bf16 once, relative to the maximum after every 64 keys, as in the mma.sync kernel of attention.cu, which has the same
+// blocks: both round the same weights the same way. (Other roundings make decoders with few large experts choose other experts for
+// nearly tied rows.) The output is then rescaled whenever a maximum grows.
 //
 // LATENT: the same for prompt runs of latent attention over expanded keys and values (latent_attention.cu has the layout): a
 // tile is 128 tokens of one head, a key is 128 numbers of its expanded row and the 64 rotated ones of its cache row, and the
 // keys of a sequence are consecutive rows, so that a box holds 128 of them. With 128 KB of shared memory one CTA fits an SM.
-// Measured on B200 (1965 MHz), mma.sync -> here: 3000 tokens of 16 heads, window 1024, 199 -> 94 us; 4096 without, 604 -> 215 us.
 //
-// Measured on B200 (1965 MHz) against the mma.sync kernel of attention.cu (64 rows per CTA, every warp re-reading all of K and V
-// from shared memory): 4096 tokens of 16 heads, window 1024, soft cap 371 -> 137 us; 3000 tokens, sinks 432 -> 111 us. That kernel
-// stays for other head sizes, page sizes that do not divide 128 keys, unaligned rows, prompts of few keys, and for attention without
-// options, whose weights are rounded to bf16 relative to a running maximum per 64 keys: another order of blocks rounds them
-// differently, and decoders with few large experts then choose other experts for nearly tied rows.
+// Measured on B200 (1965 MHz) against the mma.sync kernel of attention.cu (64 rows per CTA, every warp re-reading all of K and V from
+// shared memory), and this one with one score buffer of 128 keys between: 4096 tokens of 16 heads, window 1024, soft cap 366 -> 131 -> 96
+// us; 3000 tokens, sinks 219 -> 64 -> 48 us; latent, 4096 tokens of 16 heads 208 -> 157 us; without options, 4096 tokens of 32 heads in
+// three prompts 390 -> 111 us. Bound by the issue slots of its softmax. The mma.sync kernel stays for other head sizes, page sizes that
+// do not divide 128 keys, unaligned rows and prompts of few keys.
 #include <string.h>
 
 #include "attn_common.cuh"
@@ -30,6 +32,7 @@
 namespace dmoe {
 
 constexpr int kFaRows = 128, kFaKeys = 128, kFaDim = 128;
+constexpr int kFaSub = 64;                          // keys per step
 constexpr int kFaThreads = 192;
 constexpr int kFaHalf = 128 * 128;                  // bytes of 128 rows x 64 bf16
 constexpr int kFaTile = 2 * kFaHalf;                // one of Q, K, V
@@ -46,7 +49,7 @@ __device__ __forceinline__ void fa_load(uint32_t dst, const CUtensorMap* m, int 
 }
 
 // LATENT: tmK is the map of the expanded keys and values, tmV that of the cache rows, base the row of position 0 per tile
-template <int KIND>
+template <int KIND, bool EXACT>
 __global__ void __launch_bounds__(kFaThreads, KIND == FA_LATENT ? 1 : 2)
 prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                   const __nv_bfloat16* __restrict__ q, long long ld_q, const int* __restrict__ block_tables, int max_blocks,
@@ -58,14 +61,16 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 2 * kQk + kFaTile);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
   int* abort_word = reinterpret_cast<int*>(tmem_slot + 1);
   const uint32_t sq = smem_u32(smem), sk = sq + kQk, sv = sk + kQk;
-  // K / V landed, K / V consumed, scores ready, weights ready, output accumulated
-  const uint32_t k_full = smem_u32(bars), v_full = k_full + 8, k_empty = k_full + 16, v_empty = k_full + 24, s_full = k_full + 32,
-                 p_full = k_full + 40, o_full = k_full + 48;
+  // K / V landed, K / V consumed, output accumulated; scores ready and weights ready in each of two buffers; output complete. A thread
+  // that waits for the output of a step knows that the step before is complete, so that the parity says which step is meant; the end
+  // has a barrier of its own, because warps come to it one or two steps late
+  const uint32_t k_full = smem_u32(bars), v_full = k_full + 8, k_empty = k_full + 16, v_empty = k_full + 24, o_full = k_full + 32,
+                 s_full = k_full + 40, p_full = k_full + 56, o_done = k_full + 72;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   // tiles of a prompt are in order of position: the longest run first
   const int4 tile = tiles[n_tiles - 1 - blockIdx.x / n_kv];
   const int hkv = blockIdx.x % n_kv, gq = ext.gq;
@@ -75,10 +80,13 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
   // first key block: from the first key that anyone sees, at the start of a page
   const int first = first_key(pos0, ext.window, ext.chunk), kbase = LAT ? first : first / kFaKeys * kFaKeys;
   const int nkb = (kmax - kbase + kFaKeys - 1) / kFaKeys;
+  // uniform for the compiler; steps of 64 keys that anyone sees
+  const int blocks = __shfl_sync(0xffffffffu, nkb, 0), first_block = __shfl_sync(0xffffffffu, kbase, 0);
+  const int steps = __shfl_sync(0xffffffffu, (kmax - kbase + kFaSub - 1) / kFaSub, 0);
 
   if (threadIdx.x == 0) {
     *abort_word = 0;
-    for (int i = 0; i < 7; ++i) mbar_init(k_full + 8 * i, i == 5 ? 4 : 1);      // weights: one arrival per softmax warp
+    for (int i = 0; i < 10; ++i) mbar_init(k_full + 8 * i, i == 7 || i == 8 ? 4 : 1);      // weights: one arrival per softmax warp
     mbar_fence_init();
   }
   if (warp == 1) {
@@ -102,26 +110,30 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t t_s = *tmem_slot, t_o = t_s + kFaKeys;      // scores / weights [128 columns], output [128 columns]
+  const uint32_t t_s = __shfl_sync(0xffffffffu, *tmem_slot, 0), t_o = t_s + 2 * kFaSub;      // scores / weights [2 x 64 columns], output [128 columns]
 
   if (warp == 0) {
     // ------------------------------------------------------------ loads
     if (LAT) {
       // one box of 128 keys per 64 numbers
-      if (lane == 0) {
-        const int at = base[n_tiles - 1 - blockIdx.x / n_kv], col = hkv * (2 * kFaDim);
-        for (int j = 0; j < nkb; ++j) {
-          const int row = at + kbase + j * kFaKeys;
-          if (!mbar_wait(k_empty, (j & 1) ^ 1, abort_word)) break;
+      const int at = __shfl_sync(0xffffffffu, base[n_tiles - 1 - blockIdx.x / n_kv], 0) + first_block, col = hkv * (2 * kFaDim);
+      for (int j = 0; j < blocks; ++j) {
+        const int row = at + j * kFaKeys;
+        if (!mbar_wait_warp(k_empty, (j & 1) ^ 1, abort_word)) break;
+        if (elect_one()) {
           mbar_expect_tx(k_full, kQk);
           fa_load(sk, &tmK, col, row, k_full);
           fa_load(sk + kFaHalf, &tmK, col + 64, row, k_full);
           fa_load(sk + 2 * kFaHalf, &tmV, rankp, row, k_full);
-          if (!mbar_wait(v_empty, (j & 1) ^ 1, abort_word)) break;
+        }
+        __syncwarp();
+        if (!mbar_wait_warp(v_empty, (j & 1) ^ 1, abort_word)) break;
+        if (elect_one()) {
           mbar_expect_tx(v_full, kFaTile);
           fa_load(sv, &tmK, col + kFaDim, row, v_full);
           fa_load(sv + kFaHalf, &tmK, col + kFaDim + 64, row, v_full);
         }
+        __syncwarp();
       }
     } else {
       // lane = (page of the block, half of the head)
@@ -137,85 +149,96 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
 #pragma unroll
         for (int kv = 0; kv < 2; ++kv) {
           const uint32_t full = kv ? v_full : k_full;
-          ok = ok && mbar_wait(kv ? v_empty : k_empty, (j & 1) ^ 1, abort_word);
-          if (!__all_sync(0xffffffffu, ok)) break;
+          ok = ok && mbar_wait_warp(kv ? v_empty : k_empty, (j & 1) ^ 1, abort_word);
+          if (!ok) break;
           if (lane == 0) mbar_expect_tx(full, there * block_size * 256);
           __syncwarp();
           if (mine) tma_load_3d((kv ? sv : sk) + at, kv ? &tmV : &tmK, half * 64, hkv, slot, full);
         }
-        if (!__all_sync(0xffffffffu, ok)) break;
+        if (!ok) break;
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMAs
-    if (lane == 0) {
-      constexpr uint32_t id_qk = umma_idesc_bf16(kFaRows, kFaKeys);
-      constexpr uint32_t id_pv = umma_idesc_bf16(kFaRows, kFaDim) | (1u << 16);      // V is MN-major
-      for (int j = 0; j < nkb; ++j) {
-        const uint32_t ph = j & 1;
-        if (!mbar_wait(k_full, ph, abort_word)) break;
-        // the scores overwrite the previous block's weights, which the product before reads from tensor memory. The order of two
-        // products is only given for the same accumulator, so that one has to be complete
-        if (j > 0 && !mbar_wait(o_full, ph ^ 1, abort_word)) break;
-        tc_fence_after();
+    // ------------------------------------------------------------ MMAs (the warp converged, an elected lane issues)
+    constexpr uint32_t id_qk = umma_idesc_bf16(kFaRows, kFaSub);
+    constexpr uint32_t id_pv = umma_idesc_bf16(kFaRows, kFaDim) | (1u << 16);      // V is MN-major
+    const auto scores = [&](int t) {      // step t; its buffer is free
+      if ((t & 1) == 0 && !mbar_wait_warp(k_full, (t >> 1) & 1, abort_word)) return false;
+      tc_fence_after();
+      if (elect_one()) {
+        const uint32_t k0 = sk + (t & 1) * kFaSub * 128;
 #pragma unroll
         for (int k = 0; k < kQd / kUmmaK; ++k) {
           const uint32_t off = (k >> 2) * kFaHalf + (k & 3) * 32;
-          umma_f16(t_s, umma_desc_sw128(sq + off), umma_desc_sw128(sk + off), id_qk, k > 0 ? 1u : 0u);
+          umma_f16(t_s + (t & 1) * kFaSub, umma_desc_sw128(sq + off), umma_desc_sw128(k0 + off), id_qk, k > 0 ? 1u : 0u);
         }
-        umma_commit(s_full);
-        umma_commit(k_empty);
-        if (!mbar_wait(p_full, ph, abort_word)) break;
-        if (!mbar_wait(v_full, ph, abort_word)) break;
-        tc_fence_after();
-#pragma unroll
-        for (int part = 0; part < 2; ++part)
-#pragma unroll
-          for (int k = 0; k < kFaKeys / kUmmaK; ++k)
-            umma_f16_ta(t_o, t_s + part * (kFaKeys / 2) + k * (kUmmaK / 2), umma_desc_sw128_mn(sv + k * kUmmaK * 128, kFaHalf),
-                        id_pv, (j > 0 || part > 0 || k > 0) ? 1u : 0u);
-        umma_commit(o_full);
-        umma_commit(v_empty);
+        umma_commit(s_full + 8 * (t & 1));
+        if ((t & 1) != 0 || t == steps - 1) umma_commit(k_empty);
       }
+      __syncwarp();
+      return true;
+    };
+    bool ok = scores(0) && (steps < 2 || scores(1));
+    for (int t = 0; ok && t < steps; ++t) {
+      ok = mbar_wait_warp(p_full + 8 * (t & 1), (t >> 1) & 1, abort_word);
+      if (ok && (t & 1) == 0) ok = mbar_wait_warp(v_full, (t >> 1) & 1, abort_word);
+      if (!ok) break;
+      tc_fence_after();
+      if (elect_one()) {
+        const uint32_t p0 = t_s + (t & 1) * kFaSub, v0 = sv + (t & 1) * kFaSub * 128;
+#pragma unroll
+        for (int part = 0; part < (EXACT ? 1 : 2); ++part)
+#pragma unroll
+          for (int k = 0; k < kFaSub / kUmmaK; ++k)
+            umma_f16_ta(t_o, p0 + part * (kFaSub / 2) + k * (kUmmaK / 2), umma_desc_sw128_mn(v0 + k * kUmmaK * 128, kFaHalf), id_pv,
+                        (t > 0 || part > 0 || k > 0) ? 1u : 0u);
+        umma_commit(o_full);
+        if (t == steps - 1) umma_commit(o_done);
+        if ((t & 1) != 0 || t == steps - 1) umma_commit(v_empty);
+      }
+      __syncwarp();
+      // the next scores of this buffer overwrite the weights that this product reads from tensor memory. The order of two products is
+      // only given for the same accumulator, so it has to be complete
+      if (t + 2 < steps) ok = mbar_wait_warp(o_full, t & 1, abort_word) && scores(t + 2);
     }
   } else {
     // ------------------------------------------------------------ softmax: one query row per thread
     const uint32_t lanes = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const int qpos = pos0 + tok;
-    const float temp = query_temperature(ext, qpos);
-    const int lo = first_key(qpos, ext.window, ext.chunk);
-    // blocks that need no mask: all keys visible to the first and the last token of the tile
-    const int lo_last = first_key(kmax - 1, ext.window, ext.chunk);
+    const float temp = EXACT ? 1.f : query_temperature(ext, qpos);
+    const int lo = EXACT ? 0 : first_key(qpos, ext.window, ext.chunk);
+    // steps that need no mask: all keys visible to the first and the last token of the tile
+    const int lo_last = EXACT ? 0 : first_key(kmax - 1, ext.window, ext.chunk);
     const float scale = scale_log2 * temp;
     float m = -INFINITY, l = 0.f;
     bool ok = true;
-    for (int j = 0; j < nkb; ++j) {
-      const int key0 = kbase + j * kFaKeys;
-      if (!mbar_wait(s_full, j & 1, abort_word)) { ok = false; break; }
-      if (j > 0 && !mbar_wait(o_full, (j - 1) & 1, abort_word)) { ok = false; break; }      // complete by now
+    for (int t = 0; t < steps; ++t) {
+      const int key0 = kbase + t * kFaSub;
+      const uint32_t buf = t_s + lanes + (t & 1) * kFaSub;
+      if (!mbar_wait(s_full + 8 * (t & 1), (t >> 1) & 1, abort_word)) { ok = false; break; }
       tc_fence_after();
-      uint32_t s[4][32];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) tmem_ld32(t_s + lanes + i * 32, s[i]);
+      uint32_t s[2][32];
+      tmem_ld32(buf, s[0]);
+      tmem_ld32(buf + 32, s[1]);
       tmem_ld_wait();
-      const bool masked = key0 + kFaKeys - 1 > pos0 || key0 < lo_last;
+      const bool masked = key0 + kFaSub - 1 > pos0 || key0 < lo_last;
       float mx = -INFINITY, mul = 1.f;      // scores are s times mul: the factor goes into the exponent's subtraction where it can
-      if (ext.cap_log2 > 0.f) {
+      if (!EXACT && ext.cap_log2 > 0.f) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < 2; ++i)
 #pragma unroll
           for (int e = 0; e < 32; ++e) s[i][e] = __float_as_uint(attn_score<true>(__uint_as_float(s[i][e]) * temp, scale_log2, ext));
       } else if (scale > 0.f) {
         mul = scale;
       } else {
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < 2; ++i)
 #pragma unroll
           for (int e = 0; e < 32; ++e) s[i][e] = __float_as_uint(__uint_as_float(s[i][e]) * scale);
       }
       if (masked) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < 2; ++i)
 #pragma unroll
           for (int e = 0; e < 32; ++e) {
             const int key = key0 + i * 32 + e;
@@ -223,7 +246,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
           }
       }
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int i = 0; i < 2; ++i) {
         float a = __uint_as_float(s[i][0]), b = __uint_as_float(s[i][1]);
 #pragma unroll
         for (int e = 2; e < 32; e += 2) {
@@ -233,20 +256,27 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         mx = fmaxf(mx, fmaxf(a, b));
       }
       mx *= mul;
-      const bool grow = mx > m + kFaSlack;      // true for the first finite maximum: m is -inf before it
+      const bool grow = EXACT ? mx > m : mx > m + kFaSlack;      // true for the first finite maximum: m is -inf before it
       if (__any_sync(0xffffffffu, grow)) {
         const float to = grow ? mx : m;
-        if (j > 0) {
+        if (t > 0) {
+          ok = mbar_wait_warp(o_full, (t - 1) & 1, abort_word);
+          if (!ok) break;
+          tc_fence_after();
           const float f = grow ? exp2f(m - to) : 1.f;      // -inf - finite: 0, and what it scales is 0
           l *= f;
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            uint32_t o[16];
-            tmem_ld16(t_o + lanes + i * 16, o);
+          for (int i = 0; i < 4; ++i) {
+            uint32_t o[2][16];
+            tmem_ld16(t_o + lanes + i * 32, o[0]);
+            tmem_ld16(t_o + lanes + i * 32 + 16, o[1]);
             tmem_ld_wait();
 #pragma unroll
-            for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * f);
-            tmem_st16(t_o + lanes + i * 16, o);
+            for (int h = 0; h < 2; ++h) {
+#pragma unroll
+              for (int e = 0; e < 16; ++e) o[h][e] = __float_as_uint(__uint_as_float(o[h][e]) * f);
+              tmem_st16(t_o + lanes + i * 32 + h * 16, o[h]);
+            }
           }
         }
         m = to;
@@ -254,41 +284,42 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
       const float sub = m == -INFINITY ? 0.f : m;      // a row with nothing visible yet: weights 0, not NaN
       float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int i = 0; i < 2; ++i) {
         uint32_t hi[16], rest[16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
           // exp2f and not the instruction alone, which makes 0 of weights below 2^-126
           const float p0 = exp2f(fmaf(__uint_as_float(s[i][2 * e]), mul, -sub)), p1 = exp2f(fmaf(__uint_as_float(s[i][2 * e + 1]), mul, -sub));
           sum[e & 3] += p0 + p1;
-          split2(p0, p1, hi[e], rest[e]);
+          if (EXACT) hi[e] = pack_bf16(p0, p1);
+          else split2(p0, p1, hi[e], rest[e]);
         }
-        tmem_st16(t_s + lanes + i * 16, hi);
-        tmem_st16(t_s + lanes + kFaKeys / 2 + i * 16, rest);
+        tmem_st16(buf + i * 16, hi);
+        if (!EXACT) tmem_st16(buf + kFaSub / 2 + i * 16, rest);
       }
       l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
-      if (key0 + kFaKeys > kmax) {
+      if (key0 + kFaSub > kmax) {
         // keys past the last one: their weights are 0, but 0 times whatever the page holds there need not be
-        if (!mbar_wait(v_full, j & 1, abort_word)) ok = false;
-        const int key = threadIdx.x - 64;
+        if (!mbar_wait(v_full, (t >> 1) & 1, abort_word)) ok = false;
+        const int key = (threadIdx.x - 64) & (kFaSub - 1), half = (threadIdx.x - 64) / kFaSub;
         if (key0 + key >= kmax) {
+          uint8_t* row = smem + 2 * kQk + half * kFaHalf + ((t & 1) * kFaSub + key) * 128;
 #pragma unroll
-          for (int c = 0; c < 16; ++c)
-            *reinterpret_cast<uint4*>(smem + 2 * kQk + (c >> 3) * kFaHalf + key * 128 + ((c & 7) << 4)) = make_uint4(0, 0, 0, 0);
+          for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(row + (c << 4)) = make_uint4(0, 0, 0, 0);
         }
         fence_proxy_async_smem();
       }
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(p_full);
+      if (lane == 0) mbar_arrive(p_full + 8 * (t & 1));
       if (!ok) break;
     }
-    if (ok && mbar_wait(o_full, (nkb - 1) & 1, abort_word)) {
+    if (ok && mbar_wait(o_done, 0, abort_word)) {
       tc_fence_after();
       float inv = l > 0.f ? 1.f / l : 0.f;
-      if (ext.sink != nullptr) inv = sink_inverse(m, l, ext.sink[head]);
-      if (ext.gate != nullptr && live) inv *= head_gate<__nv_bfloat16>(ext, row0 + tok, head);
+      if (!EXACT && ext.sink != nullptr) inv = sink_inverse(m, l, ext.sink[head]);
+      if (!EXACT && ext.gate != nullptr && live) inv *= head_gate<__nv_bfloat16>(ext, row0 + tok, head);
       __nv_bfloat16* y = out + static_cast<long long>(row0 + tok) * ld_out + head * kFaDim;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -337,17 +368,17 @@ static int page_map(CUtensorMap* map, const void* cache, long long slots, int n_
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : -21;
 }
 
-template <int KIND>
+template <int KIND, bool EXACT>
 static int launch_tc(const CUtensorMap& tmK, const CUtensorMap& tmV, const void* q, long long ld_q, const int* bt, int max_blocks,
                      const void* tiles, int n_tiles, int block_size, int n_kv, float scale, void* out, long long ld_out, AttnExt ext,
                      const int* base, int rankp, int* status, cudaStream_t stream) {
   constexpr int smem = fa_smem(KIND == FA_LATENT);
   static PerDeviceOnce configured;
   const int crc = configured.run([] {
-    return static_cast<int>(cudaFuncSetAttribute(prefill_tc_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    return static_cast<int>(cudaFuncSetAttribute(prefill_tc_kernel<KIND, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   });
   if (crc != 0) return crc;
-  prefill_tc_kernel<KIND><<<n_kv * n_tiles, kFaThreads, smem, stream>>>(
+  prefill_tc_kernel<KIND, EXACT><<<n_kv * n_tiles, kFaThreads, smem, stream>>>(
       tmK, tmV, static_cast<const __nv_bfloat16*>(q), ld_q, bt, max_blocks, static_cast<const int4*>(tiles), n_tiles, n_kv,
       block_size, scale * kLog2e, static_cast<__nv_bfloat16*>(out), ld_out, ext, base, rankp, status);
   return static_cast<int>(cudaGetLastError());
@@ -360,11 +391,11 @@ using namespace dmoe;
 extern "C" int dmoe_prefill_attention_tc(const void* q, long long ld_q, const void* kcache, const void* vcache, int n_blocks,
                                          const int* block_tables, int max_blocks, const void* tiles, int n_tiles, int block_size,
                                          int n_q, int n_kv, float scale, int window, int chunk, float softcap,
-                                         const float* sink, void* out, long long ld_out, const DmoeAttnExtra* extra, int* status,
-                                         void* stream_) {
+                                         const float* sink, void* out, long long ld_out, const DmoeAttnExtra* extra, int exact,
+                                         int* status, void* stream_) {
   if (n_tiles == 0) return 0;
   if (n_kv < 1 || n_q % n_kv != 0 || n_q / n_kv > kFaRows || n_tiles < 0 || static_cast<long long>(n_tiles) * n_kv > 0x7fffffff || tiles == nullptr || n_blocks < 1 ||
-      block_size < 8 || kFaKeys % block_size != 0)
+      block_size < 8 || kFaKeys % block_size != 0 || (exact && (window > 0 || chunk > 0 || softcap > 0.f || sink != nullptr || extra != nullptr)))
     return -10;
   CUtensorMap tmK, tmV;
   const long long slots = static_cast<long long>(n_blocks) * block_size;
@@ -373,7 +404,8 @@ extern "C" int dmoe_prefill_attention_tc(const void* q, long long ld_q, const vo
   if (rc != 0) return rc;
   const AttnExt ext = make_ext(scale, window, chunk, softcap, sink, n_q / n_kv, extra);
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  return launch_tc<FA_PAGED>(tmK, tmV, q, ld_q, block_tables, max_blocks, tiles, n_tiles, block_size, n_kv, scale, out, ld_out, ext, nullptr, 0, status, stream);
+  const auto launch = exact ? launch_tc<FA_PAGED, true> : launch_tc<FA_PAGED, false>;
+  return launch(tmK, tmV, q, ld_q, block_tables, max_blocks, tiles, n_tiles, block_size, n_kv, scale, out, ld_out, ext, nullptr, 0, status, stream);
 }
 
 extern "C" int dmoe_latent_prefill_tc(const void* q, long long ld_q, const void* kv, long long ld_kv, const void* lat, long long ld_lat,
@@ -388,6 +420,6 @@ extern "C" int dmoe_latent_prefill_tc(const void* q, long long ld_q, const void*
     return -20;
   const DmoeAttnExtra extra = {gate, ld_gate, 0.f, 0};
   const AttnExt ext = make_ext(scale, window, 0, 0.f, sink, 1, &extra);
-  return launch_tc<FA_LATENT>(tmKV, tmL, q, ld_q, nullptr, 0, tiles, n_tiles, kFaKeys, heads, scale, out, ld_out, ext, base, rankp, status,
+  return launch_tc<FA_LATENT, false>(tmKV, tmL, q, ld_q, nullptr, 0, tiles, n_tiles, kFaKeys, heads, scale, out, ld_out, ext, base, rankp, status,
                               static_cast<cudaStream_t>(stream));
 }

@@ -44,6 +44,7 @@ class StepBuffers(TokenBuffers):
         self.ctx_len_decode = z(cap, dt=torch.int32)
         self.n_prefill_tiles = 0
         self.n_loose: Optional[int] = None
+        self.reach: Optional[int] = None
 
 
 class FusedModelExecutor(StepExecutor):
@@ -94,7 +95,7 @@ class FusedModelExecutor(StepExecutor):
         cfg = self.cfg
         meta = AttnMeta(buf.positions[:T], buf.slots[:T], self.block_tables, buf.bt_row[:T], buf.ctx_len[:T],
                         max_ctx=max_ctx, prefill_tiles=buf.prefill_tiles, n_prefill_tiles=buf.n_prefill_tiles,
-                        ctx_len_decode=buf.ctx_len_decode[:T], n_loose=buf.n_loose)
+                        ctx_len_decode=buf.ctx_len_decode[:T], n_loose=buf.n_loose, prefill_reach=buf.reach)
         resid = buf.resid[:T]
         F.embed(buf.ids[:T], self.embed_w, out=resid)
         parts = None
@@ -131,8 +132,9 @@ class FusedModelExecutor(StepExecutor):
                 buf.n_prefill_tiles, buf.n_loose = len(tiles), F.loose_rows(covered)
                 buf.prefill_tiles[:len(tiles)].copy_(tiles.pin_memory(), non_blocking=True)
                 cd = torch.as_tensor(ctx_len).clone()
+                buf.reach = int(cd[covered].max())
                 cd[covered] = 0
                 buf.ctx_len_decode[:T].copy_(cd.pin_memory(), non_blocking=True)
 
     def _end_prefill(self, buf: StepBuffers) -> None:
-        buf.n_prefill_tiles, buf.n_loose = 0, None
+        buf.n_prefill_tiles, buf.n_loose, buf.reach = 0, None, None

@@ -42,6 +42,8 @@ class AttnMeta:
     ctx_len_decode: Optional[torch.Tensor] = None
     # with tiles: rows from here on are all covered by them (None: not known)
     n_loose: Optional[int] = None
+    # keys that a tile looks at, at most (None: not known)
+    prefill_reach: Optional[int] = None
 
 
 @dataclass
@@ -182,7 +184,8 @@ class MoEAttention(torch.nn.Module):
         if tiled:
             # prompt segments: one pass over the sequence's K / V per tile of query rows instead of one per row
             F.prefill_attention(qkv[:, :self.q_size], kc, vc, meta.block_tables, meta.prefill_tiles,
-                                meta.n_prefill_tiles, self.num_heads, self.num_kv_heads, self.head_dim, attn)
+                                meta.n_prefill_tiles, self.num_heads, self.num_kv_heads, self.head_dim, attn,
+                                reach=meta.prefill_reach)
         if self.tp_size == 1:
             return gemm.linear(attn, self.o_w, residual=resid, out=resid)
         part = self._tp_reduce(gemm.linear(attn, self.o_w))

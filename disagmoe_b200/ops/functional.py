@@ -462,7 +462,7 @@ def loose_rows(covered: torch.Tensor) -> int:
 
 
 def _prefill_on_tcgen05(q, kcache, vcache, out, hd: int, vd: int) -> bool:
-    """Shapes of csrc/kernels/prefill_attention.cu (attention with options): heads of 128, pages that divide a block of 128 keys,
+    """Shapes of csrc/kernels/prefill_attention.cu: heads of 128, pages that divide a block of 128 keys,
     16-byte rows."""
     bs = kcache.shape[1]
     return hd == vd == 128 and bs >= 8 and 128 % bs == 0 and q.stride(0) % 8 == 0 and out.stride(0) % 8 == 0 and \
@@ -521,7 +521,7 @@ def prefill_attention(q: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tenso
     """Causal attention of the prompt tokens named by ``tiles`` (device int32 [>= n_tiles, 4], see
     :func:`build_prefill_tiles`) over the paged cache, which already holds their own K / V; writes their rows of
     ``out``. Every tile streams its sequence's K / V once (the per-token kernel streams it once per row). ``reach``
-    (:func:`tile_reach`), where the caller knows it, chooses between two kernels of attention with options."""
+    (:func:`tile_reach`), where the caller knows it, chooses between two kernels."""
     if n_tiles == 0:
         return out
     assert q.is_cuda and tiles.is_cuda and tiles.dtype == torch.int32 and tiles.is_contiguous()
@@ -531,19 +531,20 @@ def prefill_attention(q: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tenso
     options = window or chunk or softcap or fp32_weights or sink is not None or q_temp is not None or gate is not None or \
         hd != vd or n_q // n_kv not in (1, 2, 4, 8)
     x = _attn_extra(q_temp, gate, q.dtype)
-    # A CTA of the tcgen05 kernel needs 10 us before its first result and 3 us per 128 keys then, one of the mma.sync kernel 6 us and
-    # 9 us; a chip full of them meets at fewer keys. Measured on B200 (warm, mma.sync -> tcgen05), 16 / 4 heads: one prompt of 64 tokens 7.2
-    # -> 12.9 us, 192: 15.2 -> 17.1, 256: 19.3 -> 16.3; 16 prompts of 64 9.5 -> 13.5, of 100 20.5 -> 17.0; 48 of 64 23 -> 27, of 96 40 -> 31;
-    # window 64: one prompt of 1000 13.5 -> 18.5, 4 of 500 24.4 -> 22.4, one of 3000 35.0 -> 34.3; window 200: of 1000 25.7 -> 22.6.
-    if options and (reach is None or reach > 192 or reach >= 95 and n_tiles * n_kv >= 192) and \
-            _prefill_on_tcgen05(q, kcache, vcache, out, hd, vd):
+    # A CTA of the tcgen05 kernel needs 7 us before its first result and 1 us per 64 keys then, one of the mma.sync kernel 5 us and
+    # more per key; a chip full of them meets at fewer keys. Measured on B200 (warm, mma.sync -> tcgen05; without options, with sinks), 32 / 8
+    # heads: one prompt of 64 tokens 6.2 -> 8.8, 7.8 -> 9.9; 128: 8.6 -> 9.9, 11.6 -> 11.0; 160: 11.4 -> 11.3, 15.2 -> 12.4; 192: 11.9 -> 11.1, 16.2
+    # -> 12.0; 16 prompts of 96 23.5 -> 20.7, 31.1 -> 23.4; 16 / 16 heads: 16 of 96 15.6 -> 12.2, 20.8 -> 14.0, 48 of 64 18.0 -> 21.9, 25.0 -> 25.6;
+    # 32 / 8 heads, prompts of 682, 1463 and 1951 tokens 390 -> 111. Without options the mma.sync kernel stays where the reach is not known.
+    far = options if reach is None else reach > 128 or reach > 64 and n_tiles * n_kv >= 192
+    if far and _prefill_on_tcgen05(q, kcache, vcache, out, hd, vd):
         from .gemm import scratch
         _lib.check(_lib.lib().dmoe_prefill_attention_tc(
             _vp(q), c_ll(q.stride(0)), _vp(kcache), _vp(vcache), c_int(kcache.shape[0]), _vp(block_tables),
             c_int(block_tables.stride(0)), _vp(tiles), c_int(n_tiles), c_int(kcache.shape[1]), c_int(n_q), c_int(n_kv),
             c_float(scale), c_int(window or 0), c_int(chunk or 0), c_float(softcap or 0.0), _vp(sink),
-            _vp(out), c_ll(out.stride(0)), ctypes.byref(x) if x else None, _vp(scratch(q.device).status), _st()),
-            "dmoe_prefill_attention_tc")
+            _vp(out), c_ll(out.stride(0)), ctypes.byref(x) if x else None, c_int(0 if options else 1), _vp(scratch(q.device).status),
+            _st()), "dmoe_prefill_attention_tc")
         return out
     if options:
         _lib.check(_lib.lib().dmoe_prefill_attention_ext(

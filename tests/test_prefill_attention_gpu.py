@@ -78,6 +78,19 @@ def test_short_reach(opt):
     _close(*_run(8, 2, 16, segs=segs, reach=90, **opt), tol=2 ** -7)
 
 
+@pytest.mark.parametrize("n_q,n_kv", [(2, 2), (8, 2), (8, 1)])
+@pytest.mark.parametrize("scale", [None, 0.7])
+def test_without_options(n_q, n_kv, scale):
+    """Long prompts take this kernel, others (or of unknown reach) the mma.sync one: both round the weights to bf16 in the same places."""
+    opt = {} if scale is None else dict(scale=scale)
+    (far, ref), (near, _) = (_run(n_q, n_kv, 16, reach=r, **opt) for r in (129, 128))
+    # fp32 weights would give 2^-7 as above; bf16 weights add 2^-9 of the absolute sum of the weighted values
+    _close(far, ref, tol=2 ** -6)
+    # sums in another order: now and then an output on the other side of a tie, one unit of the last place or 2^-7 apart
+    _close(far, near, tol=2 ** -7)
+    assert float((far != near).float().mean()) < 0.05
+
+
 def test_many_key_blocks():
     """Two CTAs per SM, each with up to 32 key blocks: scores of a block take the place of the weights before."""
     # fp32 softmax weights: one rounding of the output, 2^-9 relative, and twice that for the bf16 reference it is compared in
