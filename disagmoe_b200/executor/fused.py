@@ -17,6 +17,7 @@ from __future__ import annotations
 
 from typing import Dict, List, Optional
 
+import numpy as np
 import torch
 
 from ..config import CacheConfig, ModelConfig
@@ -25,6 +26,7 @@ from ..models.attention import AttnMeta, MoEAttention
 from ..models.experts import MoEExperts
 from ..ops import functional as F
 from ..ops import gemm
+from ..ops._lib import Uploads
 from .step import StepExecutor, TokenBuffers
 
 
@@ -40,8 +42,8 @@ class StepBuffers(TokenBuffers):
         self.dispatch = F.DispatchBuffers(cap * k, H, E, device, dtype)
         self.parts_base = torch.tensor([self.parts.data_ptr()], dtype=torch.int64, device=device)
         # prompt segments of the current step for the tiled causal attention kernel (filled by prefill())
-        self.prefill_tiles = z(cap, 4, dt=torch.int32)
-        self.ctx_len_decode = z(cap, dt=torch.int32)
+        self.prefill_tiles: Optional[torch.Tensor] = None
+        self.ctx_len_decode: Optional[torch.Tensor] = None
         self.n_prefill_tiles = 0
         self.n_loose: Optional[int] = None
         self.reach: Optional[int] = None
@@ -95,7 +97,7 @@ class FusedModelExecutor(StepExecutor):
         cfg = self.cfg
         meta = AttnMeta(buf.positions[:T], buf.slots[:T], self.block_tables, buf.bt_row[:T], buf.ctx_len[:T],
                         max_ctx=max_ctx, prefill_tiles=buf.prefill_tiles, n_prefill_tiles=buf.n_prefill_tiles,
-                        ctx_len_decode=buf.ctx_len_decode[:T], n_loose=buf.n_loose, prefill_reach=buf.reach)
+                        ctx_len_decode=buf.ctx_len_decode, n_loose=buf.n_loose, prefill_reach=buf.reach)
         resid = buf.resid[:T]
         F.embed(buf.ids[:T], self.embed_w, out=resid)
         parts = None
@@ -123,18 +125,16 @@ class FusedModelExecutor(StepExecutor):
         F.argmax(logits, out=buf.next_ids[:T])
         return buf.next_ids[:T], (logits if want_logits else None)
 
-    def _begin_prefill(self, buf: StepBuffers, T: int, positions, ctx_len, bt_row) -> None:
+    def _begin_prefill(self, buf: StepBuffers, T: int, positions, ctx_len, bt_row, up: Uploads) -> None:
         buf.n_prefill_tiles = 0
         if self.device.type == "cuda":
             a0 = self.attn[self.layer_ids[0]]
-            tiles, covered = F.build_prefill_tiles(bt_row, positions, F.prefill_tile_tokens(a0.num_heads, a0.num_kv_heads))
+            rows, pos = np.asarray(bt_row), np.asarray(positions)
+            tiles, covered = F.prefill_tiles(F.token_runs(rows, pos), rows, pos, F.prefill_tile_tokens(a0.num_heads, a0.num_kv_heads))
             if len(tiles):
-                buf.n_prefill_tiles, buf.n_loose = len(tiles), F.loose_rows(covered)
-                buf.prefill_tiles[:len(tiles)].copy_(tiles.pin_memory(), non_blocking=True)
-                cd = torch.as_tensor(ctx_len).clone()
-                buf.reach = int(cd[covered].max())
-                cd[covered] = 0
-                buf.ctx_len_decode[:T].copy_(cd.pin_memory(), non_blocking=True)
+                ctx = np.asarray(ctx_len)
+                buf.n_prefill_tiles, buf.n_loose, buf.reach = len(tiles), F.loose_rows(covered), int(ctx[covered].max())
+                buf.prefill_tiles, buf.ctx_len_decode = up(tiles), up(np.where(covered, 0, ctx).astype(np.int32))
 
     def _end_prefill(self, buf: StepBuffers) -> None:
-        buf.n_prefill_tiles, buf.n_loose, buf.reach = 0, None, None
+        buf.n_prefill_tiles, buf.n_loose, buf.reach, buf.prefill_tiles, buf.ctx_len_decode = 0, None, None, None, None

@@ -19,6 +19,7 @@ from __future__ import annotations
 import math
 from typing import Dict, List, Optional, Tuple
 
+import numpy as np
 import torch
 
 from ..config import AttentionSpec, LatentAttentionSpec, SideBySideSpec
@@ -27,7 +28,7 @@ from ..models.mixers import (GatedFeedForward, LatentTables, RoutedBuffers, Rout
                              make_mixer)
 from ..ops import functional as F
 from ..ops import gemm
-from ..ops._lib import upload
+from ..ops._lib import Uploads
 from ..ops.recurrent import MAX_TAPS, RecurrentState, SegmentTables, build_segments, decode_segments
 from .step import StepExecutor, TokenBuffers
 
@@ -143,12 +144,13 @@ class LayerListExecutor(StepExecutor):
         return LayerListBuffers(self.cfg, cap, self.device, self.dtype, min(cap, self.max_batch_size), self.mixers)
 
     # ---- one iteration ----------------------------------------------------------------------------------------------
-    def _begin_prefill(self, buf: LayerListBuffers, T: int, positions, ctx_len, bt_row) -> None:
-        buf.segments = build_segments(bt_row, positions, self.device)
+    def _begin_prefill(self, buf: LayerListBuffers, T: int, positions, ctx_len, bt_row, up: Uploads) -> None:
+        rows, pos = np.asarray(bt_row), np.asarray(positions)
+        runs = F.token_runs(rows, pos)
+        buf.segments = build_segments(rows, pos, self.device, runs, up)
         buf.prefill_tiles, buf.ctx_len_decode, buf.n_untiled = {}, None, T
-        buf.latent = {k: LatentTables.prefill(m, bt_row, positions, self.device, self.dtype)
-                      for k, m in self.latent_specs.items()}
-        buf.block_offs = self._block_offs(T)
+        buf.latent = {k: LatentTables.prefill(m, rows, pos, self.device, self.dtype, runs, up) for k, m in self.latent_specs.items()}
+        buf.block_offs = self._block_offs(T, up)
         built, longest = {}, 0
         for mixer in self.attentions:
             m = mixer.spec
@@ -156,16 +158,16 @@ class LayerListExecutor(StepExecutor):
                 continue
             n = F.prefill_tile_tokens(m.heads, m.kv_heads)
             if n not in built:
-                built[n] = F.build_prefill_tiles(bt_row, positions, n)
+                built[n] = F.prefill_tiles(runs, rows, pos, n)
             tiles, covered = built[n]
             if not len(tiles):
                 continue
             if n not in buf.prefill_tiles:
-                buf.prefill_tiles[n] = (upload(tiles, self.device), len(tiles), {})
-                cd = torch.as_tensor(ctx_len).clone()
-                longest = int(cd[covered].max())
-                cd[covered] = 0              # which rows are tiled does not depend on the tile size
-                buf.ctx_len_decode, buf.n_untiled = upload(cd, self.device), F.loose_rows(covered)
+                buf.prefill_tiles[n] = (up(tiles), len(tiles), {})
+                if buf.ctx_len_decode is None:      # which rows are tiled does not depend on the tile size
+                    ctx = np.asarray(ctx_len)
+                    longest = int(ctx[covered].max())
+                    buf.ctx_len_decode, buf.n_untiled = up(np.where(covered, 0, ctx).astype(np.int32)), F.loose_rows(covered)
             reach = buf.prefill_tiles[n][2]
             if (m.window, m.chunk) not in reach:
                 reach[m.window, m.chunk] = F.tile_reach(longest, n, m.window, m.chunk)
@@ -173,14 +175,16 @@ class LayerListExecutor(StepExecutor):
     def _end_prefill(self, buf: LayerListBuffers) -> None:
         buf.segments, buf.prefill_tiles, buf.ctx_len_decode, buf.latent, buf.block_offs = None, {}, None, {}, {}
 
-    def _block_offs(self, T: int) -> Dict[int, torch.Tensor]:
-        return {n: upload(torch.arange(n + 1, dtype=torch.int32) * T, self.device) for n in self.blocks_of_rows}
+    def _block_offs(self, T: int, up: Uploads) -> Dict[int, torch.Tensor]:
+        return {n: up(np.arange(n + 1, dtype=np.int32) * np.int32(T)) for n in self.blocks_of_rows}
 
     def _decode_tables(self, T: int) -> Tuple[Dict[Tuple, LatentTables], Dict[int, torch.Tensor]]:
         """Latent tables and block offsets, made once per batch size: graphs replay on them."""
         if T not in self.decode_tables:
-            self.decode_tables[T] = ({k: LatentTables.decode(m, T, self.device) for k, m in self.latent_specs.items()},
-                                     self._block_offs(T))
+            up = Uploads(self.device)
+            self.decode_tables[T] = ({k: LatentTables.decode(m, T, self.device, up) for k, m in self.latent_specs.items()},
+                                     self._block_offs(T, up))
+            up.flush()
             if self.device.type == "cuda":
                 torch.cuda.current_stream(self.device).synchronize()      # the uploads: other streams read the tables as well
         return self.decode_tables[T]

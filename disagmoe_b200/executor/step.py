@@ -6,6 +6,7 @@ from __future__ import annotations
 
 from typing import Dict, List, Optional
 
+import numpy as np
 import torch
 
 from ..config import CacheConfig, ModelConfig
@@ -47,6 +48,7 @@ class StepExecutor:
         self.graphs: Dict[int, torch.cuda.CUDAGraph] = {}
         self.graph_sizes: List[int] = []
         self.graph_launches: Dict[int, int] = {}
+        self.table_ints = 1 << 14             # room for the host tables of a prompt step; grows with them
 
     # ---- supplied by a model family -----------------------------------------------------------------------------
     def _load(self, state_dict) -> None:
@@ -65,8 +67,8 @@ class StepExecutor:
         """Runs the first T rows of ``buf``; returns (next ids, logits or None) of ``buf.out_rows`` (or of all rows)."""
         raise NotImplementedError
 
-    def _begin_prefill(self, buf: TokenBuffers, T: int, positions, ctx_len, bt_row) -> None:
-        """Host-side tables of a packed batch of prompt (and decode) rows."""
+    def _begin_prefill(self, buf: TokenBuffers, T: int, positions, ctx_len, bt_row, up: _lib.Uploads) -> None:
+        """Host-side tables of a packed batch of prompt (and decode) rows; the caller flushes their uploads."""
 
     def _end_prefill(self, buf: TokenBuffers) -> None:
         """Undoes ``_begin_prefill``: the decode path (and its graphs) may share the buffers."""
@@ -109,9 +111,12 @@ class StepExecutor:
         self._fill(buf, T, ids, positions, slots, ctx_len, bt_row)
         if buf.copied is not None:
             buf.copied.record(torch.cuda.current_stream(self.device))
-        self._begin_prefill(buf, T, positions, ctx_len, bt_row)
+        up = _lib.Uploads(self.device, self.table_ints)
+        self._begin_prefill(buf, T, positions, ctx_len, bt_row, up)
         if out_rows is not None:
-            buf.out_rows = _lib.upload(torch.tensor(out_rows, dtype=torch.int32), self.device)
+            buf.out_rows = up(np.array(out_rows, dtype=np.int32))
+        up.flush()
+        self.table_ints = max(self.table_ints, up.ints)
         try:
             return self._forward(buf, T, int(ctx_len.max()), want_logits)
         finally:

@@ -17,7 +17,7 @@ from ..config import (AttentionSpec, ChannelDeltaSpec, GatedLinearSpec, GatedUni
                       LayerListConfig, MatrixMemorySpec, SideBySideSpec, WkvSpec)
 from ..ops import functional as F
 from ..ops import gemm
-from ..ops._lib import upload
+from ..ops._lib import Uploads
 from ..ops.recurrent import (GatedUnit, Recurrence, RecurrentState, SegmentTables, recurrent_attention, unit_recurrence)
 from .attention import AttnMeta
 from .experts import ExpertStack
@@ -65,31 +65,38 @@ class LatentTables:
         return m.heads, m.window, latent_layout(m).min_run(), m.gate      # gated layers write the weights of the records
 
     @staticmethod
-    def _per_head(rows: torch.Tensor, heads: int, device):
+    def _per_head(rows: np.ndarray, heads: int, up: Uploads):
         """Tables of the per-head GEMMs over [heads, n, .] rows whose outputs go to rows (batch row, head)."""
         n = len(rows)
-        recs = torch.zeros(heads * n, 4, dtype=torch.int32)
-        recs[:, 1] = (rows[None].long() * heads + torch.arange(heads)[:, None]).reshape(-1).int()
-        recs[:, 2] = torch.ones(1).view(torch.int32)
-        return upload(torch.arange(heads + 1, dtype=torch.int32) * n, device), upload(recs, device)
+        recs = np.zeros((heads * n, 4), dtype=np.int32)
+        recs[:, 1] = (rows[None] * heads + np.arange(heads, dtype=np.int32)[:, None]).reshape(-1)
+        recs[:, 2] = np.ones(1, dtype=np.float32).view(np.int32)
+        return up(np.arange(heads + 1, dtype=np.int32) * np.int32(n)), up(recs)
 
     @classmethod
-    def decode(cls, m: LatentAttentionSpec, T: int, device) -> "LatentTables":
-        return cls(T, None, None, *cls._per_head(torch.arange(T), m.heads, device))
+    def decode(cls, m: LatentAttentionSpec, T: int, device, up: Optional[Uploads] = None) -> "LatentTables":
+        """``up``: uploads that the caller flushes."""
+        own = up or Uploads(device, 8 * T * m.heads + 64)
+        t = cls(T, None, None, *cls._per_head(np.arange(T, dtype=np.int32), m.heads, own))
+        if up is None:
+            own.flush()
+        return t
 
     @classmethod
-    def prefill(cls, m: LatentAttentionSpec, bt_row, positions, device, dtype) -> "LatentTables":
+    def prefill(cls, m: LatentAttentionSpec, bt_row, positions, device, dtype, runs=None, up: Optional[Uploads] = None) -> "LatentTables":
+        """``runs``: :func:`ops.functional.token_runs` of the batch where these are known; ``up`` as in :meth:`decode`."""
         lay, T = latent_layout(m), len(positions)
         if not (device.type == "cuda" and lay.tiled(dtype)):
-            return cls.decode(m, T, device)
-        tiles, covered = F.build_prefill_tiles(bt_row, positions, 128, lay.min_run())
-        if len(tiles) == 0:
-            return cls.decode(m, T, device)
-        rows = (~covered).nonzero()[:, 0].int()
-        loose = torch.full((T,), -1, dtype=torch.int32)
-        loose[rows.long()] = torch.arange(len(rows), dtype=torch.int32)
+            return cls.decode(m, T, device, up)
+        bt_row, positions = np.asarray(bt_row), np.asarray(positions)
+        tl, covered = F.prefill_tiles(F.token_runs(bt_row, positions) if runs is None else runs, bt_row, positions, 128, lay.min_run())
+        if len(tl) == 0:
+            return cls.decode(m, T, device, up)
+        own = up or Uploads(device)
+        rows = np.nonzero(~covered)[0].astype(np.int32)
+        loose = np.full(T, -1, dtype=np.int32)
+        loose[rows] = np.arange(len(rows), dtype=np.int32)
         # runs of tiles: the keys of a run start a window before its first token and end with its last
-        tl = tiles.numpy()
         n, row, pos = tl[:, 1], tl[:, 2], tl[:, 3]
         begins = np.nonzero(np.r_[True, (row[1:] != row[:-1]) | (pos[1:] != pos[:-1] + n[:-1])])[0]
         ends = np.r_[begins[1:], len(tl)] - 1
@@ -99,13 +106,13 @@ class LatentTables:
         keys = np.empty((at[-1], 2), dtype=np.int32)
         for i, (a, b) in enumerate(zip(at[:-1], at[1:])):
             keys[a:b, 0], keys[a:b, 1] = row[begins[i]], np.arange(lo[i], hi[i])
-        base = torch.from_numpy(np.repeat(at[:-1] - lo, ends - begins + 1).astype(np.int32))
-        keys = torch.from_numpy(keys)
-        up = lambda x: upload(x, device)
-        t = cls(len(rows), up(loose), up(rows), None, None, up(tiles), up(base), len(tiles),
-                F.tile_reach(int(hi.max()), 128, m.window), up(keys), len(keys))
+        base = np.repeat(at[:-1] - lo, ends - begins + 1).astype(np.int32)
+        t = cls(len(rows), own(loose), own(rows), None, None, own(tl), own(base), len(tl),
+                F.tile_reach(int(hi.max()), 128, m.window), own(keys), len(keys))
         if len(rows):
-            t.offs, t.recs = cls._per_head(rows, m.heads, device)
+            t.offs, t.recs = cls._per_head(rows, m.heads, own)
+        if up is None:
+            own.flush()
         return t
 
 

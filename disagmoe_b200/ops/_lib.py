@@ -8,6 +8,7 @@ from __future__ import annotations
 import ctypes
 import os
 
+import numpy as np
 import torch
 
 _LIB = None
@@ -137,14 +138,40 @@ def lib():
 
 def stream_ptr() -> int:
     """The current stream of the current device, without the Python stream object (every launch asks for it)."""
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
-def upload(t: torch.Tensor, device) -> torch.Tensor:
-    """A host table on the device. To a GPU it goes through pinned memory, in stream order: a copy from pageable memory makes the
-    host wait for everything that is queued, and a step has several tables."""
-    kind = getattr(device, "type", None) or torch.device(device).type
-    return t.pin_memory().to(device, non_blocking=True) if kind == "cuda" and torch.cuda.is_available() else t.to(device)
+class Uploads:
+    """The host tables of one step on the device by one copy instead of one per table (a copy and its pinned buffer cost 20 us of host
+    time, and a copy from pageable memory would wait for everything that is queued): a call takes an int32 array and returns the device tensor that :meth:`flush` fills, in stream order. The staging memory is
+    allocated per step; torch keeps it until the copy that reads it is done. On the CPU the arrays themselves."""
+
+    def __init__(self, device, ints: int = 1 << 14):
+        self.device = torch.device(device) if isinstance(device, str) else device
+        self.cuda = self.device.type == "cuda" and torch.cuda.is_available()
+        self.ints, self.at, self.host = ints, 0, None
+
+    def __call__(self, a: np.ndarray) -> torch.Tensor:
+        assert a.dtype == np.int32
+        if not self.cuda:
+            return torch.from_numpy(np.ascontiguousarray(a))
+        n = a.size
+        if self.host is None or self.at + n > self.ints:
+            self.flush()
+            self.ints = max(self.ints, n)
+            self.host = torch.empty(self.ints, dtype=torch.int32, pin_memory=True)
+            self.view, self.dev = self.host.numpy(), torch.empty(self.ints, dtype=torch.int32, device=self.device)
+        at = self.at
+        self.view[at:at + n] = a.reshape(-1)
+        self.at = at + (n + 3 & ~3)               # tables start on 16-byte boundaries
+        t = self.dev[at:at + n]
+        return t if a.ndim == 1 else t.view(a.shape)
+
+    def flush(self) -> None:
+        if self.at:
+            n = min(self.at, self.ints)
+            self.dev[:n].copy_(self.host[:n], non_blocking=True)
+        self.at, self.host = 0, None
 
 
 LAUNCHES = 0   # entry-point calls that launched kernels of this library (a graph replay adds its captured count)

@@ -455,9 +455,10 @@ def prefill_tile_tokens(n_q: int, n_kv: int) -> int:
     return 128 // (n_q // n_kv) if n_q % n_kv == 0 and n_q // n_kv <= 64 else 0
 
 
-def loose_rows(covered: torch.Tensor) -> int:
+def loose_rows(covered) -> int:
     """How many leading rows of a batch the per-token kernel has to look at: up to the last one that no tile covers."""
-    rows = (~covered).nonzero()
+    import numpy as np
+    rows = np.nonzero(~np.asarray(covered))[0]
     return int(rows[-1]) + 1 if len(rows) else 0
 
 
@@ -472,11 +473,27 @@ def _prefill_on_tcgen05(q, kcache, vcache, out, hd: int, vd: int) -> bool:
 def token_runs(bt_row, positions):
     """(first row, end row) of every run of consecutive rows of one sequence at consecutive positions."""
     import numpy as np
-    rows, pos = np.asarray(bt_row, dtype=np.int64), np.asarray(positions, dtype=np.int64)
+    rows, pos = np.asarray(bt_row), np.asarray(positions)
     if len(rows) == 0:
         return []
-    brk = np.nonzero((rows[1:] != rows[:-1]) | (pos[1:] != pos[:-1] + 1))[0] + 1
-    return list(zip([0] + brk.tolist(), brk.tolist() + [len(rows)]))
+    brk = (np.nonzero((rows[1:] != rows[:-1]) | (pos[1:] != pos[:-1] + 1))[0] + 1).tolist()
+    return list(zip([0] + brk, brk + [len(rows)]))
+
+
+def prefill_tiles(runs, rows, pos, tile_tokens: int, min_len: int = 8):
+    """:func:`build_prefill_tiles` of runs that are known (:func:`token_runs`), on numpy arrays."""
+    import numpy as np
+    covered, tiles = np.zeros(len(rows), dtype=bool), []
+    for a, b in runs if tile_tokens > 0 else ():
+        if b - a < min_len:
+            continue
+        covered[a:b] = True
+        t = np.empty((-(-(b - a) // tile_tokens), 4), dtype=np.int32)
+        t0 = t[:, 0] = np.arange(a, b, tile_tokens)
+        t[:, 1], t[:, 2], t[:, 3] = tile_tokens, rows[a], pos[t0]
+        t[-1, 1] = b - t0[-1]
+        tiles.append(t)
+    return (np.concatenate(tiles) if tiles else np.zeros((0, 4), dtype=np.int32)), covered
 
 
 def build_prefill_tiles(bt_row, positions, tile_tokens: int, min_len: int = 8):
@@ -487,21 +504,9 @@ def build_prefill_tiles(bt_row, positions, tile_tokens: int, min_len: int = 8):
     rows go to the tiled kernel. Returns (tiles int32 CPU tensor [n, 4] = (first row, tokens, block-table row, first
     position), covered bool CPU tensor [T]): rows not covered stay with the per-token kernel."""
     import numpy as np
-    rows = np.asarray(bt_row, dtype=np.int64)
-    pos = np.asarray(positions, dtype=np.int64)
-    T = len(rows)
-    covered = np.zeros(T, dtype=bool)
-    tiles = []
-    if T == 0 or tile_tokens <= 0:
-        return torch.zeros(0, 4, dtype=torch.int32), torch.from_numpy(covered)
-    for a, b in token_runs(rows, pos):
-        if b - a < min_len:
-            continue
-        covered[a:b] = True
-        t0 = np.arange(a, b, tile_tokens)
-        tiles.append(np.stack([t0, np.minimum(tile_tokens, b - t0), np.full_like(t0, rows[a]), pos[t0]], 1))
-    t = torch.from_numpy(np.concatenate(tiles).astype(np.int32)) if tiles else torch.zeros(0, 4, dtype=torch.int32)
-    return t, torch.from_numpy(covered)
+    rows, pos = np.asarray(bt_row, dtype=np.int64), np.asarray(positions, dtype=np.int64)
+    tiles, covered = prefill_tiles(token_runs(rows, pos), rows, pos, tile_tokens, min_len)
+    return torch.from_numpy(tiles), torch.from_numpy(covered)
 
 
 def tile_reach(longest: int, tile_tokens: int, window: Optional[int] = None, chunk: Optional[int] = None) -> int:

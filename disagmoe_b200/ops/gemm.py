@@ -31,7 +31,7 @@ _num_sms_cache = {}
 
 def num_sms(device=None) -> int:
     """SM count of a CUDA device (read once per device)."""
-    idx = torch.device(device).index if device is not None else None
+    idx = None if device is None else device.index if isinstance(device, torch.device) else torch.device(device).index
     if idx is None:
         idx = torch.cuda.current_device() if torch.cuda.is_available() else -1
     if idx not in _num_sms_cache:
@@ -57,7 +57,7 @@ _scratch = {}
 
 
 def scratch(device) -> _Scratch:
-    key = torch.device(device).index or 0
+    key = (device.index if isinstance(device, torch.device) else torch.device(device).index) or 0
     if key not in _scratch:
         _scratch[key] = _Scratch(torch.device("cuda", key))
     return _scratch[key]

@@ -49,20 +49,25 @@ class SegmentTables:
         return self.singles.tolist() + self.multi.tolist()
 
 
-def build_segments(bt_row, positions, device) -> SegmentTables:
-    """Tables of a batch given on the host (rows of one sequence are consecutive, as every scheduler emits them)."""
+def build_segments(bt_row, positions, device, runs=None, up: Optional[_lib.Uploads] = None) -> SegmentTables:
+    """Tables of a batch given on the host (rows of one sequence are consecutive, as every scheduler emits them). ``runs``: its
+    :func:`token_runs` where these are known; ``up``: uploads that the caller flushes."""
     rows, pos = np.asarray(bt_row), np.asarray(positions)
     singles, multi, chunks = [], [], []
-    for a, b in token_runs(rows, pos):
+    for a, b in token_runs(rows, pos) if runs is None else runs:
         seg = (a, b - a, int(rows[a]), int(pos[a]))
         if b - a == 1:
             singles.append(seg)
             continue
         chunks += [(c, min(CHUNK, b - c), len(multi), i) for i, c in enumerate(range(a, b, CHUNK))]
         multi.append(seg)
-    table = torch.from_numpy(np.array(singles + multi + chunks, dtype=np.int32).reshape(-1, 4))
-    if torch.device(device).type == "cuda":
-        table = _lib.upload(table, device)
+    table = np.array(singles + multi + chunks, dtype=np.int32).reshape(-1, 4)
+    if up is None:
+        up = _lib.Uploads(device, max(4, table.size))
+        table = up(table)
+        up.flush()
+    else:
+        table = up(table)
     s, m = len(singles), len(multi)
     return SegmentTables(s, m, len(chunks), max((x[1] for x in multi), default=0), table[:s], table[s:s + m], table[s + m:])
 
