@@ -165,7 +165,8 @@ typedef struct DmoeGemm {
   float act_limit;
   int act_cols;
   int unit_weights;   // combine: the records' weights are left out
-  // != 0: the tokens are the M operand (gemm_wide.cu: CTA pairs on tiles of 256 tokens x 256 weight rows) where the launch
+  // != 0: the tokens are the M operand (gemm_wide.cu: CTA pairs on tiles of 256 tokens x 256 weight rows, or x `wide` of them where
+  // that is more than 1: a multiple of 32 up to 256, of the head size with rope_table, 256 with w_blocked) where the launch
   // allows it: no multi-GPU hooks, splitk <= 1, no pair, 16-byte aligned output rows; other launches ignore it. bn, streamk,
   // ws and counters are unused then.
   int wide;

@@ -12,7 +12,8 @@
 //
 // Warp roles (192 threads per CTA): warp 0 TMA producer (its own CTA's operands), warp 1 TMEM owner and, in the even CTA,
 // MMA issuer for both, warps 2..5 epilogue of the CTA's 128 accumulator lanes. Two accumulators of 256 columns fill TMEM:
-// the epilogue of a tile runs under the next one's main loop. Persistent: pair p runs tiles p, p + pairs, ...; tiles are
+// the epilogue of a tile runs under the next one's main loop. Dense launches may take tiles of fewer weight rows (any multiple of
+// 32), so that their count fills whole waves of pairs. Persistent: pair p runs tiles p, p + pairs, ...; tiles are
 // numbered group after group with the token tile fastest, so that concurrent pairs share a weight tile in L2.
 //
 // Measured on B200 against gemm.cu, see ops/gemm.py: want_wide, which holds the rule that chooses between the two.
@@ -24,16 +25,16 @@ namespace dmoe {
 
 constexpr int kWThreads = 192;
 constexpr int kWTokens = 2 * kBM;                        // tokens per tile
-constexpr int kWCols = 256;                              // accumulator columns = weight rows per tile
+constexpr int kWCols = 256;                              // accumulator columns = weight rows per tile, at most
 constexpr int kWSub = 2;                                 // K blocks per stage
-constexpr int kWStages = 3;
-constexpr int kWOperandBytes = kBM * kBK * 2;            // 128 rows x 64 bf16: one CTA's tokens or its half of the weights
-constexpr int kWSubBytes = 2 * kWOperandBytes;           // tokens, then weights of one K block
-constexpr int kWStageBytes = kWSub * kWSubBytes;
+constexpr int kWMaxStages = 4;
+constexpr int kWStageRoom = 208 * 1024;                  // three stages of 256 or four of 160 columns
+constexpr int kWOperandBytes = kBM * kBK * 2;            // 128 rows x 64 bf16: one CTA's tokens
 constexpr int kWBarBytes = 256;
-constexpr int kWSmemBytes = kWStages * kWStageBytes + 1024 /*alignment slack*/ + kWBarBytes + (2 * kMaxGroups + 1) * 4;
+constexpr int kWSmemBytes = kWStageRoom + 1024 /*alignment slack*/ + kWBarBytes + (2 * kMaxGroups + 1) * 4;
 
 struct WideArgs {
+  int cols, stages;      // weight rows per tile: a multiple of 32 up to kWCols
   const int* offs;
   int G, T, F, K, w_rows, w_blocked;
   void* Y;
@@ -92,26 +93,28 @@ __global__ void __launch_bounds__(kWThreads, 1)
 gemm_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const WideArgs a) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + kWStages * kWStageBytes);
-  uint64_t* empty_bar = full_bar + kWStages;
-  uint64_t* tfull_bar = empty_bar + kWStages;      // [2]
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + kWStageRoom);
+  uint64_t* empty_bar = full_bar + kWMaxStages;
+  uint64_t* tfull_bar = empty_bar + kWMaxStages;      // [2]
   uint64_t* tempty_bar = tfull_bar + 2;            // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
   int* abort_word = reinterpret_cast<int*>(tmem_slot + 1);
-  int* s_start = reinterpret_cast<int*>(smem + kWStages * kWStageBytes + kWBarBytes);      // [G] first row
+  int* s_start = reinterpret_cast<int*>(smem + kWStageRoom + kWBarBytes);      // [G] first row
   int* s_tile0 = s_start + kMaxGroups;                                                     // [G + 1] first tile
 
   const int prank = __shfl_sync(0xffffffffu, static_cast<int>(cluster_ctarank()), 0);
   const bool leader = prank == 0;
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
-  constexpr int kFeat = EPI == EPI_SWIGLU ? kWCols / 2 : kWCols;      // output features per tile
-  const int NT = (a.F + kFeat - 1) / kFeat;
+  const int feat = EPI == EPI_SWIGLU ? a.cols / 2 : a.cols;           // output features per tile
+  const int half = a.cols / 2, w_bytes = half * kBK * 2;              // weight rows that a CTA stages
+  const int sub_bytes = kWOperandBytes + w_bytes, stage_bytes = kWSub * sub_bytes;      // tokens, then weights of one K block
+  const int NT = (a.F + feat - 1) / feat;
   const int kblocks = (a.K + kBK - 1) / kBK;
 
   if (threadIdx.x == 0) {
     *abort_word = 0;
-    for (int s = 0; s < kWStages; ++s) {
+    for (int s = 0; s < a.stages; ++s) {
       mbar_init(smem_u32(&full_bar[s]), 1);
       mbar_init(smem_u32(&empty_bar[s]), 1);
     }
@@ -183,18 +186,18 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       // a weight tile that one token tile reads streams through L2, one that several read stays
       const bool once = __shfl_sync(0xffffffffu, s_tile0[u.g + 1] - s_tile0[u.g], 0) == NT;
       const int xrow = __shfl_sync(0xffffffffu, u.row0, 0) + prank * kBM;
-      const int wrow = __shfl_sync(0xffffffffu, u.g * a.w_rows + u.n * kFeat, 0) + prank * (EPI == EPI_SWIGLU ? a.F : kBM);
+      const int wrow = __shfl_sync(0xffffffffu, u.g * a.w_rows + u.n * feat, 0) + prank * (EPI == EPI_SWIGLU ? a.F : half);
       for (int i = 0; i < steps; ++i) {
         ok = mbar_wait_warp(smem_u32(&empty_bar[stage]), phase ^ 1, abort_word);
         if (!ok) break;
-        const uint32_t fb = full0 + 8 * stage, st = smem_u32(smem) + stage * kWStageBytes;
+        const uint32_t fb = full0 + 8 * stage, st = smem_u32(smem) + stage * stage_bytes;
         const int kb = i * kWSub, n = min(kWSub, kblocks - kb);
         if (elect_one()) {
-          if (leader) mbar_expect_tx(smem_u32(&full_bar[stage]), n * (both ? 4 : 3) * kWOperandBytes);
+          if (leader) mbar_expect_tx(smem_u32(&full_bar[stage]), n * ((both ? 2 : 1) * kWOperandBytes + 2 * w_bytes));
 #pragma unroll
           for (int j = 0; j < kWSub; ++j) {
             if (j < n) {
-              const uint32_t sx = st + j * kWSubBytes;
+              const uint32_t sx = st + j * sub_bytes;
               const int x = a.w_blocked ? 0 : (kb + j) * kBK, y = a.w_blocked ? (wrow / kBM * kblocks + kb + j) * kBM : wrow;
               tma_load_2d_pair(sx + kWOperandBytes, &tmW, x, y, fb, once ? pol_first : pol_last);
               if (mine) tma_load_2d_pair(sx, &tmX, (kb + j) * kBK, xrow, fb, pol_last);
@@ -202,13 +205,13 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
           }
         }
         __syncwarp();
-        if (++stage == kWStages) { stage = 0; phase ^= 1; }
+        if (++stage == a.stages) { stage = 0; phase ^= 1; }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (the even CTA's)
     if (leader) {
-      constexpr uint32_t idesc = umma_idesc_bf16(2 * kBM, kWCols);
+      const uint32_t idesc = umma_idesc_bf16(2 * kBM, a.cols);
       const int tiles = __shfl_sync(0xffffffffu, s_tile0[a.G], 0);
       int stage = 0, it = 0;
       uint32_t phase = 0;
@@ -223,13 +226,13 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
           ok = mbar_wait_warp(smem_u32(&full_bar[stage]), phase, abort_word);
           if (!ok) break;
           tc_fence_after();
-          const uint32_t st = smem_u32(smem) + stage * kWStageBytes;
+          const uint32_t st = smem_u32(smem) + stage * stage_bytes;
           const int n = min(kWSub, kblocks - i * kWSub);
           if (elect_one()) {
 #pragma unroll
             for (int j = 0; j < kWSub; ++j) {
               if (j < n) {
-                const uint64_t da = umma_desc_sw128(st + j * kWSubBytes), db = umma_desc_sw128(st + j * kWSubBytes + kWOperandBytes);
+                const uint64_t da = umma_desc_sw128(st + j * sub_bytes), db = umma_desc_sw128(st + j * sub_bytes + kWOperandBytes);
 #pragma unroll
                 for (int k = 0; k < kBK / kUmmaK; ++k)
                   umma_f16_pair(d0, da + 2 * k, db + 2 * k, idesc, (i > 0 || j > 0 || k > 0) ? 1u : 0u);
@@ -238,7 +241,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
             umma_commit_both(smem_u32(&empty_bar[stage]));
           }
           __syncwarp();
-          if (++stage == kWStages) { stage = 0; phase ^= 1; }
+          if (++stage == a.stages) { stage = 0; phase ^= 1; }
         }
         if (ok && elect_one()) umma_commit_both(smem_u32(&tfull_bar[buf]));
         __syncwarp();
@@ -256,7 +259,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       const int first = prank * kBM + q * 32;      // first token of this warp inside the tile
       const bool ok_row = first + lane < u.ntok;
       const long long t = u.row0 + first + lane;
-      const int f0 = u.n * kFeat;
+      const int f0 = u.n * feat;
       const uint32_t back = mapa_rank(smem_u32(&tempty_bar[buf]), 0);
       // after a warp's last read of the accumulator
       const auto hand_back = [&]() {
@@ -269,27 +272,27 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         continue;
       }
       if (EPI == EPI_SWIGLU) {
-        const int chunks = min(kFeat / 32, (a.F - f0 + 31) / 32);
+        const int cols = min(feat, a.F - f0), chunks = (cols + 31) / 32;
         const float s = a.recs != nullptr && ok_row ? __int_as_float(__ldg(&a.recs[t].z)) : 1.f;
         __nv_bfloat16* y = static_cast<__nv_bfloat16*>(a.Y) + t * a.ldy + f0;
 #pragma unroll 1
         for (int c = 0; c < chunks; ++c) {
           uint32_t g[32], up[32];
           tmem_ld32(t0 + c * 32, g);
-          tmem_ld32(t0 + kFeat + c * 32, up);
+          tmem_ld32(t0 + feat + c * 32, up);
           tmem_ld_wait();
           if (c == chunks - 1) hand_back();
           float o[32], x[32];
 #pragma unroll
           for (int j = 0; j < 32; ++j) { o[j] = __uint_as_float(g[j]) * s; x[j] = __uint_as_float(up[j]) * s; }
           gated(o, x, a.act, a.act_limit);
-          if (ok_row) store32(y + c * 32, o, a.F - f0 - c * 32);
+          if (ok_row) store32(y + c * 32, o, cols - c * 32);
         }
       } else if (EPI == EPI_PLAIN && a.rope_table != nullptr) {
         // QKV: rotation partners are hd / 2 columns apart in the same lane. The accumulator is rounded to bf16 before the
         // rotation, as the unfused path stores and re-reads it. Whole heads: 256 columns hold 2 or 4 of them.
         const int half = a.hd >> 1, hc = half >> 5;              // 32-column chunks per half head
-        const int heads = min(kWCols, a.F - f0) / a.hd;
+        const int heads = min(a.cols, a.F - f0) / a.hd;
         int pos = ok_row ? __ldg(a.positions + t) : 0;
         pos = pos < 0 ? 0 : (pos >= a.rope_max_pos ? a.rope_max_pos - 1 : pos);
         const long long slot = ok_row && a.slots != nullptr ? __ldg(a.slots + t) : -1;
@@ -337,7 +340,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
           }
         }
       } else {
-        const int cols = min(kWCols, a.F - f0), chunks = (cols + 31) / 32;
+        const int cols = min(a.cols, a.F - f0), chunks = (cols + 31) / 32;
         int4 rec = make_int4(0, -1, 0, 0);
         __nv_bfloat16* y = nullptr;
         float w = 1.f;
@@ -450,6 +453,10 @@ static int launch_wide(const CUtensorMap& tmW, const CUtensorMap& tmX, const Wid
 int gemm_wide(const DmoeGemm* d, cudaStream_t stream) {
   WideArgs a;
   memset(&a, 0, sizeof(a));
+  a.cols = d->wide > 1 ? d->wide : kWCols;
+  if (a.cols < 64 || a.cols > kWCols || a.cols % 32 != 0 || (d->w_blocked && a.cols != kWCols) || (d->rope_table != nullptr && a.cols % d->hd != 0)) return -11;
+  const int sub = kWOperandBytes + a.cols / 2 * kBK * 2;
+  a.stages = kWStageRoom / (kWSub * sub) < kWMaxStages ? kWStageRoom / (kWSub * sub) : kWMaxStages;
   a.offs = d->offs;
   a.G = d->G; a.T = d->T; a.F = d->F; a.K = d->K;
   a.w_rows = d->epi == EPI_SWIGLU ? 2 * d->F : d->F;
@@ -469,11 +476,11 @@ int gemm_wide(const DmoeGemm* d, cudaStream_t stream) {
   const long long ldx = d->ldx > 0 ? d->ldx : d->K, rows = static_cast<long long>(d->G) * a.w_rows;
   if (a.w_blocked) {
     if (make_map_2d(&tmW, d->W, rows * (d->K / kBK), kBK, kBK, kBM) != 0) return -20;
-  } else if (make_map_2d(&tmW, d->W, rows, d->K, d->K, kBM) != 0) {
+  } else if (make_map_2d(&tmW, d->W, rows, d->K, d->K, a.cols / 2) != 0) {
     return -20;
   }
   if (make_map_2d(&tmX, d->X, d->T, d->K, ldx, kBM) != 0) return -21;
-  const int feat = d->epi == EPI_SWIGLU ? kWCols / 2 : kWCols;
+  const int feat = d->epi == EPI_SWIGLU ? a.cols / 2 : a.cols;
   // upper bound of the tile count (group sizes live on the device): every group may add one ragged tile
   const long long tiles = static_cast<long long>((d->F + feat - 1) / feat) * ((d->T + kWTokens - 1) / kWTokens + (d->offs ? d->G : 0));
   if (tiles > (1 << 30)) return -11;

@@ -143,8 +143,9 @@ def stream_ptr() -> int:
 
 class Uploads:
     """The host tables of one step on the device by one copy instead of one per table (a copy and its pinned buffer cost 20 us of host
-    time, and a copy from pageable memory would wait for everything that is queued): a call takes an int32 array and returns the device tensor that :meth:`flush` fills, in stream order. The staging memory is
-    allocated per step; torch keeps it until the copy that reads it is done. On the CPU the arrays themselves."""
+    time, and a copy from pageable memory would wait for everything that is queued): a call takes an int32 array and returns the
+    device tensor that :meth:`flush` fills, in stream order. The staging memory is allocated per step; torch keeps it until the
+    copy that reads it is done. On the CPU the arrays themselves."""
 
     def __init__(self, device, ints: int = 1 << 14):
         self.device = torch.device(device) if isinstance(device, str) else device

@@ -190,11 +190,22 @@ def want_wide(epi: int, T: int, F: int, K: int, G: int, sms: int) -> bool:
     return units >= sms or wide < 1.4 + dense_cost(T, F, K, sms)[0]
 
 
-def dense_wide_cost(T: int, F: int, K: int, epi: int, sms: int) -> float:
-    """us of a dense product in csrc/kernels/gemm_wide.cu, fitted to the sweep of :func:`split_plan` (within 6 % on average)."""
-    feat = 128 if epi == EPI_SWIGLU else 256
-    waves = -(-(-(-F // feat) * -(-T // 256)) // max(1, sms // 2))
-    return 2.7 + waves * (4.3 + 0.31 * -(-K // 64))
+@lru_cache(maxsize=4096)
+def dense_wide(T: int, F: int, K: int, epi: int, sms: int, hd: int = 0):
+    """(us, weight rows per tile) of a dense product in csrc/kernels/gemm_wide.cu: of the tile sizes the one whose count fills whole
+    waves of CTA pairs best; ``hd``: heads that a tile has to hold whole. Fitted to a sweep on B200 (42 sizes, T 66 .. 4096, K 16 .. 10944;
+    error 6 %, the choice is 0.8 % slower than the best size on average). Measured with 256 rows -> with the choice, us: 2500 x 2048 x 2048
+    27.9 -> 20.7 (80 tiles for 74 pairs -> 130 smaller ones), 2500 x 2048 x 5632 66.5 -> 45.4, 3000 x 2048 x 2048 27.8 -> 23.2, 2500 x 4096 x
+    2048 40.2 -> 34.6, 1111 x 6144 x 2048 30.7 -> 28.7, 724 x 3664 x 2048 18.2 -> 14.4, SwiGLU 1111 x 2816 x 2048 28.6 -> 25.1."""
+    pairs, best = max(1, sms // 2), None
+    for cols in (256, 224, 192, 160, 128):
+        if hd and cols % hd:
+            continue
+        waves = -(-(-(-F // (cols // 2 if epi == EPI_SWIGLU else cols)) * -(-T // 256)) // pairs)
+        cost = 6.1 + waves * (2.3 * cols / 256 + (0.05 + 0.254 * cols / 256) * -(-K // 64))
+        if best is None or cost < best[0]:
+            best = (cost, cols)
+    return best
 
 
 # CTAs of csrc/kernels/gemm_split.cu that a B200 holds at once in clusters of 1 .. 8, with the small amount of shared memory (two per
@@ -258,12 +269,16 @@ def _split_plan(T: int, F: int, K: int, epi: int, sms: int):
 
 
 @lru_cache(maxsize=4096)
-def _dense_plan(T: int, F: int, K: int, epi: int, sms: int):
-    """(wide, split plan) of a dense launch on one GPU that leaves the choice of kernel to this module."""
+def _dense_plan(T: int, F: int, K: int, epi: int, sms: int, hd: int = 0):
+    """(weight rows per tile of gemm_wide.cu or 0, split plan or None) of a dense launch on one GPU that leaves the choice of kernel to
+    this module; ``hd``: see :func:`dense_wide`."""
     wide, plan = want_wide(epi, T, F, K, 1, sms), split_plan(T, F, K, epi, sms)
-    if plan is not None and (not wide or plan[0] < dense_wide_cost(T, F, K, epi, sms)):
-        return False, plan
-    return wide, None
+    if not wide:
+        return 0, plan
+    cost, cols = dense_wide(T, F, K, epi, sms, hd)
+    # up to 256 tokens every weight is read once, from HBM, which the model of the pair kernel leaves out (256 x 6144 x 4096: 23 us there,
+    # 20 us in the other)
+    return (0, plan) if plan is not None and (T <= 256 or plan[0] < cost) else (cols, None)
 
 
 def _wide_rows(F: int, out: Optional[torch.Tensor], residual: Optional[torch.Tensor], comm: "Optional[GemmComm]") -> bool:
@@ -355,13 +370,13 @@ def rope_table(max_pos: int, hd: int, theta: float, device) -> torch.Tensor:
 
 def _launch(W, X, Y, R, offs, recs, bases, G, T, F, K, epi, bn, splitk, ldy, y_f32, comm: Optional[GemmComm] = None,
             streamk: bool = False, pair: bool = False, w_blocked: bool = False, act: int = 0, act_limit: float = 0.0,
-            act_cols: int = 0, unit_weights: bool = False, wide: bool = False, cluster: int = 0):
+            act_cols: int = 0, unit_weights: bool = False, wide: int = 0, cluster: int = 0):
     s = scratch(X.device)
     d = _lib.DmoeGemm()           # zeros: only what a launch has is filled in
     if cluster:
         d.cluster = cluster
     if wide:
-        d.wide = 1
+        d.wide = int(wide)        # True, or the weight rows per tile
     if act:
         d.act, d.act_limit, d.act_cols = act, act_limit, act_cols
     if unit_weights:
@@ -494,7 +509,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, residual: Optional[torch.Tensor] = 
     if wide is None and not cluster:
         wide = False
         if not (bn or splitk or pair) and _wide_rows(F, out, residual, comm):
-            wide, plan = _dense_plan(T, F, K, EPI_PLAIN, sms)
+            wide, plan = _dense_plan(T, F, K, EPI_PLAIN, sms, comm.rope.hd if comm is not None and comm.rope is not None else 0)
             if plan is not None:
                 _, bn, cluster = plan
     if cluster:

@@ -1,0 +1,64 @@
+"""Tiles of 64 .. 256 weight rows of the pair GEMM (csrc/kernels/gemm_wide.cu): edges of tokens, weight rows, K blocks and stages."""
+import pytest
+import torch
+
+from disagmoe_b200.ops import gemm, reference
+
+pytestmark = pytest.mark.gpu
+
+
+def _bf(*s):
+    return torch.randn(*s, device="cuda").to(torch.bfloat16)
+
+
+def _close(y, ref, K):
+    """One rounding of the output (half a unit: 2^-8 relative) and fp32 sums of K products of size 1 / K in any order."""
+    bad = ((y.double() - ref).abs() > ref.abs() * 2.0 ** -8 + 2.0 ** -22 * K ** 0.5 + 1e-6).sum().item()
+    assert bad == 0 and gemm.check_status() == 0, f"{bad} of {ref.numel()} off, max {(y.double() - ref).abs().max().item():.3g}"
+
+
+@pytest.mark.parametrize("cols", [64, 96, 128, 160, 192, 224, 256])
+@pytest.mark.parametrize("T,N,K", [(1, 8, 8), (129, 168, 64), (257, 520, 136), (700, 1320, 712)])
+def test_tile_sizes(T, N, K, cols):
+    torch.manual_seed(T + cols)
+    x, w, r = _bf(T, K), _bf(N, K) * K ** -0.5, _bf(T, N)
+    ref = x.double() @ w.double().T
+    out = torch.full((T + 1, N + 8), 7.0, dtype=torch.bfloat16, device="cuda")
+    gemm.linear(x, w, out=out[:T, :N], wide=cols)
+    _close(out[:T, :N], ref, K)
+    assert bool((out[T] == 7.0).all()) and bool((out[:, N:] == 7.0).all())
+    y = r.clone()
+    gemm.linear(x, w, residual=y, out=y, wide=cols)
+    _close(y, ref + r.double(), K)
+    w2 = _bf(2 * N, K) * K ** -0.5
+    h = x.double() @ w2.double().T
+    out.fill_(7.0)
+    gemm.swiglu_linear(x, w2, out=out[:T, :N], wide=cols)
+    _close(out[:T, :N], h[:, :N] * torch.sigmoid(h[:, :N]) * h[:, N:], K)
+    assert bool((out[T] == 7.0).all()) and bool((out[:, N:] == 7.0).all())
+
+
+@pytest.mark.parametrize("hd,cols", [(64, 64), (64, 192), (64, 256), (128, 128), (128, 256)])
+def test_heads_stay_whole(hd, cols):
+    torch.manual_seed(cols)
+    T, K, n_q, n_kv, bs = 300, 256, 5, 2, 16
+    N = (n_q + 2 * n_kv) * hd
+    x, w = _bf(T, K), _bf(N, K) * K ** -0.5
+    pos = torch.randint(0, 500, (T,), device="cuda", dtype=torch.int32)
+    slots = torch.randperm(400, device="cuda")[:T]
+    caches = [torch.zeros(25, bs, n_kv, hd, dtype=torch.bfloat16, device="cuda") for _ in range(4)]
+    table, y = gemm.rope_table(512, hd, 1e4, "cuda"), torch.zeros(T, N, dtype=torch.bfloat16, device="cuda")
+    gemm.linear(x, w, out=y, wide=cols, comm=gemm.GemmComm(rope=gemm.RopeAppend(table, pos, slots, *caches[:2], n_q, n_kv, hd)))
+    z = gemm.linear(x, w, wide=256)
+    reference.rope_kv_append(z, pos, slots, *caches[2:], n_q, n_kv, hd, 1e4)
+    # the reference rotates in fp32 with its own sines: a unit of the last place of bf16
+    for a, b in ((y[:, :n_q * hd], z[:, :n_q * hd]), (caches[0], caches[2]), (caches[1], caches[3])):
+        torch.testing.assert_close(a.float(), b.float(), rtol=2 ** -7, atol=2 ** -7)
+    assert gemm.check_status() == 0
+
+
+def test_chosen_tiles():
+    assert gemm.dense_wide(2500, 2048, 2048, gemm.EPI_PLAIN, 148)[1] == 160      # 130 tiles in two waves of 74 pairs, 80 of 256 rows
+    assert gemm.dense_wide(4096, 4096, 4096, gemm.EPI_PLAIN, 148, 128)[1] % 128 == 0
+    x, w = _bf(2500, 512), _bf(2048, 512) * 512 ** -0.5
+    _close(gemm.linear(x, w), x.double() @ w.double().T, 512)
