@@ -10,9 +10,9 @@
 //
 // The weights are the M operand (gemm.cu says why); the token tile is any multiple of 16 up to 256 rows, so that one wave of
 // CTAs can be made to fit the chip at any number of tokens. For SwiGLU a tile is 64 gate and the matching 64 up rows: they meet
-// again when the partial rows are added up. Up to 80 tokens a CTA takes 112 KB of shared memory, so that two of them share an SM.
+// again when the partial rows are added up. Up to 128 tokens a CTA takes 112 KB of shared memory, so that two of them share an SM.
 //
-// A stage holds two K blocks: a round of the issuing warp (wait, MMAs, commit) takes about 400 cycles however small the MMAs are.
+// A stage holds two K blocks (one from 96 tokens on, where two CTAs share an SM): a round of the issuing warp (wait, MMAs, commit) takes about 400 cycles however small the MMAs are.
 // Warp roles as in gemm.cu: warp 0 TMA producer, warp 1 TMEM owner and MMA issuer, warps 2..5 accumulator readers; all six add up.
 // ops/gemm.py: split_plan holds the rule that chooses bn, S and this kernel, with both sides measured.
 #include <string.h>
@@ -28,12 +28,12 @@ constexpr int kSThreads = 192;
 constexpr int kSSmallSmem = 112 * 1024 + 512;            // two CTAs per SM
 constexpr int kSLargeSmem = 226 * 1024;
 constexpr int kSWBytes = kBM * kBK * 2;                  // weights of one K block
-constexpr int kSSub = 2;                                 // K blocks per stage
+constexpr int kSSub = 2;                                 // K blocks per stage (one where two stages of two do not fit)
 constexpr int kSMaxStages = 6;
 constexpr int kSRow = kBM * 4;                           // bytes of a token's partial sums
 
 struct SplitArgs {
-  int T, F, K, bn, splits, per;      // per: K blocks per CTA
+  int T, F, K, bn, splits, per, sub;      // per: K blocks per CTA, sub: per stage
   int stages, recv_off, alias;       // recv_off: partial rows of this CTA's tokens; alias: they lie over the stages
   int tmem_cols;
   void* Y;
@@ -124,7 +124,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   constexpr int kFeat = EPI == EPI_SWIGLU ? kBM / 2 : kBM;      // output features per tile
-  const int x_bytes = a.bn * kBK * 2, stage_bytes = kSSub * (kSWBytes + x_bytes);
+  const int x_bytes = a.bn * kBK * 2, stage_bytes = a.sub * (kSWBytes + x_bytes);
   __shared__ uint64_t bars[2 * kSMaxStages + 2];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_word;
@@ -136,7 +136,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
   const int tpr = (ntok + a.splits - 1) / a.splits;             // tokens of the tile that a CTA adds up
   const int tok0 = rank * tpr, own = max(0, min(tpr, ntok - tok0));
   const int kblocks = (a.K + kBK - 1) / kBK;
-  const int kb0 = rank * a.per, nkb = min(a.per, kblocks - kb0), steps = (nkb + kSSub - 1) / kSSub;
+  const int kb0 = rank * a.per, nkb = min(a.per, kblocks - kb0), steps = (nkb + a.sub - 1) / a.sub;
   const bool cluster = a.splits > 1;
   float* parts = reinterpret_cast<float*>(smem);                     // [tokens][kBM], over the stages once these are consumed
   float* recv = reinterpret_cast<float*>(smem + a.recv_off);         // [splits - 1][tpr][kBM]: the others' partial rows of this CTA's tokens
@@ -174,8 +174,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     uint32_t phase = 0;
     for (int i = 0; i < steps; ++i) {
       if (!mbar_wait_warp(empty + 8 * stage, phase ^ 1, &abort_word)) break;
-      const uint32_t fb = full + 8 * stage, st = smem_u32(smem) + stage * stage_bytes, sx = st + kSSub * kSWBytes;
-      const int x = (kb0 + i * kSSub) * kBK, n = min(kSSub, nkb - i * kSSub);
+      const uint32_t fb = full + 8 * stage, st = smem_u32(smem) + stage * stage_bytes, sx = st + a.sub * kSWBytes;
+      const int x = (kb0 + i * a.sub) * kBK, n = min(a.sub, nkb - i * a.sub);
       if (elect_one()) {
         mbar_expect_tx(fb, n * (kSWBytes + x_bytes));
 #pragma unroll
@@ -198,8 +198,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     for (int i = 0; i < steps; ++i) {
       if (!mbar_wait_warp(full + 8 * stage, phase, &abort_word)) break;
       tc_fence_after();
-      const uint32_t st = smem_u32(smem) + stage * stage_bytes, sx = st + kSSub * kSWBytes;
-      const int n = min(kSSub, nkb - i * kSSub);
+      const uint32_t st = smem_u32(smem) + stage * stage_bytes, sx = st + a.sub * kSWBytes;
+      const int n = min(a.sub, nkb - i * a.sub);
       if (elect_one()) {
 #pragma unroll
         for (int j = 0; j < kSSub; ++j) {
@@ -392,27 +392,28 @@ int gemm_split(const DmoeGemm* d, cudaStream_t stream) {
   a.per = (kblocks + a.splits - 1) / a.splits;
   a.splits = (kblocks + a.per - 1) / a.per;      // no share may be empty
   // A CTA's partial rows lie over its stages; those it receives behind them where that leaves all of its share or two stages, else over
-  // them too.
-  const int stage = kSSub * (kSWBytes + bn * kBK * 2), steps = (a.per + kSSub - 1) / kSSub, most = std::min(steps, kSMaxStages), want = std::min(steps, 2);
-  const int parts = bn * kSRow, recv = (a.splits - 1) * ((bn + a.splits - 1) / a.splits) * kSRow;
-  // The large amount of shared memory (one CTA per SM) has more stages in flight, which counts where each is fetched from HBM: 1.1 us
-  // per round trip. It is taken where all CTAs find place at once, and where the small one is too small.
+  // them too. The large amount of shared memory (one CTA per SM) has more stages in flight, which counts where each is fetched from
+  // HBM: 1.1 us per round trip. It is taken where all CTAs find place at once, and where the small one is too small.
   const long long mt = (d->F + feat - 1) / feat, nt = (d->T + bn - 1) / bn;
   const bool spread = a.per > 2 * kSSub && a.splits * mt * nt <= large_capacity(a.splits);
-  int smem = 0;
-  for (int size : {spread ? kSLargeSmem : kSSmallSmem, kSLargeSmem}) {
-    const int room = size - 1024 /*alignment*/;
+  const int parts = bn * kSRow, recv = (a.splits - 1) * ((bn + a.splits - 1) / a.splits) * kSRow;
+  const auto fits = [&](int room, int sub) {
+    const int stage = sub * (kSWBytes + bn * kBK * 2), steps = (a.per + sub - 1) / sub, most = std::min(steps, kSMaxStages), want = std::min(steps, sub == 1 ? 3 : 2);
     const int beside = std::min(most, (room - recv) / stage), over = std::min(most, room / stage);
     if (beside >= want && beside * stage >= parts) {
       a.alias = 0; a.stages = beside; a.recv_off = beside * stage;
     } else if (over >= want && parts + recv <= room) {
       a.alias = 1; a.stages = over; a.recv_off = parts;
     } else {
-      continue;
+      return false;
     }
-    smem = size;
-    break;
-  }
+    a.sub = sub;
+    return true;
+  };
+  const int small = kSSmallSmem - 1024 /*alignment*/, large = kSLargeSmem - 1024;
+  int smem = 0;
+  if (!spread && (fits(small, kSSub) || (bn <= 128 && fits(small, 1)))) smem = kSSmallSmem;
+  else if (fits(large, kSSub)) smem = kSLargeSmem;
   if (smem == 0) return -11;
   a.tmem_cols = 32;
   while (a.tmem_cols < bn) a.tmem_cols *= 2;

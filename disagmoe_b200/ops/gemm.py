@@ -216,15 +216,15 @@ _SPLIT_LARGE = (148, 148, 135, 132, 130, 132, 105, 120)
 
 def split_plan(T: int, F: int, K: int, epi: int, sms: int):
     """(cost in us, token tile, CTAs per cluster) of a dense product in csrc/kernels/gemm_split.cu, or None where other kernels are
-    faster: all its CTAs have to find place at once, or it has one tile of up to 64 tokens and the weights stream through it (an LM
+    faster: all its CTAs have to find place at once, or it has one tile of up to 128 tokens and the weights stream through it (an LM
     head).
 
     The cost model is fitted to a sweep on B200 (T 1 .. 4096, F 16 .. 151936, K 16 .. 14336; launches back to back, weights from HBM); its
     choice is 2.8 % slower than the best tile and cluster on average. Measured, this module's other kernels -> the choice, us: 1 x 4096 x
     4096 13.9 -> 9.7, 37 x 2048 x 2048 10.3 -> 6.6, 37 x 6144 x 2048 14.6 -> 9.6, 37 x 2048 x 5632 14.1 -> 9.1, SwiGLU 37 x 5632 x 2048 17.7
     -> 11.8, 96 x 2048 x 10944 22.6 -> 14.5, 256 x 4096 x 4096 22.0 -> 16.0, 576 x 2048 x 5632 29.4 -> 22.0, 1111 x 2048 x 2048 17.8 -> 14.7, 3
-    x 32000 x 4096 54.1 -> 42.4, 37 x 151936 x 2048 111 -> 104. A second wave costs as much as the first: 96 x 10944 x 2048 SwiGLU (171
-    CTAs of one per SM) 22.6 -> 26.3, 1111 x 2816 x 2048 SwiGLU 28.6 -> 36.4, 192 x 32000 x 2048 32.5 -> 42.5.
+    x 32000 x 4096 54.1 -> 42.4, 37 x 151936 x 2048 111 -> 104, 96 x 102400 x 2048 88.5 -> 78.0, 66 x 151936 x 2048 128 -> 110. A second wave costs as much as the first: 200 x 10944 x 2048 SwiGLU (171
+    CTAs of one per SM) 23.0 -> 40.6, 1111 x 2816 x 2048 SwiGLU 28.6 -> 36.4, 192 x 32000 x 2048 32.5 -> 42.5.
 
     Sizes are rounded up to a grid of tokens, so that few plans serve prompts of all lengths."""
     grid = 16 if T <= 256 else 32 if T <= 1024 else 64
@@ -239,7 +239,7 @@ def _split_plan(T: int, F: int, K: int, epi: int, sms: int):
     stream = F * K * (4 if gate else 2) / 6.6e6
     best = None
     if mt > small[0]:
-        shapes = [(1, T)] if T <= 64 else []
+        shapes = [(1, T)] if T <= 128 else []
     elif mt * -(-T // 256) > small[0]:
         shapes = []
     else:
@@ -252,11 +252,13 @@ def _split_plan(T: int, F: int, K: int, epi: int, sms: int):
         per = -(-kblocks // S)
         if -(-kblocks // per) != S:
             continue                      # a smaller cluster has the same shares
-        units, steps, stage = mt * S * -(-T // bn), -(-per // 2), 32768 + 256 * bn
-        one = bn > 80 or (per > 4 and units <= large[S - 1])      # one CTA per SM
+        units = mt * S * -(-T // bn)
+        one = bn > 128 or (per > 4 and units <= large[S - 1])      # one CTA per SM
+        sub = 2 if one or bn <= 80 else 1                          # K blocks per stage
+        steps, stage = -(-per // sub), sub * (16384 + 128 * bn)
         cap = (large if one else small)[S - 1]
-        if units > cap and (S > 1 or bn < T or T > 64):
-            continue
+        if units > cap and (S > 1 or bn < T or T > 128) or not one and bn > 80 and S > 1:
+            continue                      # the latter: stages of one K block and the exchange, 256 x 4096 x 4096 16.1 -> 20.6 us
         waves, shared = -(-units // cap), 2 if not one and units > sms else 1
         flight = min(steps, (230400 if one else 114176) // stage, 6)
         body = max(waves * steps * max(0.226, shared * stage / 1.27e5, 0.81 / flight), stream)

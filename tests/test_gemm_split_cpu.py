@@ -7,11 +7,15 @@ from disagmoe_b200.ops import gemm
 
 
 def _fits(bn, S, per):
-    """Restates the kernel's shared memory: stages of two K blocks, a CTA's partial rows over them, those it receives beside or over."""
-    steps, stage, parts, recv = -(-per // 2), 2 * (128 * 64 * 2 + bn * 128), bn * 512, (S - 1) * -(-bn // S) * 512
-    room = 226 * 1024 - 1024
-    beside, over = min(steps, 6, max(0, room - recv) // stage), min(steps, 6, room // stage)
-    return (beside >= min(steps, 2) and beside * stage >= parts) or (over >= min(steps, 2) and parts + recv <= room)
+    """Restates the kernel's shared memory: stages of one or two K blocks, a CTA's partial rows over them, those it receives beside or
+    over, in the amount that lets two CTAs share an SM or in the one that does not."""
+    parts, recv = bn * 512, (S - 1) * -(-bn // S) * 512
+    for room, sub in ((112 * 1024 + 512 - 1024, 2), (112 * 1024 + 512 - 1024, 1), (226 * 1024 - 1024, 2)):
+        stage, steps = sub * (16384 + bn * 128), -(-per // sub)
+        want, beside, over = min(steps, 3 if sub == 1 else 2), min(steps, 6, max(0, room - recv) // stage), min(steps, 6, room // stage)
+        if (beside >= want and beside * stage >= parts) or (over >= want and parts + recv <= room):
+            return True
+    return False
 
 
 @pytest.mark.parametrize("epi", [gemm.EPI_PLAIN, gemm.EPI_SWIGLU])
@@ -29,12 +33,12 @@ def test_plans_fit_the_kernel(epi):
         kblocks = -(-K // 64)
         assert 16 <= bn <= 256 and bn % 16 == 0 and 1 <= S <= min(8, kblocks) and _fits(bn, S, -(-kblocks // S))
         tiles = -(-F // (64 if epi == gemm.EPI_SWIGLU else 128)) * -(-T // bn)
-        assert S * tiles <= 296 or (S == 1 and T <= 64 and bn >= T)      # one wave, or one tile of tokens that weights stream through
+        assert S * tiles <= 296 or (S == 1 and T <= 128 and bn >= T)      # one wave, or one tile of tokens that weights stream through
     assert found > 300
 
 
 def test_refused_where_a_second_wave_would_start():
     assert gemm.split_plan(4096, 4096, 4096, gemm.EPI_PLAIN, 148) is None
     assert gemm.split_plan(192, 32000, 2048, gemm.EPI_PLAIN, 148) is None
-    assert gemm.split_plan(96, 10944, 2048, gemm.EPI_SWIGLU, 148) is None
+    assert gemm.split_plan(200, 10944, 2048, gemm.EPI_SWIGLU, 148) is None
     assert gemm.split_plan(1, 151936, 2048, gemm.EPI_PLAIN, 148)[1:] == (16, 1)

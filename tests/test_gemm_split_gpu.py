@@ -19,7 +19,7 @@ def _close(y, ref, K, bits=8):
     assert bad == 0 and gemm.check_status() == 0, f"{bad} of {ref.numel()} off, max {(y.double() - ref).abs().max().item():.3g}"
 
 
-@pytest.mark.parametrize("bn,cluster", [(16, 1), (16, 8), (32, 4), (48, 5), (80, 2), (96, 3), (128, 2), (208, 8), (256, 1)])
+@pytest.mark.parametrize("bn,cluster", [(16, 1), (16, 8), (32, 4), (48, 5), (80, 2), (96, 1), (96, 3), (112, 8), (128, 1), (128, 2), (208, 8), (256, 1)])
 @pytest.mark.parametrize("T,N,K", [(1, 8, 8), (15, 136, 72), (17, 128, 64), (97, 264, 520), (300, 144, 1096), (33, 1024, 2048)])
 def test_tiles_and_clusters(T, N, K, bn, cluster):
     torch.manual_seed(T + N + K)
