@@ -194,9 +194,9 @@ def want_wide(epi: int, T: int, F: int, K: int, G: int, sms: int) -> bool:
 def dense_wide(T: int, F: int, K: int, epi: int, sms: int, hd: int = 0):
     """(us, weight rows per tile) of a dense product in csrc/kernels/gemm_wide.cu: of the tile sizes the one whose count fills whole
     waves of CTA pairs best; ``hd``: heads that a tile has to hold whole. Fitted to a sweep on B200 (42 sizes, T 66 .. 4096, K 16 .. 10944;
-    error 6 %, the choice is 0.8 % slower than the best size on average). Measured with 256 rows -> with the choice, us: 2500 x 2048 x 2048
-    27.9 -> 20.7 (80 tiles for 74 pairs -> 130 smaller ones), 2500 x 2048 x 5632 66.5 -> 45.4, 3000 x 2048 x 2048 27.8 -> 23.2, 2500 x 4096 x
-    2048 40.2 -> 34.6, 1111 x 6144 x 2048 30.7 -> 28.7, 724 x 3664 x 2048 18.2 -> 14.4, SwiGLU 1111 x 2816 x 2048 28.6 -> 25.1."""
+    error 7 %, the choice is 1 % slower than the best size on average). Measured with 256 rows -> with the choice, us: 2500 x 2048 x 2048
+    27.8 -> 20.0 (80 tiles for 74 pairs -> 130 smaller ones), 2500 x 2048 x 5632 62.6 -> 43.6, 3000 x 2048 x 2048 27.5 -> 22.8, 2500 x 4096 x
+    2048 39.3 -> 33.5, 1111 x 6144 x 2048 29.8 -> 27.6, 724 x 3664 x 2048 18.3 -> 14.3, SwiGLU 1111 x 2816 x 2048 29.3 -> 26.4."""
     pairs, best = max(1, sms // 2), None
     for cols in (256, 224, 192, 160, 128):
         if hd and cols % hd:

@@ -38,6 +38,23 @@ def test_tile_sizes(T, N, K, cols):
     assert bool((out[T] == 7.0).all()) and bool((out[:, N:] == 7.0).all())
 
 
+@pytest.mark.parametrize("sizes", [[33, 0, 1, 31, 257, 32, 300], [64, 255, 7]])
+def test_rows_of_the_next_group_stay(sizes):
+    """Whole warps of a group go out as boxes of 32 rows; a remainder may not reach into the next group or past the last."""
+    torch.manual_seed(len(sizes))
+    G, N, K, T = len(sizes), 328, 136, sum(sizes) + 40
+    x, w13 = _bf(T, K), _bf(G, 2 * N, K) * K ** -0.5
+    offs = torch.tensor([0, *sizes], device="cuda").cumsum(0).to(torch.int32)
+    for op, w in ((gemm.grouped_linear, w13[:, :N].contiguous()), (gemm.grouped_swiglu, w13)):
+        out = torch.full((T + 1, N + 8), 7.0, dtype=torch.bfloat16, device="cuda")
+        op(x, w, offs, out=out[:T, :N], wide=True)
+        for g in range(G):
+            a, b = sum(sizes[:g]), sum(sizes[:g + 1])
+            h = x[a:b].double() @ w[g].double().T
+            _close(out[a:b, :N], h if op is gemm.grouped_linear else h[:, :N] * torch.sigmoid(h[:, :N]) * h[:, N:], K)
+        assert bool((out[sum(sizes):] == 7.0).all()) and bool((out[:, N:] == 7.0).all())
+
+
 @pytest.mark.parametrize("hd,cols", [(64, 64), (64, 192), (64, 256), (128, 128), (128, 256)])
 def test_heads_stay_whole(hd, cols):
     torch.manual_seed(cols)
