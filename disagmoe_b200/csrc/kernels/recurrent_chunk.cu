@@ -71,19 +71,47 @@ __device__ __forceinline__ void store_acc_frag(uint8_t* tile, int lane, const fl
   store_frag(tile + kFrag, lane, l);
 }
 
+// 2^x; a result below the normal numbers (2^-126) is 0
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// N consecutive bf16 of a row, as they are
 template <int N>
-__device__ __forceinline__ void load_bf16(const __nv_bfloat16* p, float* f) {
-  if (N == 4) {
-    const uint2 r = *reinterpret_cast<const uint2*>(p);
-    const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.x));
-    const float2 y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.y));
-    f[0] = x.x; f[N - 3] = x.y; f[N - 2] = y.x; f[N - 1] = y.y;
-  } else if (N == 2) {
-    const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
-    f[0] = x.x; f[N - 1] = x.y;
+struct Raw { using T = unsigned short; };
+template <>
+struct Raw<2> { using T = uint32_t; };
+template <>
+struct Raw<4> { using T = uint2; };
+__device__ __forceinline__ void unpack(unsigned short r, float (&f)[1]) { f[0] = __uint_as_float(static_cast<uint32_t>(r) << 16); }
+__device__ __forceinline__ void unpack(uint32_t r, float (&f)[2]) {
+  f[0] = __uint_as_float(r << 16);
+  f[1] = __uint_as_float(r & 0xffff0000u);
+}
+__device__ __forceinline__ void unpack(const uint2& r, float (&f)[4]) {
+  f[0] = __uint_as_float(r.x << 16);
+  f[1] = __uint_as_float(r.x & 0xffff0000u);
+  f[2] = __uint_as_float(r.y << 16);
+  f[3] = __uint_as_float(r.y & 0xffff0000u);
+}
+// N consecutive fp32 of shared memory, aligned to their size
+template <int N>
+__device__ __forceinline__ void load_f32(const float* p, float (&f)[N]) {
+  if constexpr (N == 4) {
+    const float4 v = *reinterpret_cast<const float4*>(p);
+    f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w;
+  } else if constexpr (N == 2) {
+    const float2 v = *reinterpret_cast<const float2*>(p);
+    f[0] = v.x; f[1] = v.y;
   } else {
-    f[0] = __bfloat162float(p[0]);
+    f[0] = p[0];
   }
+}
+// Byte of 16-byte piece c of row t in a [64][DP] bf16 matrix without padding: ldmatrix of 8 rows meets no bank twice
+template <int DP>
+__device__ __forceinline__ uint32_t raw_at(int t, int c) {
+  return t * DP * 2 + ((c ^ (DP >= 64 ? t & 7 : (t >> 1) & 3)) << 4);
 }
 // hi / lo planes of N consecutive fp32 values
 template <int N>
@@ -105,14 +133,25 @@ __device__ __forceinline__ void store_split(__nv_bfloat16* hi, __nv_bfloat16* lo
   }
 }
 
-// T = (I + A)^-1 for a strictly lower triangular A [64][65]: 16 x 16 diagonal blocks by forward substitution, then the
-// blocks below them, one block diagonal after the other: T_IJ = -T_II sum_{J <= K < I} A_IK T_KJ. `m` is scratch
-// [3][16][17]. All 256 threads; T is complete after the last barrier.
-__device__ __forceinline__ void invert_unit_lower(const float* A, float* T, float* m) {
-  constexpr int LD = kChunk + 1;
+// T = (I + A)^-1 for a strictly lower triangular A [64][kLdA]: 16 x 16 diagonal blocks by forward substitution, then the
+// blocks below them, one block diagonal after the other: T_IJ = -T_II sum_{J <= K < I} A_IK T_KJ. Blocks above the diagonal are not
+// written. All 256 threads, one element of a block each; T is complete after the last barrier. Both factors of a product are read
+// along the sum, 16 bytes at a time (T and the sums also lie transposed, `tt` [64][kLdA] and `mt` [3][16][kLdM]): element by element
+// this was bound by its shared memory loads (17 thousand of the 109 thousand cycles of a chunk with 128 channels).
+constexpr int kLdA = kChunk + 4, kLdM = 20;
+__device__ __forceinline__ float dot16(float s, const float* x, const float* y, float sign) {
+#pragma unroll
+  for (int k = 0; k < 16; k += 4) {
+    const float4 a = *reinterpret_cast<const float4*>(x + k), b = *reinterpret_cast<const float4*>(y + k);
+    s += sign * a.x * b.x;
+    s += sign * a.y * b.y;
+    s += sign * a.z * b.z;
+    s += sign * a.w * b.w;
+  }
+  return s;
+}
+__device__ __forceinline__ void invert_unit_lower(const float* A, float* T, float* tt, float* mt) {
   const int tid = threadIdx.x;
-  for (int i = tid; i < kChunk * LD; i += kChunkThreads) T[i] = 0.f;
-  __syncthreads();
   if (tid < kChunk) {
     const int o = tid / 16 * 16, c = tid % 16;
     float x[16];
@@ -120,30 +159,40 @@ __device__ __forceinline__ void invert_unit_lower(const float* A, float* T, floa
     for (int i = 0; i < 16; ++i) {
       float s = i == c ? 1.f : 0.f;
 #pragma unroll
-      for (int j = 0; j < i; ++j) s -= A[(o + i) * LD + o + j] * x[j];
+      for (int j = 0; j < i; j += 4) {
+        const float4 r = *reinterpret_cast<const float4*>(A + (o + i) * kLdA + o + j);
+        s -= r.x * x[j];
+        if (j + 1 < i) s -= r.y * x[j + 1];
+        if (j + 2 < i) s -= r.z * x[j + 2];
+        if (j + 3 < i) s -= r.w * x[j + 3];
+      }
       x[i] = i >= c ? s : 0.f;
-      T[(o + i) * LD + o + c] = x[i];
     }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) T[(o + i) * kLdA + o + c] = x[i];
+#pragma unroll
+    for (int i = 0; i < 16; i += 4)
+      *reinterpret_cast<float4*>(tt + (o + c) * kLdA + o + i) = make_float4(x[i], x[i + 1], x[i + 2], x[i + 3]);
   }
   __syncthreads();
   const int i = tid / 16, j = tid % 16;
+#pragma unroll
   for (int dist = 1; dist < 4; ++dist) {
+#pragma unroll
     for (int I = dist; I < 4; ++I) {
       const int J = I - dist;
       float s = 0.f;
-      for (int K = J; K < I; ++K) {
 #pragma unroll
-        for (int k = 0; k < 16; ++k) s += A[(16 * I + i) * LD + 16 * K + k] * T[(16 * K + k) * LD + 16 * J + j];
-      }
-      m[(J * 16 + i) * 17 + j] = s;
+      for (int K = J; K < I; ++K) s = dot16(s, A + (16 * I + i) * kLdA + 16 * K, tt + (16 * J + j) * kLdA + 16 * K, 1.f);
+      mt[(J * 16 + j) * kLdM + i] = s;
     }
     __syncthreads();
+#pragma unroll
     for (int I = dist; I < 4; ++I) {
       const int J = I - dist;
-      float s = 0.f;
-#pragma unroll
-      for (int k = 0; k < 16; ++k) s -= T[(16 * I + i) * LD + 16 * I + k] * m[(J * 16 + k) * 17 + j];
-      T[(16 * I + i) * LD + 16 * J + j] = s;
+      const float s = dot16(0.f, T + (16 * I + i) * kLdA + 16 * I, mt + (J * 16 + j) * kLdM, -1.f);
+      T[(16 * I + i) * kLdA + 16 * J + j] = s;
+      tt[(16 * J + j) * kLdA + 16 * I + i] = s;
     }
     __syncthreads();
   }
@@ -153,30 +202,41 @@ template <int DP, int MODE>
 struct PrepSmem {
   static constexpr bool DELTA = MODE == kDelta;
   static constexpr int kKs = DP + 8;
+  static constexpr int kSb = DP + 8;         // row stride of the decays: the four rows of a half warp's float2 loads lie 8 banks apart
   static constexpr int kKn = 2 * kChunk * kKs * 2, kTX = DELTA ? 4 * kChunk * kPs * 2 : 0;
   static constexpr int kRegion = kKn > kTX ? kKn : kTX;
-  static constexpr int kBytes = 4 * kChunk * DP + 3 * 4 * kChunk + kRegion + (DELTA ? 2 * 4 * kChunk * (kChunk + 1) : 0) +
-                                (MODE == kBonus ? 4 * 4 * DP : 0) + 16;
+  // behind the region: A and T, where the rows of k and q lie before them; the rows of q; or the decays of a bonus' tiles
+  static constexpr int kBehind = DELTA ? 2 * 4 * kChunk * kLdA : MODE == kBonus ? 4 * 4 * DP : 2 * kChunk * DP;
+  static constexpr int kBytes = 4 * kChunk * kSb + 3 * 4 * kChunk + 4 * DP + kRegion + kBehind + 16;
 };
 
+// Bound by what its 16 warps per SM issue and wait for, not by memory (a delta chunk of 128 channels and values reads 80 KB and writes
+// 144 KB: 35 us for 1024 of them at the copy rate). Of the 109 thousand cycles that such a chunk took, rows read from global memory as
+// fragments need them, decays in rows that meet in the same banks, two exponentials where a product does, a branch per token's
+// decay, logits fetched eight at a time, norms reduced one by one and the inversion's loads made up more than a third. Recurrence as a
+// whole (preparation, scan, norm), 4096 tokens x 16 heads of 128 x 128, before -> now, us: delta rule 359 -> 263, plain write 221 ->
+// 198, bonus 228 -> 202; 700 tokens x 32 heads of 64 x 64: 68 -> 54, 38.6 -> 34.3, 36.7 -> 34.8.
 template <int DP, int MODE>
 __global__ void __launch_bounds__(kChunkThreads, MODE == kBonus && DP <= 64 ? 3 : 2)
 chunk_prep_kernel(const DmoeRecur a, const int4* __restrict__ chunks, uint8_t* __restrict__ ws, long long ws_stride, int h0) {
   using L = ChunkWs<DP>;
   using SM = PrepSmem<DP, MODE>;
   constexpr bool DELTA = MODE == kDelta, BONUS = MODE == kBonus;
-  constexpr int PL = DP / 32, KS = DP / 16, MT = DP / 16, LDA = kChunk + 1, ROWS = kChunk / 8;
+  constexpr int PL = DP / 32, KS = DP / 16, MT = DP / 16, LDA = kLdA, ROWS = kChunk / 8, SB = SM::kSb;
   extern __shared__ __align__(16) uint8_t s_raw[];
-  float* s_b = reinterpret_cast<float*>(s_raw);                 // [64][DP] running log2 decay
-  float* s_fq = s_b + kChunk * DP;                              // [64] factors of the raw q and k rows
+  float* s_b = reinterpret_cast<float*>(s_raw);                 // [64][SB] running log2 decay
+  float* s_fq = s_b + kChunk * SB;                              // [64] factors of the raw q and k rows
   float* s_fk = s_fq + kChunk;
   float* s_beta = s_fk + kChunk;                                // delta: write strengths; bonus: P_tt
-  uint8_t* region = reinterpret_cast<uint8_t*>(s_beta + kChunk);
+  float* s_em = s_beta + kChunk;                                // [DP] decay up to the middle
+  uint8_t* region = reinterpret_cast<uint8_t*>(s_em + DP);
   __nv_bfloat16* s_kh = reinterpret_cast<__nv_bfloat16*>(region);          // scaled k rows, hi then lo plane
   __nv_bfloat16* s_kl = s_kh + kChunk * SM::kKs;
   float* s_A = reinterpret_cast<float*>(region + SM::kRegion);
   float* s_T = s_A + kChunk * LDA;
   float* s_step = s_A;                                          // bonus: [4][DP] decay over tile i of 16 tokens
+  uint8_t* raw_k = reinterpret_cast<uint8_t*>(s_A);             // rows of k and q, until A and T take their places
+  uint8_t* raw_q = reinterpret_cast<uint8_t*>(DELTA ? s_T : s_A);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tq = lane & 3;
   const int lm_mi = lane >> 3, lm_r = lane & 7;
@@ -188,76 +248,99 @@ chunk_prep_kernel(const DmoeRecur a, const int4* __restrict__ chunks, uint8_t* _
   const __nv_bfloat16* kp = static_cast<const __nv_bfloat16*>(a.k) + row0 * a.ldk + hk * D;
   uint8_t* w = ws + (static_cast<long long>(blockIdx.x) * gridDim.y + blockIdx.y) * ws_stride;
 
-  // ---- this warp's rows of k (and q, for its norm); loads first, they are used below
+  // ---- this warp's rows of k and q and this thread's decay logits: all loads first, they are used below
   const int t0 = warp * ROWS, d0 = lane * PL;
-  float k[ROWS][PL];
+  using Rw = typename Raw<PL>::T;
+  Rw rk[ROWS], rq[ROWS];
 #pragma unroll
   for (int i = 0; i < ROWS; ++i) {
-#pragma unroll
-    for (int e = 0; e < PL; ++e) k[i][e] = 0.f;
-    if (t0 + i < n && d0 < D) load_bf16<PL>(kp + (t0 + i) * a.ldk + d0, k[i]);
+    const bool in = t0 + i < n && d0 < D;
+    rk[i] = in ? *reinterpret_cast<const Rw*>(kp + (t0 + i) * a.ldk + d0) : Rw{};
+    rq[i] = in ? *reinterpret_cast<const Rw*>(qp + (t0 + i) * a.ldq + d0) : Rw{};
   }
   // ---- log2 decays and their running sums; a thread keeps one channel
   {
     constexpr int NG = kChunkThreads / DP, LEN = kChunk / NG;
-    const float scale = decay_scale(a, h);
-    const int d = tid % DP, gi = tid / DP;
-    const float bias = d < D ? a.z_bias[h * D + d] : 0.f;
+    float* s_end = reinterpret_cast<float*>(region);             // [NG][DP]
+    const int d = tid % DP, gi = tid / DP, at = gi * LEN;
     const float* zp = a.z + row0 * a.ldz + h * D + d;
-    float run = 0.f;
+    float run[LEN];
 #pragma unroll
-    for (int t8 = 0; t8 < LEN; t8 += 8) {
-      float z[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int t = gi * LEN + t8 + j;
-        z[j] = t < n && d < D ? zp[t * a.ldz] : 0.f;
-      }
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int t = gi * LEN + t8 + j;
-        if (t < n && d < D) run += kLog2e * log_decay(a.decay_kind, z[j] + bias, scale);
-        s_b[t * DP + d] = run;
-      }
-    }
+    for (int j = 0; j < LEN; ++j) run[j] = at + j < n && d < D ? zp[(at + j) * a.ldz] : 0.f;
+    const float scale = decay_scale(a, h), bias = d < D ? a.z_bias[h * D + d] : 0.f;
     if (tid < kChunk)
       s_beta[tid] = DELTA && tid < n
                         ? 1.f / (1.f + expf(-__bfloat162float(static_cast<const __nv_bfloat16*>(a.beta)[(row0 + tid) * a.ldb + h])))
                         : 0.f;
+    // without a branch per token, so that the chains of the tokens overlap
+    const auto logs = [&](int kind) {
+#pragma unroll
+      for (int j = 0; j < LEN; ++j) run[j] = log_decay(kind, run[j] + bias, scale);
+    };
+    if (a.decay_kind == 0) logs(0);
+    else if (a.decay_kind == 1) logs(1);
+    else logs(2);
+    float sum = 0.f;
+#pragma unroll
+    for (int j = 0; j < LEN; ++j) {
+      if (at + j < n && d < D) sum += kLog2e * run[j];
+      run[j] = sum;
+    }
+    s_end[tid] = sum;
     __syncthreads();
     float before = 0.f;
-    for (int j = 0; j < gi; ++j) before += s_b[((j + 1) * LEN - 1) * DP + d];
-    __syncthreads();
-    if (gi > 0) {
-#pragma unroll 8
-      for (int t = gi * LEN; t < (gi + 1) * LEN; ++t) s_b[t * DP + d] += before;
-    }
+    for (int j = 0; j < gi; ++j) before += s_end[j * DP + d];
+#pragma unroll
+    for (int j = 0; j < LEN; ++j) s_b[(at + j) * SB + d] = gi > 0 ? run[j] + before : run[j];
   }
-  // ---- factors of the rows: scale and unit norms; with a bonus the diagonal of P
-  if (DELTA || BONUS) {
-    float q[ROWS][PL], bonus[PL];
+  // ---- rows as they are for the products below; factors of the rows: scale and unit norms; with a bonus the diagonal of P
+  float k[ROWS][PL];
 #pragma unroll
-    for (int e = 0; e < PL; ++e) bonus[e] = BONUS && d0 < D ? a.bonus[h * D + d0 + e] : 0.f;
+  for (int i = 0; i < ROWS; ++i) {
+    unpack(rk[i], k[i]);
+    const uint32_t o = raw_at<DP>(t0 + i, d0 / 8) + d0 % 8 * 2;
+    if (DELTA) *reinterpret_cast<Rw*>(raw_k + o) = rk[i];
+    if (!BONUS) *reinterpret_cast<Rw*>(raw_q + o) = rq[i];
+  }
+  if (BONUS) {
+    float bonus[PL];
+#pragma unroll
+    for (int e = 0; e < PL; ++e) bonus[e] = d0 < D ? a.bonus[h * D + d0 + e] : 0.f;
 #pragma unroll
     for (int i = 0; i < ROWS; ++i) {
+      float q[PL], qq = 0.f;
+      unpack(rq[i], q);
 #pragma unroll
-      for (int e = 0; e < PL; ++e) q[i][e] = 0.f;
-      if (t0 + i < n && d0 < D) load_bf16<PL>(qp + (t0 + i) * a.ldq + d0, q[i]);
+      for (int e = 0; e < PL; ++e) qq += q[e] * (k[i][e] * bonus[e]);
+      qq = warp_sum(qq);
+      if (lane == 0) { s_fq[t0 + i] = a.qscale; s_fk[t0 + i] = 1.f; s_beta[t0 + i] = qq * a.qscale; }
+    }
+  } else if (DELTA) {
+    // 16 sums over the lanes: every exchange halves the sums that a lane still holds, so that lane l ends with the sum l / 2
+    float v[2 * ROWS];
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+      float q[PL];
+      unpack(rq[i], q);
+      v[i] = v[ROWS + i] = 0.f;
+#pragma unroll
+      for (int e = 0; e < PL; ++e) { v[i] += q[e] * q[e]; v[ROWS + i] += k[i][e] * k[i][e]; }
     }
 #pragma unroll
-    for (int i = 0; i < ROWS; ++i) {
-      float qq = 0.f, kk = 0.f;
-      if (BONUS) {
+    for (int o = 16; o > 1; o >>= 1) {
+      const bool up = lane & o;
 #pragma unroll
-        for (int e = 0; e < PL; ++e) qq += q[i][e] * (k[i][e] * bonus[e]);
-        qq = warp_sum(qq);
-        if (lane == 0) { s_fq[t0 + i] = a.qscale; s_fk[t0 + i] = 1.f; s_beta[t0 + i] = qq * a.qscale; }
-        continue;
+      for (int i = 0; i < o / 2; ++i) {
+        const float send = up ? v[i] : v[i + o / 2], keep = up ? v[i + o / 2] : v[i];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
       }
+    }
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+    const float f = (lane < 16 ? a.qscale : 1.f) / sqrtf(v[0] + 1e-6f);
+    if (!(lane & 1)) (lane < 16 ? s_fq + t0 : s_fk + t0 - ROWS)[lane / 2] = f;
 #pragma unroll
-      for (int e = 0; e < PL; ++e) { qq += q[i][e] * q[i][e]; kk += k[i][e] * k[i][e]; }
-      const float fk = 1.f / sqrtf(warp_sum(kk) + 1e-6f), fq = a.qscale / sqrtf(warp_sum(qq) + 1e-6f);
-      if (lane == 0) { s_fq[t0 + i] = fq; s_fk[t0 + i] = fk; }
+    for (int i = 0; i < ROWS; ++i) {
+      const float fk = __shfl_sync(0xffffffffu, f, 2 * (ROWS + i));
 #pragma unroll
       for (int e = 0; e < PL; ++e) k[i][e] *= fk;
     }
@@ -266,24 +349,27 @@ chunk_prep_kernel(const DmoeRecur a, const int4* __restrict__ chunks, uint8_t* _
     s_fk[t0 + lane] = 1.f;
   }
   __syncthreads();
-  bool wide = false;
+  bool wide = false, faint = false;
   if (tid < DP) {
-    const float m = s_b[kMid * DP + tid];
+    const float m = s_b[kMid * SB + tid];
     if (BONUS) {
       float from = 0.f;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const float end = s_b[(16 * i + 15) * DP + tid];
+        const float end = s_b[(16 * i + 15) * SB + tid];
         wide = wide || from - end > kMaxTileShift;
-        s_step[i * DP + tid] = exp2f(end - from);
+        s_step[i * DP + tid] = ex2(end - from);
         from = end;
       }
     } else {
-      wide = s_b[tid] - m > kMaxShift || m - s_b[(kChunk - 1) * DP + tid] > kMaxShift;
+      wide = s_b[tid] - m > kMaxShift || m - s_b[(kChunk - 1) * SB + tid] > kMaxShift;
+      faint = m < -kMaxTileShift;
+      s_em[tid] = ex2(m);
     }
-    reinterpret_cast<float*>(w + L::kDec)[tid] = exp2f(s_b[(kChunk - 1) * DP + tid]);
+    reinterpret_cast<float*>(w + L::kDec)[tid] = ex2(s_b[(kChunk - 1) * SB + tid]);
   }
   const bool slow = __syncthreads_or(wide);
+  const bool direct = !BONUS && (__syncthreads_or(faint) || slow);      // e^b is not e^(b - m) e^m in fp32
 
   // ---- k e^(b_end - b): through shared memory into transposed fragments
   auto stage_k = [&] {
@@ -293,21 +379,34 @@ chunk_prep_kernel(const DmoeRecur a, const int4* __restrict__ chunks, uint8_t* _
   };
   float to_mid[PL];                                  // e^(m - b_end)
   float k_tile[BONUS ? ROWS : 1][PL];                // k e^(b at the end of its tile - b)
+  float end[PL];
+  load_f32<PL>(s_b + (kChunk - 1) * SB + d0, end);
+  if (BONUS) {
+    float tile[PL], rest[PL];
+    load_f32<PL>(s_b + (warp / 2 * 16 + 15) * SB + d0, tile);
 #pragma unroll
-  for (int e = 0; e < PL; ++e) {
-    const float end = s_b[(kChunk - 1) * DP + d0 + e];
-    if (BONUS) {
-      const float tile = s_b[(warp / 2 * 16 + 15) * DP + d0 + e], rest = exp2f(end - tile);
+    for (int e = 0; e < PL; ++e) rest[e] = ex2(end[e] - tile[e]);
 #pragma unroll
-      for (int i = 0; i < ROWS; ++i) {
-        k_tile[BONUS ? i : 0][e] = k[i][e] * exp2f(tile - s_b[(t0 + i) * DP + d0 + e]);
-        k[i][e] = k_tile[BONUS ? i : 0][e] * rest;
+    for (int i = 0; i < ROWS; ++i) {
+      float b[PL];
+      load_f32<PL>(s_b + (t0 + i) * SB + d0, b);
+#pragma unroll
+      for (int e = 0; e < PL; ++e) {
+        k_tile[BONUS ? i : 0][e] = k[i][e] * ex2(tile[e] - b[e]);
+        k[i][e] = k_tile[BONUS ? i : 0][e] * rest[e];
       }
-      continue;
     }
-    to_mid[e] = slow ? 0.f : exp2f(s_b[kMid * DP + d0 + e] - end);
+  } else {
+    load_f32<PL>(s_b + kMid * SB + d0, to_mid);
 #pragma unroll
-    for (int i = 0; i < ROWS; ++i) k[i][e] *= exp2f(end - s_b[(t0 + i) * DP + d0 + e]);
+    for (int e = 0; e < PL; ++e) to_mid[e] = slow ? 0.f : ex2(to_mid[e] - end[e]);
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+      float b[PL];
+      load_f32<PL>(s_b + (t0 + i) * SB + d0, b);
+#pragma unroll
+      for (int e = 0; e < PL; ++e) k[i][e] *= ex2(end[e] - b[e]);
+    }
   }
   stage_k();
   __syncthreads();
@@ -364,11 +463,11 @@ chunk_prep_kernel(const DmoeRecur a, const int4* __restrict__ chunks, uint8_t* _
             const int r = j & 1 ? r1 : r0, c = ks * 16 + 2 * tq + (j >> 1) * 8;
             x[j] = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw[kk][j]));
             float2 b = make_float2(0.f, 0.f);
-            if (r > 0) b = *reinterpret_cast<const float2*>(s_b + (r - 1) * DP + c);
+            if (r > 0) b = *reinterpret_cast<const float2*>(s_b + (r - 1) * SB + c);
             float2 m = make_float2(0.f, 0.f);
-            if (from >= 0) m = *reinterpret_cast<const float2*>(s_b + (16 * from + 15) * DP + c);
-            x[j].x *= a.qscale * exp2f(b.x - m.x);
-            x[j].y *= a.qscale * exp2f(b.y - m.y);
+            if (from >= 0) m = *reinterpret_cast<const float2*>(s_b + (16 * from + 15) * SB + c);
+            x[j].x *= a.qscale * ex2(b.x - m.x);
+            x[j].y *= a.qscale * ex2(b.y - m.y);
           }
           uint32_t ah[4], al[4];
 #pragma unroll
@@ -418,82 +517,81 @@ chunk_prep_kernel(const DmoeRecur a, const int4* __restrict__ chunks, uint8_t* _
         store_acc_frag(w + L::kP + (mi * 4 + kg) * 2 * kFrag, lane, acc[i][0], acc[i][1]);
       }
     }
-  } else {                                           // warps 0-3; A (warps 4-7)
-    const int mi = warp & 3;
+  } else {
+    // Warps 0-3; A (warps 4-7), the row tiles the other way round: a tile has products with those up to its own, and warps w and
+    // w + 4 share a part of the SM. Rows through ldmatrix; read from global memory as the fragments need them (16 bytes of 8 rows) a
+    // warp's loads alone took a fifth of this section
     const bool second = warp >= 4;
-    if (!second || (DELTA && !slow)) {
-      const int r0 = mi * 16 + g, r1 = r0 + 8;
-      const __nv_bfloat16* src = second ? kp : qp;
-      const long long ld = second ? a.ldk : a.ldq;
+    const int mi = second ? 7 - warp : warp;
+    const bool works = !second || (DELTA && !slow);
+    float acc[8][4];
+    const int r0 = mi * 16 + g, r1 = r0 + 8;
+    if (works) {
+      const uint32_t raw = smem_u32(second ? raw_k : raw_q);
       const float f0 = second ? s_fk[r0] : s_fq[r0], f1 = second ? s_fk[r1] : s_fq[r1];
-      float acc[8][4];
 #pragma unroll
       for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
       const uint32_t bh = smem_u32(s_kh), bl = smem_u32(s_kl);
+#pragma unroll 2
+      for (int ks = 0; ks < KS; ++ks) {
+        uint32_t rows[4], ah[4], al[4], zh[4], zl[4];
+        ldmatrix_x4(raw + raw_at<DP>(mi * 16 + (lm_mi & 1) * 8 + lm_r, ks * 2 + (lm_mi >> 1)), rows[0], rows[1], rows[2], rows[3]);
 #pragma unroll
-      for (int kb = 0; kb < KS; kb += 4) {           // raw values of up to four k tiles in flight
-        uint32_t raw[4][4];
-#pragma unroll
-        for (int kk = 0; kk < 4 && kb + kk < KS; ++kk)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int r = j & 1 ? r1 : r0, c = (kb + kk) * 16 + 2 * tq + (j >> 1) * 8;
-            raw[kk][j] = r < n && c < D ? *reinterpret_cast<const uint32_t*>(src + r * ld + c) : 0u;
-          }
-#pragma unroll
-        for (int kk = 0; kk < 4 && kb + kk < KS; ++kk) {
-          const int ks = kb + kk;
-          uint32_t ah[4], al[4], zh[4], zl[4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int r = j & 1 ? r1 : r0, c = ks * 16 + 2 * tq + (j >> 1) * 8;
-            const float f = j & 1 ? f1 : f0;
-            float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw[kk][j]));
-            x.x *= f;
-            x.y *= f;
-            const float2 b = *reinterpret_cast<const float2*>(s_b + r * DP + c);
-            const float2 m = *reinterpret_cast<const float2*>(s_b + kMid * DP + c);
-            split2(x.x * exp2f(b.x - m.x), x.y * exp2f(b.y - m.y), ah[j], al[j]);
-            if (!second) split2(x.x * exp2f(b.x), x.y * exp2f(b.y), zh[j], zl[j]);
-          }
+        for (int j = 0; j < 4; ++j) {
+          const int r = j & 1 ? r1 : r0, c = ks * 16 + 2 * tq + (j >> 1) * 8;
+          const float f = j & 1 ? f1 : f0;
+          float x[2];
+          unpack(rows[j], x);
+          x[0] *= f;
+          x[1] *= f;
+          const float2 b = *reinterpret_cast<const float2*>(s_b + r * SB + c);
+          const float2 m = *reinterpret_cast<const float2*>(s_b + kMid * SB + c);
+          const float e0 = ex2(b.x - m.x), e1 = ex2(b.y - m.y);
+          split2(x[0] * e0, x[1] * e1, ah[j], al[j]);
           if (!second) {
-            store_frag(w + L::kQ + (mi * KS + ks) * 2 * kFrag, lane, zh);
-            store_frag(w + L::kQ + ((mi * KS + ks) * 2 + 1) * kFrag, lane, zl);
-          }
-          if (slow) continue;
-#pragma unroll
-          for (int kg = 0; kg < 4; ++kg) {
-            if (kg <= mi) {
-              const uint32_t off = ((kg * 16 + (lm_mi >> 1) * 8 + lm_r) * SM::kKs + ks * 16 + (lm_mi & 1) * 8) * 2;
-              uint32_t h0_, h1_, h2_, h3_, l0_, l1_, l2_, l3_;
-              ldmatrix_x4(bh + off, h0_, h1_, h2_, h3_);
-              ldmatrix_x4(bl + off, l0_, l1_, l2_, l3_);
-              mma_split(acc[2 * kg], ah, al, h0_, h1_, l0_, l1_);
-              mma_split(acc[2 * kg + 1], ah, al, h2_, h3_, l2_, l3_);
-            }
-          }
-        }
-      }
-      if (!slow) {
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-          const int c = nt * 8 + 2 * tq, edge = second ? -1 : 0;        // A is strictly below the diagonal
-          if (c > r0 + edge) acc[nt][0] = 0.f;
-          if (c + 1 > r0 + edge) acc[nt][1] = 0.f;
-          if (c > r1 + edge) acc[nt][2] = 0.f;
-          if (c + 1 > r1 + edge) acc[nt][3] = 0.f;
-          if (DELTA && second) {
-            s_A[r0 * LDA + c] = acc[nt][0] * s_beta[r0];
-            s_A[r0 * LDA + c + 1] = acc[nt][1] * s_beta[r0];
-            s_A[r1 * LDA + c] = acc[nt][2] * s_beta[r1];
-            s_A[r1 * LDA + c + 1] = acc[nt][3] * s_beta[r1];
+            float2 em = *reinterpret_cast<const float2*>(s_em + c);
+            em.x *= e0;
+            em.y *= e1;
+            if (direct) em = make_float2(ex2(b.x), ex2(b.y));
+            split2(x[0] * em.x, x[1] * em.y, zh[j], zl[j]);
           }
         }
         if (!second) {
-#pragma unroll
-          for (int kg = 0; kg < 4; ++kg)
-            store_acc_frag(w + L::kP + (mi * 4 + kg) * 2 * kFrag, lane, acc[2 * kg], acc[2 * kg + 1]);
+          store_frag(w + L::kQ + (mi * KS + ks) * 2 * kFrag, lane, zh);
+          store_frag(w + L::kQ + ((mi * KS + ks) * 2 + 1) * kFrag, lane, zl);
         }
+        if (slow) continue;
+#pragma unroll
+        for (int kg = 0; kg < 4; ++kg) {
+          if (kg <= mi) {
+            const uint32_t off = ((kg * 16 + (lm_mi >> 1) * 8 + lm_r) * SM::kKs + ks * 16 + (lm_mi & 1) * 8) * 2;
+            uint32_t h0_, h1_, h2_, h3_, l0_, l1_, l2_, l3_;
+            ldmatrix_x4(bh + off, h0_, h1_, h2_, h3_);
+            ldmatrix_x4(bl + off, l0_, l1_, l2_, l3_);
+            mma_split(acc[2 * kg], ah, al, h0_, h1_, l0_, l1_);
+            mma_split(acc[2 * kg + 1], ah, al, h2_, h3_, l2_, l3_);
+          }
+        }
+      }
+    }
+    if (DELTA) __syncthreads();                      // the rows of k are read: A takes their place
+    if (works && !slow) {
+#pragma unroll
+      for (int nt = 0; nt < 8; ++nt) {
+        const int c = nt * 8 + 2 * tq, edge = second ? -1 : 0;        // A is strictly below the diagonal
+        if (c > r0 + edge) acc[nt][0] = 0.f;
+        if (c + 1 > r0 + edge) acc[nt][1] = 0.f;
+        if (c > r1 + edge) acc[nt][2] = 0.f;
+        if (c + 1 > r1 + edge) acc[nt][3] = 0.f;
+        if (DELTA && second) {
+          *reinterpret_cast<float2*>(s_A + r0 * LDA + c) = make_float2(acc[nt][0] * s_beta[r0], acc[nt][1] * s_beta[r0]);
+          *reinterpret_cast<float2*>(s_A + r1 * LDA + c) = make_float2(acc[nt][2] * s_beta[r1], acc[nt][3] * s_beta[r1]);
+        }
+      }
+      if (!second) {
+#pragma unroll
+        for (int kg = 0; kg < 4; ++kg)
+          store_acc_frag(w + L::kP + (mi * 4 + kg) * 2 * kFrag, lane, acc[2 * kg], acc[2 * kg + 1]);
       }
     }
   }
@@ -504,7 +602,7 @@ chunk_prep_kernel(const DmoeRecur a, const int4* __restrict__ chunks, uint8_t* _
       if ((BONUS ? j < t : j <= t) && t < n) {
         const int tr = BONUS ? t - 1 : t;              // place of the read-out
         for (int d = 0; d < D; ++d) {
-          const float e = __bfloat162float(kp[j * a.ldk + d]) * s_fk[j] * exp2f(s_b[tr * DP + d] - s_b[j * DP + d]);
+          const float e = __bfloat162float(kp[j * a.ldk + d]) * s_fk[j] * ex2(s_b[tr * SB + d] - s_b[j * SB + d]);
           p += __bfloat162float(qp[t * a.ldq + d]) * e;
           if (DELTA) kk += __bfloat162float(kp[t * a.ldk + d]) * e;
         }
@@ -529,7 +627,7 @@ chunk_prep_kernel(const DmoeRecur a, const int4* __restrict__ chunks, uint8_t* _
   const int nd = (DP + 63) / 64, nv = (V + 63) / 64;
   const __nv_bfloat16* vp = static_cast<const __nv_bfloat16*>(a.v) + row0 * a.ldv + h * V;
   float* w_u = reinterpret_cast<float*>(w + L::kU);
-  const int mi = warp & 3, nh = warp >> 2;
+  const int nh = warp >> 2, mi = nh ? 7 - warp : warp;      // T is triangular: as above
   uint32_t raw[8];                                   // the next 64-column tile of k or v: rows tid / 32 + 8 i
   auto fetch = [&](int x) {
     const bool keys = x < nd;
@@ -542,10 +640,12 @@ chunk_prep_kernel(const DmoeRecur a, const int4* __restrict__ chunks, uint8_t* _
     }
   };
   fetch(0);
-  invert_unit_lower(s_A, s_T, reinterpret_cast<float*>(s_xh));
+  invert_unit_lower(s_A, s_T, reinterpret_cast<float*>(s_xh), reinterpret_cast<float*>(s_th));
   for (int i = tid; i < kChunk * kChunk / 2; i += kChunkThreads) {
     const int t = i / (kChunk / 2), c = i % (kChunk / 2) * 2;
-    const float v[2] = {s_T[t * LDA + c], s_T[t * LDA + c + 1]};
+    if (c / 16 > t / 16) continue;
+    float v[2];
+    load_f32<2>(s_T + t * LDA + c, v);
     store_split<2>(s_th + t * kPs + c, s_tl + t * kPs + c, v);
   }
   for (int x = 0; x < nd + nv; ++x) {
@@ -558,8 +658,10 @@ chunk_prep_kernel(const DmoeRecur a, const int4* __restrict__ chunks, uint8_t* _
       float v[2] = {r.x * s_beta[t], r.y * s_beta[t]};
       if (keys) {
         const float f = -s_fk[t];
-        v[0] *= cc < DP ? f * exp2f(s_b[t * DP + cc]) : 0.f;
-        v[1] *= cc < DP ? f * exp2f(s_b[t * DP + cc + 1]) : 0.f;
+        float2 b = make_float2(0.f, 0.f);
+        if (cc < DP) b = *reinterpret_cast<const float2*>(s_b + t * SB + cc);
+        v[0] *= cc < DP ? f * ex2(b.x) : 0.f;
+        v[1] *= cc < DP ? f * ex2(b.y) : 0.f;
       }
       store_split<2>(s_xh + t * kPs + c, s_xl + t * kPs + c, v);
     }
