@@ -1117,9 +1117,13 @@ static int run_chunks(const DmoeRecur& a, const void* chunks, int n_chunks, uint
   long long per = ws_bytes / (stride * n_chunks);               // heads whose chunks fit the workspace at a time
   if (per < 1) return -15;
   if (per > a.heads) per = a.heads;
-  // narrower value tiles where the wide ones would leave SMs idle
-  const long long wide = static_cast<long long>(a.n_segs) * per * ((a.vdim + 31) / 32);
-  const bool narrow = a.vdim <= 16 || wide < device_num_sms();
+  // Value tiles of 16 or 32 columns: a chunk of 32 takes 1.2 times as long as one of 16 (delta rule 1.4 times), one CTA fits an SM and
+  // walks all chunks of its segment, so the launch takes as long as its waves. Measured over the whole recurrence, 2048 tokens, heads
+  // of 128 x 128, tiles of 16 -> 32, us: 16 heads (one wave both ways, 4096 tokens) plain 201 -> 218, delta 263 -> 325; 20 heads (two
+  // waves -> one) 158 -> 127, 223 -> 198; 32 heads 206 -> 155, 270 -> 239; 40 heads (three -> two) 285 -> 240, 366 -> 366.
+  const long long sms = device_num_sms(), extra = MODE == kMemory ? 1 : 0;
+  const auto waves = [&](int vt) { return (a.n_segs * per * ((a.vdim + vt - 1) / vt + extra) + sms - 1) / sms; };
+  const bool narrow = a.vdim <= 16 || waves(16) * 5 < waves(32) * (DELTA ? 7 : 6);
   for (int h0 = 0; h0 < a.heads; h0 += static_cast<int>(per)) {
     const int hn = a.heads - h0 < per ? a.heads - h0 : static_cast<int>(per);
     int rc;

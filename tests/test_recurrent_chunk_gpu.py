@@ -47,3 +47,24 @@ def test_fading(delta, H, G, D, V, T, fade):
     g = gate.view(T, H, V).double()
     o = o * torch.sigmoid(g) * g
     assert (out.view(T, H, V).double() - o).norm() < 2.0 ** -8 * o.norm()      # one rounding to bf16: at most 2^-8 of every value
+
+
+@pytest.mark.parametrize("delta", [False, True])
+def test_value_tiles_agree(delta):
+    """20 heads take value tiles of 32 columns (one wave of CTAs), 10 heads those of 16: the same sums in the same order."""
+    torch.manual_seed(3)
+    T, H, D, V = 150, 20, 72, 120
+    bf = lambda *s: torch.randn(*s, device="cuda").to(torch.bfloat16)
+    q, k, v, gate, beta, z = bf(T, H * D), bf(T, H * D), bf(T, H * V), bf(T, H * V), bf(T, H), torch.randn(T, H * D, device="cuda")
+    bias, log = torch.randn(H * D, device="cuda"), 0.3 * torch.randn(H, device="cuda")
+
+    def run(a, b):
+        d, e = slice(a * D, b * D), slice(a * V, b * V)
+        r = Recurrence(b - a, b - a, D, V, delta, bias[d], torch.ones(V, device="cuda"), 1e-6, a_log=log[a:b] if delta else None)
+        s = r.new_state(1, torch.bfloat16, "cuda")
+        return recurrent_attention(r, q[:, d], k[:, d], v[:, e], gate[:, e], beta[:, a:b] if delta else None, z[:, d], s,
+                                   build_segments([0] * T, range(T), "cuda")), s.S[0]
+    out, S = run(0, H)
+    for a in (0, 10):
+        o, s = run(a, a + 10)
+        assert torch.equal(o, out[:, a * V:(a + 10) * V]) and torch.equal(s, S[a:a + 10])
