@@ -214,8 +214,8 @@ struct PrepSmem {
 // 144 KB: 35 us for 1024 of them at the copy rate). Of the 109 thousand cycles that such a chunk took, rows read from global memory as
 // fragments need them, decays in rows that meet in the same banks, two exponentials where a product does, a branch per token's
 // decay, logits fetched eight at a time, norms reduced one by one and the inversion's loads made up more than a third. Recurrence as a
-// whole (preparation, scan, norm), 4096 tokens x 16 heads of 128 x 128, before -> now, us: delta rule 359 -> 263, plain write 221 ->
-// 198, bonus 228 -> 202; 700 tokens x 32 heads of 64 x 64: 68 -> 54, 38.6 -> 34.3, 36.7 -> 34.8.
+// whole (preparation, scan, norm), 4096 tokens x 16 heads of 128 x 128, before -> now, us: delta rule 359 -> 261, plain write 221 ->
+// 198, bonus 228 -> 200; 700 tokens x 32 heads of 64 x 64: 68 -> 54, 38.6 -> 34.3, 36.7 -> 34.8.
 template <int DP, int MODE>
 __global__ void __launch_bounds__(kChunkThreads, MODE == kBonus && DP <= 64 ? 3 : 2)
 chunk_prep_kernel(const DmoeRecur a, const int4* __restrict__ chunks, uint8_t* __restrict__ ws, long long ws_stride, int h0) {
@@ -831,7 +831,7 @@ chunk_prep_head_kernel(const DmoeRecur a, const int4* __restrict__ chunks, uint8
 // the state and u, the right operands that every warp shares, go through shared memory.
 template <int DP, int VT, int MODE>
 __global__ void __launch_bounds__(kChunkThreads, 1)
-chunk_scan_kernel(const DmoeRecur a, const uint8_t* __restrict__ ws, long long ws_stride, int h0, int n_heads) {
+chunk_scan_kernel(const DmoeRecur a, const uint8_t* __restrict__ ws, long long ws_stride, int h0, int n_heads, bool ahead) {
   using L = ChunkWs<DP>;
   constexpr bool DELTA = MODE == kDelta, MEM = MODE == kMemory;
   constexpr int NT = VT / 8, KS = DP / 16, MT = DP / 16, VS = VT + 8;
@@ -963,6 +963,8 @@ chunk_scan_kernel(const DmoeRecur a, const uint8_t* __restrict__ ws, long long w
   __syncthreads();
 
   for (int c = 0; c < nc; ++c) {
+    if (ahead && blockIdx.z == 0 && tid == 0 && c + 3 < nc)      // one value tile for all of the head
+      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(base(c + 3)), "r"(static_cast<uint32_t>(ws_stride)) : "memory");
     if (!DELTA && tid < kChunk * NT) {                           // u = v
       *reinterpret_cast<uint4*>(p_u[0] + tid / NT * VS + tid % NT * 8) = vnext;
       if (c + 1 < nc) fetch_v(c + 1);
@@ -1104,9 +1106,13 @@ static int launch_prep_head(const DmoeRecur& a, const void* chunks, int n_chunks
 }
 
 template <int DP, int VT, int MODE>
-static int launch_scan(const DmoeRecur& a, const uint8_t* ws, long long stride, int h0, int hn, cudaStream_t stream) {
+static int launch_scan(const DmoeRecur& a, const uint8_t* ws, long long stride, int h0, int hn, int n_chunks, cudaStream_t stream) {
   const dim3 grid(a.n_segs, hn, (a.vdim + VT - 1) / VT + (MODE == kMemory ? 1 : 0));
-  chunk_scan_kernel<DP, VT, MODE><<<grid, kChunkThreads, 0, stream>>>(a, ws, stride, h0, hn);
+  // What the preparation wrote is still in the L2 where it is small. Above that a chunk's left operands are asked for three chunks
+  // before their turn: 4096 tokens x 16 heads of 128 x 128 (84 MB; delta rule 147 MB), whole recurrence, plain 201 -> 184 us, bonus 203 ->
+  // 186, delta 263 -> 257; 2048 tokens x 20 heads (53 MB) 126.8 -> 125.4; below 32 MB equal or 1 % slower
+  const bool ahead = stride * n_chunks * hn > (32ll << 20);
+  chunk_scan_kernel<DP, VT, MODE><<<grid, kChunkThreads, 0, stream>>>(a, ws, stride, h0, hn, ahead);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1133,8 +1139,8 @@ static int run_chunks(const DmoeRecur& a, const void* chunks, int n_chunks, uint
     if (rc != 0) return rc;
     // the scan of a bonus is that of the plain write
     constexpr int SCAN = MODE == kBonus ? kPlain : MODE;
-    rc = narrow ? launch_scan<DP, 16, SCAN>(a, ws, stride, h0, hn, stream)
-                : launch_scan<DP, 32, SCAN>(a, ws, stride, h0, hn, stream);
+    rc = narrow ? launch_scan<DP, 16, SCAN>(a, ws, stride, h0, hn, n_chunks, stream)
+                : launch_scan<DP, 32, SCAN>(a, ws, stride, h0, hn, n_chunks, stream);
     if (rc != 0) return rc;
   }
   return 0;

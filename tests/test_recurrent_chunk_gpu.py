@@ -68,3 +68,22 @@ def test_value_tiles_agree(delta):
     for a in (0, 10):
         o, s = run(a, a + 10)
         assert torch.equal(o, out[:, a * V:(a + 10) * V]) and torch.equal(s, S[a:a + 10])
+
+
+def test_operands_asked_for_ahead():
+    """A workspace of more than 32 MB (asked for ahead of its turn) gives what its heads give alone."""
+    torch.manual_seed(4)
+    T, H, D, V = 1600, 17, 128, 16
+    bf = lambda *s: torch.randn(*s, device="cuda").to(torch.bfloat16)
+    q, k, v, gate, z = bf(T, H * D), bf(T, H * D), bf(T, H * V), bf(T, H * V), torch.randn(T, H * D, device="cuda") + 3.0
+
+    def run(a, b):
+        d, e = slice(a * D, b * D), slice(a * V, b * V)
+        r = Recurrence(b - a, b - a, D, V, False, torch.zeros((b - a) * D, device="cuda"), torch.ones(V, device="cuda"), 1e-6)
+        s = r.new_state(1, torch.bfloat16, "cuda")
+        return recurrent_attention(r, q[:, d].contiguous(), k[:, d].contiguous(), v[:, e].contiguous(), gate[:, e].contiguous(), None,
+                                   z[:, d].contiguous(), s, build_segments([0] * T, range(T), "cuda")), s.S[0]
+    out, S = run(0, H)
+    for a in (0, 16):
+        o, s = run(a, a + 1)
+        assert torch.equal(o, out[:, a * V:(a + 1) * V]) and torch.equal(s, S[a:a + 1])
