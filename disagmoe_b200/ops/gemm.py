@@ -159,7 +159,8 @@ def want_wide(epi: int, T: int, F: int, K: int, G: int, sms: int) -> bool:
 
     Dense: a cost model of both, in us, fitted to a sweep on B200 (K 1024 .. 5632, F 256 .. 32000, T 8 .. 2048; the choice is within
     8 % of the better of these two kernels, K below 1024 within 15 %). A wide tile takes 0.31 us per K block whatever part of it is
-    used, the other kernel what its SM pulls from L2. Measured (bf16, other kernel -> wide): 4096 x 6144 x 4096 201 -> 149 us (1381
+    used, the other kernel what its SM pulls from L2. Measured (bf16, other kernel -> wide tiles of 256 rows; :func:`dense_wide` then takes
+    narrower ones, :func:`split_plan` a third kernel): 4096 x 6144 x 4096 201 -> 149 us (1381
     TFLOP/s), 2500 x 4096 x 2048 106 -> 40, 1111 x 6144 x 2048 79 -> 31, 256 x 32000 x 4096 89 -> 58; SwiGLU 1024 x 5632 x 2048 59 ->
     42. A few rows of SwiGLU gain by the wider tile's faster K blocks (1 row, 2048 x 4096 38 -> 32, 16 rows, 8192 x 7168 82 -> 65),
     but pay 2 us more per launch (1 row, 2048 x 256 11.2 -> 12.6, 4096 x 1024 17.4 -> 17.4), and more where the tiles of a wave want
