@@ -55,6 +55,32 @@ def test_rows_of_the_next_group_stay(sizes):
         assert bool((out[sum(sizes):] == 7.0).all()) and bool((out[:, N:] == 7.0).all())
 
 
+@pytest.mark.parametrize("blocked", [False, True])
+@pytest.mark.parametrize("sizes", [[5, 64, 128, 65, 0, 129, 385], [1], [127, 32]])
+def test_tail_tiles(sizes, blocked):
+    """Tiles of up to 128 tokens (64 per CTA, both halves of the columns in one TMEM): plain, fp32, gated and combining."""
+    torch.manual_seed(sum(sizes))
+    G, N, K, T = len(sizes), 384, 192, sum(sizes)
+    x, w13, w = _bf(T, K), _bf(G, 2 * N, K) * K ** -0.5, _bf(G, N, K) * K ** -0.5
+    offs = torch.tensor([0, *sizes], device="cuda").cumsum(0).to(torch.int32)
+    lay = gemm.block_weight if blocked else lambda t: t
+    kw = dict(wide=True, w_blocked=blocked)
+    up, y, y32 = gemm.grouped_swiglu(x, lay(w13), offs, **kw), gemm.grouped_linear(x, lay(w), offs, **kw), \
+        gemm.grouped_linear(x, lay(w), offs, out_dtype=torch.float32, **kw)
+    recs, weight, to = torch.zeros(T, 4, dtype=torch.int32, device="cuda"), torch.rand(T, device="cuda"), torch.randperm(T, device="cuda")
+    recs[:, 1], recs[:, 2] = to.int(), weight.view(torch.int32)
+    out = torch.full((T + 1, N), 7.0, dtype=torch.bfloat16, device="cuda")
+    gemm.grouped_combine(x, lay(w), offs, recs, torch.tensor([out.data_ptr()], device="cuda"), N, **kw)
+    assert bool((out[T] == 7.0).all())
+    for g in range(G):
+        a, b = sum(sizes[:g]), sum(sizes[:g + 1])
+        h, r = x[a:b].double() @ w13[g].double().T, x[a:b].double() @ w[g].double().T
+        _close(up[a:b], h[:, :N] * torch.sigmoid(h[:, :N]) * h[:, N:], K)
+        _close(y[a:b], r, K)
+        _close(y32[a:b], r, K)
+        _close(out[to[a:b]], r * weight[a:b, None].double(), K)
+
+
 @pytest.mark.parametrize("hd,cols", [(64, 64), (64, 192), (64, 256), (128, 128), (128, 256)])
 def test_heads_stay_whole(hd, cols):
     torch.manual_seed(cols)
