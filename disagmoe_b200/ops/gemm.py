@@ -166,9 +166,12 @@ def want_wide(epi: int, T: int, F: int, K: int, G: int, sms: int) -> bool:
     but pay 2 us more per launch (1 row, 2048 x 256 11.2 -> 12.6, 4096 x 1024 17.4 -> 17.4), and more where the tiles of a wave want
     more than HBM gives (1 row, 8192 x 1024 17.4 -> 19.3, 8192 x 7168 69 -> 78; 8 rows, 8192 x 4096 47 -> 49).
 
-    Grouped (only the mean group size is known): up to 128 tokens the other kernel's tile fits a group and streams the weights
-    at HBM speed, beyond that it needs a second tile per group. Measured at 64 experts of 1408 x 2048, SwiGLU: 120 tokens each
-    140 -> 154 us, 150: 187 -> 160; 8 experts of 14336 x 4096: 128 tokens 344 -> 393, 160: 456 -> 391. Down-projections with
+    Grouped (only the mean group size is known): up to 128 tokens both kernels read the weights once; the wide one has a half product for
+    such groups and no transposing epilogue, the other one smaller units, which counts where few experts have long rows of tiles. Sweep
+    over 20 shapes at 40 .. 128 tokens per expert (other kernel / wide): SwiGLU with F K to 6 million 0.99 .. 1.57 (64 x 1408 x 2048, 104
+    tokens 133 -> 126 us; 16 x 2816 x 2048, 96 tokens 69 -> 64), above that 0.93 .. 1.1 (8 x 14336 x 4096: 40 tokens 290 -> 309, 128: 354 ->
+    339); down-projections to K 5632 1.00 .. 1.70 (16 x (2048 x 2816), 96 tokens 46 -> 37), 8 x (4096 x 14336): 64 tokens 155 -> 157, 96: 183 ->
+    159. Beyond 128 tokens the other kernel needs a second tile per group (8 x 14336 x 4096, SwiGLU, 160: 533 -> 369). Down-projections with
     short K loops are bound by the other kernel's transposing epilogue at any size. Sweep over 8 .. 64 experts, F 2048 .. 6144, K 512
     .. 7168, 2 rows in all .. 140 per expert: with F K to 4.4 million 0.92 .. 1.9 times as fast, 1.17 on average (60 x (2048 x 1408):
     16 rows 46 -> 34, 148 rows 81 -> 70; 8 x (4096 x 1024): 74 rows 28 -> 25); above that a badly filled wave of long tiles can make it
@@ -176,7 +179,9 @@ def want_wide(epi: int, T: int, F: int, K: int, G: int, sms: int) -> bool:
     1.5; 60 x (4096 x 2048): 64 rows 136 -> 131); from K 2816 on nothing is gained (8 x (4096 x 14336): 2 rows 47 -> 77, 128 rows 149 -> 181)."""
     kblocks, pairs = (K + 63) // 64, max(1, sms // 2)
     if G > 1:
-        return T >= 144 * G or (epi != EPI_SWIGLU and K <= 2048 and (F * K <= 4_400_000 or G >= 60))
+        if epi == EPI_SWIGLU:
+            return T >= 128 * G or (T >= 40 * G and F * K <= 6_000_000)
+        return T >= 88 * G or (T >= 40 * G and K <= 6144) or (K <= 2048 and (F * K <= 4_400_000 or G >= 60))
     if T < 64 and epi != EPI_SWIGLU:
         return False
     if T <= 32 and (K < 1024 or F > 4096 and K < (8192 if T <= 8 else 4096)):      # SwiGLU: see above

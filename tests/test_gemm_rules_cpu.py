@@ -22,6 +22,15 @@ def test_measured_choices(epi, T, F, K, G, wide):
     assert gemm.want_wide(epi, T, F, K, G, SMS) is wide
 
 
+@pytest.mark.parametrize("epi,per,F,K,G,wide", [
+    (gemm.EPI_SWIGLU, 104, 1408, 2048, 64, True), (gemm.EPI_SWIGLU, 39, 1408, 2048, 64, False), (gemm.EPI_SWIGLU, 127, 14336, 4096, 8, False),
+    (gemm.EPI_SWIGLU, 128, 14336, 4096, 8, True), (gemm.EPI_SWIGLU, 64, 6144, 2048, 16, False), (gemm.EPI_COMBINE, 87, 4096, 14336, 8, False),
+    (gemm.EPI_COMBINE, 88, 4096, 14336, 8, True), (gemm.EPI_PLAIN, 40, 6144, 2048, 16, True), (gemm.EPI_COMBINE, 39, 6144, 2048, 16, False),
+])
+def test_measured_choices_per_expert(epi, per, F, K, G, wide):
+    assert gemm.want_wide(epi, per * G, F, K, G, SMS) is wide
+
+
 @pytest.mark.parametrize("G", [1, 2, 8, 64])
 def test_stream_k_of_no_expected_rows(G):
     """An expert rank whose share of the arriving rows rounds to none still asks for a rule: 32 tiles leave most SMs idle."""
