@@ -71,12 +71,6 @@ __device__ __forceinline__ void store_acc_frag(uint8_t* tile, int lane, const fl
   store_frag(tile + kFrag, lane, l);
 }
 
-// 2^x; a result below the normal numbers (2^-126) is 0
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 // N consecutive bf16 of a row, as they are
 template <int N>
 struct Raw { using T = unsigned short; };
@@ -207,15 +201,17 @@ struct PrepSmem {
   static constexpr int kRegion = kKn > kTX ? kKn : kTX;
   // behind the region: A and T, where the rows of k and q lie before them; the rows of q; or the decays of a bonus' tiles
   static constexpr int kBehind = DELTA ? 2 * 4 * kChunk * kLdA : MODE == kBonus ? 4 * 4 * DP : 2 * kChunk * DP;
-  static constexpr int kBytes = 4 * kChunk * kSb + 3 * 4 * kChunk + 4 * DP + kRegion + kBehind + 16;
+  static constexpr int kBytes = 4 * kChunk * kSb + 3 * 4 * kChunk + kRegion + kBehind + 16;
 };
 
 // Bound by what its 16 warps per SM issue and wait for, not by memory (a delta chunk of 128 channels and values reads 80 KB and writes
 // 144 KB: 35 us for 1024 of them at the copy rate). Of the 109 thousand cycles that such a chunk took, rows read from global memory as
-// fragments need them, decays in rows that meet in the same banks, two exponentials where a product does, a branch per token's
-// decay, logits fetched eight at a time, norms reduced one by one and the inversion's loads made up more than a third. Recurrence as a
-// whole (preparation, scan, norm), 4096 tokens x 16 heads of 128 x 128, before -> now, us: delta rule 359 -> 261, plain write 221 ->
-// 198, bonus 228 -> 200; 700 tokens x 32 heads of 64 x 64: 68 -> 54, 38.6 -> 34.3, 36.7 -> 34.8.
+// fragments need them, decays in rows that meet in the same banks, a branch per token's decay, logits fetched eight at a time, norms
+// reduced one by one and the inversion's loads made up more than a third. Recurrence as a whole (preparation, scan with its operands
+// asked for ahead, norm), 4096 tokens x 16 heads of 128 x 128, before -> now, us: delta rule 360 -> 262, plain write 221 -> 183, bonus 228
+// -> 188; 700 tokens x 32 heads of 64 x 64: 68 -> 54, 38.4 -> 34.6, 36.7 -> 35.2.
+// exp2f and not the instruction alone, which makes 0 of decays below 2^-126 (1 to 2 % of these times); e^b of a read-out as one
+// exponential and not as e^(b - m) e^m, which is rounded three times.
 template <int DP, int MODE>
 __global__ void __launch_bounds__(kChunkThreads, MODE == kBonus && DP <= 64 ? 3 : 2)
 chunk_prep_kernel(const DmoeRecur a, const int4* __restrict__ chunks, uint8_t* __restrict__ ws, long long ws_stride, int h0) {
@@ -228,8 +224,7 @@ chunk_prep_kernel(const DmoeRecur a, const int4* __restrict__ chunks, uint8_t* _
   float* s_fq = s_b + kChunk * SB;                              // [64] factors of the raw q and k rows
   float* s_fk = s_fq + kChunk;
   float* s_beta = s_fk + kChunk;                                // delta: write strengths; bonus: P_tt
-  float* s_em = s_beta + kChunk;                                // [DP] decay up to the middle
-  uint8_t* region = reinterpret_cast<uint8_t*>(s_em + DP);
+  uint8_t* region = reinterpret_cast<uint8_t*>(s_beta + kChunk);
   __nv_bfloat16* s_kh = reinterpret_cast<__nv_bfloat16*>(region);          // scaled k rows, hi then lo plane
   __nv_bfloat16* s_kl = s_kh + kChunk * SM::kKs;
   float* s_A = reinterpret_cast<float*>(region + SM::kRegion);
@@ -349,7 +344,7 @@ chunk_prep_kernel(const DmoeRecur a, const int4* __restrict__ chunks, uint8_t* _
     s_fk[t0 + lane] = 1.f;
   }
   __syncthreads();
-  bool wide = false, faint = false;
+  bool wide = false;
   if (tid < DP) {
     const float m = s_b[kMid * SB + tid];
     if (BONUS) {
@@ -358,18 +353,15 @@ chunk_prep_kernel(const DmoeRecur a, const int4* __restrict__ chunks, uint8_t* _
       for (int i = 0; i < 4; ++i) {
         const float end = s_b[(16 * i + 15) * SB + tid];
         wide = wide || from - end > kMaxTileShift;
-        s_step[i * DP + tid] = ex2(end - from);
+        s_step[i * DP + tid] = exp2f(end - from);
         from = end;
       }
     } else {
       wide = s_b[tid] - m > kMaxShift || m - s_b[(kChunk - 1) * SB + tid] > kMaxShift;
-      faint = m < -kMaxTileShift;
-      s_em[tid] = ex2(m);
     }
-    reinterpret_cast<float*>(w + L::kDec)[tid] = ex2(s_b[(kChunk - 1) * SB + tid]);
+    reinterpret_cast<float*>(w + L::kDec)[tid] = exp2f(s_b[(kChunk - 1) * SB + tid]);
   }
   const bool slow = __syncthreads_or(wide);
-  const bool direct = !BONUS && (__syncthreads_or(faint) || slow);      // e^b is not e^(b - m) e^m in fp32
 
   // ---- k e^(b_end - b): through shared memory into transposed fragments
   auto stage_k = [&] {
@@ -385,27 +377,27 @@ chunk_prep_kernel(const DmoeRecur a, const int4* __restrict__ chunks, uint8_t* _
     float tile[PL], rest[PL];
     load_f32<PL>(s_b + (warp / 2 * 16 + 15) * SB + d0, tile);
 #pragma unroll
-    for (int e = 0; e < PL; ++e) rest[e] = ex2(end[e] - tile[e]);
+    for (int e = 0; e < PL; ++e) rest[e] = exp2f(end[e] - tile[e]);
 #pragma unroll
     for (int i = 0; i < ROWS; ++i) {
       float b[PL];
       load_f32<PL>(s_b + (t0 + i) * SB + d0, b);
 #pragma unroll
       for (int e = 0; e < PL; ++e) {
-        k_tile[BONUS ? i : 0][e] = k[i][e] * ex2(tile[e] - b[e]);
+        k_tile[BONUS ? i : 0][e] = k[i][e] * exp2f(tile[e] - b[e]);
         k[i][e] = k_tile[BONUS ? i : 0][e] * rest[e];
       }
     }
   } else {
     load_f32<PL>(s_b + kMid * SB + d0, to_mid);
 #pragma unroll
-    for (int e = 0; e < PL; ++e) to_mid[e] = slow ? 0.f : ex2(to_mid[e] - end[e]);
+    for (int e = 0; e < PL; ++e) to_mid[e] = slow ? 0.f : exp2f(to_mid[e] - end[e]);
 #pragma unroll
     for (int i = 0; i < ROWS; ++i) {
       float b[PL];
       load_f32<PL>(s_b + (t0 + i) * SB + d0, b);
 #pragma unroll
-      for (int e = 0; e < PL; ++e) k[i][e] *= ex2(end[e] - b[e]);
+      for (int e = 0; e < PL; ++e) k[i][e] *= exp2f(end[e] - b[e]);
     }
   }
   stage_k();
@@ -466,8 +458,8 @@ chunk_prep_kernel(const DmoeRecur a, const int4* __restrict__ chunks, uint8_t* _
             if (r > 0) b = *reinterpret_cast<const float2*>(s_b + (r - 1) * SB + c);
             float2 m = make_float2(0.f, 0.f);
             if (from >= 0) m = *reinterpret_cast<const float2*>(s_b + (16 * from + 15) * SB + c);
-            x[j].x *= a.qscale * ex2(b.x - m.x);
-            x[j].y *= a.qscale * ex2(b.y - m.y);
+            x[j].x *= a.qscale * exp2f(b.x - m.x);
+            x[j].y *= a.qscale * exp2f(b.y - m.y);
           }
           uint32_t ah[4], al[4];
 #pragma unroll
@@ -546,15 +538,8 @@ chunk_prep_kernel(const DmoeRecur a, const int4* __restrict__ chunks, uint8_t* _
           x[1] *= f;
           const float2 b = *reinterpret_cast<const float2*>(s_b + r * SB + c);
           const float2 m = *reinterpret_cast<const float2*>(s_b + kMid * SB + c);
-          const float e0 = ex2(b.x - m.x), e1 = ex2(b.y - m.y);
-          split2(x[0] * e0, x[1] * e1, ah[j], al[j]);
-          if (!second) {
-            float2 em = *reinterpret_cast<const float2*>(s_em + c);
-            em.x *= e0;
-            em.y *= e1;
-            if (direct) em = make_float2(ex2(b.x), ex2(b.y));
-            split2(x[0] * em.x, x[1] * em.y, zh[j], zl[j]);
-          }
+          split2(x[0] * exp2f(b.x - m.x), x[1] * exp2f(b.y - m.y), ah[j], al[j]);
+          if (!second) split2(x[0] * exp2f(b.x), x[1] * exp2f(b.y), zh[j], zl[j]);
         }
         if (!second) {
           store_frag(w + L::kQ + (mi * KS + ks) * 2 * kFrag, lane, zh);
@@ -602,7 +587,7 @@ chunk_prep_kernel(const DmoeRecur a, const int4* __restrict__ chunks, uint8_t* _
       if ((BONUS ? j < t : j <= t) && t < n) {
         const int tr = BONUS ? t - 1 : t;              // place of the read-out
         for (int d = 0; d < D; ++d) {
-          const float e = __bfloat162float(kp[j * a.ldk + d]) * s_fk[j] * ex2(s_b[tr * SB + d] - s_b[j * SB + d]);
+          const float e = __bfloat162float(kp[j * a.ldk + d]) * s_fk[j] * exp2f(s_b[tr * SB + d] - s_b[j * SB + d]);
           p += __bfloat162float(qp[t * a.ldq + d]) * e;
           if (DELTA) kk += __bfloat162float(kp[t * a.ldk + d]) * e;
         }
@@ -660,8 +645,8 @@ chunk_prep_kernel(const DmoeRecur a, const int4* __restrict__ chunks, uint8_t* _
         const float f = -s_fk[t];
         float2 b = make_float2(0.f, 0.f);
         if (cc < DP) b = *reinterpret_cast<const float2*>(s_b + t * SB + cc);
-        v[0] *= cc < DP ? f * ex2(b.x) : 0.f;
-        v[1] *= cc < DP ? f * ex2(b.y) : 0.f;
+        v[0] *= cc < DP ? f * exp2f(b.x) : 0.f;
+        v[1] *= cc < DP ? f * exp2f(b.y) : 0.f;
       }
       store_split<2>(s_xh + t * kPs + c, s_xl + t * kPs + c, v);
     }

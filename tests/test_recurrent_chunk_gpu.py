@@ -49,6 +49,49 @@ def test_fading(delta, H, G, D, V, T, fade):
     assert (out.view(T, H, V).double() - o).norm() < 2.0 ** -8 * o.norm()      # one rounding to bf16: at most 2^-8 of every value
 
 
+@pytest.mark.parametrize("drops", [{1: 75.0, 40: 16.0}, {1: 45.0, 40: 46.0}])
+@pytest.mark.parametrize("kind,D,V", [("plain", 128, 16), ("plain", 40, 24), ("bonus", 128, 16), ("bonus", 64, 40), ("delta", 72, 16)])
+def test_decays_below_the_normal_range(kind, D, V, drops):
+    """A state and a write that fade by 2^-131 within a chunk (to a subnormal factor) still count: both are as large as fp32 and bf16 have
+    them. The first drops leave pairs of tokens to products, the second ones are evaluated pair by pair."""
+    torch.manual_seed(D)
+    T, H, pos0 = 64, 2, 100
+    bf = lambda *s: (1.0 + torch.rand(*s, device="cuda")).to(torch.bfloat16)
+    q, k, v, gate, beta = 2.0 ** 20 * bf(T, H * D), 2.0 ** 20 * bf(T, H * D), torch.zeros(T, H * V, device="cuda").bfloat16(), bf(T, H * V), bf(T, H)
+    v[0] = 2.0 ** 100 * bf(H * V)
+    q[0] = 0.0                                             # its read-out would be no fp32 number
+    if kind == "delta":
+        k.zero_()                                          # nothing written or taken back: the state fades
+    z = torch.full((T, H * D), -80.0, device="cuda")       # a factor of 1
+    for t, x in drops.items():
+        z[t] = x
+    bonus = torch.rand(H, D, device="cuda") if kind == "bonus" else None
+    r = Recurrence(H, H, D, V, kind == "delta", torch.zeros(H * D, device="cuda"), torch.ones(V, device="cuda"), 1e-30, bonus=bonus,
+                   a_log=torch.zeros(H, device="cuda") if kind == "delta" else None)
+    state = r.new_state(1, torch.bfloat16, "cuda")
+    state.S[0] = 2.0 ** 120 * (1.0 + torch.rand(H, D, V, device="cuda"))
+    S = state.S[0].double()
+    out = recurrent_attention(r, q, k, v, gate, beta if kind == "delta" else None, z if kind == "delta" else -z, state,
+                              build_segments([0] * T, range(pos0, pos0 + T), "cuda"))
+    qq, kk, vv = q.view(T, H, D).double(), k.view(T, H, D).double(), v.view(T, H, V).double()
+    keep, o = 1 / (1 + torch.exp(z.double().view(T, H, D, 1))), []
+    for t in range(T):
+        if bonus is not None:
+            o.append(torch.einsum("hd,hdv->hv", qq[t], S + (bonus.double() * kk[t])[..., None] * vv[t][:, None]))
+        S = S * keep[t] + kk[t][..., None] * vv[t][:, None]
+        if bonus is None:
+            o.append(torch.einsum("hd,hdv->hv", qq[t], S))
+    # running sums of 131 in fp32 are off by 2^-17 (relative, in the power), the power itself keeps 18 bits below the normal range, and
+    # both factors of a product 16 or more
+    assert float(((state.S[0].double() - S).abs() / S).max()) < 2.0 ** -12
+    if kind != "delta":
+        o = torch.stack(o)[41:]                            # behind the second drop
+        o = o / torch.sqrt((o * o).mean(-1, keepdim=True) + 1e-30)
+        g = gate.view(T, H, V).double()[41:]
+        o = o * torch.sigmoid(g) * g
+        assert float(((out.view(T, H, V)[41:].double() - o).abs() / o).max()) < 2.0 ** -7
+
+
 @pytest.mark.parametrize("delta", [False, True])
 def test_value_tiles_agree(delta):
     """20 heads take value tiles of 32 columns (one wave of CTAs), 10 heads those of 16: the same sums in the same order."""
