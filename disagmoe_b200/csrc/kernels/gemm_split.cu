@@ -165,10 +165,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
   pdl_trigger();      // behind the allocation: a CTA of the next launch never holds TMEM that this one still needs
   // partial rows may be sent to a CTA that runs (or, over the stages, to one whose MMAs are done)
   if (cluster && !a.alias) cluster_arrive_relaxed();
+  // all warps: the time limits below count from here, and the launch before may wait for a peer longer than they allow
+  pdl_wait();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    pdl_wait();
     const uint64_t pol_w = gridDim.z == 1 ? l2_policy_evict_first() : l2_policy_evict_last(), pol_x = l2_policy_evict_last();
     int stage = 0;
     uint32_t phase = 0;
@@ -246,7 +247,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     }
     __syncwarp();
   }
-  pdl_wait();      // everything below reads and writes what other launches may
   if (cluster && own > 0) mbar_wait(rfull, 0, &abort_word);
   __syncwarp();
   if (cluster) cluster_arrive_relaxed();      // all that this CTA waits for has come

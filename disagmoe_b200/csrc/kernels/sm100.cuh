@@ -370,9 +370,10 @@ struct PerDeviceOnce {
 // ---------------------------------------------------------------- programmatic dependent launch
 // With DMOE_PDL=1 the per-layer kernels are launched with the programmatic-stream-serialization attribute: a kernel
 // may become resident (and run the part of its prologue that touches no global data) while its predecessor in the
-// stream is still draining. Every such kernel calls pdl_trigger() first (its own successor may start early too) and
-// pdl_wait() before it reads anything a predecessor wrote; pdl_wait() returns once the predecessor grid has completed
-// and its writes are visible. Without the attribute both are no-ops.
+// stream is still draining. Every such kernel calls pdl_trigger() (its own successor may start early too) first, or behind its
+// allocation where it allocates tensor memory without waiting for its predecessor, and pdl_wait() with all warps before it reads
+// anything a predecessor wrote and before its first bounded wait, whose limit would count the predecessor's time as well; pdl_wait()
+// returns once the predecessor grid has completed and its writes are visible. Without the attribute both are no-ops.
 inline bool pdl_enabled() {
   static const bool v = [] {
     const char* e = getenv("DMOE_PDL");

@@ -86,3 +86,33 @@ def test_launch_that_does_not_qualify():
     """Rows that do not move 16 bytes at a time keep the kernel that stores them one by one."""
     x, w = _bf(9, 128), _bf(20, 128)
     _close(gemm.linear(x, w, bn=16, cluster=2, out_dtype=torch.float32), x.double() @ w.double().T, 128 * 128, bits=20)
+
+
+LATE = """
+import torch
+from disagmoe_b200.ops import _lib, functional as F, gemm
+bf = lambda *s: torch.randn(*s, device="cuda").to(torch.bfloat16)
+z = lambda n: torch.zeros(n, dtype=torch.int32, device="cuda")
+x, w, resid, dst, status = bf(37, 512), bf(1024, 512), bf(4, 256), bf(4, 256), z(1)
+ptr, flags, epoch, ticket = torch.tensor([dst.data_ptr()], device="cuda"), z(1), z(1), z(1)
+want = [gemm.linear(x, w, bn=48, cluster=c) for c in (1, 4)]
+_lib.lib().dmoe_set_flag_wait_cycles(2_300_000_000)
+for c, y in zip((1, 4), want):
+    status.zero_()
+    torch.cuda.synchronize()
+    F.norm_gather(resid, None, bf(256), 1e-6, None, ptr, 1, 0, 256, 4, 256, wait_flags=flags, n_wait=1, wait_epoch=epoch, ticket=ticket, status=status)
+    got = gemm.linear(x, w, bn=48, cluster=c)
+    assert int(status) == 2 and gemm.check_status() == 0 and torch.equal(got, y), (c, int(status))
+"""
+
+
+def test_limits_count_from_the_end_of_the_launch_before():
+    """Started while its predecessor still waits for a peer (here for a flag that nothing sets, until its own limit of 1.2 s), the kernel
+    does not count that time against its barriers' limits of a second."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    out = subprocess.run([sys.executable, "-c", LATE], env={**os.environ, "DMOE_PDL": "1", "PYTHONPATH": root}, capture_output=True, text=True,
+                         timeout=300)
+    assert out.returncode == 0, out.stderr[-2000:]
