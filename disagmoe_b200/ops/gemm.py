@@ -155,28 +155,27 @@ def want_streamk(epi: int, F: int, G: int, T: int, bn: int, sms: int) -> bool:
 
 @lru_cache(maxsize=4096)
 def want_wide(epi: int, T: int, F: int, K: int, G: int, sms: int) -> bool:
-    """Should the tokens be the M operand (csrc/kernels/gemm_wide.cu, 256 x 256 tiles on CTA pairs) instead of the weights?
+    """Should the tokens be the M operand (csrc/kernels/gemm_wide.cu, CTA pairs) instead of the weights (csrc/kernels/gemm.cu)?
 
-    Dense: a cost model of both, in us, fitted to a sweep on B200 (K 1024 .. 5632, F 256 .. 32000, T 8 .. 2048; the choice is within
-    8 % of the better of these two kernels, K below 1024 within 15 %). A wide tile takes 0.31 us per K block whatever part of it is
-    used, the other kernel what its SM pulls from L2. Measured (bf16, other kernel -> wide tiles of 256 rows; :func:`dense_wide` then takes
-    narrower ones, :func:`split_plan` a third kernel): 4096 x 6144 x 4096 201 -> 149 us (1381
-    TFLOP/s), 2500 x 4096 x 2048 106 -> 40, 1111 x 6144 x 2048 79 -> 31, 256 x 32000 x 4096 89 -> 58; SwiGLU 1024 x 5632 x 2048 59 ->
-    42. A few rows of SwiGLU gain by the wider tile's faster K blocks (1 row, 2048 x 4096 38 -> 32, 16 rows, 8192 x 7168 82 -> 65),
-    but pay 2 us more per launch (1 row, 2048 x 256 11.2 -> 12.6, 4096 x 1024 17.4 -> 17.4), and more where the tiles of a wave want
-    more than HBM gives (1 row, 8192 x 1024 17.4 -> 19.3, 8192 x 7168 69 -> 78; 8 rows, 8192 x 4096 47 -> 49).
+    Dense: for launches that fit no :func:`split_plan` (:func:`_dense_plan`; one group of a grouped product counts as well). A cost model of
+    both, in us, of an earlier state of the two kernels: tiles of 256 weight rows, 0.31 us per K block of 64 whatever part of a tile is
+    used, against what an SM of the other kernel pulls from L2; the pair kernel has become the faster of them since (4096 x 6144 x 4096
+    then 201 against 149 us, now 228 against 140), so that the line is on the safe side for it. A few rows of SwiGLU gain by the wider
+    tile's faster K blocks (1 row, 2048 x 4096 38 -> 32, 16 rows, 8192 x 7168 82 -> 65), but pay 2 us more per launch (1 row, 2048 x 256
+    11.2 -> 12.6, 4096 x 1024 17.4 -> 17.4), and more where the tiles of a wave want more than HBM gives (1 row, 8192 x 1024 17.4 -> 19.3,
+    8192 x 7168 69 -> 78; 8 rows, 8192 x 4096 47 -> 49).
 
     Grouped (only the mean group size is known): up to 128 tokens both kernels read the weights once; the wide one has a half product for
-    such groups and no transposing epilogue, the other one smaller units, which counts where few experts have long rows of tiles. Sweep
-    over 20 shapes at 40 .. 128 tokens per expert (other kernel / wide): SwiGLU with F K to 6 million 0.99 .. 1.57 (64 x 1408 x 2048, 104
-    tokens 133 -> 126 us; 16 x 2816 x 2048, 96 tokens 69 -> 64), above that 0.93 .. 1.1 (8 x 14336 x 4096: 40 tokens 290 -> 309, 128: 354 ->
-    339); down-projections to K 5632 1.00 .. 1.70 (16 x (2048 x 2816), 96 tokens 46 -> 37), 8 x (4096 x 14336): 64 tokens 155 -> 157, 96: 183 ->
-    159. Beyond 128 tokens the other kernel needs a second tile per group (8 x 14336 x 4096, SwiGLU, 160: 533 -> 369). Down-projections with
-    short K loops are bound by the other kernel's transposing epilogue at any size. Sweep over 8 .. 64 experts, F 2048 .. 6144, K 512
-    .. 7168, 2 rows in all .. 140 per expert: with F K to 4.4 million 0.92 .. 1.9 times as fast, 1.17 on average (60 x (2048 x 1408):
-    16 rows 46 -> 34, 148 rows 81 -> 70; 8 x (4096 x 1024): 74 rows 28 -> 25); above that a badly filled wave of long tiles can make it
-    0.8 times as fast with few experts (16 x (6144 x 2048): 24 rows 74 -> 88), while 60 and 64 experts still gain to K 2048 (0.96 ..
-    1.5; 60 x (4096 x 2048): 64 rows 136 -> 131); from K 2816 on nothing is gained (8 x (4096 x 14336): 2 rows 47 -> 77, 128 rows 149 -> 181)."""
+    such groups and no transposing epilogue, the other one smaller units, which counts where few experts have long rows of tiles. From 40
+    tokens per expert on, sweep over 20 shapes at 40 .. 128 (other kernel -> wide, us): SwiGLU with F K to 6 million 0.99 .. 1.57 times as
+    fast (64 x 1408 x 2048, 104 tokens 133 -> 126; 16 x 2816 x 2048, 96 tokens 69 -> 64), above that 0.93 .. 1.1 (8 x 14336 x 4096: 40 tokens
+    290 -> 309, 128: 354 -> 339); down-projections to K 5632 1.00 .. 1.70 (16 x (2048 x 2816), 96 tokens 46 -> 37), 8 x (4096 x 14336): 64
+    tokens 155 -> 157, 96: 183 -> 159. Beyond 128 tokens the other kernel needs a second tile per group (8 x 14336 x 4096, SwiGLU, 160: 533 ->
+    369). Below 40 tokens short K loops are bound by the other kernel's transposing epilogue: sweep over 8 .. 64 experts, F 2048 .. 6144, K
+    512 .. 7168, before the half products and both kernels' present issue loops: with F K to 4.4 million 0.92 .. 1.9 times as fast, 1.17 on
+    average (60 x (2048 x 1408): 16 rows 46 -> 34; 8 x (4096 x 1024): 74 rows 28 -> 25); above that a badly filled wave of long tiles can
+    make it 0.8 times as fast with few experts (16 x (6144 x 2048): 24 rows 74 -> 88), while 60 and 64 experts still gain to K 2048; from K
+    2816 on nothing was gained there (8 x (4096 x 14336): 2 rows 47 -> 77)."""
     kblocks, pairs = (K + 63) // 64, max(1, sms // 2)
     if G > 1:
         if epi == EPI_SWIGLU:
@@ -279,14 +278,20 @@ def _split_plan(T: int, F: int, K: int, epi: int, sms: int):
 @lru_cache(maxsize=4096)
 def _dense_plan(T: int, F: int, K: int, epi: int, sms: int, hd: int = 0):
     """(weight rows per tile of gemm_wide.cu or 0, split plan or None) of a dense launch on one GPU that leaves the choice of kernel to
-    this module; ``hd``: see :func:`dense_wide`."""
-    wide, plan = want_wide(epi, T, F, K, 1, sms), split_plan(T, F, K, epi, sms)
-    if not wide:
+    this module; ``hd``: see :func:`dense_wide`.
+
+    Up to 128 tokens the split kernel where it has a plan: the pair kernel would work half its rows for nothing, and its model leaves out
+    that all of the weights come from HBM. Beyond, the cheaper of both models. Sweep of 267 sizes with a plan on B200 (T 2 .. 4096, F 256 ..
+    14336, K 256 .. 14336): the choice is 0.5 % slower than the best tile of either kernel on average, 17 % at most. Split -> pairs, us: 512 x
+    4096 x 14336 61 -> 52, 1000 x 2048 x 14336 58 -> 49, 512 x 4096 x 11008 49 -> 40, 200 x 12288 x 4096 35 -> 27, SwiGLU 230 x 4344 x 5768 50 ->
+    40; the other way 200 x 2048 x 14336 21 and 44, 300 x 2048 x 14336 29 and 44."""
+    plan = split_plan(T, F, K, epi, sms)
+    if plan is not None and T <= 128:
         return 0, plan
+    if plan is None and not want_wide(epi, T, F, K, 1, sms):
+        return 0, None
     cost, cols = dense_wide(T, F, K, epi, sms, hd)
-    # up to 256 tokens every weight is read once, from HBM, which the model of the pair kernel leaves out (256 x 6144 x 4096: 23 us there,
-    # 20 us in the other)
-    return (0, plan) if plan is not None and (T <= 256 or plan[0] < cost) else (cols, None)
+    return (0, plan) if plan is not None and plan[0] < cost else (cols, None)
 
 
 def _wide_rows(F: int, out: Optional[torch.Tensor], residual: Optional[torch.Tensor], comm: "Optional[GemmComm]") -> bool:

@@ -31,6 +31,25 @@ def test_measured_choices_per_expert(epi, per, F, K, G, wide):
     assert gemm.want_wide(epi, per * G, F, K, G, SMS) is wide
 
 
+@pytest.mark.parametrize("epi,T,F,K,pairs", [
+    (gemm.EPI_PLAIN, 512, 4096, 14336, True), (gemm.EPI_PLAIN, 1000, 2048, 14336, True), (gemm.EPI_PLAIN, 512, 4096, 11008, True),
+    (gemm.EPI_PLAIN, 200, 12288, 4096, True), (gemm.EPI_SWIGLU, 230, 4344, 5768, True), (gemm.EPI_PLAIN, 660, 3064, 11816, True),
+    (gemm.EPI_PLAIN, 200, 2048, 14336, False), (gemm.EPI_PLAIN, 300, 2048, 14336, False), (gemm.EPI_PLAIN, 128, 4096, 14336, False),
+    (gemm.EPI_PLAIN, 256, 4096, 4096, False), (gemm.EPI_PLAIN, 4096, 6144, 4096, True), (gemm.EPI_PLAIN, 96, 102400, 2048, False),
+])
+def test_dense_products_take_the_faster_of_both_kernels(epi, T, F, K, pairs):
+    """Sizes that were measured in both: a plan of the split kernel is no reason to leave the pairs' cost out."""
+    cols, plan = gemm._dense_plan(T, F, K, epi, SMS)
+    assert (cols > 0) is pairs and (plan is None) is pairs
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+def test_pair_tiles_hold_whole_heads(hd):
+    for T in (200, 512, 700, 1111, 4096):
+        cols, plan = gemm._dense_plan(T, 48 * hd, 14336, gemm.EPI_PLAIN, SMS, hd)
+        assert cols % hd == 0 and (cols > 0 or plan is not None)
+
+
 @pytest.mark.parametrize("G", [1, 2, 8, 64])
 def test_stream_k_of_no_expected_rows(G):
     """An expert rank whose share of the arriving rows rounds to none still asks for a rule: 32 tiles leave most SMs idle."""
