@@ -250,6 +250,7 @@ class AttentionRank:
         self.status = gemm.scratch(dev).status
         self.active = [B] * S.n_mb      # rows of every micro-batch that the next launches process (<= B)
         self.n_pre = [0] * S.n_mb       # prompt tiles of every micro-batch for the tiled causal attention kernel
+        self.reach = [0] * S.n_mb       # and the keys that the longest of their prompts looks at
 
     def set_active(self, m: int, T: int) -> None:
         """The next launches of micro-batch m process its first T rows (1 <= T <= batch): a serving step fills the
@@ -269,9 +270,10 @@ class AttentionRank:
         tiles, covered = F.build_prefill_tiles(bt_row, positions, F.prefill_tile_tokens(a0.num_heads, a0.num_kv_heads))
         self.n_pre[m] = len(tiles)
         if len(tiles):
-            d = self.mb[m]
+            d, ctx = self.mb[m], torch.as_tensor(ctx_len)
+            self.reach[m] = int(ctx[covered].max())
             d["pre_tiles"][:len(tiles)].copy_(tiles, non_blocking=True)
-            cd = torch.as_tensor(ctx_len).clone()
+            cd = ctx.clone()
             cd[covered] = 0
             d["ctx_dec"][:len(cd)].copy_(cd, non_blocking=True)
         return len(tiles)
@@ -357,7 +359,7 @@ class AttentionRank:
                               splits=F.pick_attn_splits(T, a.num_kv_heads, cfg.max_seq_len, self.block_size))
             if n_pre:
                 F.prefill_attention(qkv[:, :a.q_size], kc, vc, meta.block_tables, d["pre_tiles"], n_pre, a.num_heads,
-                                    a.num_kv_heads, a.head_dim, attn)
+                                    a.num_kv_heads, a.head_dim, attn, reach=self.reach[m])
         if "o_proj" not in parts:
             return
         _lib.TAG = "o_proj"
