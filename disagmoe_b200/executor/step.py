@@ -13,6 +13,8 @@ from ..config import CacheConfig, ModelConfig
 from ..ops import _lib
 from ..utils.utils import get_graph_batch_size, graph_batch_sizes
 
+TABLE_INTS = 1 << 14       # least room for the host tables of a prompt step
+
 
 class TokenBuffers:
     """Static inputs and outputs for up to ``cap`` tokens (CUDA graphs replay on fixed addresses)."""
@@ -48,7 +50,7 @@ class StepExecutor:
         self.graphs: Dict[int, torch.cuda.CUDAGraph] = {}
         self.graph_sizes: List[int] = []
         self.graph_launches: Dict[int, int] = {}
-        self.table_ints = 1 << 14             # room for the host tables of a prompt step; grows with them
+        self.table_ints = TABLE_INTS          # room for the host tables of a prompt step
 
     # ---- supplied by a model family -----------------------------------------------------------------------------
     def _load(self, state_dict) -> None:
@@ -116,7 +118,8 @@ class StepExecutor:
         if out_rows is not None:
             buf.out_rows = up(np.array(out_rows, dtype=np.int32))
         up.flush()
-        self.table_ints = max(self.table_ints, up.ints)
+        # the next step of this size goes up in one copy; after a long one the room halves from step to step
+        self.table_ints = max(TABLE_INTS, up.total, self.table_ints // 2)
         try:
             return self._forward(buf, T, int(ctx_len.max()), want_logits)
         finally:

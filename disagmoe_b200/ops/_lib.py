@@ -145,12 +145,13 @@ class Uploads:
     """The host tables of one step on the device by one copy instead of one per table (a copy and its pinned buffer cost 20 us of host
     time, and a copy from pageable memory would wait for everything that is queued): a call takes an int32 array and returns the
     device tensor that :meth:`flush` fills, in stream order. The staging memory is allocated per step; torch keeps it until the
-    copy that reads it is done. On the CPU the arrays themselves."""
+    copy that reads it is done. ``total``: the room (in ints) with which the tables so far would have gone up in one copy. On the CPU the
+    arrays themselves."""
 
     def __init__(self, device, ints: int = 1 << 14):
         self.device = torch.device(device) if isinstance(device, str) else device
         self.cuda = self.device.type == "cuda" and torch.cuda.is_available()
-        self.ints, self.at, self.host = ints, 0, None
+        self.ints, self.at, self.host, self.total = ints, 0, None, 0
 
     def __call__(self, a: np.ndarray) -> torch.Tensor:
         assert a.dtype == np.int32
@@ -165,6 +166,7 @@ class Uploads:
         at = self.at
         self.view[at:at + n] = a.reshape(-1)
         self.at = at + (n + 3 & ~3)               # tables start on 16-byte boundaries
+        self.total += self.at - at
         t = self.dev[at:at + n]
         return t if a.ndim == 1 else t.view(a.shape)
 
