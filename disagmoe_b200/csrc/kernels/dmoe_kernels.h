@@ -178,6 +178,8 @@ typedef struct DmoeGemm {
 
 int dmoe_gemm(const DmoeGemm* desc, void* stream);
 int dmoe_gemm_pick_bn(int tokens_per_group_hint, int epi);
+// CTAs of gemm_split.cu that the current device holds at once in clusters of 1 .. 8 CTAs, one per SM (large) or two; 0: unknown
+int dmoe_gemm_split_ctas(int splits, int large);
 long long dmoe_gemm_workspace_bytes(int T, int F, int bn, int splitk);
 
 // ---- row kernels (elementwise.cu) -------------------------------------------------------------------

@@ -27,6 +27,7 @@ namespace dmoe {
 constexpr int kSThreads = 192;
 constexpr int kSSmallSmem = 112 * 1024 + 512;            // two CTAs per SM
 constexpr int kSLargeSmem = 226 * 1024;
+constexpr int kSStaticSmem = 256;                        // barriers and the like, at most
 constexpr int kSWBytes = kBM * kBK * 2;                  // weights of one K block
 constexpr int kSSub = 2;                                 // K blocks per stage (one where two stages of two do not fit)
 constexpr int kSMaxStages = 6;
@@ -327,31 +328,38 @@ static int configure_split() {
   });
 }
 
-// CTAs in clusters of `splits` that are on the chip at once with the large amount of shared memory (asked for once per device)
-static int large_capacity(int splits) {
-  static std::atomic<int> cache[kMaxDevicesPerProcess][9];
+// What the driver is asked about in place of gemm_split_kernel: of a kernel that allocates tensor memory it counts one CTA per SM
+// whatever it needs, where two do share an SM (tiles of 16 tokens, K 512, in L2: 148 CTAs 5.3 us, 149 5.9, 296 6.9, 297 9.2).
+__global__ void __launch_bounds__(kSThreads) split_room_kernel() {}
+
+// CTAs in clusters of `splits` that are on the chip at once with the large or the small amount of shared memory (asked for once per
+// device: clusters stay inside a group of SMs, whose sizes differ from chip to chip); 0 where the driver does not say
+static int split_capacity(int splits, bool large) {
+  static std::atomic<int> cache[kMaxDevicesPerProcess][2][9];
   int dev = 0;
-  if (splits < 2) return device_num_sms();
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevicesPerProcess) return 0;
-  int n = cache[dev][splits].load(std::memory_order_relaxed);
-  if (n == 0) {
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3(splits, 1, 1);
-    cfg.blockDim = dim3(kSThreads, 1, 1);
-    cfg.dynamicSmemBytes = kSLargeSmem;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = splits;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int clusters = 0;
-    if (configure_split<EPI_PLAIN>() != 0 || cudaOccupancyMaxActiveClusters(&clusters, gemm_split_kernel<EPI_PLAIN>, &cfg) != cudaSuccess) return 0;
-    n = clusters > 0 ? clusters * splits : -1;
-    cache[dev][splits].store(n, std::memory_order_relaxed);
+  if (splits < 1 || splits > 8 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevicesPerProcess) return 0;
+  int n = cache[dev][large][splits].load(std::memory_order_relaxed);
+  if (n != 0) return n;
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(splits, 1, 1);
+  cfg.blockDim = dim3(kSThreads, 1, 1);
+  cfg.dynamicSmemBytes = (large ? kSLargeSmem : kSSmallSmem) + kSStaticSmem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = splits;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int clusters = 0;
+  if (cudaFuncSetAttribute(split_room_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(cfg.dynamicSmemBytes)) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&clusters, split_room_kernel, &cfg) != cudaSuccess) {
+    cudaGetLastError();      // not the error of the next launch
+    return 0;
   }
+  n = clusters * splits;
+  cache[dev][large][splits].store(n, std::memory_order_relaxed);
   return n;
 }
 
@@ -395,7 +403,7 @@ int gemm_split(const DmoeGemm* d, cudaStream_t stream) {
   // them too. The large amount of shared memory (one CTA per SM) has more stages in flight, which counts where each is fetched from
   // HBM: 1.1 us per round trip. It is taken where all CTAs find place at once, and where the small one is too small.
   const long long mt = (d->F + feat - 1) / feat, nt = (d->T + bn - 1) / bn;
-  const bool spread = a.per > 2 * kSSub && a.splits * mt * nt <= large_capacity(a.splits);
+  const bool spread = a.per > 2 * kSSub && a.splits * mt * nt <= split_capacity(a.splits, true);
   const int parts = bn * kSRow, recv = (a.splits - 1) * ((bn + a.splits - 1) / a.splits) * kSRow;
   const auto fits = [&](int room, int sub) {
     const int stage = sub * (kSWBytes + bn * kBK * 2), steps = (a.per + sub - 1) / sub, most = std::min(steps, kSMaxStages), want = std::min(steps, sub == 1 ? 3 : 2);
@@ -434,3 +442,6 @@ int gemm_split(const DmoeGemm* d, cudaStream_t stream) {
 }
 
 }  // namespace dmoe
+
+// CTAs of the split GEMM that the current device holds at once in clusters of `splits` (1 .. 8), one per SM (`large`) or two; 0: unknown
+extern "C" int dmoe_gemm_split_ctas(int splits, int large) { return dmoe::split_capacity(splits, large != 0); }

@@ -213,13 +213,34 @@ def dense_wide(T: int, F: int, K: int, epi: int, sms: int, hd: int = 0):
     return best
 
 
-# CTAs of csrc/kernels/gemm_split.cu that a B200 holds at once in clusters of 1 .. 8, with the small amount of shared memory (two per
-# SM) and the large one; fewer than two per SM and one, because a cluster stays inside a group of SMs
+# CTAs of csrc/kernels/gemm_split.cu that a B200 held at once in clusters of 1 .. 8, with the small amount of shared memory (two per
+# SM) and the large one; fewer than two per SM and one, because a cluster stays inside a group of SMs. For rules without a device
+# (:func:`split_ctas` asks the one at hand)
 _SPLIT_SMALL = (296, 296, 279, 284, 280, 270, 259, 264)
 _SPLIT_LARGE = (148, 148, 135, 132, 130, 132, 105, 120)
 
 
-def split_plan(T: int, F: int, K: int, epi: int, sms: int):
+_split_ctas_cache = {}
+
+
+def split_ctas(device):
+    """(small, large): the two tables above for a CUDA device, as its driver says (asked for once per device)."""
+    idx = device.index if device.index is not None else torch.cuda.current_device()
+    if idx not in _split_ctas_cache:
+        with torch.cuda.device(idx):
+            tables = [tuple(_lib.lib().dmoe_gemm_split_ctas(n, large) for n in range(1, 9)) for large in (0, 1)]
+        if min(map(min, tables)) <= 0:
+            tables = _scaled_ctas(num_sms(torch.device("cuda", idx)))
+        _split_ctas_cache[idx] = tuple(tables)
+    return _split_ctas_cache[idx]
+
+
+@lru_cache(maxsize=16)
+def _scaled_ctas(sms: int):
+    return tuple(tuple(n * sms // 148 for n in t) for t in (_SPLIT_SMALL, _SPLIT_LARGE))
+
+
+def split_plan(T: int, F: int, K: int, epi: int, sms: int, ctas=None):
     """(cost in us, token tile, CTAs per cluster) of a dense product in csrc/kernels/gemm_split.cu, or None where other kernels are
     faster: all its CTAs have to find place at once, or it has one tile of up to 128 tokens and the weights stream through it (an LM
     head).
@@ -231,16 +252,16 @@ def split_plan(T: int, F: int, K: int, epi: int, sms: int):
     x 32000 x 4096 54.1 -> 42.4, 37 x 151936 x 2048 111 -> 104, 96 x 102400 x 2048 88.5 -> 78.0, 66 x 151936 x 2048 128 -> 110. A second wave costs as much as the first: 200 x 10944 x 2048 SwiGLU (171
     CTAs of one per SM) 23.0 -> 40.6, 1111 x 2816 x 2048 SwiGLU 28.6 -> 36.4, 192 x 32000 x 2048 32.5 -> 42.5.
 
-    Sizes are rounded up to a grid of tokens, so that few plans serve prompts of all lengths."""
+    ``ctas``: :func:`split_ctas`. Sizes are rounded up to a grid of tokens, so that few plans serve prompts of all lengths."""
     grid = 16 if T <= 256 else 32 if T <= 1024 else 64
-    return _split_plan(-(-T // grid) * grid, F, K, epi, sms)
+    return _split_plan(-(-T // grid) * grid, F, K, epi, sms, ctas or _scaled_ctas(sms))
 
 
 @lru_cache(maxsize=4096)
-def _split_plan(T: int, F: int, K: int, epi: int, sms: int):
+def _split_plan(T: int, F: int, K: int, epi: int, sms: int, ctas):
     gate = epi == EPI_SWIGLU
     mt, kblocks = -(-F // (64 if gate else 128)), -(-K // 64)
-    small, large = ([n * sms // 148 for n in t] for t in (_SPLIT_SMALL, _SPLIT_LARGE))
+    small, large = ctas
     stream = F * K * (4 if gate else 2) / 6.6e6
     best = None
     if mt > small[0]:
@@ -276,7 +297,7 @@ def _split_plan(T: int, F: int, K: int, epi: int, sms: int):
 
 
 @lru_cache(maxsize=4096)
-def _dense_plan(T: int, F: int, K: int, epi: int, sms: int, hd: int = 0):
+def _dense_plan(T: int, F: int, K: int, epi: int, sms: int, hd: int = 0, ctas=None):
     """(weight rows per tile of gemm_wide.cu or 0, split plan or None) of a dense launch on one GPU that leaves the choice of kernel to
     this module; ``hd``: see :func:`dense_wide`.
 
@@ -285,7 +306,7 @@ def _dense_plan(T: int, F: int, K: int, epi: int, sms: int, hd: int = 0):
     14336, K 256 .. 14336): the choice is 0.5 % slower than the best tile of either kernel on average, 17 % at most. Split -> pairs, us: 512 x
     4096 x 14336 61 -> 52, 1000 x 2048 x 14336 58 -> 49, 512 x 4096 x 11008 49 -> 40, 200 x 12288 x 4096 35 -> 27, SwiGLU 230 x 4344 x 5768 50 ->
     40; the other way 200 x 2048 x 14336 21 and 44, 300 x 2048 x 14336 29 and 44."""
-    plan = split_plan(T, F, K, epi, sms)
+    plan = split_plan(T, F, K, epi, sms, ctas)
     if plan is not None and T <= 128:
         return 0, plan
     if plan is None and not want_wide(epi, T, F, K, 1, sms):
@@ -522,7 +543,8 @@ def linear(x: torch.Tensor, w: torch.Tensor, residual: Optional[torch.Tensor] = 
     if wide is None and not cluster:
         wide = False
         if not (bn or splitk or pair) and _wide_rows(F, out, residual, comm):
-            wide, plan = _dense_plan(T, F, K, EPI_PLAIN, sms, comm.rope.hd if comm is not None and comm.rope is not None else 0)
+            wide, plan = _dense_plan(T, F, K, EPI_PLAIN, sms, comm.rope.hd if comm is not None and comm.rope is not None else 0,
+                                     split_ctas(x.device))
             if plan is not None:
                 _, bn, cluster = plan
     if cluster:
@@ -732,7 +754,7 @@ def swiglu_linear(x: torch.Tensor, w13: torch.Tensor, out: Optional[torch.Tensor
     if wide is None and not cluster:
         wide = False
         if not bn:
-            wide, plan = _dense_plan(T, I, K, EPI_SWIGLU, num_sms(x.device))
+            wide, plan = _dense_plan(T, I, K, EPI_SWIGLU, num_sms(x.device), 0, split_ctas(x.device))
             if plan is not None and _wide_rows(I, out, None, None):
                 _, bn, cluster = plan
     if cluster:

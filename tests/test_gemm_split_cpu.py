@@ -42,3 +42,18 @@ def test_refused_where_a_second_wave_would_start():
     assert gemm.split_plan(192, 32000, 2048, gemm.EPI_PLAIN, 148) is None
     assert gemm.split_plan(200, 10944, 2048, gemm.EPI_SWIGLU, 148) is None
     assert gemm.split_plan(1, 151936, 2048, gemm.EPI_PLAIN, 148)[1:] == (16, 1)
+
+
+def test_plans_follow_what_the_device_holds():
+    """On a chip whose groups of SMs hold fewer clusters of 4 and 5 no plan asks for more of them than find place at once."""
+    small, large = (list(t) for t in (gemm._SPLIT_SMALL, gemm._SPLIT_LARGE))
+    for n in (3, 4):
+        small[n], large[n] = small[n] // 2, large[n] // 2
+    changed = 0
+    for T, F, K in ((37, 2048, 5632), (96, 2048, 4096), (128, 1024, 8192), (48, 6144, 4096), (200, 2048, 14336), (16, 4096, 4096)):
+        _, bn, S = gemm.split_plan(T, F, K, gemm.EPI_PLAIN, 148, (tuple(small), tuple(large)))
+        per = -(-(-(-K // 64)) // S)
+        cap = large if bn > 128 or (per > 4 and S * -(-F // 128) * -(-T // bn) <= large[S - 1]) else small
+        assert S * -(-F // 128) * -(-T // bn) <= cap[S - 1]
+        changed += (bn, S) != gemm.split_plan(T, F, K, gemm.EPI_PLAIN, 148)[1:]
+    assert changed > 0

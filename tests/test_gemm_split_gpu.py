@@ -82,6 +82,19 @@ def test_chosen_plan_agrees_with_the_other_kernels(T, N, K, gate):
     assert gemm.check_status() == 0
 
 
+def test_rule_and_kernel_agree_on_what_the_device_holds():
+    """The rule counts waves with the driver's answers; an answer that the driver does not give is no error of a later launch."""
+    small, large = gemm.split_ctas(torch.device("cuda"))
+    sms = gemm.num_sms("cuda")
+    assert small[0] == 2 * sms and large[0] == sms
+    for n in range(1, 9):
+        assert sms // 2 < large[n - 1] <= sms and large[n - 1] % n == 0 and sms < small[n - 1] <= 2 * sms and small[n - 1] % n == 0
+    from disagmoe_b200.ops import _lib
+    assert [_lib.lib().dmoe_gemm_split_ctas(n, 1) for n in (0, 9, -1)] == [0, 0, 0]
+    x, w = _bf(4, 64), _bf(8, 64)
+    _close(gemm.linear(x, w), x.double() @ w.double().T, 64 * 64)
+
+
 def test_launch_that_does_not_qualify():
     """Rows that do not move 16 bytes at a time keep the kernel that stores them one by one."""
     x, w = _bf(9, 128), _bf(20, 128)
