@@ -265,7 +265,7 @@ def _split_plan(T: int, F: int, K: int, epi: int, sms: int, ctas):
     stream = F * K * (4 if gate else 2) / 6.6e6
     best = None
     if mt > small[0]:
-        shapes = [(1, T)] if T <= 128 else []
+        shapes = [(1, T)] if T <= 128 and mt <= 65535 else []      # tiles of weight rows are the grid's second dimension
     elif mt * -(-T // 256) > small[0]:
         shapes = []
     else:

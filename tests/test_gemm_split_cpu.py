@@ -57,3 +57,9 @@ def test_plans_follow_what_the_device_holds():
         assert S * -(-F // 128) * -(-T // bn) <= cap[S - 1]
         changed += (bn, S) != gemm.split_plan(T, F, K, gemm.EPI_PLAIN, 148)[1:]
     assert changed > 0
+
+
+def test_more_weight_rows_than_the_grid_has_tiles_stay_with_the_other_kernel():
+    assert gemm.split_plan(1, 65535 * 128, 8, gemm.EPI_PLAIN, 148) is not None and gemm.split_plan(1, 65535 * 128 + 8, 8, gemm.EPI_PLAIN, 148) is None
+    assert gemm._dense_plan(1, 65535 * 128 + 8, 8, gemm.EPI_PLAIN, 148) == (0, None)
+    assert gemm.split_plan(1, 65535 * 64 + 8, 8, gemm.EPI_SWIGLU, 148) is None
