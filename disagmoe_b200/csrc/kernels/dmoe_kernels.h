@@ -166,13 +166,13 @@ typedef struct DmoeGemm {
   int act_cols;
   int unit_weights;   // combine: the records' weights are left out
   // != 0: the tokens are the M operand (gemm_wide.cu: CTA pairs on tiles of 256 tokens x 256 weight rows, or x `wide` of them where
-  // that is more than 1: a multiple of 32 up to 256, of the head size with rope_table, 256 with w_blocked) where the launch
+  // that is more than 1: a multiple of 32 from 64 to 256, of the head size with rope_table, 256 with w_blocked) where the launch
   // allows it: no multi-GPU hooks, splitk <= 1, no pair, 16-byte aligned output rows; other launches ignore it. bn, streamk,
   // ws and counters are unused then.
   int wide;
-  // > 0: one tile of 128 weight rows x bn tokens (any multiple of 16 up to 256) per cluster of `cluster` CTAs (1 .. 8) that share
-  // K (gemm_split.cu) where the launch qualifies as above, is dense, plain or SwiGLU, and its weights are row-major; otherwise the
-  // launch picks a token tile of its own
+  // > 0: one tile of 128 weight rows x bn tokens (a multiple of 16 up to 256, up to 240 from 5 CTAs on; at most 65535 tiles of either)
+  // per cluster of `cluster` CTAs (more than 8 count as 8) that share K (gemm_split.cu) where the launch qualifies as above, is
+  // dense, plain or SwiGLU, and its weights are row-major; otherwise the launch picks a token tile of its own
   int cluster;
 } DmoeGemm;
 

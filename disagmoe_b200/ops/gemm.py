@@ -240,6 +240,10 @@ def _scaled_ctas(sms: int):
     return tuple(tuple(n * sms // 148 for n in t) for t in (_SPLIT_SMALL, _SPLIT_LARGE))
 
 
+def _split_tile(T: int) -> int:
+    return -(-min(T, 128) // 16) * 16
+
+
 def split_plan(T: int, F: int, K: int, epi: int, sms: int, ctas=None):
     """(cost in us, token tile, CTAs per cluster) of a dense product in csrc/kernels/gemm_split.cu, or None where other kernels are
     faster: all its CTAs have to find place at once, or it has one tile of up to 128 tokens and the weights stream through it (an LM
@@ -507,7 +511,8 @@ def linear(x: torch.Tensor, w: torch.Tensor, residual: Optional[torch.Tensor] = 
            silu_cols: int = 0, wide: Optional[bool] = None, cluster: Optional[int] = None) -> torch.Tensor:
     """y[T, F] = x[T, K] @ w[F, K].T (+ residual[T, F]); ``tanh``: of the product; ``silu_cols``: silu of the first so
     many columns. ``pair``: CTA pairs (tcgen05 cta_group::2) on tiles of 256 weight rows x ``bn`` (128 / 256) tokens, whole tiles.
-    ``cluster``: tiles of 128 weight rows x ``bn`` tokens (any multiple of 16), K cut over so many CTAs (csrc/kernels/gemm_split.cu)."""
+    ``cluster``: tiles of 128 weight rows x ``bn`` tokens (any multiple of 16 up to 256, up to 240 from 5 CTAs on, where partial rows sent
+    and received share the memory; 0: those of the batch, 128 at most), K cut over so many CTAs (csrc/kernels/gemm_split.cu)."""
     T, K = x.shape
     F = w.shape[0]
     if not x.is_cuda:
@@ -548,6 +553,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, residual: Optional[torch.Tensor] = 
             if plan is not None:
                 _, bn, cluster = plan
     if cluster:
+        bn = bn or _split_tile(T)
         _launch(w, x, out, residual, None, None, None, 1, T, F, K, EPI_PLAIN, bn, 1, out.stride(0), out.dtype == torch.float32, comm,
                 act=ACT_TANH if tanh else ACT_SILU if silu_cols else 0, act_cols=silu_cols, cluster=cluster)
         return out
@@ -758,6 +764,7 @@ def swiglu_linear(x: torch.Tensor, w13: torch.Tensor, out: Optional[torch.Tensor
             if plan is not None and _wide_rows(I, out, None, None):
                 _, bn, cluster = plan
     if cluster:
+        bn = bn or _split_tile(T)
         _launch(w13, x, out, None, None, None, None, 1, T, I, K, EPI_SWIGLU, bn, 1, out.stride(0), False, act=ACTS[act], cluster=cluster)
         return out
     bn = bn or pick_bn(T, EPI_SWIGLU)

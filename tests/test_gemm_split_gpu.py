@@ -95,6 +95,16 @@ def test_rule_and_kernel_agree_on_what_the_device_holds():
     _close(gemm.linear(x, w), x.double() @ w.double().T, 64 * 64)
 
 
+@pytest.mark.parametrize("T", [1, 37, 300])
+def test_tile_of_its_own_choice(T):
+    x, w, w13 = _bf(T, 520), _bf(264, 520), _bf(528, 520)
+    bn = min(-(-T // 16) * 16, 128)
+    assert torch.equal(gemm.linear(x, w, cluster=3), gemm.linear(x, w, bn=bn, cluster=3))
+    assert torch.equal(gemm.swiglu_linear(x, w13, cluster=3), gemm.swiglu_linear(x, w13, bn=bn, cluster=3))
+    for S in range(1, 9):                                  # the widest tile that every cluster takes
+        _close(gemm.linear(x, w, bn=256 if S < 5 else 240, cluster=S, out_dtype=torch.float32), x.double() @ w.double().T, 520 * 520, bits=20)
+
+
 def test_launch_that_does_not_qualify():
     """Rows that do not move 16 bytes at a time keep the kernel that stores them one by one."""
     x, w = _bf(9, 128), _bf(20, 128)
