@@ -6,23 +6,33 @@ import pytest
 from disagmoe_b200.ops import gemm
 
 
-def _fits(bn, S, per):
-    """Restates the kernel's shared memory: stages of one or two K blocks, a CTA's partial rows over them, those it receives beside or
-    over, in the amount that lets two CTAs share an SM or in the one that does not."""
+def _layout(bn, S, per, units):
+    """Restates how the kernel lays out its shared memory, in its order of choice: one CTA per SM where all of a launch find place that way
+    and a share is long; else the amount with which two share an SM, stages of two K blocks, or of one up to 128 tokens; else the large
+    amount. Partial rows lie over the stages; those received beside them, or over them too. Returns (large, stages), or None: refused."""
     parts, recv = bn * 512, (S - 1) * -(-bn // S) * 512
-    for room, sub in ((112 * 1024 + 512 - 1024, 2), (112 * 1024 + 512 - 1024, 1), (226 * 1024 - 1024, 2)):
+    small, large = 112 * 1024 + 512 - 1024, 226 * 1024 - 1024
+
+    def fits(room, sub):
         stage, steps = sub * (16384 + bn * 128), -(-per // sub)
         want, beside, over = min(steps, 3 if sub == 1 else 2), min(steps, 6, max(0, room - recv) // stage), min(steps, 6, room // stage)
-        if (beside >= want and beside * stage >= parts) or (over >= want and parts + recv <= room):
-            return True
-    return False
+        if beside >= want and beside * stage >= parts:
+            return beside
+        return over if over >= want and parts + recv <= room else 0
+    spread = per > 4 and units <= gemm._SPLIT_LARGE[S - 1]
+    if not spread:
+        n = fits(small, 2) or (bn <= 128 and fits(small, 1))
+        if n:
+            return False, n
+    n = fits(large, 2)
+    return (True, n) if n else None
 
 
 @pytest.mark.parametrize("epi", [gemm.EPI_PLAIN, gemm.EPI_SWIGLU])
 def test_plans_fit_the_kernel(epi):
     rng = random.Random(epi)
-    found = 0
-    for _ in range(1500):
+    found, clusters = 0, set()
+    for _ in range(3000):
         T, F, K = (int(2 ** rng.uniform(0, hi)) for hi in (12, 17, 14))
         F, K = max(8, F // 8 * 8), max(8, K // 8 * 8)
         plan = gemm.split_plan(T, F, K, epi, 148)
@@ -31,10 +41,23 @@ def test_plans_fit_the_kernel(epi):
         found += 1
         _, bn, S = plan
         kblocks = -(-K // 64)
-        assert 16 <= bn <= 256 and bn % 16 == 0 and 1 <= S <= min(8, kblocks) and _fits(bn, S, -(-kblocks // S))
-        tiles = -(-F // (64 if epi == gemm.EPI_SWIGLU else 128)) * -(-T // bn)
-        assert S * tiles <= 296 or (S == 1 and T <= 128 and bn >= T)      # one wave, or one tile of tokens that weights stream through
-    assert found > 300
+        per = -(-kblocks // S)
+        units = S * -(-F // (64 if epi == gemm.EPI_SWIGLU else 128)) * -(-T // bn)
+        assert 16 <= bn <= 256 and bn % 16 == 0 and 1 <= S <= min(8, kblocks) and -(-kblocks // per) == S
+        layout = _layout(bn, S, per, units)
+        assert layout is not None, (T, F, K, plan)
+        # one wave of what the device holds, or one tile of tokens that weights stream through
+        assert units <= (gemm._SPLIT_LARGE if layout[0] else gemm._SPLIT_SMALL)[S - 1] or (S == 1 and T <= 128 and bn >= T), (T, F, K, plan)
+        clusters.add(S)
+    assert found > 600 and clusters == set(range(1, 9))
+
+
+def test_limits_of_explicit_tiles():
+    """Every tile of up to 240 tokens in every cluster, 256 up to 4 CTAs, whatever the length of a share."""
+    for S in range(1, 9):
+        for bn in range(16, 257, 16):
+            refused = [per for per in range(1, 300) if any(_layout(bn, S, per, u) is None for u in (1, 1000))]
+            assert not refused or (bn == 256 and S >= 5)
 
 
 def test_refused_where_a_second_wave_would_start():

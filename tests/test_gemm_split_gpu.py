@@ -50,6 +50,24 @@ def test_gated(T, I, K, bn, cluster):
     _close(gemm.swiglu_linear(x, w, bn=bn, cluster=cluster), ref, K)
 
 
+@pytest.mark.parametrize("T,N,K,bn,cluster", [(1, 8, 64, 16, 1), (37, 72, 520, 48, 3), (150, 200, 1024, 144, 4)])
+def test_other_epilogues(T, N, K, bn, cluster):
+    torch.manual_seed(T)
+    kw = dict(bn=bn, cluster=cluster)
+    x, w, r, w13 = _bf(T, K), _bf(N, K) * K ** -0.5, _bf(T, N), _bf(2 * N, K) * K ** -0.5
+    h = x.double() @ w.double().T
+    _close(gemm.linear(x, w, tanh=True, **kw), torch.tanh(h), K)
+    # out_tanh is good to 2^-22 (1 - 2 / (e + 1), e to 2^-21): within the absolute part of the bound
+    _close(gemm.linear(x, w, tanh=True, out_dtype=torch.float32, **kw), torch.tanh(h), K, bits=22)
+    _close(gemm.linear(x, w, residual=r, out_dtype=torch.float32, **kw), h + r.double(), K, bits=22)
+    g, u = (x.double() @ w13.double().T).split(N, 1)
+    # the error of the gate's product counts |u| <= 4 times: 16 K under the root
+    _close(gemm.swiglu_linear(x, w13, act="gelu_tanh", **kw), torch.nn.functional.gelu(g, approximate="tanh") * u, 16 * K)
+    out, m = torch.empty(T, N, dtype=torch.bfloat16, device="cuda"), g.clamp(max=0.75)
+    gemm._launch(w13, x, out, None, None, None, None, 1, T, N, K, gemm.EPI_SWIGLU, bn, 1, N, False, act=gemm.ACTS["clamped"], act_limit=0.75, cluster=cluster)
+    _close(out, m * torch.sigmoid(1.702 * m) * (u.clamp(-0.75, 0.75) + 1.0), 16 * K)
+
+
 @pytest.mark.parametrize("hd,n_q,n_kv", [(128, 4, 1), (64, 6, 2)])
 @pytest.mark.parametrize("T,bn,cluster", [(1, 16, 4), (50, 32, 3), (200, 112, 2)])
 def test_rope_append(T, bn, cluster, hd, n_q, n_kv):
@@ -72,10 +90,12 @@ def test_rope_append(T, bn, cluster, hd, n_q, n_kv):
 
 
 @pytest.mark.parametrize("T,N,K,gate", [(1, 4096, 4096, False), (37, 6144, 2048, False), (64, 32000, 512, False), (65, 2816, 1024, True),
-                                        (300, 2048, 1096, False), (1111, 1024, 256, False)])
+                                        (300, 2048, 1096, False), (1111, 1024, 256, False), (37, 2048, 2048, False), (96, 1024, 4096, False),
+                                        (200, 2048, 4096, False), (65, 1408, 2048, True), (150, 704, 4096, True), (20, 256, 11008, False)])
 def test_chosen_plan_agrees_with_the_other_kernels(T, N, K, gate):
     torch.manual_seed(N)
-    assert gemm.split_plan(T, N, K, gemm.EPI_SWIGLU if gate else gemm.EPI_PLAIN, gemm.num_sms("cuda")) is not None
+    assert gemm.split_plan(T, N, K, gemm.EPI_SWIGLU if gate else gemm.EPI_PLAIN, gemm.num_sms("cuda"),
+                           gemm.split_ctas(torch.device("cuda"))) is not None
     x, w = _bf(T, K), _bf(2 * N if gate else N, K) * K ** -0.5
     y, z = (gemm.swiglu_linear(x, w), gemm.swiglu_linear(x, w, wide=False)) if gate else (gemm.linear(x, w), gemm.linear(x, w, wide=False))
     torch.testing.assert_close(y.float(), z.float(), rtol=2 ** -7, atol=2 ** -9)      # two roundings of nearly equal sums

@@ -38,6 +38,27 @@ def test_tile_sizes(T, N, K, cols):
     assert bool((out[T] == 7.0).all()) and bool((out[:, N:] == 7.0).all())
 
 
+@pytest.mark.parametrize("cols", [64, 128, 160, 256])
+@pytest.mark.parametrize("T,N,K", [(1, 8, 64), (150, 200, 520), (300, 328, 1024)])
+def test_other_epilogues(T, N, K, cols):
+    torch.manual_seed(T + cols)
+    x, w, r, w13 = _bf(T, K), _bf(N, K) * K ** -0.5, _bf(T, N), _bf(2 * N, K) * K ** -0.5
+    h = x.double() @ w.double().T
+    # the bound's 2^-8 of the output is more than fp32 outputs need; what they add is the order of their sums
+    _close(gemm.linear(x, w, wide=cols, tanh=True), torch.tanh(h), K)
+    _close(gemm.linear(x, w, wide=cols, tanh=True, out_dtype=torch.float32), torch.tanh(h), K)
+    _close(gemm.linear(x, w, wide=cols, residual=r, out_dtype=torch.float32), h + r.double(), K)
+    silu = h.clone()
+    silu[:, :N // 2] *= torch.sigmoid(silu[:, :N // 2])
+    _close(gemm.linear(x, w, wide=cols, silu_cols=N // 2), silu, K)
+    g, u = (x.double() @ w13.double().T).split(N, 1)
+    # the error of the gate's product counts |u| <= 4 times: 16 K under the root
+    _close(gemm.swiglu_linear(x, w13, wide=cols, act="gelu_tanh"), torch.nn.functional.gelu(g, approximate="tanh") * u, 16 * K)
+    out, m = torch.empty(T, N, dtype=torch.bfloat16, device="cuda"), g.clamp(max=0.75)
+    gemm._launch(w13, x, out, None, None, None, None, 1, T, N, K, gemm.EPI_SWIGLU, 128, 1, N, False, act=gemm.ACTS["clamped"], act_limit=0.75, wide=cols)
+    _close(out, m * torch.sigmoid(1.702 * m) * (u.clamp(-0.75, 0.75) + 1.0), 16 * K)
+
+
 @pytest.mark.parametrize("sizes", [[33, 0, 1, 31, 257, 32, 300], [64, 255, 7]])
 def test_rows_of_the_next_group_stay(sizes):
     """Whole warps of a group go out as boxes of 32 rows; a remainder may not reach into the next group or past the last."""
