@@ -353,7 +353,8 @@ static int split_capacity(int splits, bool large) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   int clusters = 0;
-  if (cudaFuncSetAttribute(split_room_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(cfg.dynamicSmemBytes)) != cudaSuccess ||
+  // always the large amount: another thread may ask about the other one at the same time
+  if (cudaFuncSetAttribute(split_room_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSLargeSmem + kSStaticSmem) != cudaSuccess ||
       cudaOccupancyMaxActiveClusters(&clusters, split_room_kernel, &cfg) != cudaSuccess) {
     cudaGetLastError();      // not the error of the next launch
     return 0;
