@@ -12,8 +12,9 @@
 // CTAs can be made to fit the chip at any number of tokens. For SwiGLU a tile is 64 gate and the matching 64 up rows: they meet
 // again when the partial rows are added up. Up to 128 tokens a CTA takes 112 KB of shared memory, so that two of them share an SM.
 //
-// A stage holds two K blocks (one from 96 tokens on, where two CTAs share an SM): a round of the issuing warp (wait, MMAs, commit) takes about 400 cycles however small the MMAs are.
-// Warp roles as in gemm.cu: warp 0 TMA producer, warp 1 TMEM owner and MMA issuer, warps 2..5 accumulator readers; all six add up.
+// A stage holds two K blocks (one from 96 tokens on, where two CTAs share an SM): a round of the issuing warp (wait, MMAs, commit)
+// takes about 400 cycles however small the MMAs are. Warp roles as in gemm.cu: warp 0 TMA producer, warp 1 TMEM owner and MMA issuer,
+// warps 2..5 accumulator readers; all six add up.
 // ops/gemm.py: split_plan holds the rule that chooses bn, S and this kernel, with both sides measured.
 #include <string.h>
 
@@ -88,9 +89,9 @@ __device__ __forceinline__ uint4 pack_row8(const float (&x)[8]) {
   return pk;
 }
 
-// QKV: features f0 .. f0 + 7 of token t, whose partial sums are `at` floats behind the first. A tile holds whole heads, so the rotation partner of a
-// feature is half a head away in the same partial rows. Sums are rounded to bf16 before the rotation, as the unfused path stores and
-// re-reads them.
+// QKV: features f0 .. f0 + 7 of token t, whose partial sums are `at` floats behind the first. A tile holds whole heads, so the rotation
+// partner of a feature is half a head away in the same partial rows. Sums are rounded to bf16 before the rotation, as the unfused path
+// stores and re-reads them.
 __device__ __forceinline__ void rope_item(const SplitArgs& a, const PartialRows& rows, int at, int f0, long long t) {
   const int half = a.hd >> 1, d0 = f0 % a.hd, head = f0 / a.hd;
   const bool lower = d0 < half, rot = head < a.n_q + a.n_kv;
@@ -140,7 +141,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
   const int kb0 = rank * a.per, nkb = min(a.per, kblocks - kb0), steps = (nkb + a.sub - 1) / a.sub;
   const bool cluster = a.splits > 1;
   float* parts = reinterpret_cast<float*>(smem);                     // [tokens][kBM], over the stages once these are consumed
-  float* recv = reinterpret_cast<float*>(smem + a.recv_off);         // [splits - 1][tpr][kBM]: the others' partial rows of this CTA's tokens
+  float* recv = reinterpret_cast<float*>(smem + a.recv_off);         // [splits - 1][tpr][kBM]: the others' rows of this CTA's tokens
 
   if (threadIdx.x == 0) {
     abort_word = 0;
@@ -243,8 +244,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     if (warp == 0 && lane < a.splits && lane != rank && *const_cast<volatile int*>(&abort_word) == 0) {
       const int rows = min(tpr, ntok - lane * tpr);
       if (rows > 0)
-        bulk_to_cluster(mapa_rank(smem_u32(recv) + (rank < lane ? rank : rank - 1) * tpr * kSRow, lane), smem_u32(parts) + lane * tpr * kSRow,
-                        rows * kSRow, mapa_rank(rfull, lane));
+        bulk_to_cluster(mapa_rank(smem_u32(recv) + (rank < lane ? rank : rank - 1) * tpr * kSRow, lane),
+                        smem_u32(parts) + lane * tpr * kSRow, rows * kSRow, mapa_rank(rfull, lane));
     }
     __syncwarp();
   }
@@ -407,7 +408,8 @@ int gemm_split(const DmoeGemm* d, cudaStream_t stream) {
   const bool spread = a.per > 2 * kSSub && a.splits * mt * nt <= split_capacity(a.splits, true);
   const int parts = bn * kSRow, recv = (a.splits - 1) * ((bn + a.splits - 1) / a.splits) * kSRow;
   const auto fits = [&](int room, int sub) {
-    const int stage = sub * (kSWBytes + bn * kBK * 2), steps = (a.per + sub - 1) / sub, most = std::min(steps, kSMaxStages), want = std::min(steps, sub == 1 ? 3 : 2);
+    const int stage = sub * (kSWBytes + bn * kBK * 2), steps = (a.per + sub - 1) / sub;
+    const int most = std::min(steps, kSMaxStages), want = std::min(steps, sub == 1 ? 3 : 2);
     const int beside = std::min(most, (room - recv) / stage), over = std::min(most, room / stage);
     if (beside >= want && beside * stage >= parts) {
       a.alias = 0; a.stages = beside; a.recv_off = beside * stage;

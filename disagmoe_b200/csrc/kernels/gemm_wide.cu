@@ -14,9 +14,8 @@
 // time and 24 instead of 32 KB per K block: the tokens of a CTA then lie in lanes 0 .. 63 with the accumulator columns of the even
 // CTA's weight rows and in lanes 64 .. 127 with those of the odd one's; for SwiGLU each CTA stages 64 gate and the matching 64 up rows.
 // Full product -> this (with the turn of WideTurn), us: 64 experts of 1408 x 2048, SwiGLU, 104 rows each 150 -> 126, 281: 264 -> 236,
-// their down-projections 77 -> 66 and 137 -> 125; 8 experts of 14336 x 4096, 281 rows 626 -> 562 and 346 -> 318; whole prompt steps:
-// Supinex 3000 tokens 2615 -> 2391, DeepSeek-V2-Lite 1111 1167 -> 1138, Qwen-MoE 64 + 512 1476 -> 1436. Results equal bit for bit. Tiles of
-// 256 weight rows only: dense launches of narrower ones have too few tails to shorten a wave.
+// their down-projections 77 -> 66 and 137 -> 125; 8 experts of 14336 x 4096, 281 rows 626 -> 562 and 346 -> 318. Results equal
+// bit for bit. Tiles of 256 weight rows only: dense launches of narrower ones have too few tails to shorten a wave.
 //
 // Warp roles (192 threads per CTA): warp 0 TMA producer (its own CTA's operands), warp 1 TMEM owner and, in the even CTA,
 // MMA issuer for both, warps 2..5 epilogue of the CTA's 128 accumulator lanes. Two accumulators of 256 columns fill TMEM:
@@ -224,7 +223,8 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         const uint32_t fb = full0 + 8 * stage, st = smem_u32(smem) + stage * stage_bytes;
         const int kb = i * kWSub, n = min(kWSub, kblocks - kb);
         if (elect_one()) {
-          if (leader) mbar_expect_tx(smem_u32(&full_bar[stage]), n * ((both ? 2 : 1) * kWOperandBytes + 2 * w_bytes));      // a tail: two halves
+          // a tail has two halves of one operand's token rows
+          if (leader) mbar_expect_tx(smem_u32(&full_bar[stage]), n * ((both ? 2 : 1) * kWOperandBytes + 2 * w_bytes));
 #pragma unroll
           for (int j = 0; j < kWSub; ++j) {
             if (j < n) {
@@ -303,9 +303,8 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const uint4 v = pack8(o + 8 * i);
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(base + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4)), "r"(v.x), "r"(v.y),
-                     "r"(v.z), "r"(v.w)
-                     : "memory");
+        const uint32_t at = base + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4);
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
       }
       fence_proxy_async_smem();
       __syncwarp();
@@ -361,7 +360,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         }
       } else if (EPI == EPI_PLAIN && a.rope_table != nullptr) {
         // QKV: rotation partners are hd / 2 columns apart in the same lane. The accumulator is rounded to bf16 before the
-        // rotation, as the unfused path stores and re-reads it. Whole heads: 256 columns hold 2 or 4 of them.
+        // rotation, as the unfused path stores and re-reads it. A tile holds whole heads (gemm_wide checks its columns).
         const int half = a.hd >> 1, hc = half >> 5;              // 32-column chunks per half head
         const int heads = min(a.cols, a.F - f0) / a.hd;
         int pos = ok_row ? __ldg(a.positions + t) : 0;
@@ -498,8 +497,8 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
 }
 
 template <int EPI>
-static int launch_wide(const CUtensorMap& tmW, const CUtensorMap& tmX, const CUtensorMap& tmY, const CUtensorMap& tmW64, const CUtensorMap& tmX64,
-                       const WideArgs& a, int smem, int max_tiles, cudaStream_t stream) {
+static int launch_wide(const CUtensorMap& tmW, const CUtensorMap& tmX, const CUtensorMap& tmY, const CUtensorMap& tmW64,
+                       const CUtensorMap& tmX64, const WideArgs& a, int smem, int max_tiles, cudaStream_t stream) {
   static PerDeviceOnce configured;
   const int crc = configured.run([] {
     return static_cast<int>(cudaFuncSetAttribute(gemm_wide_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWSmemMax));
@@ -539,7 +538,9 @@ int gemm_wide(const DmoeGemm* d, cudaStream_t stream) {
   WideArgs a;
   memset(&a, 0, sizeof(a));
   a.cols = d->wide > 1 ? d->wide : kWCols;
-  if (a.cols < 64 || a.cols > kWCols || a.cols % 32 != 0 || (d->w_blocked && a.cols != kWCols) || (d->rope_table != nullptr && a.cols % d->hd != 0)) return -11;
+  if (a.cols < 64 || a.cols > kWCols || a.cols % 32 != 0 || (d->w_blocked && a.cols != kWCols) ||
+      (d->rope_table != nullptr && a.cols % d->hd != 0))
+    return -11;
   const int stage_bytes = kWSub * (kWOperandBytes + a.cols / 2 * kBK * 2);
   a.stages = kWMaxStages;
   while (wide_smem(a.stages, stage_bytes, d->G) > kWSmemMax) --a.stages;
@@ -573,7 +574,8 @@ int gemm_wide(const DmoeGemm* d, cudaStream_t stream) {
   a.tails = a.cols == kWCols && d->rope_table == nullptr;
   if (a.tails && make_map_2d(&tmX64, d->X, d->T, d->K, ldx, 64) != 0) return -21;
   if (a.tails && d->epi == EPI_SWIGLU) {
-    if ((a.w_blocked ? make_map_2d(&tmW64, d->W, rows * (d->K / kBK), kBK, kBK, 64) : make_map_2d(&tmW64, d->W, rows, d->K, d->K, 64)) != 0) return -20;
+    if ((a.w_blocked ? make_map_2d(&tmW64, d->W, rows * (d->K / kBK), kBK, kBK, 64) : make_map_2d(&tmW64, d->W, rows, d->K, d->K, 64)) != 0)
+      return -20;
   }
   a.put = d->epi != EPI_COMBINE && !d->y_f32 && d->rope_table == nullptr && d->Y != nullptr;
   if (a.put && make_put_map(&tmY, d->Y, d->T, d->F, d->ldy) != 0) return -22;

@@ -110,7 +110,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t t_s = __shfl_sync(0xffffffffu, *tmem_slot, 0), t_o = t_s + 2 * kFaSub;      // scores / weights [2 x 64 columns], output [128 columns]
+  // scores / weights [2 x 64 columns], output [128 columns]
+  const uint32_t t_s = __shfl_sync(0xffffffffu, *tmem_slot, 0), t_o = t_s + 2 * kFaSub;
 
   if (warp == 0) {
     // ------------------------------------------------------------ loads
@@ -394,9 +395,10 @@ extern "C" int dmoe_prefill_attention_tc(const void* q, long long ld_q, const vo
                                          const float* sink, void* out, long long ld_out, const DmoeAttnExtra* extra, int exact,
                                          int* status, void* stream_) {
   if (n_tiles == 0) return 0;
-  if (n_kv < 1 || n_q % n_kv != 0 || n_q / n_kv > kFaRows || n_tiles < 0 || static_cast<long long>(n_tiles) * n_kv > 0x7fffffff || tiles == nullptr || n_blocks < 1 ||
-      block_size < 8 || kFaKeys % block_size != 0 || (exact && (window > 0 || chunk > 0 || softcap > 0.f || sink != nullptr || extra != nullptr)))
+  if (n_kv < 1 || n_q % n_kv != 0 || n_q / n_kv > kFaRows || n_tiles < 0 || static_cast<long long>(n_tiles) * n_kv > 0x7fffffff ||
+      tiles == nullptr || n_blocks < 1 || block_size < 8 || kFaKeys % block_size != 0)
     return -10;
+  if (exact && (window > 0 || chunk > 0 || softcap > 0.f || sink != nullptr || extra != nullptr)) return -10;
   CUtensorMap tmK, tmV;
   const long long slots = static_cast<long long>(n_blocks) * block_size;
   int rc = page_map(&tmK, kcache, slots, n_kv, block_size);
@@ -405,7 +407,8 @@ extern "C" int dmoe_prefill_attention_tc(const void* q, long long ld_q, const vo
   const AttnExt ext = make_ext(scale, window, chunk, softcap, sink, n_q / n_kv, extra);
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   const auto launch = exact ? launch_tc<FA_PAGED, true> : launch_tc<FA_PAGED, false>;
-  return launch(tmK, tmV, q, ld_q, block_tables, max_blocks, tiles, n_tiles, block_size, n_kv, scale, out, ld_out, ext, nullptr, 0, status, stream);
+  return launch(tmK, tmV, q, ld_q, block_tables, max_blocks, tiles, n_tiles, block_size, n_kv, scale, out, ld_out, ext, nullptr, 0, status,
+                stream);
 }
 
 extern "C" int dmoe_latent_prefill_tc(const void* q, long long ld_q, const void* kv, long long ld_kv, const void* lat, long long ld_lat,

@@ -537,10 +537,11 @@ def prefill_attention(q: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tenso
         hd != vd or n_q // n_kv not in (1, 2, 4, 8)
     x = _attn_extra(q_temp, gate, q.dtype)
     # A CTA of the tcgen05 kernel needs 7 us before its first result and 1 us per 64 keys then, one of the mma.sync kernel 5 us and
-    # more per key; a chip full of them meets at fewer keys. Measured on B200 (warm, mma.sync -> tcgen05; without options, with sinks), 32 / 8
-    # heads: one prompt of 64 tokens 6.2 -> 8.8, 7.8 -> 9.9; 128: 8.6 -> 9.9, 11.6 -> 11.0; 160: 11.4 -> 11.3, 15.2 -> 12.4; 192: 11.9 -> 11.1, 16.2
-    # -> 12.0; 16 prompts of 96 23.5 -> 20.7, 31.1 -> 23.4; 16 / 16 heads: 16 of 96 15.6 -> 12.2, 20.8 -> 14.0, 48 of 64 18.0 -> 21.9, 25.0 -> 25.6;
-    # 32 / 8 heads, prompts of 682, 1463 and 1951 tokens 390 -> 111. Without options the mma.sync kernel stays where the reach is not known.
+    # more per key; a chip full of them meets at fewer keys. Measured on B200 (warm, mma.sync -> tcgen05; without options, with sinks),
+    # 32 / 8 heads: one prompt of 64 tokens 6.2 -> 8.8, 7.8 -> 9.9; 128: 8.6 -> 9.9, 11.6 -> 11.0; 160: 11.4 -> 11.3, 15.2 -> 12.4; 192:
+    # 11.9 -> 11.1, 16.2 -> 12.0; 16 prompts of 96 23.5 -> 20.7, 31.1 -> 23.4; 16 / 16 heads: 16 of 96 15.6 -> 12.2, 20.8 -> 14.0, 48 of
+    # 64 18.0 -> 21.9, 25.0 -> 25.6; 32 / 8 heads, prompts of 682, 1463 and 1951 tokens 390 -> 111. Without options the mma.sync kernel
+    # stays where the reach is not known.
     far = options if reach is None else reach > 128 or reach > 64 and n_tiles * n_kv >= 192
     if far and _prefill_on_tcgen05(q, kcache, vcache, out, hd, vd):
         from .gemm import scratch

@@ -1,4 +1,5 @@
-"""bf16 GEMMs on the tcgen05 kernel of ``csrc/kernels/gemm.cu``.
+"""bf16 GEMMs on the tcgen05 kernels of ``csrc/kernels``: ``gemm.cu``, for prompt-sized batches ``gemm_wide.cu``, for dense products that
+these two cannot fill the chip with ``gemm_split.cu``; :func:`want_wide` and :func:`_dense_plan` choose.
 
 ``linear``          y = x @ w.T (+ residual)                         -- reference: disagmoe/models/linear.py:131-136
 ``grouped_swiglu``  act = silu(x @ w13[g][:I].T) * (x @ w13[g][I:].T)   -- reference: disagmoe/models/experts.py:84-88
@@ -8,7 +9,7 @@
                     row (and GPU) it came from                         -- reference: disagmoe/frontend/engine.py:731-734
 
 Weights are K-contiguous ``[groups, out, in]``. CPU tensors take a plain PyTorch path (used by the fp32 CPU
-configuration and as the numerical reference); CUDA tensors always run the sm_100a kernels: bf16 the tcgen05 kernel, fp32
+configuration and as the numerical reference); CUDA tensors always run the sm_100a kernels: bf16 the tcgen05 kernels, fp32
 operands (and bf16 operands whose rows are not 16-byte aligned) the CUDA-core kernel of ``csrc/kernels/layer_ops.cu``.
 """
 from __future__ import annotations
@@ -157,21 +158,21 @@ def want_streamk(epi: int, F: int, G: int, T: int, bn: int, sms: int) -> bool:
 def want_wide(epi: int, T: int, F: int, K: int, G: int, sms: int) -> bool:
     """Should the tokens be the M operand (csrc/kernels/gemm_wide.cu, CTA pairs) instead of the weights (csrc/kernels/gemm.cu)?
 
-    Dense: for launches that fit no :func:`split_plan` (:func:`_dense_plan`; one group of a grouped product counts as well). A cost model of
-    both, in us, of an earlier state of the two kernels: tiles of 256 weight rows, 0.31 us per K block of 64 whatever part of a tile is
-    used, against what an SM of the other kernel pulls from L2; the pair kernel has become the faster of them since (4096 x 6144 x 4096
-    then 201 against 149 us, now 228 against 140), so that the line is on the safe side for it. A few rows of SwiGLU gain by the wider
-    tile's faster K blocks (1 row, 2048 x 4096 38 -> 32, 16 rows, 8192 x 7168 82 -> 65), but pay 2 us more per launch (1 row, 2048 x 256
-    11.2 -> 12.6, 4096 x 1024 17.4 -> 17.4), and more where the tiles of a wave want more than HBM gives (1 row, 8192 x 1024 17.4 -> 19.3,
-    8192 x 7168 69 -> 78; 8 rows, 8192 x 4096 47 -> 49).
+    Dense: for launches that fit no :func:`split_plan` (:func:`_dense_plan`; one group of a grouped product counts as well). A cost
+    model of both, in us, of an earlier state of the two kernels: tiles of 256 weight rows, 0.31 us per K block of 64 whatever part of
+    a tile is used, against what an SM of the other kernel pulls from L2; the pair kernel has become the faster of them since (4096 x
+    6144 x 4096 then 201 against 149 us, now 228 against 140), so that the line is on the safe side for it. A few rows of SwiGLU gain
+    by the wider tile's faster K blocks (1 row, 2048 x 4096 38 -> 32, 16 rows, 8192 x 7168 82 -> 65), but pay 2 us more per launch (1
+    row, 2048 x 256 11.2 -> 12.6, 4096 x 1024 17.4 -> 17.4), and more where the tiles of a wave want more than HBM gives (1 row, 8192 x
+    1024 17.4 -> 19.3, 8192 x 7168 69 -> 78; 8 rows, 8192 x 4096 47 -> 49).
 
-    Grouped (only the mean group size is known): up to 128 tokens both kernels read the weights once; the wide one has a half product for
-    such groups and no transposing epilogue, the other one smaller units, which counts where few experts have long rows of tiles. From 40
-    tokens per expert on, sweep over 20 shapes at 40 .. 128 (other kernel -> wide, us): SwiGLU with F K to 6 million 0.99 .. 1.57 times as
-    fast (64 x 1408 x 2048, 104 tokens 133 -> 126; 16 x 2816 x 2048, 96 tokens 69 -> 64), above that 0.93 .. 1.1 (8 x 14336 x 4096: 40 tokens
-    290 -> 309, 128: 354 -> 339); down-projections to K 5632 1.00 .. 1.70 (16 x (2048 x 2816), 96 tokens 46 -> 37), 8 x (4096 x 14336): 64
-    tokens 155 -> 157, 96: 183 -> 159. Beyond 128 tokens the other kernel needs a second tile per group (8 x 14336 x 4096, SwiGLU, 160: 533 ->
-    369). Below 40 tokens short K loops are bound by the other kernel's transposing epilogue: sweep over 8 .. 64 experts, F 2048 .. 6144, K
+    Grouped (only the mean group size is known): up to 128 tokens both kernels read the weights once; the wide one has a half product
+    for such groups and no transposing epilogue, the other one smaller units, which counts where few experts have long rows of tiles.
+    From 40 tokens per expert on, sweep over 20 shapes at 40 .. 128 (other kernel -> wide, us): SwiGLU with F K to 6 million 0.99 ..
+    1.57 times as fast (64 x 1408 x 2048, 104 tokens 133 -> 126; 16 x 2816 x 2048, 96 tokens 69 -> 64), above that 0.93 .. 1.1 (8 x
+    14336 x 4096: 40 tokens 290 -> 309, 128: 354 -> 339); down-projections to K 5632 1.00 .. 1.70 (16 x (2048 x 2816), 96 tokens 46 ->
+    37), 8 x (4096 x 14336): 64 tokens 155 -> 157, 96: 183 -> 159. Beyond 128 tokens the other kernel needs a second tile per group (8
+    x 14336 x 4096, SwiGLU, 160: 533 -> 369). Below 40 tokens short K loops are bound by the other kernel's transposing epilogue: sweep over 8 .. 64 experts, F 2048 .. 6144, K
     512 .. 7168, before the half products and both kernels' present issue loops: with F K to 4.4 million 0.92 .. 1.9 times as fast, 1.17 on
     average (60 x (2048 x 1408): 16 rows 46 -> 34; 8 x (4096 x 1024): 74 rows 28 -> 25); above that a badly filled wave of long tiles can
     make it 0.8 times as fast with few experts (16 x (6144 x 2048): 24 rows 74 -> 88), while 60 and 64 experts still gain to K 2048; from K
@@ -198,8 +199,8 @@ def want_wide(epi: int, T: int, F: int, K: int, G: int, sms: int) -> bool:
 @lru_cache(maxsize=4096)
 def dense_wide(T: int, F: int, K: int, epi: int, sms: int, hd: int = 0):
     """(us, weight rows per tile) of a dense product in csrc/kernels/gemm_wide.cu: of the tile sizes the one whose count fills whole
-    waves of CTA pairs best; ``hd``: heads that a tile has to hold whole. Fitted to a sweep on B200 (42 sizes, T 66 .. 4096, K 16 .. 10944;
-    error 7 %, the choice is 1 % slower than the best size on average). Measured with 256 rows -> with the choice, us: 2500 x 2048 x 2048
+    waves of CTA pairs best; ``hd``: heads that a tile has to hold whole. Fitted to a sweep on B200 (42 sizes, T 66 .. 4096, K 16 ..
+    10944, harness of benchmark/ops/dense_gemm.py; error 7 %, the choice is 1 % slower than the best size on average). Measured with 256 rows -> with the choice, us: 2500 x 2048 x 2048
     27.8 -> 20.0 (80 tiles for 74 pairs -> 130 smaller ones), 2500 x 2048 x 5632 62.6 -> 43.6, 3000 x 2048 x 2048 27.5 -> 22.8, 2500 x 4096 x
     2048 39.3 -> 33.5, 1111 x 6144 x 2048 29.8 -> 27.6, 724 x 3664 x 2048 18.3 -> 14.3, SwiGLU 1111 x 2816 x 2048 29.3 -> 26.4."""
     pairs, best = max(1, sms // 2), None
@@ -249,12 +250,13 @@ def split_plan(T: int, F: int, K: int, epi: int, sms: int, ctas=None):
     faster: all its CTAs have to find place at once, or it has one tile of up to 128 tokens and the weights stream through it (an LM
     head).
 
-    The cost model is fitted to a sweep on B200 (T 1 .. 4096, F 16 .. 151936, K 16 .. 14336; launches back to back, weights from HBM); its
-    choice is 2.8 % slower than the best tile and cluster on average. Measured, this module's other kernels -> the choice, us: 1 x 4096 x
-    4096 13.9 -> 9.7, 37 x 2048 x 2048 10.3 -> 6.6, 37 x 6144 x 2048 14.6 -> 9.6, 37 x 2048 x 5632 14.1 -> 9.1, SwiGLU 37 x 5632 x 2048 17.7
-    -> 11.8, 96 x 2048 x 10944 22.6 -> 14.5, 256 x 4096 x 4096 22.0 -> 16.0, 576 x 2048 x 5632 29.4 -> 22.0, 1111 x 2048 x 2048 17.8 -> 14.7, 3
-    x 32000 x 4096 54.1 -> 42.4, 37 x 151936 x 2048 111 -> 104, 96 x 102400 x 2048 88.5 -> 78.0, 66 x 151936 x 2048 128 -> 110. A second wave costs as much as the first: 200 x 10944 x 2048 SwiGLU (171
-    CTAs of one per SM) 23.0 -> 40.6, 1111 x 2816 x 2048 SwiGLU 28.6 -> 36.4, 192 x 32000 x 2048 32.5 -> 42.5.
+    The cost model is fitted to a sweep on B200 (T 1 .. 4096, F 16 .. 151936, K 16 .. 14336; launches back to back, weights from HBM:
+    benchmark/ops/dense_gemm.py); its choice is 2.8 % slower than the best tile and cluster on average. Measured, this module's other
+    kernels -> the choice, us: 1 x 4096 x 4096 13.9 -> 9.7, 37 x 2048 x 2048 10.3 -> 6.6, 37 x 6144 x 2048 14.6 -> 9.6, 37 x 2048 x
+    5632 14.1 -> 9.1, SwiGLU 37 x 5632 x 2048 17.7 -> 11.8, 96 x 2048 x 10944 22.6 -> 14.5, 256 x 4096 x 4096 22.0 -> 16.0, 576 x 2048 x
+    5632 29.4 -> 22.0, 1111 x 2048 x 2048 17.8 -> 14.7, 3 x 32000 x 4096 54.1 -> 42.4, 37 x 151936 x 2048 111 -> 104, 96 x 102400 x 2048
+    88.5 -> 78.0, 66 x 151936 x 2048 128 -> 110. A second wave costs as much as the first: 200 x 10944 x 2048 SwiGLU (171 CTAs of one
+    per SM) 23.0 -> 40.6, 1111 x 2816 x 2048 SwiGLU 28.6 -> 36.4, 192 x 32000 x 2048 32.5 -> 42.5.
 
     ``ctas``: :func:`split_ctas`. Sizes are rounded up to a grid of tokens, so that few plans serve prompts of all lengths."""
     grid = 16 if T <= 256 else 32 if T <= 1024 else 64
@@ -307,9 +309,9 @@ def _dense_plan(T: int, F: int, K: int, epi: int, sms: int, hd: int = 0, ctas=No
 
     Up to 128 tokens the split kernel where it has a plan: the pair kernel would work half its rows for nothing, and its model leaves out
     that all of the weights come from HBM. Beyond, the cheaper of both models. Sweep of 267 sizes with a plan on B200 (T 2 .. 4096, F 256 ..
-    14336, K 256 .. 14336): the choice is 0.5 % slower than the best tile of either kernel on average, 17 % at most. Split -> pairs, us: 512 x
-    4096 x 14336 61 -> 52, 1000 x 2048 x 14336 58 -> 49, 512 x 4096 x 11008 49 -> 40, 200 x 12288 x 4096 35 -> 27, SwiGLU 230 x 4344 x 5768 50 ->
-    40; the other way 200 x 2048 x 14336 21 and 44, 300 x 2048 x 14336 29 and 44."""
+    14336, K 256 .. 14336): the choice is 0.5 % slower than the best tile of either kernel on average, 17 % at most. Split -> pairs, us:
+    512 x 4096 x 14336 61 -> 52, 1000 x 2048 x 14336 58 -> 49, 512 x 4096 x 11008 49 -> 40, 200 x 12288 x 4096 35 -> 27, SwiGLU 230 x
+    4344 x 5768 50 -> 40; the other way 200 x 2048 x 14336 21 and 44, 300 x 2048 x 14336 29 and 44."""
     plan = split_plan(T, F, K, epi, sms, ctas)
     if plan is not None and T <= 128:
         return 0, plan
