@@ -202,13 +202,17 @@ def dense_wide(T: int, F: int, K: int, epi: int, sms: int, hd: int = 0):
     waves of CTA pairs best; ``hd``: heads that a tile has to hold whole. Fitted to a sweep on B200 (42 sizes, T 66 .. 4096, K 16 ..
     10944, harness of benchmark/ops/dense_gemm.py; error 7 %, the choice is 1 % slower than the best size on average). Measured with 256 rows -> with the choice, us: 2500 x 2048 x 2048
     27.8 -> 20.0 (80 tiles for 74 pairs -> 130 smaller ones), 2500 x 2048 x 5632 62.6 -> 43.6, 3000 x 2048 x 2048 27.5 -> 22.8, 2500 x 4096 x
-    2048 39.3 -> 33.5, 1111 x 6144 x 2048 29.8 -> 27.6, 724 x 3664 x 2048 18.3 -> 14.3, SwiGLU 1111 x 2816 x 2048 29.3 -> 26.4."""
+    2048 39.3 -> 33.5, 1111 x 6144 x 2048 29.8 -> 27.6, 724 x 3664 x 2048 18.3 -> 14.3, SwiGLU 1111 x 2816 x 2048 29.3 -> 26.4.
+
+    The 0.9 us of a tile that do not shrink with it count where K is short: without them 1386 x 26112 x 64 took 128 rows (46.3 us, 37.4 with
+    256) and SwiGLU 622 x 19584 x 384 160 (38.2 and 31.9). Over 230 sizes (T 129 .. 4096, F 256 .. 32000, K 64 .. 11000) the choice is 0.24 %
+    slower than the best size on average (0.72 % without), 8 % at most (24 %)."""
     pairs, best = max(1, sms // 2), None
     for cols in (256, 224, 192, 160, 128):
         if hd and cols % hd:
             continue
         waves = -(-(-(-F // (cols // 2 if epi == EPI_SWIGLU else cols)) * -(-T // 256)) // pairs)
-        cost = 6.1 + waves * (2.3 * cols / 256 + (0.05 + 0.254 * cols / 256) * -(-K // 64))
+        cost = 6.1 + waves * (0.9 + 1.4 * cols / 256 + (0.05 + 0.254 * cols / 256) * -(-K // 64))
         if best is None or cost < best[0]:
             best = (cost, cols)
     return best

@@ -86,3 +86,12 @@ def test_reach_of_prompt_tiles():
         reach = F.tile_reach(100, 32, window, chunk)
         assert most <= reach <= min(100, 32 + min(window or 100, chunk or 100) - 1)
     assert F.tile_reach(90, 32) == 90 and F.tile_reach(90, 32, window=10) == 41
+
+
+@pytest.mark.parametrize("epi,T,F,K,cols", [
+    (gemm.EPI_PLAIN, 1386, 26112, 64, (224, 256)), (gemm.EPI_SWIGLU, 622, 19584, 384, (256,)), (gemm.EPI_PLAIN, 1601, 14336, 192, (224, 256)),
+    (gemm.EPI_PLAIN, 1601, 14360, 200, (224, 256)), (gemm.EPI_PLAIN, 2500, 2048, 2048, (160,)), (gemm.EPI_PLAIN, 2500, 2048, 5632, (160,)),
+])
+def test_tile_widths_of_short_and_long_products(epi, T, F, K, cols):
+    """Measured: many tiles of short K pay for each tile, whatever its width; long ones gain by tiles that fill their waves."""
+    assert gemm.dense_wide(T, F, K, epi, SMS)[1] in cols
