@@ -172,11 +172,12 @@ def want_wide(epi: int, T: int, F: int, K: int, G: int, sms: int) -> bool:
     1.57 times as fast (64 x 1408 x 2048, 104 tokens 133 -> 126; 16 x 2816 x 2048, 96 tokens 69 -> 64), above that 0.93 .. 1.1 (8 x
     14336 x 4096: 40 tokens 290 -> 309, 128: 354 -> 339); down-projections to K 5632 1.00 .. 1.70 (16 x (2048 x 2816), 96 tokens 46 ->
     37), 8 x (4096 x 14336): 64 tokens 155 -> 157, 96: 183 -> 159. Beyond 128 tokens the other kernel needs a second tile per group (8
-    x 14336 x 4096, SwiGLU, 160: 533 -> 369). Below 40 tokens short K loops are bound by the other kernel's transposing epilogue: sweep over 8 .. 64 experts, F 2048 .. 6144, K
-    512 .. 7168, before the half products and both kernels' present issue loops: with F K to 4.4 million 0.92 .. 1.9 times as fast, 1.17 on
-    average (60 x (2048 x 1408): 16 rows 46 -> 34; 8 x (4096 x 1024): 74 rows 28 -> 25); above that a badly filled wave of long tiles can
-    make it 0.8 times as fast with few experts (16 x (6144 x 2048): 24 rows 74 -> 88), while 60 and 64 experts still gain to K 2048; from K
-    2816 on nothing was gained there (8 x (4096 x 14336): 2 rows 47 -> 77)."""
+    x 14336 x 4096, SwiGLU, 160: 533 -> 369). Below 40 tokens short K loops are bound by the other kernel's transposing epilogue:
+    sweep over 8 .. 64 experts, F 2048 .. 6144, K 512 .. 7168, before the half products and both kernels' present issue loops: with F
+    K to 4.4 million 0.92 .. 1.9 times as fast, 1.17 on average (60 x (2048 x 1408): 16 rows 46 -> 34; 8 x (4096 x 1024): 74 rows 28
+    -> 25); above that a badly filled wave of long tiles can make it 0.8 times as fast with few experts (16 x (6144 x 2048): 24 rows
+    74 -> 88), while 60 and 64 experts still gain to K 2048; from K 2816 on nothing was gained there (8 x (4096 x 14336): 2 rows 47 ->
+    77)."""
     kblocks, pairs = (K + 63) // 64, max(1, sms // 2)
     if G > 1:
         if epi == EPI_SWIGLU:
@@ -200,19 +201,21 @@ def want_wide(epi: int, T: int, F: int, K: int, G: int, sms: int) -> bool:
 def dense_wide(T: int, F: int, K: int, epi: int, sms: int, hd: int = 0):
     """(us, weight rows per tile) of a dense product in csrc/kernels/gemm_wide.cu: of the tile sizes the one whose count fills whole
     waves of CTA pairs best; ``hd``: heads that a tile has to hold whole. Fitted to a sweep on B200 (42 sizes, T 66 .. 4096, K 16 ..
-    10944, harness of benchmark/ops/dense_gemm.py; error 7 %, the choice is 1 % slower than the best size on average). Measured with 256 rows -> with the choice, us: 2500 x 2048 x 2048
-    27.8 -> 20.0 (80 tiles for 74 pairs -> 130 smaller ones), 2500 x 2048 x 5632 62.6 -> 43.6, 3000 x 2048 x 2048 27.5 -> 22.8, 2500 x 4096 x
-    2048 39.3 -> 33.5, 1111 x 6144 x 2048 29.8 -> 27.6, 724 x 3664 x 2048 18.3 -> 14.3, SwiGLU 1111 x 2816 x 2048 29.3 -> 26.4.
+    10944, harness of benchmark/ops/dense_gemm.py; error 7 %, the choice is 1 % slower than the best size on average). Measured with
+    256 rows -> with the choice, us: 2500 x 2048 x 2048 27.8 -> 20.0 (80 tiles for 74 pairs -> 130 smaller ones), 2500 x 2048 x 5632
+    62.6 -> 43.6, 3000 x 2048 x 2048 27.5 -> 22.8, 2500 x 4096 x 2048 39.3 -> 33.5, 1111 x 6144 x 2048 29.8 -> 27.6, 724 x 3664 x 2048
+    18.3 -> 14.3, SwiGLU 1111 x 2816 x 2048 29.3 -> 26.4.
 
-    The 0.9 us of a tile that do not shrink with it count where K is short: without them 1386 x 26112 x 64 took 128 rows (46.3 us, 37.4 with
-    256) and SwiGLU 622 x 19584 x 384 160 (38.2 and 31.9). Over 230 sizes (T 129 .. 4096, F 256 .. 32000, K 64 .. 11000) the choice is 0.24 %
-    slower than the best size on average (0.72 % without), 8 % at most (24 %)."""
+    The 0.9 us of a tile that do not shrink with it count where K is short: without them 1386 x 26112 x 64 took 128 rows (46.3 us,
+    37.4 with 256) and SwiGLU 622 x 19584 x 384 160 (38.2 and 31.9). Over 230 sizes (T 129 .. 4096, F 256 .. 32000, K 64 .. 11000) the
+    choice is 0.24 % slower than the best size on average (0.72 % without), 8 % at most (24 %)."""
     pairs, best = max(1, sms // 2), None
+    rows = 1.15 if K % 16 else 1.0            # rows that start inside a sector of 32 bytes: 102 sizes
     for cols in (256, 224, 192, 160, 128):
         if hd and cols % hd:
             continue
         waves = -(-(-(-F // (cols // 2 if epi == EPI_SWIGLU else cols)) * -(-T // 256)) // pairs)
-        cost = 6.1 + waves * (0.9 + 1.4 * cols / 256 + (0.05 + 0.254 * cols / 256) * -(-K // 64))
+        cost = 6.1 + waves * (0.9 + 1.4 * cols / 256 + rows * (0.05 + 0.254 * cols / 256) * -(-K // 64))
         if best is None or cost < best[0]:
             best = (cost, cols)
     return best
@@ -273,6 +276,9 @@ def _split_plan(T: int, F: int, K: int, epi: int, sms: int, ctas):
     mt, kblocks = -(-F // (64 if gate else 128)), -(-K // 64)
     small, large = ctas
     stream = F * K * (4 if gate else 2) / 6.6e6
+    # bytes per us that a CTA loads. Rows that start inside a sector of 32 bytes (K not a multiple of 16) come at 0.57 of the rate (85
+    # sizes, root of the mean square error 23 -> 11 %): fewer and larger token tiles then, 58 x 9152 x 5864 35.4 -> 25.9 us
+    load = 7.3e4 if K % 16 else 1.27e5
     best = None
     if mt > small[0]:
         shapes = [(1, T)] if T <= 128 and mt <= 65535 else []      # tiles of weight rows are the grid's second dimension
@@ -297,7 +303,7 @@ def _split_plan(T: int, F: int, K: int, epi: int, sms: int, ctas):
             continue                      # the latter: stages of one K block and the exchange, 256 x 4096 x 4096 16.1 -> 20.6 us
         waves, shared = -(-units // cap), 2 if not one and units > sms else 1
         flight = min(steps, (230400 if one else 114176) // stage, 6)
-        body = max(waves * steps * max(0.226, shared * stage / 1.27e5, 0.81 / flight), stream)
+        body = max(waves * steps * max(0.226, shared * stage / load, 0.81 / flight), stream)
         adds = -(-(-(-bn // S) * (8 if gate else 16)) // 192)
         cost = 3.4 + body + 0.0098 * bn + (0.0167 * bn if S > 1 else 0.0) + waves * adds * 0.285 + (0.51 if shared > 1 else 0.0) + \
             (0.1 if bn < T else 0.0)
@@ -315,9 +321,12 @@ def _dense_plan(T: int, F: int, K: int, epi: int, sms: int, hd: int = 0, ctas=No
     that all of the weights come from HBM. Beyond, the cheaper of both models. Sweep of 267 sizes with a plan on B200 (T 2 .. 4096, F 256 ..
     14336, K 256 .. 14336): the choice is 0.5 % slower than the best tile of either kernel on average, 17 % at most. Split -> pairs, us:
     512 x 4096 x 14336 61 -> 52, 1000 x 2048 x 14336 58 -> 49, 512 x 4096 x 11008 49 -> 40, 200 x 12288 x 4096 35 -> 27, SwiGLU 230 x
-    4344 x 5768 50 -> 40; the other way 200 x 2048 x 14336 21 and 44, 300 x 2048 x 14336 29 and 44."""
+    4344 x 5768 50 -> 40; the other way 200 x 2048 x 14336 21 and 44, 300 x 2048 x 14336 29 and 44.
+
+    Rows that start inside a sector of 32 bytes (K not a multiple of 16) load more slowly, in the split kernel above all (see the models);
+    beyond 64 tokens the pairs can then be the faster ones: SwiGLU 128 x 8024 x 1752 21 -> 19.5, 120 x 11840 x 1304 27 -> 22."""
     plan = split_plan(T, F, K, epi, sms, ctas)
-    if plan is not None and T <= 128:
+    if plan is not None and T <= (64 if K % 16 else 128):
         return 0, plan
     if plan is None and not want_wide(epi, T, F, K, 1, sms):
         return 0, None

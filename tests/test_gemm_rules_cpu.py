@@ -95,3 +95,14 @@ def test_reach_of_prompt_tiles():
 def test_tile_widths_of_short_and_long_products(epi, T, F, K, cols):
     """Measured: many tiles of short K pay for each tile, whatever its width; long ones gain by tiles that fill their waves."""
     assert gemm.dense_wide(T, F, K, epi, SMS)[1] in cols
+
+
+@pytest.mark.parametrize("epi,T,F,K,pairs,bn", [
+    (gemm.EPI_PLAIN, 58, 9152, 5864, False, 64), (gemm.EPI_PLAIN, 48, 9152, 5864, False, 48),
+    (gemm.EPI_SWIGLU, 128, 8024, 1752, True, 0), (gemm.EPI_SWIGLU, 120, 11840, 1304, True, 0), (gemm.EPI_SWIGLU, 64, 8024, 1752, False, 64),
+    (gemm.EPI_SWIGLU, 128, 5632, 2048, False, 128), (gemm.EPI_PLAIN, 96, 5120, 88, False, 32), (gemm.EPI_PLAIN, 1, 4104, 4088, False, 16),
+])
+def test_rows_inside_a_sector_load_more_slowly(epi, T, F, K, pairs, bn):
+    """Measured choices where K is not a multiple of 16 (one that is beside them): weights are not loaded once per cut of the tokens."""
+    cols, plan = gemm._dense_plan(T, F, K, epi, SMS)
+    assert (cols > 0) is pairs and (plan is None or plan[1] == bn)
