@@ -5,7 +5,8 @@
 // output chunk has to be transposed through shared memory. Here a cluster of two CTAs computes a tile of 256 tokens x 256
 // weight rows with tcgen05.mma.cta_group::2: each CTA stages its own 128 token rows and HALF of the weight rows (32 KB per
 // 512 tensor cycles). A stage holds two K blocks, three stages fit: a round of the issuing warp takes about 400 cycles, and
-// was what bounded a K block when every block had a round of its own. A TMEM lane is a token, so an epilogue thread owns
+// was what bounded a K block when every block had a round of its own (SwiGLU of K up to 512 takes 1 to 5 % longer so: 2952 x 2816 x 256
+// 20.0 -> 20.7 us; 3000 x 5632 x 1024 59 -> 51, 1024 x 5632 x 2048 42.1 -> 38.6). A TMEM lane is a token, so an epilogue thread owns
 // consecutive features of one output row: no transposition, no barrier between the epilogue warps. For SwiGLU the even CTA
 // stages 128 gate rows and the odd one the matching 128 up rows; gate and up of a feature then sit 128 TMEM columns apart
 // in the same lane.
@@ -295,7 +296,8 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     // 32 columns from x of the warp's 32 rows from y. A lane has a row, so plain stores are 16 bytes of 32 rows, four times; through
     // 64-byte swizzled shared memory (no bank is met twice) the copy engine writes rows of 64 bytes while the next columns are read
     // from TMEM. Plain stores -> this, us: 2500 x 7184 x 2048 54.7 -> 52.6, 3000 x 4096 x 512 20.4 -> 19.5, 576 x 6144 x 2048 20.0 ->
-    // 18.8, 2500 x 2048 x 1024 15.4 -> 14.3; median of 42 sizes 2 % (SwiGLU, where the gate bounds the epilogue: equal)
+    // 18.8, 2500 x 2048 x 1024 15.4 -> 14.3; median of 42 sizes 2 %; SwiGLU 2952 x 2816 x
+    // 256 21.3 -> 20.7, 4096 x 14336 x 1024 169 -> 161
     const auto put = [&](const float (&o)[32], int x, int y) {
       if (lane == 0) bulk_wait_read<1>();
       __syncwarp();

@@ -313,9 +313,10 @@ def _split_plan(T: int, F: int, K: int, epi: int, sms: int, ctas):
 
 
 @lru_cache(maxsize=4096)
-def _dense_plan(T: int, F: int, K: int, epi: int, sms: int, hd: int = 0, ctas=None):
+def _dense_plan(T: int, F: int, K: int, epi: int, sms: int, hd: int = 0, device: Optional[torch.device] = None):
     """(weight rows per tile of gemm_wide.cu or 0, split plan or None) of a dense launch on one GPU that leaves the choice of kernel to
-    this module; ``hd``: see :func:`dense_wide`.
+    this module; ``hd``: see :func:`dense_wide`; ``device``: whose :func:`split_ctas` count, and part of the key under which every launch finds
+    its plan (the tables themselves took 0.5 us to hash: 2 % of prompt steps that the host bounds).
 
     Up to 128 tokens the split kernel where it has a plan: the pair kernel would work half its rows for nothing, and its model leaves out
     that all of the weights come from HBM. Beyond, the cheaper of both models. Sweep of 267 sizes with a plan on B200 (T 2 .. 4096, F 256 ..
@@ -325,7 +326,7 @@ def _dense_plan(T: int, F: int, K: int, epi: int, sms: int, hd: int = 0, ctas=No
 
     Rows that start inside a sector of 32 bytes (K not a multiple of 16) load more slowly, in the split kernel above all (see the models);
     beyond 64 tokens the pairs can then be the faster ones: SwiGLU 128 x 8024 x 1752 21 -> 19.5, 120 x 11840 x 1304 27 -> 22."""
-    plan = split_plan(T, F, K, epi, sms, ctas)
+    plan = split_plan(T, F, K, epi, sms, None if device is None else split_ctas(device))
     if plan is not None and T <= (64 if K % 16 else 128):
         return 0, plan
     if plan is None and not want_wide(epi, T, F, K, 1, sms):
@@ -563,8 +564,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, residual: Optional[torch.Tensor] = 
     if wide is None and not cluster:
         wide = False
         if not (bn or splitk or pair) and _wide_rows(F, out, residual, comm):
-            wide, plan = _dense_plan(T, F, K, EPI_PLAIN, sms, comm.rope.hd if comm is not None and comm.rope is not None else 0,
-                                     split_ctas(x.device))
+            wide, plan = _dense_plan(T, F, K, EPI_PLAIN, sms, comm.rope.hd if comm is not None and comm.rope is not None else 0, x.device)
             if plan is not None:
                 _, bn, cluster = plan
     if cluster:
@@ -775,7 +775,7 @@ def swiglu_linear(x: torch.Tensor, w13: torch.Tensor, out: Optional[torch.Tensor
     if wide is None and not cluster:
         wide = False
         if not bn:
-            wide, plan = _dense_plan(T, I, K, EPI_SWIGLU, num_sms(x.device), 0, split_ctas(x.device))
+            wide, plan = _dense_plan(T, I, K, EPI_SWIGLU, num_sms(x.device), 0, x.device)
             if plan is not None and _wide_rows(I, out, None, None):
                 _, bn, cluster = plan
     if cluster:

@@ -86,3 +86,16 @@ def test_more_weight_rows_than_the_grid_has_tiles_stay_with_the_other_kernel():
     assert gemm.split_plan(1, 65535 * 128, 8, gemm.EPI_PLAIN, 148) is not None and gemm.split_plan(1, 65535 * 128 + 8, 8, gemm.EPI_PLAIN, 148) is None
     assert gemm._dense_plan(1, 65535 * 128 + 8, 8, gemm.EPI_PLAIN, 148) == (0, None)
     assert gemm.split_plan(1, 65535 * 64 + 8, 8, gemm.EPI_SWIGLU, 148) is None
+
+
+def test_a_launch_finds_its_plan_without_the_tables(monkeypatch):
+    """The tables of a device are asked for once per plan, and each device has plans of its own."""
+    import torch
+    asked = []
+    monkeypatch.setattr(gemm, "split_ctas", lambda device: asked.append(device.index) or gemm._scaled_ctas(148 if device.index == 0 else 74))
+    gemm._dense_plan.cache_clear()
+    try:
+        a, b = ([gemm._dense_plan(16, 4096, 4104, gemm.EPI_PLAIN, 148, 0, torch.device("cuda", i)) for _ in range(3)] for i in (0, 1))
+    finally:
+        gemm._dense_plan.cache_clear()
+    assert asked == [0, 1] and a[0] == a[2] and b[0] == b[2] and a[0] != b[0]
