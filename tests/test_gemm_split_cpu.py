@@ -95,7 +95,7 @@ def test_a_launch_finds_its_plan_without_the_tables(monkeypatch):
     monkeypatch.setattr(gemm, "split_ctas", lambda device: asked.append(device.index) or gemm._scaled_ctas(148 if device.index == 0 else 74))
     gemm._dense_plan.cache_clear()
     try:
-        a, b = ([gemm._dense_plan(16, 4096, 4104, gemm.EPI_PLAIN, 148, 0, torch.device("cuda", i)) for _ in range(3)] for i in (0, 1))
+        a, b = ([gemm._dense_plan(64, 4096, 4096, gemm.EPI_PLAIN, 148, 0, torch.device("cuda", i)) for _ in range(3)] for i in (0, 1))
     finally:
         gemm._dense_plan.cache_clear()
     assert asked == [0, 1] and a[0] == a[2] and b[0] == b[2] and a[0] != b[0]
